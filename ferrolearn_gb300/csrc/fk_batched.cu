@@ -3,16 +3,11 @@
 //
 // Layout in HBM: every problem's rows packed into one f32 buffer (16-byte
 // aligned starts); per fit (problem p, run r) an n_p-long int32 scratch pair
-// (labels | members, reused as the k-means++ D^2 and running-sum arrays) and
-// two k x d centre buffers that alternate between iterations.
+// (labels | members) and two k x d centre buffers that alternate between
+// iterations.
 //
 // Launches:
-//   batch_kpp_kernel     one persistent launch; a CTA takes the next fit from
-//                        a work queue (largest first) and runs greedy
-//                        k-means++ for it exactly as kmeans.rs:169-253 in f32:
-//                        the running sum is the reference's sequential fold
-//                        (one lane, the values broadcast by shuffles), each
-//                        trial's potential likewise, trials in parallel warps.
+//   k-means++            every fit's seeding together (fk_kpp.cu).
 //   batch_assign_kernel  per Lloyd iteration, one persistent launch per
 //                        (d, k) bucket over a queue of (fit, row range) items,
 //                        largest fits first; the fit's centres in shared
@@ -54,7 +49,7 @@ struct BFit {
     int32_t n, d, k, max_iter;
     float tol;
     int32_t first_item, n_items;
-    int32_t trials, prob;
+    int32_t prob, pad;
     uint64_t seed;
 };
 
@@ -67,30 +62,11 @@ struct BItem {
     int32_t fit, lo, hi, pad;
 };
 
-constexpr int KPP_T = 256;
-constexpr int KPP_TILE = 8192;  // floats of shared memory for a tile of rows (padded stride d + 1)
-static_assert(KPP_TILE % 256 == 0, "tile prefetch assumes 256 threads");
 constexpr int ASSIGN_T = 128;
 constexpr int UPDATE_T = 256;
 constexpr int NBUCKETS = 20;  // d in {8, 16, 32, 64, other} x k in {<=16, <=32, <=64, >64}
 constexpr int NVARIANTS = 5;  // (rows per thread, centres per pass): (1,1) (2,1) (1,2) (2,2) (4,1)
 constexpr int MAX_K = 1024, MAX_D = 256, MAX_KD = 32768;
-
-__device__ __forceinline__ uint64_t dev_splitmix64(uint64_t &s) {
-    uint64_t z = (s += 0x9E3779B97F4A7C15ULL);
-    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ULL;
-    z = (z ^ (z >> 27)) * 0x94D049BB133111EBULL;
-    return z ^ (z >> 31);
-}
-__device__ __forceinline__ double dev_uniform(uint64_t &s) {
-    return (double)(dev_splitmix64(s) >> 11) * (1.0 / 9007199254740992.0);
-}
-__device__ __forceinline__ int dev_range(double u, int n) {
-    long long i = (long long)floor(u * (double)n);
-    if (i < 0) i = 0;
-    if (i >= n) i = n - 1;
-    return (int)i;
-}
 
 // squared_euclidean (kmeans.rs:159-163) in f32: left fold, no FMA.
 __device__ __forceinline__ float sqeuc_f32(const float *__restrict__ a, const float *__restrict__ b, int d) {
@@ -100,224 +76,6 @@ __device__ __forceinline__ float sqeuc_f32(const float *__restrict__ a, const fl
         acc = __fadd_rn(acc, __fmul_rn(t, t));
     }
     return acc;
-}
-
-// ------------------------------------------------------------- k-means++ --
-// First index i with cum[i] >= thr (cum is non-decreasing); n - 1 if none.
-__device__ int first_reaching(const float *__restrict__ cum, int n, float thr) {
-    int lo = 0, hi = n;  // answer in [lo, hi]
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (cum[mid] >= thr) hi = mid;
-        else lo = mid + 1;
-    }
-    return lo < n ? lo : n - 1;
-}
-
-// Sequential f32 fold of v[0..n) by one warp (the reference's in-order
-// sum): the warp stages 256 values at a time in its shared-memory slice
-// (coalesced loads, one batch ahead), then every lane runs the same chain
-// over broadcast reads; with cum, lane 0 also records each running value in
-// the slice and the warp writes them out coalesced.
-constexpr int FOLD_N = 256;
-
-__device__ float warp_serial_fold(const float *__restrict__ v, int n, float *__restrict__ cum,
-                                  float *__restrict__ stage, float *__restrict__ cbuf) {
-    const int lane = threadIdx.x & 31;
-    float run = 0.f;
-    float cur[FOLD_N / 32], nxt[FOLD_N / 32];
-#pragma unroll
-    for (int b = 0; b < FOLD_N / 32; b++) cur[b] = b * 32 + lane < n ? v[b * 32 + lane] : 0.f;
-    for (int base = 0; base < n; base += FOLD_N) {
-#pragma unroll
-        for (int b = 0; b < FOLD_N / 32; b++) {
-            const int i = base + FOLD_N + b * 32 + lane;
-            nxt[b] = i < n ? v[i] : 0.f;
-        }
-        __syncwarp();
-#pragma unroll
-        for (int b = 0; b < FOLD_N / 32; b++) stage[b * 32 + lane] = cur[b];
-        __syncwarp();
-        const int m = min(FOLD_N, n - base);
-        if (m == FOLD_N) {
-#pragma unroll 16
-            for (int q = 0; q < FOLD_N / 4; q++) {
-                const float4 f = reinterpret_cast<const float4 *>(stage)[q];
-                run = __fadd_rn(run, f.x);
-                if (cum && lane == 0) cbuf[4 * q] = run;
-                run = __fadd_rn(run, f.y);
-                if (cum && lane == 0) cbuf[4 * q + 1] = run;
-                run = __fadd_rn(run, f.z);
-                if (cum && lane == 0) cbuf[4 * q + 2] = run;
-                run = __fadd_rn(run, f.w);
-                if (cum && lane == 0) cbuf[4 * q + 3] = run;
-            }
-        } else {
-            for (int e = 0; e < m; e++) {
-                run = __fadd_rn(run, stage[e]);
-                if (cum && lane == 0) cbuf[e] = run;
-            }
-        }
-        if (cum) {
-            __syncwarp();
-#pragma unroll
-            for (int b = 0; b < FOLD_N / 32; b++)
-                if (b * 32 + lane < m) cum[base + b * 32 + lane] = cbuf[b * 32 + lane];
-        }
-#pragma unroll
-        for (int b = 0; b < FOLD_N / 32; b++) cur[b] = nxt[b];
-    }
-    return run;
-}
-
-// Distances (direct form) of every row to ntr candidate rows (crow, ntr x d,
-// shared memory) over tiles of rows staged in shared memory (coalesced loads,
-// padded stride d + 1: conflict-free reads; the next tile is loaded into
-// registers while the current one is scored); the (row, candidate) pairs of
-// a tile are spread evenly over the threads. mode 0: mind[i] = d(x_i,
-// crow[0]); mode 1: nd[t n + i] = min(d(x_i, crow[t]), mind[i]).
-constexpr int KPP_PF = KPP_TILE / 256;  // prefetched floats per thread
-
-__device__ void tile_distances(const float *__restrict__ x, int n, int d, const float *__restrict__ crow, int ntr,
-                               int mode, float *__restrict__ mind, float *__restrict__ nd, float *__restrict__ tile) {
-    const int tid = threadIdx.x;
-    const int TR = KPP_TILE / (d + 1) < 256 ? KPP_TILE / (d + 1) : 256;  // rows per tile
-    float pf[KPP_PF];
-    auto fetch = [&](int i0) {
-        const int cnt = min(TR, n - i0) * d;
-#pragma unroll
-        for (int u = 0; u < KPP_PF; u++) {
-            const int e = tid + u * KPP_T;
-            pf[u] = e < cnt ? x[(int64_t)i0 * d + e] : 0.f;
-        }
-    };
-    if (n > 0) fetch(0);
-    for (int i0 = 0; i0 < n; i0 += TR) {
-        const int rows = min(TR, n - i0);
-        __syncthreads();
-#pragma unroll
-        for (int u = 0; u < KPP_PF; u++) {
-            const int e = tid + u * KPP_T;
-            if (e < rows * d) {
-                const int rr = e / d, j = e - rr * d;
-                tile[rr * (d + 1) + j] = pf[u];
-            }
-        }
-        __syncthreads();
-        if (i0 + TR < n) fetch(i0 + TR);
-        for (int pr = tid; pr < rows * ntr; pr += KPP_T) {
-            const int r = pr % rows, t = pr / rows;
-            const float *xr = tile + r * (d + 1);
-            const float *cr = crow + t * d;
-            float acc = 0.f;
-            for (int j = 0; j < d; j++) {
-                const float df = __fsub_rn(xr[j], cr[j]);
-                acc = __fadd_rn(acc, __fmul_rn(df, df));
-            }
-            const int i = i0 + r;
-            if (mode == 0) {
-                mind[i] = acc;
-            } else {
-                const float mv = mind[i];
-                nd[(int64_t)t * n + i] = acc < mv ? acc : mv;
-            }
-        }
-    }
-    __syncthreads();
-}
-
-// One CTA per fit. Per new centre: the running sum of D^2 (warp 0), the
-// thresholds and candidates (thread 0), one pass over the rows computing
-// min(d(x, candidate t), D^2) for every trial t into nd (the CTA's scratch),
-// the trials' potentials (one warp each, sequential folds), the choice, and
-// D^2 <- nd[best].
-__global__ void __launch_bounds__(KPP_T) batch_kpp_kernel(const float *__restrict__ X, const BFit *__restrict__ fits,
-                                                          const int *__restrict__ order, int nf, int *counter,
-                                                          int *__restrict__ lab, int *__restrict__ mem,
-                                                          float *__restrict__ C, float *__restrict__ nd_all,
-                                                          int64_t nd_stride) {
-    __shared__ int q_sh, idx_sh;
-    __shared__ float total_sh;
-    __shared__ int cand_sh[16];
-    __shared__ float pot_sh[16], thr_sh[16];
-    __shared__ float crow[8 * MAX_D];
-    __shared__ float tile[KPP_TILE];
-    __shared__ __align__(16) float fold_sm[KPP_T / 32][2 * FOLD_N];
-    const int tid = threadIdx.x, warp = tid >> 5;
-    float *stage = fold_sm[warp], *cbuf = fold_sm[warp] + FOLD_N;
-    float *nd = nd_all + (int64_t)blockIdx.x * nd_stride;
-    uint64_t rng = 0;  // thread 0 only
-    while (true) {
-        if (tid == 0) q_sh = atomicAdd(counter, 1);
-        __syncthreads();
-        const int q = q_sh;
-        __syncthreads();
-        if (q >= nf) break;
-        const BFit F = fits[order[q]];
-        const int n = F.n, d = F.d, k = F.k, trials = F.trials;
-        const float *x = X + F.x_off;
-        float *mind = reinterpret_cast<float *>(lab + F.s_off);
-        float *cum = reinterpret_cast<float *>(mem + F.s_off);
-        float *cen = C + F.c_off;  // buffer 0
-        if (tid == 0) {
-            rng = F.seed;
-            idx_sh = dev_range(dev_uniform(rng), n);
-        }
-        __syncthreads();
-        for (int j = tid; j < d; j += KPP_T) {
-            const float v = x[(int64_t)idx_sh * d + j];
-            cen[j] = v;
-            crow[j] = v;
-        }
-        __syncthreads();
-        if (k > 1) tile_distances(x, n, d, crow, 1, 0, mind, nullptr, tile);
-        for (int c = 1; c < k; c++) {
-            if (warp == 0) {
-                const float total = warp_serial_fold(mind, n, cum, stage, cbuf);  // the reference's sequential f32 sum
-                if ((tid & 31) == 0) total_sh = total;
-            }
-            __syncthreads();
-            const float total = total_sh;
-            if (total <= 0.f) {  // kmeans.rs:202-206: a uniform random row (NaN falls through)
-                if (tid == 0) idx_sh = dev_range(dev_uniform(rng), n);
-                __syncthreads();
-                for (int j = tid; j < d; j += KPP_T) cen[(int64_t)c * d + j] = x[(int64_t)idx_sh * d + j];
-                __syncthreads();
-                continue;
-            }
-            if (tid == 0)  // the draws in order, one per trial (kmeans.rs:213-214)
-                for (int t = 0; t < trials; t++) thr_sh[t] = __fmul_rn(__double2float_rn(dev_uniform(rng)), total);
-            __syncthreads();
-            if (tid < trials) cand_sh[tid] = first_reaching(cum, n, thr_sh[tid]);
-            __syncthreads();
-            for (int e = tid; e < trials * d; e += KPP_T) {
-                const int t = e / d, j = e - t * d;
-                crow[t * d + j] = x[(int64_t)cand_sh[t] * d + j];
-            }
-            __syncthreads();
-            tile_distances(x, n, d, crow, trials, 1, mind, nd, tile);
-            for (int t = warp; t < trials; t += KPP_T / 32) {
-                const float pot = warp_serial_fold(nd + (int64_t)t * n, n, nullptr, stage, cbuf);
-                if ((tid & 31) == 0) pot_sh[t] = pot;
-            }
-            __syncthreads();
-            if (tid == 0) {  // strictly smallest potential, first trial on ties (kmeans.rs:239-243)
-                int best = 0;
-                float bp = pot_sh[0];
-                for (int t = 1; t < trials; t++)
-                    if (pot_sh[t] < bp) {
-                        bp = pot_sh[t];
-                        best = t;
-                    }
-                idx_sh = best;
-            }
-            __syncthreads();
-            const int best = idx_sh;
-            for (int j = tid; j < d; j += KPP_T) cen[(int64_t)c * d + j] = crow[best * d + j];
-            for (int i = tid; i < n; i += KPP_T) mind[i] = nd[(int64_t)best * n + i];
-            __syncthreads();
-        }
-    }
 }
 
 // ------------------------------------------------------------ assignment --
@@ -856,7 +614,6 @@ fk_status batched_fit_impl(Ctx &ctx, fk_batch_problem *P, int64_t np, int reduct
             F.k = (int32_t)q.n_clusters;
             F.max_iter = (int32_t)q.max_iter;
             F.tol = (float)q.tol;
-            F.trials = kpp_trials_host(q.n_clusters);
             F.seed = q.random_state + (uint64_t)r;
             F.prob = (int32_t)p;
             fits.push_back(F);
@@ -896,7 +653,7 @@ fk_status batched_fit_impl(Ctx &ctx, fk_batch_problem *P, int64_t np, int reduct
     BState *dstate = (BState *)ctx.get(BUF_BSTATE, sizeof(BState) * (size_t)nf);
     BItem *ditems = (BItem *)ctx.get(BUF_BITEMS, sizeof(BItem) * items.size() + 16);
     double *dpart = (double *)ctx.get(BUF_BPART, sizeof(double) * items.size() + 16);
-    int *dorder = (int *)ctx.get(BUF_BORDER, sizeof(int) * (size_t)(2 * nf) + 16);
+    int *dorder = (int *)ctx.get(BUF_BORDER, sizeof(int) * (size_t)nf + 16);
     int *dctr = (int *)ctx.get(BUF_BCTR, sizeof(int) * 32);
     int *dlab = (int *)ctx.get(BUF_BLAB, sizeof(int) * (size_t)soff + 16);
     int *dmem = (int *)ctx.get(BUF_BMEM, sizeof(int) * (size_t)soff + 16);
@@ -921,9 +678,7 @@ fk_status batched_fit_impl(Ctx &ctx, fk_batch_problem *P, int64_t np, int reduct
     }
     if (!items.empty())
         FK_CUDA(cudaMemcpyAsync(ditems, items.data(), sizeof(BItem) * items.size(), cudaMemcpyHostToDevice, s));
-    std::vector<int> orders(byc);
-    orders.insert(orders.end(), kpp_order.begin(), kpp_order.end());
-    FK_CUDA(cudaMemcpyAsync(dorder, orders.data(), sizeof(int) * orders.size(), cudaMemcpyHostToDevice, s));
+    FK_CUDA(cudaMemcpyAsync(dorder, byc.data(), sizeof(int) * byc.size(), cudaMemcpyHostToDevice, s));
     std::vector<BState> st0(nf);
     int active = 0;
     for (int f = 0; f < nf; f++) {
@@ -948,21 +703,21 @@ fk_status batched_fit_impl(Ctx &ctx, fk_batch_problem *P, int64_t np, int reduct
     }
     FK_CUDA(cudaEventRecord(ev[1], s));
 
-    // ---- k-means++ (one persistent launch)
+    // ---- k-means++ (fk_kpp.cu): every fit's seeding, a centre of each per step
     if (!kpp_order.empty()) {
-        const int grid = std::min((int)kpp_order.size(), ctx.num_sms * 2);
-        int64_t nmax_kpp = 1;
-        for (int f : kpp_order) nmax_kpp = std::max<int64_t>(nmax_kpp, fits[f].n);
-        const int64_t nd_stride = 8 * nmax_kpp;  // trials <= 8 (k <= 1024)
-        float *nd = (float *)ctx.get(BUF_BND, sizeof(float) * (size_t)(nd_stride * grid));
-        batch_kpp_kernel<<<grid, KPP_T, 0, s>>>(X, dfits, dorder + nf, (int)kpp_order.size(), dctr + 30, dlab, dmem,
-                                                dC, nd, nd_stride);
-        FK_LAUNCH_CHECK();
-        // k-means++ used the label arrays as scratch: fits that run no
-        // iteration report all-zero labels (kmeans.rs:459-466)
-        for (int f = 0; f < nf; f++)
-            if (fits[f].max_iter == 0)
-                FK_CUDA(cudaMemsetAsync(dlab + fits[f].s_off, 0, sizeof(int) * (size_t)fits[f].n, s));
+        std::vector<KppJob> jobs;
+        for (int f : kpp_order) {
+            KppJob j;
+            j.x = X + fits[f].x_off;
+            j.n = fits[f].n;
+            j.d = fits[f].d;
+            j.k = fits[f].k;
+            j.seed = fits[f].seed;
+            j.centers = dC + fits[f].c_off;  // buffer 0
+            j.nan_direct = false;
+            jobs.push_back(j);
+        }
+        run_kmeanspp<float>(ctx, jobs, nullptr);
     }
     FK_CUDA(cudaEventRecord(ev[2], s));
 

@@ -447,13 +447,40 @@ fk_status fit_impl(fk_ctx *ctxp, const TX *x_in, int64_t n, int64_t d, const fk_
     const TC *init = init_in ? stage_in<TC>(ctx, BUF_INIT, init_in, kd * (size_t)p->n_init) : nullptr;
     const double *draws_dev = nullptr;
     int64_t n_draws = 0;
-    if (!init) {
-        // k-means++ draws: caller's flat stream, or splitmix64 per run.
-        n_draws = p->draws ? p->n_draws : 1 + (k - 1) * kpp_trials_host(k);
-        if (p->draws) draws_dev = stage_in<double>(ctx, BUF_DRAWS, p->draws, (size_t)n_draws);
+    if (!init && p->draws) {
+        n_draws = p->n_draws;
+        draws_dev = stage_in<double>(ctx, BUF_DRAWS, p->draws, (size_t)n_draws);
     }
     int64_t draws_pos = 0;
-    std::vector<double> hdraws;
+    // k-means++ reads rows of F: the f32 rows of the f32x64 forms are widened
+    // exactly first
+    const TC *xk = nullptr;
+    TC *seeds = nullptr;
+    if (!init) {
+        Timer t(timing, ctx, rep ? &rep->ms_init : nullptr);
+        if constexpr (std::is_same<TX, TC>::value) {
+            xk = x;
+        } else {
+            TC *xw = (TC *)ctx.get(BUF_XC, sizeof(TC) * (size_t)n * d);
+            launch_convert<TX, TC>(x, (int64_t)n * d, xw, s);
+            xk = xw;
+        }
+        if (!p->draws) {
+            // the restarts' streams are independent: all seedings run together
+            seeds = (TC *)ctx.get(BUF_KPPC, sizeof(TC) * kd * (size_t)p->n_init);
+            std::vector<KppJob> jobs((size_t)p->n_init);
+            for (int64_t run = 0; run < p->n_init; run++) {
+                KppJob &j = jobs[(size_t)run];
+                j.x = xk;
+                j.n = n;
+                j.d = (int)d;
+                j.k = (int)k;
+                j.seed = (p->has_random_state ? p->random_state : 0) + (uint64_t)run;
+                j.centers = seeds + (size_t)run * kd;
+            }
+            run_kmeanspp<TC>(ctx, jobs, nullptr);
+        }
+    }
 
     bool have = false;
     TC best_inertia = FMax<TC>::v();
@@ -468,38 +495,27 @@ fk_status fit_impl(fk_ctx *ctxp, const TX *x_in, int64_t n, int64_t d, const fk_
     for (int64_t run = 0; run < p->n_init; run++) {
         if (init) {
             FK_CUDA(cudaMemcpyAsync(cb3[0], init + (size_t)run * kd, sizeof(TC) * kd, cudaMemcpyDeviceToDevice, s));
+        } else if (seeds) {
+            FK_CUDA(cudaMemcpyAsync(cb3[0], seeds + (size_t)run * kd, sizeof(TC) * kd, cudaMemcpyDeviceToDevice, s));
         } else {
+            // the caller's stream: each run continues where the last one stopped
             Timer t(timing, ctx, rep ? &rep->ms_init : nullptr);
-            const double *dr;
-            int64_t ndr;
-            if (p->draws) {
-                if (draws_pos >= n_draws) {
-                    set_error("injected draw stream exhausted before run %lld", (long long)run);
-                    fail(FK_ERR_INVALID_PARAMETER);
-                }
-                dr = draws_dev + draws_pos;
-                ndr = n_draws - draws_pos;
-            } else {
-                uint64_t seed = (p->has_random_state ? p->random_state : 0) + (uint64_t)run;
-                hdraws.resize((size_t)n_draws);
-                host_draws(seed, n_draws, hdraws.data());
-                double *dd = (double *)ctx.get(BUF_DRAWS, sizeof(double) * (size_t)n_draws);
-                FK_CUDA(cudaMemcpyAsync(dd, hdraws.data(), sizeof(double) * (size_t)n_draws,
-                                        cudaMemcpyHostToDevice, s));
-                FK_CUDA(cudaStreamSynchronize(s));  // hdraws is reused next run
-                dr = dd;
-                ndr = n_draws;
+            if (draws_pos >= n_draws) {
+                set_error("injected draw stream exhausted before run %lld", (long long)run);
+                fail(FK_ERR_INVALID_PARAMETER);
             }
+            std::vector<KppJob> jobs(1);
+            KppJob &j = jobs[0];
+            j.x = xk;
+            j.n = n;
+            j.d = (int)d;
+            j.k = (int)k;
+            j.draws = draws_dev + draws_pos;
+            j.n_draws = n_draws - draws_pos;
+            j.centers = cb3[0];
             int64_t used = 0;
-            if constexpr (std::is_same<TX, TC>::value) {
-                run_kmeanspp<TC>(ctx, x, n, (int)d, (int)k, dr, ndr, cb3[0], &used);
-            } else {
-                // k-means++ on the exactly widened matrix.
-                TC *xw = (TC *)ctx.get(BUF_XC, sizeof(TC) * (size_t)n * d);
-                launch_convert<TX, TC>(x, (int64_t)n * d, xw, s);
-                run_kmeanspp<TC>(ctx, xw, n, (int)d, (int)k, dr, ndr, cb3[0], &used);
-            }
-            if (p->draws) draws_pos += used;
+            run_kmeanspp<TC>(ctx, jobs, &used);
+            draws_pos += used;
         }
         int64_t n_iter = 0;
         TC inertia = FMax<TC>::v();
@@ -794,21 +810,21 @@ fk_status kpp_impl(fk_ctx *ctxp, const T *x_in, int64_t n, int64_t d, int64_t k,
     ctx.bind();
     cudaStream_t s = ctx.stream;
     const T *x = stage_in<T>(ctx, BUF_X, x_in, (size_t)n * d);
-    std::vector<double> hd;
-    const double *dr;
-    if (draws) {
-        dr = stage_in<double>(ctx, BUF_DRAWS, draws, (size_t)n_draws);
-    } else {
-        n_draws = 1 + (k - 1) * kpp_trials_host(k);
-        hd.resize((size_t)n_draws);
-        host_draws(seed, n_draws, hd.data());
-        double *dd = (double *)ctx.get(BUF_DRAWS, sizeof(double) * (size_t)n_draws);
-        FK_CUDA(cudaMemcpyAsync(dd, hd.data(), sizeof(double) * (size_t)n_draws, cudaMemcpyHostToDevice, s));
-        dr = dd;
-    }
     T *o = is_device_ptr(centers_out) ? centers_out : (T *)ctx.get(BUF_OUT, sizeof(T) * (size_t)k * d);
+    std::vector<KppJob> jobs(1);
+    KppJob &j = jobs[0];
+    j.x = x;
+    j.n = n;
+    j.d = (int)d;
+    j.k = (int)k;
+    if (draws) {
+        j.draws = stage_in<double>(ctx, BUF_DRAWS, draws, (size_t)n_draws);
+        j.n_draws = n_draws;
+    }
+    j.seed = seed;
+    j.centers = o;
     int64_t used = 0;
-    run_kmeanspp<T>(ctx, x, n, (int)d, (int)k, dr, n_draws, o, &used);
+    run_kmeanspp<T>(ctx, jobs, &used);
     if (o != centers_out) copy_out<T>(ctx, centers_out, o, (size_t)k * d);
     FK_CUDA(cudaStreamSynchronize(s));
     if (draws_used) *draws_used = used;
@@ -938,13 +954,29 @@ fk_status minibatch_impl(fk_ctx *ctxp, const T *x_in, int64_t n, int64_t d, cons
     std::vector<int32_t> hidx;
     std::unordered_map<int64_t, int64_t> moved;
     std::vector<int64_t> pool;
-    std::vector<double> hdraws;
     const std::vector<long long> ones((size_t)k, 1LL);  // per-centre counts start at 1 (:543)
     const uint64_t base = p->has_random_state ? p->random_state : 0;
     const T tol = (T)p->tol;
     bool have = false;
     T best_inertia = FMax<T>::v();
     int64_t best_iter = 0, best_run = 0;
+    // k-means++ of every run together (their streams are independent)
+    T *seeds = nullptr;
+    std::vector<int64_t> seed_draws((size_t)p->n_init, 0);
+    if (!init && p->init == FK_MB_INIT_KMEANS_PLUS_PLUS) {
+        seeds = (T *)ctx.get(BUF_KPPC, sizeof(T) * kd * (size_t)p->n_init);
+        std::vector<KppJob> jobs((size_t)p->n_init);
+        for (int64_t run = 0; run < p->n_init; run++) {
+            KppJob &j = jobs[(size_t)run];
+            j.x = x;
+            j.n = n;
+            j.d = (int)d;
+            j.k = (int)k;
+            j.seed = base + (uint64_t)run * 1000003ULL;
+            j.centers = seeds + (size_t)run * kd;
+        }
+        run_kmeanspp<T>(ctx, jobs, seed_draws.data());
+    }
     for (int64_t run = 0; run < p->n_init; run++) {
         const uint64_t seed = base + (uint64_t)run * 1000003ULL;
         int64_t pos = 0;  // stream position after the initial centres
@@ -959,12 +991,8 @@ fk_status minibatch_impl(fk_ctx *ctxp, const T *x_in, int64_t n, int64_t d, cons
             launch_gather_rows<T>(x, (int)d, didx, k, c, s);
             FK_CUDA(cudaStreamSynchronize(s));  // hidx is refilled below
         } else {
-            const int64_t n_draws = 1 + (k - 1) * kpp_trials_host(k);
-            hdraws.resize((size_t)n_draws);
-            host_draws(seed, n_draws, hdraws.data());
-            double *dd = (double *)ctx.get(BUF_DRAWS, sizeof(double) * (size_t)n_draws);
-            FK_CUDA(cudaMemcpyAsync(dd, hdraws.data(), sizeof(double) * (size_t)n_draws, cudaMemcpyHostToDevice, s));
-            run_kmeanspp<T>(ctx, x, n, (int)d, (int)k, dd, n_draws, c, &pos);  // synchronises
+            FK_CUDA(cudaMemcpyAsync(c, seeds + (size_t)run * kd, sizeof(T) * kd, cudaMemcpyDeviceToDevice, s));
+            pos = seed_draws[(size_t)run];
         }
         FK_CUDA(cudaMemcpyAsync(counts, ones.data(), sizeof(long long) * (size_t)k, cudaMemcpyHostToDevice, s));
         UniformStream g(seed, pos);

@@ -148,7 +148,7 @@ struct MixedPlan {
 enum BufSlot {
     BUF_X = 0, BUF_XC, BUF_C0, BUF_C1, BUF_CBEST, BUF_LABELS, BUF_LBEST, BUF_MIND,
     BUF_MEMBERS, BUF_SEGHIST, BUF_SCAN_TMP, BUF_COUNTS, BUF_PARTIAL, BUF_SCALARS,
-    BUF_OUT, BUF_OUT2, BUF_KPP0, BUF_KPP1, BUF_KPP2, BUF_KPP3, BUF_DRAWS,
+    BUF_OUT, BUF_OUT2, BUF_KPP0, BUF_KPP1, BUF_KPP2, BUF_DRAWS,
     BUF_XB, BUF_XNORM, BUF_CB, BUF_CAUX, BUF_TOP2, BUF_FLAGS, BUF_FULL, BUF_CF32, BUF_CF32C, BUF_FIXPART,
     BUF_XB2, BUF_EX, BUF_XAUG, BUF_ROWSCALE, BUF_ROWINFO2, BUF_STATS2, BUF_CB2, BUF_CAUG2,
     BUF_HALF2, BUF_INERTIA2, BUF_C2, BUF_XSTATE, BUF_XCOUNTS, BUF_MOVED, BUF_MOVED_ENT, BUF_MOVED_HIST, BUF_MOVED_TMP,
@@ -158,7 +158,8 @@ enum BufSlot {
     BUF_BK_FOLD, BUF_BK_LABELS, BUF_BK_XSEG, BUF_BK_CHAINS, BUF_BK_FRES, BUF_BK_FCNT, BUF_FOLD_SUM, BUF_FOLD_CNT,
     BUF_FOLD_MAP, BUF_MASKS, BUF_THRESH, BUF_FLOORS, BUF_SHIFT, BUF_THMAIN, BUF_TH2, BUF_CNT2, BUF_LIST3,
     BUF_SLOT3, BUF_TH3, BUF_XB3,
-    BUF_BX, BUF_BFITS, BUF_BSTATE, BUF_BITEMS, BUF_BPART, BUF_BORDER, BUF_BCTR, BUF_BLAB, BUF_BMEM, BUF_BCEN, BUF_BND, BUF_BXOFF,
+    BUF_BX, BUF_BFITS, BUF_BSTATE, BUF_BITEMS, BUF_BPART, BUF_BORDER, BUF_BCTR, BUF_BLAB, BUF_BMEM, BUF_BCEN, BUF_BXOFF,
+    BUF_KPPC,
     BUF_PF_X32, BUF_PF_XERR, BUF_PF_C32, BUF_PF_CERR, BUF_PF_LIST, BUF_PF_CNT,
     BUF_COUNT
 };
@@ -410,9 +411,25 @@ template <typename T>
 void run_exact_folds(Ctx &ctx, const FoldChain *chains, int nchains, int64_t m, const int *active, T *result,
                      long long *count);
 
+// One seeding: x (n x d of F, device) into centers (k x d, device). draws: an
+// injected uniform stream (device, 0 past its n_draws), or null for the
+// library's stream of seed. nan_direct: a NaN total takes a random row, as a
+// total of zero does (KMeans::fit), or goes through the trials (batched fits).
+struct KppJob {
+    const void *x;
+    const float *x32 = nullptr, *xerr = nullptr;  // set by run_kmeanspp
+    int64_t n;
+    int d, k;
+    const double *draws = nullptr;
+    int64_t n_draws = 0;
+    uint64_t seed = 0;
+    void *centers;
+    bool nan_direct = true;
+};
+// All seedings together, a centre of each per step; in f64 they share one x.
+// draws_used (nullable): the draws each consumed. Synchronises.
 template <typename T>
-void run_kmeanspp(Ctx &ctx, const T *x, int64_t n, int d, int k, const double *draws_dev,
-                  int64_t n_draws, T *centers_out, int64_t *draws_used);
+void run_kmeanspp(Ctx &ctx, std::vector<KppJob> &jobs, int64_t *draws_used);
 
 // Mixed-precision assignment (BF16 / FP8 tcgen05 approximate pass, FP32 and
 // FP64 exact re-check) of X stored as f32. Results identical to the FP64

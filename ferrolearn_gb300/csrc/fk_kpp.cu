@@ -1,5 +1,7 @@
 // fk_kpp.cu -- greedy k-means++ on the GPU (kmeans.rs:169-253), with the
-// reference's arithmetic: every sum is the sequential left fold in F.
+// reference's arithmetic: every sum is the sequential left fold in F. Many
+// seedings (the restarts of a fit, the fits of a batch) run together, one
+// centre of each per step.
 //
 // The reference forms three sums per new centre, each a left fold in F from
 // zero in row order: the total of the D^2 array (kmeans.rs:201), the running
@@ -15,42 +17,54 @@
 //   therefore a map P -> P + a[P & 1], and so is any run of elements: these
 //   maps compose (associatively), and a composed map is exact whenever the
 //   final P stays below the binade's top (the sum only grows, so every
-//   intermediate stayed inside too).
+//   intermediate stayed inside too). A run without an exact half is a plain
+//   integer sum, in any order.
 //
-// kpp_compose_kernel forms, per chunk of KPP_CH values, the composed map for
-// the three binades around the chunk's estimated starting sum (an f64 prefix
-// of chunk sums; the estimate only steers speed, never the result).
-// kpp_walk_kernel then walks the chunks with one warp per fold: a chunk whose
-// map applies is one integer add; otherwise (the sum changes binade inside
-// it, or is zero or non-finite) the warp walks the chunk 32 values at a time
-// with a warp scan of the same maps, taking one exact F addition at each
-// element where the binade changes. Every state it records is bit for bit
-// the reference's running sum.
-//
-// Per new centre: kpp_select_kernel resolves the previous centre's trials
-// (strictly smallest potential, first trial on ties: kmeans.rs:239-243),
-// draws the thresholds u * total in F (:213-214) and finds each trial's
-// candidate (the first row whose running sum reaches its threshold: a 32-ary
-// search over the recorded chunk states, then the chunk walked exactly);
-// kpp_trials_kernel forms min(D^2, d(x, candidate)) for every trial in one
-// pass over X (direct-form distances, no FMA, identical to the reference; in
-// f64, kpp_trials_f64f_kernel bounds them in FP32 first and forms the FP64
-// distance only where the candidate may come closer than D^2);
-// compose and walk give every trial's potential and its chunk states, which
-// the next centre's search uses (the chosen trial's D^2 array becomes the new
-// one without a copy: two buffers alternate). A non-positive total takes one
-// uniform draw as a random row (:202-206).
+// Per new centre, four launches over all seedings:
+//   kpp_pairs_kernel    the trials' candidates against the centres so far: a
+//                       lower bound of each squared distance, as the row
+//                       threshold of the next kernel.
+//   kpp_trials_kernel   min(D^2, d(x, candidate)) for every trial in one pass.
+//                       A row whose D^2 (its distance to its nearest centre q)
+//                       is below a quarter of the bound of d(candidate, q)
+//                       cannot come closer (triangle inequality, with room for
+//                       every rounding): its value is copied without reading
+//                       the row. The other rows are gathered, so that the
+//                       arithmetic runs in full warps. Direct-form distances,
+//                       no FMA; in f64 they are bounded in FP32 first and
+//                       formed in FP64 only where the candidate may come
+//                       closer.
+//   kpp_compose_kernel  per chunk of KPP_CH values the composed map for the
+//                       binade of the chunk's estimated starting sum (and the
+//                       next one, when the chunk may start or end there). The
+//                       estimate, an f32 prefix of partial sums, steers speed,
+//                       never the result.
+//   kpp_walk_kernel     one CTA per fold scans the chunk maps, 1024 at a time;
+//                       a chunk whose map does not apply (the sum changes
+//                       binade in it, or is zero or not finite) is scanned
+//                       value by value, with one exact F addition where the
+//                       binade changes. Every state it records is bit for bit
+//                       the reference's running sum. The seeding's last CTA
+//                       then takes the strictly smallest potential (first
+//                       trial on ties: kmeans.rs:239-243), draws the next
+//                       thresholds u * total in F (:213-214) and finds each
+//                       trial's candidate: the first row whose running sum
+//                       reaches its threshold (a 32-ary search over the chunk
+//                       states, then that chunk walked exactly).
+// The chosen trial's D^2 array becomes the new one without a copy (two
+// buffers alternate). A non-positive total takes one uniform draw as a random
+// row (:202-206).
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
+#include <cstring>
+#include <vector>
 
 #include "fk_internal.cuh"
 
 namespace fk {
 namespace {
 
-template <typename T> __device__ __forceinline__ T kpp_sub(T a, T b);
-template <> __device__ __forceinline__ float kpp_sub(float a, float b) { return __fsub_rn(a, b); }
-template <> __device__ __forceinline__ double kpp_sub(double a, double b) { return __dsub_rn(a, b); }
 template <typename T> __device__ __forceinline__ T kpp_mul(T a, T b);
 template <> __device__ __forceinline__ float kpp_mul(float a, float b) { return __fmul_rn(a, b); }
 template <> __device__ __forceinline__ double kpp_mul(double a, double b) { return __dmul_rn(a, b); }
@@ -58,12 +72,11 @@ template <typename T> __device__ __forceinline__ T kpp_add(T a, T b);
 template <> __device__ __forceinline__ float kpp_add(float a, float b) { return __fadd_rn(a, b); }
 template <> __device__ __forceinline__ double kpp_add(double a, double b) { return __dadd_rn(a, b); }
 
-constexpr int KPP_CH = 1024;      // values per fold chunk (and rows per trial-pass CTA)
-constexpr int KPP_GROUPS = KPP_CH / 32;  // 32-value groups per chunk
-constexpr int KPP_THREADS = 256;
+constexpr int KPP_CH = 1024;      // values per fold chunk
+constexpr int KPP_THREADS = 256;  // every kernel's block
+constexpr int KPP_WARPS = KPP_THREADS / 32;
 constexpr int MAX_TRIALS = 16;
-constexpr int KPP_PAD = 4;        // row padding of the staged X tile (16 bytes of f32)
-constexpr long long KPP_SAT = 1LL << 61;  // saturated increment: never applies
+constexpr int KPP_SLAB = 64;      // features staged at a time
 
 // ---------------------------------------------------- binade arithmetic --
 template <typename T> struct Bits;
@@ -100,245 +113,203 @@ __device__ __forceinline__ bool is_inf_or_nan(T p) {
 
 // Significand of a normal value as an integer in [2^MB, 2^(MB+1)).
 template <typename T>
-__device__ __forceinline__ long long significand(T p) {
+__device__ __forceinline__ typename Bits<T>::U significand(T p) {
     using B = Bits<T>;
     const typename B::U m = ((typename B::U)1 << B::MB) - 1;
-    return (long long)((B::bits(p) & m) | ((typename B::U)1 << B::MB));
+    return (B::bits(p) & m) | ((typename B::U)1 << B::MB);
 }
 
 template <typename T>
-__device__ __forceinline__ T from_parts(int be, long long P) {
+__device__ __forceinline__ T from_parts(int be, typename Bits<T>::U P) {
     using B = Bits<T>;
     const typename B::U m = ((typename B::U)1 << B::MB) - 1;
-    return B::from(((typename B::U)be << B::MB) | ((typename B::U)P & m));
+    return B::from(((typename B::U)be << B::MB) | (P & m));
 }
 
-// Increment map of one value v >= 0 on the grid of binade be: a0 / a1 for a
-// running sum whose significand is even / odd. Integer arithmetic on the
-// value's significand m and exponent: v / ulp = m * 2^(e - be), so the
-// rounded increment is m shifted right by be - e, rounded to nearest, with
-// an exact half left to the sum's parity (ties to even).
-struct Step {
-    long long a0, a1;
-};
-
+// Increment of one value on the grid of binade be, and whether it is an exact
+// half (then rounded down here: the sum's parity decides). Values that leave
+// the binade, and negative or non-finite ones, give 2^(MB+1), which no sum in
+// the binade can take.
 template <typename T>
-__device__ __forceinline__ Step step_of(T v, int be) {
+__device__ __forceinline__ typename Bits<T>::U inc_of(T v, int be, bool &tie) {
     using B = Bits<T>;
     using U = typename B::U;
+    constexpr U OUT = (U)1 << (B::MB + 1);
     const U b = B::bits(v);
-    const int ev = (int)((b >> B::MB) & (U)B::EXPM);
-    if (ev == B::EXPM) return {KPP_SAT, KPP_SAT};  // inf or NaN
+    const int ev = (int)(b >> B::MB);  // the sign bit makes it > EXPM
+    if (ev >= B::EXPM) return (U)(b << 1) == 0 ? (U)0 : OUT;  // negative (-0 is harmless), inf, NaN
     const U mask = ((U)1 << B::MB) - 1;
-    if (b >> (sizeof(U) * 8 - 1))                   // negative: only -0 is harmless
-        return (b << 1) == 0 ? Step{0, 0} : Step{KPP_SAT, KPP_SAT};
-    U m = b & mask;
-    int e = ev;
-    if (ev == 0) {
-        if (m == 0) return {0, 0};
-        e = 1;  // subnormal: no hidden bit, the exponent of the smallest normals
-    } else {
-        m |= (U)1 << B::MB;
+    const U m = (b & mask) | (ev ? (U)1 << B::MB : (U)0);
+    const int r = be - (ev ? ev : 1);
+    if (r < 0) return m == 0 ? (U)0 : OUT;
+    if (r > B::MB + 2) return (U)0;
+    if (r == 0) return m;
+    const U half = (U)1 << (r - 1);
+    const U s = m + half;
+    const bool t = (s & ((half << 1) - 1)) == 0;
+    tie |= t;
+    return (s >> r) - (t ? (U)1 : (U)0);
+}
+
+// The map of 32 values, a lane each (dead lanes: increment 0), for binade be.
+// A tie rounds the sum to even, so the parity after it is known and every later
+// tie of the group is settled by the parities since the one before; only the
+// first tie depends on the sum's parity at the start. Saturated at 2^(MB+1).
+template <typename T>
+struct GMap {
+    typename Bits<T>::U a0, a1;
+};
+
+__device__ __forceinline__ uint32_t warp_sum(uint32_t v) { return __reduce_add_sync(0xffffffffu, v); }
+__device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
+    // values up to 2^54: two halves of 27 bits, 32 lanes
+    const uint32_t lo = (uint32_t)v & ((1u << 27) - 1u), hi = (uint32_t)(v >> 27);
+    return ((unsigned long long)__reduce_add_sync(0xffffffffu, hi) << 27) +
+           (unsigned long long)__reduce_add_sync(0xffffffffu, lo);
+}
+
+// The parity of the increments since the last tie before this lane (from lane
+// 0 if there is none), this lane's included: 1 where a tie here rounds up.
+__device__ __forceinline__ unsigned tie_up(unsigned ties, unsigned odd, int lane) {
+    const unsigned before = ties & ((1u << lane) - 1u);
+    unsigned since = odd & (0xffffffffu >> (31 - lane));
+    if (before) since &= ~(0xffffffffu >> __clz(before));
+    return (unsigned)__popc(since) & 1u;
+}
+
+template <typename T>
+__device__ __forceinline__ GMap<T> group_map(T v, bool live, int be) {
+    using U = typename Bits<T>::U;
+    constexpr U OUT = (U)1 << (Bits<T>::MB + 1);
+    const int lane = threadIdx.x & 31;
+    bool tie = false;
+    U inc = live ? inc_of(v, be, tie) : (U)0;
+    const unsigned ties = __ballot_sync(0xffffffffu, tie);
+    if (!ties) {
+        const U s = warp_sum(inc);
+        const U a = s < OUT ? s : OUT;
+        return GMap<T>{a, a};
     }
-    const int sh = e - be;
-    if (sh > 0) return {KPP_SAT, KPP_SAT};  // v >= 2^(be+1): the sum leaves the binade
-    const int r = -sh;
-    if (r == 0) return {(long long)m, (long long)m};
-    if (r > B::MB + 2) return {0, 0};  // v < ulp / 2 by far: rounds away, never a half
-    const long long q = (long long)(m >> r);
-    const U rem = m & (((U)1 << r) - 1), half = (U)1 << (r - 1);
-    if (rem > half) return {q + 1, q + 1};
-    if (rem < half) return {q, q};
-    return {q + (q & 1), q + ((q + 1) & 1)};  // exact half: the even neighbour
+    const unsigned odd = __ballot_sync(0xffffffffu, (inc & 1) != 0);
+    const int first = __ffs(ties) - 1;
+    const unsigned up = tie_up(ties, odd, lane);
+    if (tie && lane != first) inc += up;
+    const U s = warp_sum(inc);
+    const U e = (U)__shfl_sync(0xffffffffu, up, first);  // what the first tie adds to an even sum
+    const U a0 = s + e, a1 = s + (1 - e);
+    return GMap<T>{a0 < OUT ? a0 : OUT, a1 < OUT ? a1 : OUT};
 }
 
 // f then g
-__device__ __forceinline__ Step compose(Step f, Step g) {
-    const long long g0 = (f.a0 & 1) ? g.a1 : g.a0;      // even start: parity after f is f.a0's
-    const long long g1 = ((1 + f.a1) & 1) ? g.a1 : g.a0;  // odd start
-    long long h0 = f.a0 + g0, h1 = f.a1 + g1;
-    if (h0 > KPP_SAT) h0 = KPP_SAT;
-    if (h1 > KPP_SAT) h1 = KPP_SAT;
-    return {h0, h1};
+template <typename T>
+__device__ __forceinline__ GMap<T> gcompose(const GMap<T> &f, const GMap<T> &g) {
+    return GMap<T>{f.a0 + ((f.a0 & 1) ? g.a1 : g.a0), f.a1 + ((f.a1 & 1) ? g.a0 : g.a1)};
 }
 
-__device__ __forceinline__ Step shfl_up_step(Step s, int off) {
-    return {(long long)__shfl_up_sync(0xffffffffu, (unsigned long long)s.a0, off),
-            (long long)__shfl_up_sync(0xffffffffu, (unsigned long long)s.a1, off)};
-}
-__device__ __forceinline__ Step shfl_down_step(Step s, int off) {
-    return {(long long)__shfl_down_sync(0xffffffffu, (unsigned long long)s.a0, off),
-            (long long)__shfl_down_sync(0xffffffffu, (unsigned long long)s.a1, off)};
-}
-
-// One group of up to 32 values (lane i holds value i of the group, len of
-// them valid) added to the running sum p in order, exactly as the sequential
-// fold. Warp-uniform result. With thr given, *hit receives the first value
-// index whose inclusive running sum reaches *thr (-1 if none).
-template <typename T, bool SEARCH>
-__device__ T walk_group(T p, T v, int len, T thr, int *hit) {
+// Inclusive scan over the lanes of saturated maps (at most 32 * 2^(MB+1): no overflow).
+template <typename T>
+__device__ __forceinline__ GMap<T> gscan(GMap<T> m) {
     const int lane = threadIdx.x & 31;
-    constexpr long long TOP = 1LL << (Bits<T>::MB + 1);
-    int start = 0;
-    if (SEARCH) *hit = -1;
-    while (start < len) {
-        const bool live = lane >= start && lane < len;
-        const int be = normal_exp(p);
-        if (be == 0) {
-            if (p != p) return p;  // a NaN sum stays NaN and reaches no threshold
-            const T vs = __shfl_sync(0xffffffffu, v, start);
-            if (is_inf_or_nan(p)) {
-                // +inf stays +inf until a NaN value arrives, which makes it NaN
-                if (SEARCH) {
-                    const T p1 = kpp_add(p, vs);
-                    if (p1 >= thr) {
-                        *hit = start;
-                        return p1;
-                    }
-                }
-                const unsigned nanm = __ballot_sync(0xffffffffu, live && v != v);
-                if (nanm) p = __shfl_sync(0xffffffffu, v, __ffs(nanm) - 1);
-                return p;
-            }
-            // zero or subnormal sum: one exact addition
-            p = kpp_add(p, vs);
-            if (SEARCH && p >= thr) {
-                *hit = start;
-                return p;
-            }
-            start++;
-            continue;
-        }
-        const long long P = significand(p);
-        Step s = live ? step_of(v, be) : Step{0, 0};
 #pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const Step o = shfl_up_step(s, off);
-            if (lane >= off) s = compose(o, s);
-        }
-        const long long Pl = P + ((P & 1) ? s.a1 : s.a0);
-        const unsigned badm = __ballot_sync(0xffffffffu, live && !(Pl < TOP));
-        const int f0 = badm ? __ffs(badm) - 1 : len;  // first value that leaves the binade
-        if (SEARCH) {
-            const T pl = from_parts<T>(be, Pl < TOP ? Pl : P);
-            const unsigned hm = __ballot_sync(0xffffffffu, live && lane < f0 && pl >= thr);
-            if (hm) {
-                *hit = __ffs(hm) - 1;
-                return __shfl_sync(0xffffffffu, pl, *hit);
-            }
-        }
-        if (f0 > start) {
-            const long long Pb = (long long)__shfl_sync(0xffffffffu, (unsigned long long)Pl, f0 - 1);
-            p = from_parts<T>(be, Pb);
-        }
-        if (f0 >= len) return p;
-        const T vf = __shfl_sync(0xffffffffu, v, f0);
-        p = kpp_add(p, vf);  // the one exact addition where the binade changes
-        if (SEARCH && p >= thr) {
-            *hit = f0;
-            return p;
-        }
-        start = f0 + 1;
+    for (int off = 1; off < 32; off <<= 1) {
+        const GMap<T> o{__shfl_up_sync(0xffffffffu, m.a0, off), __shfl_up_sync(0xffffffffu, m.a1, off)};
+        if (lane >= off) m = gcompose(o, m);
     }
-    return p;
+    return m;
 }
 
-// Maps of one chunk or group for the three binades of its window.
-struct Map3 {
-    Step s[3];
-};
-
-__device__ __forceinline__ Step pick(const Map3 &m, int slot) {
-    return slot == 0 ? m.s[0] : (slot == 1 ? m.s[1] : m.s[2]);
+// Up to 32 values from p (normal, binade be, significand P) on, a lane each:
+// the state after each lane's value (valid up to the first that reaches 2^(MB+1)).
+template <typename T>
+__device__ __forceinline__ typename Bits<T>::U group_states(T v, bool live, int be, typename Bits<T>::U P) {
+    using U = typename Bits<T>::U;
+    const int lane = threadIdx.x & 31;
+    bool tie = false;
+    U inc = live ? inc_of(v, be, tie) : (U)0;
+    const unsigned ties = __ballot_sync(0xffffffffu, tie);
+    const unsigned odd = __ballot_sync(0xffffffffu, (inc & 1) != 0);
+    if (tie) {
+        unsigned up = tie_up(ties, odd, lane);
+        if (!(ties & ((1u << lane) - 1u))) up ^= (unsigned)(P & 1);  // the first tie: the sum's own parity counts
+        inc += up;
+    }
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const U o = __shfl_up_sync(0xffffffffu, inc, off);
+        if (lane >= off) inc += o;
+    }
+    return P + inc;
 }
 
-// Where the fold data of one buffer / trial slice live (kpp_layout on the host).
-struct FoldSlices {
-    int *elo;       // [2][ts][nch] lowest binade of each chunk's window (-1: none)
-    Map3 *cmap;     // [2][ts][nch] chunk maps
-    Map3 *gmap;     // [2][ts][nch][32] group maps
-    void *states;   // [2][ts][nch] running sum at each chunk's end (T)
+// Maps of one chunk for the binades elo and elo + 1 (elo < 0: none; cnt of
+// them built), saturated as GMap.
+template <typename T>
+struct CMap {
+    GMap<T> s[2];
+    int elo, cnt;
 };
+
+// A value as an f32 summand of the folds' estimates: F = f32 itself, F = f64
+// times 2^-esc by its bits (no FP64 conversion; out of range: 0 or inf).
+__device__ __forceinline__ float est_of(float v, int) { return v; }
+__device__ __forceinline__ float est_of(double v, int esc) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    const int e = (int)((b >> 52) & 0x7FFull) - 1023 - esc + 127;
+    if (e <= 0) return 0.f;
+    if (e >= 255) return INFINITY;
+    return __uint_as_float(((uint32_t)e << 23) | (uint32_t)((b >> 29) & 0x7FFFFFull));
+}
+// Biased exponent in F of an estimate, else 0.
+__device__ __forceinline__ int est_exp(float e, int, float) { return normal_exp(e); }
+__device__ __forceinline__ int est_exp(float e, int esc, double) {
+    const int be = normal_exp(e);
+    const int b64 = be - 127 + esc + 1023;
+    return be > 0 && b64 >= 1 && b64 < 0x7FF ? b64 : 0;
+}
 
 struct KppState {
-    long long cursor;  // uniform draws consumed so far
-    int direct;        // the current centre was a uniform random row (no trials)
-    int cur;           // buffer holding the current D^2 array ...
-    int cur_trial;     // ... and its trial slice
-    int pending;       // trial results not yet resolved into a centre
-    int wbuf;          // buffer the pending trials were written to
-    int ntr;           // their count
-    int pcentre;       // their centre index (-1: the first D^2 array)
-    int pad;
+    long long cursor;       // uniform draws consumed so far
+    int direct[2];          // centre c was a uniform random row (slot c & 1): it has no trials
+    int cur, cur_trial;     // buffer and trial slice of the current D^2 array
+    int prev_trial;         // slice (of the other buffer) of the array before it
+    int own_c;              // centre the current array was formed with (-1: the first)
+    int done;               // folds of this step already walked
+    int esc;                // exponent offset of the f64 estimates
     long long cand[MAX_TRIALS];
-    double thr[MAX_TRIALS];
-    double pot[MAX_TRIALS];  // fold of each pending trial's array (F, widened)
+    double pot[MAX_TRIALS];  // fold of each trial's array (F, widened)
     double total;            // fold of the current D^2 array
 };
 
-// The values of one chunk (clen of them) added to p in order, exactly as the
-// sequential fold: the groups' maps scanned 32 at a time, and a group whose
-// map does not apply walked value by value. With SEARCH, *hit receives the
-// index (within the chunk) of the first value whose inclusive running sum
-// reaches thr, or -1.
-template <typename T, bool SEARCH>
-__device__ T walk_chunk(T p, const T *__restrict__ cv, int clen, const Map3 *__restrict__ gm, int e_lo, T thr,
-                        int *hit) {
-    const int lane = threadIdx.x & 31;
-    constexpr long long TOP = 1LL << (Bits<T>::MB + 1);
-    const int ng = (clen + 31) / 32;
-    Map3 g{};
-    if (e_lo >= 0 && lane < ng) g = gm[lane];
-    if (SEARCH) *hit = -1;
-    int start = 0;
-    while (start < ng) {
-        const int be = normal_exp(p);
-        const int slot = be - e_lo;
-        if (!(be > 0 && e_lo >= 0 && slot >= 0 && slot < 3)) {
-            // no map for this sum: the first remaining group value by value
-            const int len = min(32, clen - start * 32);
-            const T val = lane < len ? cv[start * 32 + lane] : T(0);
-            int h = -1;
-            p = walk_group<T, SEARCH>(p, val, len, thr, &h);
-            if (SEARCH && h >= 0) {
-                *hit = start * 32 + h;
-                return p;
-            }
-            start++;
-            continue;
-        }
-        const bool live = lane >= start && lane < ng;
-        Step s = live ? pick(g, slot) : Step{0, 0};
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const Step o = shfl_up_step(s, off);
-            if (lane >= off) s = compose(o, s);
-        }
-        const long long P = significand(p);
-        const long long Pl = P + ((P & 1) ? s.a1 : s.a0);
-        const unsigned badm = __ballot_sync(0xffffffffu, live && !(Pl < TOP));
-        const int f0 = badm ? __ffs(badm) - 1 : ng;  // first group whose map does not apply
-        int gsel = f0;                                 // the group to walk value by value
-        if (SEARCH) {
-            const unsigned hm = __ballot_sync(0xffffffffu, live && lane < f0 && from_parts<T>(be, Pl) >= thr);
-            if (hm) gsel = __ffs(hm) - 1;              // the threshold is reached inside this group
-        }
-        if (gsel > start) {
-            const long long Pb = (long long)__shfl_sync(0xffffffffu, (unsigned long long)Pl, gsel - 1);
-            p = from_parts<T>(be, Pb);
-        }
-        if (gsel >= ng) return p;
-        const int len = min(32, clen - gsel * 32);
-        const T val = lane < len ? cv[gsel * 32 + lane] : T(0);
-        int h = -1;
-        p = walk_group<T, SEARCH>(p, val, len, thr, &h);
-        if (SEARCH && h >= 0) {
-            *hit = gsel * 32 + h;
-            return p;
-        }
-        start = gsel + 1;
-    }
-    return p;
+// One seeding (device copy of a KppJob and its workspace).
+template <typename T>
+struct KppFit {
+    const T *x;
+    const float *x32, *xerr;  // f32 rows (F = f32: x itself) and their rounding-error norms (F = f64)
+    const double *draws;      // injected draws (n_draws of them, 0 past the end); null: the stream of seed
+    T *centers;
+    T *chains;                // [2][trials][n] D^2 arrays
+    T *states;                // [2][trials][nch] running sum at each chunk's end
+    CMap<T> *cmaps;           // [trials][nch]
+    T *gstates;               // [2][trials][32] running sum after each 32 values of the first chunk
+    float *csum;              // [trials][tiles] estimates of the tiles' sums
+    T *thr;                   // [k] skip threshold of each centre's rows at this step
+    int32_t *own;             // [n] nearest centre so far
+    int32_t *crow;            // [k] rows chosen
+    KppState *st;
+    long long n, nch, tiles, n_draws;
+    unsigned long long seed;
+    int d, k, trials, nan_direct;
+};
+
+template <typename T>
+__device__ __forceinline__ double draw_at(const KppFit<T> &f, long long i) {
+    if (f.draws) return i < f.n_draws ? f.draws[i] : 0.0;
+    // splitmix64: draw i mixes the state after i + 1 golden-gamma steps
+    unsigned long long z = f.seed + (unsigned long long)(i + 1) * 0x9E3779B97F4A7C15ULL;
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ULL;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBULL;
+    z = z ^ (z >> 31);
+    return (double)(z >> 11) * (1.0 / 9007199254740992.0);
 }
 
 __device__ __forceinline__ long long draw_to_range(double u, long long n) {
@@ -348,164 +319,75 @@ __device__ __forceinline__ long long draw_to_range(double u, long long n) {
     return i;
 }
 
+// Work item: block blockIdx.x serves part y of seeding x (null table: one
+// seeding, part blockIdx.x).
+__device__ __forceinline__ int2 item_at(const int2 *__restrict__ items) {
+    return items ? items[blockIdx.x] : make_int2(0, (int)blockIdx.x);
+}
+
 template <typename T>
-__global__ void kpp_first_kernel(const T *__restrict__ x, long long n, int d, const double *__restrict__ draws,
-                                 long long n_draws, KppState *st, T *__restrict__ centers) {
+__global__ void kpp_first_kernel(const KppFit<T> *__restrict__ fits) {
+    const KppFit<T> f = fits[blockIdx.x];
     __shared__ long long first;
     if (threadIdx.x == 0) {
-        const double u = n_draws > 0 ? draws[0] : 0.0;
-        first = draw_to_range(u, n);
+        first = draw_to_range(draw_at(f, 0), f.n);
+        KppState *st = f.st;
         st->cursor = 1;
-        st->direct = 0;
+        st->direct[0] = st->direct[1] = 0;
+        st->cur = st->cur_trial = st->prev_trial = 0;
+        st->own_c = -1;
+        st->done = 0;
+        st->esc = 0;
         st->cand[0] = first;
-        st->pending = 1;  // the first D^2 array: no centre to resolve
-        st->wbuf = 0;
-        st->ntr = 1;
-        st->pcentre = -1;
+        f.crow[0] = (int32_t)first;
     }
     __syncthreads();
-    for (int j = threadIdx.x; j < d; j += blockDim.x) centers[j] = x[first * d + j];
+    for (int j = threadIdx.x; j < f.d; j += blockDim.x) f.centers[j] = f.x[first * f.d + j];
 }
 
-template <typename T> struct TrialTile;
-template <> struct TrialTile<float> { static constexpr int DJ = 8; };
-template <> struct TrialTile<double> { static constexpr int DJ = 4; };
-
-// Two stages of the staged tile (rows and trial candidates), filled with
-// asynchronous copies one feature round ahead.
-template <typename T, int TT>
-constexpr size_t trial_smem() {
-    return 2 * sizeof(T) * ((size_t)TrialTile<T>::DJ * (KPP_CH + KPP_PAD) + (size_t)TrialTile<T>::DJ * TT);
-}
-
-// One element from global to shared memory, asynchronously (cp.async of 4
-// or 8 bytes); ok == false writes zero (src-size 0: nothing is read).
+// Squared distances of the step's candidates to the centres so far, bounded
+// below (one warp per centre), as row thresholds (the smallest over the
+// trials): a row whose D^2 value m is its computed distance to centre q, and
+// m < thr[q], cannot come closer to any candidate. With g = (d + 4) u the relative error of a direct form, D = the
+// exact distance: D(x, q) <= m (1 + 2g), thr = L (1 - rho) / 4 with L <= D(cand,
+// q), so sqrt D(x, cand) >= sqrt L - sqrt D(x, q) >= sqrt D(x, q) (1 + rho - 2g)
+// and the computed distance to the candidate is at least m (1 + 2 rho - 8g) > m
+// for rho = (d + 8) 1e-6 (8g <= (d + 4) 4.8e-7 in f32). Bounds below 1e-30,
+// where underflow would count, and NaN skip nothing.
 template <typename T>
-__device__ __forceinline__ void cp_async_elem(T *dst, const T *src, bool ok) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-    const int n = ok ? (int)sizeof(T) : 0;
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(src), "n"((int)sizeof(T)), "r"(n)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// One CTA per chunk of KPP_CH rows, 4 rows per thread, all TT trial slots per
-// thread (ntr <= TT of them live): every trial's min(D^2, d(x, candidate))
-// (INIT: d(x, first row), the first D^2 array; kmeans.rs:188-195, 225-233)
-// with the direct form folded over the features in order, and the chunk's
-// sums (only an estimate for the fold's binade windows). The features come
-// in rounds of DJ, staged in shared memory by asynchronous copies one round
-// ahead of the arithmetic (two stages).
-template <typename T, int TT, bool INIT>
-__global__ void __launch_bounds__(KPP_THREADS)
-    kpp_trials_kernel(const T *__restrict__ x, long long n, int d, T *__restrict__ chains, int tstride,
-                      const KppState *__restrict__ st, int ntr, double *__restrict__ csum, long long nch) {
-    if (!INIT && st->direct) return;
-    constexpr int DJ = TrialTile<T>::DJ;
-    constexpr int XS = KPP_CH + KPP_PAD;  // row length of the staged tile
-    extern __shared__ __align__(16) unsigned char kpp_smem[];
-    constexpr int STAGE = DJ * XS + DJ * TT;  // elements of one stage
-    // stage q: xs = [DJ][XS] (feature-major, rows contiguous), then cs = [DJ][TT]
-    T *const stages = reinterpret_cast<T *>(kpp_smem);
-    __shared__ long long cand[TT];
-    __shared__ double red[TT][KPP_THREADS / 32];
-    const int tid = threadIdx.x;
-    if (tid < TT) cand[tid] = tid < ntr ? st->cand[tid] : 0;
-    const int cur = INIT ? 0 : st->cur, cur_trial = INIT ? 0 : st->cur_trial, wbuf = INIT ? 0 : 1 - cur;
-    const T *mind = chains + ((long long)cur * tstride + cur_trial) * n;
-    T *out = chains + (long long)wbuf * tstride * n;
-    const long long base = (long long)blockIdx.x * KPP_CH;
-    T acc[4][TT];
-#pragma unroll
-    for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int b = 0; b < TT; b++) acc[a][b] = T(0);
-    __syncthreads();  // cand
-    auto stage_round = [&](int j0, int q) {
-        T *xs = stages + q * STAGE;
-        T *cs = xs + DJ * XS;
-        const int jn = min(DJ, d - j0);
-        for (int e = tid; e < KPP_CH * DJ; e += KPP_THREADS) {
-            const int r = e / DJ, jj = e - r * DJ;
-            const long long gr = base + r;
-            const bool ok = gr < n && jj < jn;
-            cp_async_elem(xs + jj * XS + r, ok ? x + gr * d + j0 + jj : x, ok);
+__global__ void __launch_bounds__(KPP_THREADS) kpp_pairs_kernel(const KppFit<T> *__restrict__ fits, int c) {
+    const unsigned groups = (unsigned)((c + KPP_WARPS - 1) / KPP_WARPS);
+    const KppFit<T> &f = fits[blockIdx.x / groups];
+    if (f.st->direct[c & 1]) return;
+    const int lane = threadIdx.x & 31;
+    const int q = (int)(blockIdx.x % groups) * KPP_WARPS + (threadIdx.x >> 5);
+    if (q >= c) return;
+    const int d = f.d;
+    const long long rq = f.crow[q];
+    const float *xq = f.x32 + rq * d;
+    const float eq = f.xerr ? f.xerr[rq] : 0.f;
+    const float rho = (float)(d + 8) * 1e-6f;
+    float thmin = FLT_MAX;
+#pragma unroll 4
+    for (int t = 0; t < f.trials; t++) {
+        const long long rc = f.st->cand[t];
+        const float *xc = f.x32 + rc * d;
+        float s = 0.f;
+        for (int j = lane; j < d; j += 32) {
+            const float v = __fsub_rn(xc[j], xq[j]);
+            s = __fmaf_rn(v, v, s);
         }
-        for (int e = tid; e < TT * DJ; e += KPP_THREADS) {
-            const int t = e / DJ, jj = e - t * DJ;
-            const bool ok = t < ntr && jj < jn;
-            cp_async_elem(cs + jj * TT + t, ok ? x + cand[t] * d + j0 + jj : x, ok);
-        }
-        cp_async_commit();
-    };
-    stage_round(0, 0);
-    for (int j0 = 0, q = 0; j0 < d; j0 += DJ, q ^= 1) {
-        const int jn = min(DJ, d - j0);
-        if (j0 + DJ < d) {
-            stage_round(j0 + DJ, q ^ 1);  // the next round's copies fly during this round
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
-        }
-        __syncthreads();  // every thread's copies of this round have landed
-        const T *xs = stages + q * STAGE;
-        const T *cs = xs + DJ * XS;
-        for (int jj = 0; jj < jn; jj++) {
-            T xv[4], cvv[TT];
 #pragma unroll
-            for (int a = 0; a < 4; a++) xv[a] = xs[jj * XS + tid * 4 + a];
-#pragma unroll
-            for (int b = 0; b < TT; b++) cvv[b] = cs[jj * TT + b];
-#pragma unroll
-            for (int a = 0; a < 4; a++)
-#pragma unroll
-                for (int b = 0; b < TT; b++) {
-                    const T df = kpp_sub(xv[a], cvv[b]);
-                    acc[a][b] = kpp_add(acc[a][b], kpp_mul(df, df));
-                }
-        }
-        __syncthreads();  // this stage is refilled by the next round's staging
+        for (int o = 16; o >= 1; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        const float ec = f.xerr ? __fadd_ru(f.xerr[rc], eq) : 0.f;
+        const float th = 0.25f * __fsub_rd(s, bound32(s, ec, d)) * (1.0f - rho);
+        thmin = th < thmin ? th : (th >= thmin ? thmin : 0.f);  // NaN: 0
     }
-    double psum[TT];
-#pragma unroll
-    for (int b = 0; b < TT; b++) psum[b] = 0.0;
-#pragma unroll
-    for (int a = 0; a < 4; a++) {
-        const long long row = base + tid * 4 + a;
-        if (row < n) {
-            const T m = INIT ? T(0) : mind[row];
-#pragma unroll
-            for (int b = 0; b < TT; b++) {
-                if (b < ntr) {
-                    const T v = acc[a][b];
-                    const T r = INIT ? v : (v < m ? v : m);  // kmeans.rs:230-232
-                    out[(long long)b * n + row] = r;
-                    psum[b] += (double)r;
-                }
-            }
-        }
-    }
-    const int lane = tid & 31, w = tid >> 5;
-#pragma unroll
-    for (int b = 0; b < TT; b++) {
-        double v = psum[b];
-#pragma unroll
-        for (int off = 16; off >= 1; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-        if (lane == 0) red[b][w] = v;
-    }
-    __syncthreads();
-    if (tid < ntr) {
-        double v = 0.0;
-        for (int q = 0; q < KPP_THREADS / 32; q++) v += red[tid][q];
-        csum[(long long)tid * nch + blockIdx.x] = v;
-    }
+    if (lane == 0) f.thr[q] = thmin > 1e-30f && thmin < FLT_MAX ? (T)thmin : T(0);
 }
 
-// The direct form in FP64, in the reference's order (the loads run ahead of
-// the dependent adds).
-__device__ __forceinline__ double sqeuc_f64(const double *__restrict__ a, const double *__restrict__ b, int d) {
+// d(a, b), direct form in the reference's order.
+__device__ __forceinline__ double sqeuc(const double *__restrict__ a, const double *__restrict__ b, int d) {
     double v = 0.0;
 #pragma unroll 8
     for (int j = 0; j < d; j++) {
@@ -515,541 +397,1019 @@ __device__ __forceinline__ double sqeuc_f64(const double *__restrict__ a, const 
     return v;
 }
 
-constexpr int KPP_OPEN = 2048;  // listed open pairs a chunk (row within the chunk << 4 | trial)
-static_assert(KPP_CH <= 4096, "a chunk row fits the list entry's 12 bits");
+// m < thr for D^2 values and thresholds >= 0 (f64 by their bits: no FP64
+// comparison; a NaN is never below).
+__device__ __forceinline__ bool below(float m, float th) { return m < th; }
+__device__ __forceinline__ bool below(double m, double th) {
+    return (unsigned long long)__double_as_longlong(m) < (unsigned long long)__double_as_longlong(th);
+}
 
-// The f64 trial pass through FP32 bounds: the same outputs as
-// kpp_trials_kernel<double, TT, false>, bit for bit. The distances are first
-// formed in FP32 from the rows' f32 copies (t = x - c, fma), with the
-// rigorous bound b = bound32(d32, e_row + e_candidate, d) of their distance
-// from the exact distance and from the FP64 direct form. Where d32 - b (down)
-// exceeds the row's current D^2 value m, the FP64 distance v is larger too and
-// min(v, m) is m (kmeans.rs:230-232); only the other (row, trial) pairs --
-// rows the candidate may come closer to, non-finite values, values beyond the
-// f32 range -- form v with the direct form in FP64, in the reference's order.
-template <int TT>
+// 16 or 4 bytes from global to shared memory, asynchronously; ok == false
+// writes zeros (nothing is read).
+__device__ __forceinline__ void cp_async16(float *dst, const float *src, bool ok) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(ok ? 16 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async4(float *dst, const float *src, bool ok) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(ok ? 4 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Row stride (floats) of a staged slab: a multiple of 4 with an odd number of
+// 16-byte units, so that eight lanes reading 16 bytes of eight rows meet no
+// bank conflict.
+__host__ __device__ inline int slab_width(int d) { return d < KPP_SLAB ? (d + 3) / 4 * 4 : KPP_SLAB; }
+__host__ __device__ inline int slab_stride(int w) { return (w / 4) & 1 ? w + 8 : w + 4; }
+inline size_t trial_smem(int dmax, int tt) {
+    const int w = slab_width(dmax);
+    return sizeof(float) * ((size_t)KPP_THREADS * slab_stride(w) + (size_t)tt * w);
+}
+
+// One CTA per tile of `scan` rows (a divisor of KPP_CH, a multiple of 256):
+// every trial's min(D^2, d(x, candidate)) (INIT: d(x, first row), the first
+// D^2 array; kmeans.rs:188-195, 225-233), and estimates of the tile's sums.
+// First the rows' owners (nearest centre so far) are brought up to date and
+// the rows that no candidate can come closer to get their values; the others
+// are listed, then scored 256 at a time, a thread a row with all TT trials,
+// the row read from a slab of KPP_SLAB features in shared memory.
+//
+// Bound at n = 1M, d = 64, 7 trials in f32: the FP32 pipe for the listed rows
+// (3 d operations a pair), L2 for the values (8 bytes a pair).
+template <typename T, int TT, bool INIT>
 __global__ void __launch_bounds__(KPP_THREADS)
-    kpp_trials_f64f_kernel(const double *__restrict__ x, const float *__restrict__ x32,
-                           const float *__restrict__ xerr, long long n, int d, double *__restrict__ chains,
-                           int tstride, const KppState *__restrict__ st, int ntr, double *__restrict__ csum,
-                           long long nch) {
-    if (st->direct) return;
-    constexpr int DJ = TrialTile<float>::DJ;
-    constexpr int XS = KPP_CH + KPP_PAD;  // row length of the staged tile
+    kpp_trials_kernel(const KppFit<T> *__restrict__ fits, const int2 *__restrict__ items, int scan, int c) {
+    constexpr bool F64 = sizeof(T) == 8;
+    const int2 it = item_at(items);
+    const KppFit<T> &f = fits[it.x];
+    const KppState *st = f.st;
+    if (!INIT && st->direct[c & 1]) return;
+    const int d = f.d, ntr = INIT ? 1 : f.trials;
+    const long long n = f.n, base = (long long)it.y * scan;
     extern __shared__ __align__(16) unsigned char kpp_smem[];
-    constexpr int STAGE = DJ * XS + DJ * TT;  // elements of one stage
-    float *const stages = reinterpret_cast<float *>(kpp_smem);
+    const int W = slab_width(d), XS = slab_stride(W);
+    float *const xs = reinterpret_cast<float *>(kpp_smem);  // [256][XS] rows
+    float *const cs = xs + KPP_THREADS * XS;                // [TT][W] candidates
     __shared__ long long cand[TT];
     __shared__ float cerr[TT];
-    __shared__ double red[TT][KPP_THREADS / 32];
-    __shared__ double open_sum[TT];
-    __shared__ unsigned short open_pairs[KPP_OPEN];
-    __shared__ int open_n;
-    const int tid = threadIdx.x;
+    __shared__ unsigned short list[KPP_CH];
+    __shared__ unsigned short open_pairs[F64 ? KPP_THREADS * TT : 1];
+    __shared__ int list_n, open_n;
+    __shared__ float red[TT][KPP_WARPS];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     if (tid < TT) {
         cand[tid] = tid < ntr ? st->cand[tid] : 0;
-        cerr[tid] = tid < ntr ? xerr[st->cand[tid]] : 0.f;
-        open_sum[tid] = 0.0;
+        cerr[tid] = F64 && tid < ntr ? f.xerr[st->cand[tid]] : 0.f;
     }
-    if (tid == 0) open_n = 0;
-    const int cur = st->cur, cur_trial = st->cur_trial, wbuf = 1 - cur;
-    const double *mind = chains + ((long long)cur * tstride + cur_trial) * n;
-    double *out = chains + (long long)wbuf * tstride * n;
-    const long long base = (long long)blockIdx.x * KPP_CH;
-    float acc[4][TT];
+    if (tid == 0) list_n = 0;
+    const int cur = st->cur, esc = INIT ? 0 : st->esc;
+    const T *mind = f.chains + ((long long)cur * f.trials + st->cur_trial) * n + base;
+    const T *prev = f.chains + ((long long)(1 - cur) * f.trials + st->prev_trial) * n + base;
+    T *out = f.chains + (long long)(INIT ? 0 : 1 - cur) * f.trials * n + base;
+    const int rows = (int)min((long long)scan, n - base);
+    const int own_c = st->own_c;
+    float psum[TT], skipped = 0.f;
 #pragma unroll
-    for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int b = 0; b < TT; b++) acc[a][b] = 0.f;
-    __syncthreads();  // cand, cerr
-    auto stage_round = [&](int j0, int q) {
-        float *xs = stages + q * STAGE;
-        float *cs = xs + DJ * XS;
-        const int jn = min(DJ, d - j0);
-        for (int e = tid; e < KPP_CH * DJ; e += KPP_THREADS) {
-            const int r = e / DJ, jj = e - r * DJ;
-            const long long gr = base + r;
-            const bool ok = gr < n && jj < jn;
-            cp_async_elem(xs + jj * XS + r, ok ? x32 + gr * d + j0 + jj : x32, ok);
+    for (int b = 0; b < TT; b++) psum[b] = 0.f;
+    __syncthreads();
+    if (INIT) {
+        for (int i = tid; i < rows; i += KPP_THREADS) {
+            list[i] = (unsigned short)i;
+            f.own[base + i] = 0;
         }
-        for (int e = tid; e < TT * DJ; e += KPP_THREADS) {
-            const int t = e / DJ, jj = e - t * DJ;
-            const bool ok = t < ntr && jj < jn;
-            cp_async_elem(cs + jj * TT + t, ok ? x32 + cand[t] * d + j0 + jj : x32, ok);
-        }
-        cp_async_commit();
-    };
-    stage_round(0, 0);
-    for (int j0 = 0, q = 0; j0 < d; j0 += DJ, q ^= 1) {
-        const int jn = min(DJ, d - j0);
-        if (j0 + DJ < d) {
-            stage_round(j0 + DJ, q ^ 1);  // the next round's copies fly during this round
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
-        }
-        __syncthreads();  // every thread's copies of this round have landed
-        const float *xs = stages + q * STAGE;
-        const float *cs = xs + DJ * XS;
-        for (int jj = 0; jj < jn; jj++) {
-            float xv[4], cvv[TT];
-#pragma unroll
-            for (int a = 0; a < 4; a++) xv[a] = xs[jj * XS + tid * 4 + a];
-#pragma unroll
-            for (int b = 0; b < TT; b++) cvv[b] = cs[jj * TT + b];
-#pragma unroll
-            for (int a = 0; a < 4; a++)
-#pragma unroll
-                for (int b = 0; b < TT; b++) {
-                    const float df = __fsub_rn(xv[a], cvv[b]);
-                    acc[a][b] = __fmaf_rn(df, df, acc[a][b]);
-                }
-        }
-        __syncthreads();  // this stage is refilled by the next round's staging
-    }
-    // Pairs the bounds leave open are listed (row within the chunk, trial)
-    // and formed in FP64 by the whole block afterwards, one pair a thread:
-    // a warp whose lanes waited on one lane's FP64 chain would run it for
-    // nearly every row slot. A pair beyond the list's room is formed in place.
-    double psum[TT];
-#pragma unroll
-    for (int b = 0; b < TT; b++) psum[b] = 0.0;
-#pragma unroll
-    for (int a = 0; a < 4; a++) {
-        const long long row = base + tid * 4 + a;
-        if (row < n) {
-            const double m = mind[row];
-            const float er = xerr[row];
-#pragma unroll
-            for (int b = 0; b < TT; b++) {
-                if (b < ntr) {
-                    const float bnd = bound32(acc[a][b], __fadd_ru(er, cerr[b]), d);
-                    double r = m;  // v >= d32 - bnd > m: min(v, m) = m (kmeans.rs:230-232)
-                    if (!((double)__fsub_rd(acc[a][b], bnd) > m)) {
-                        const int slot = atomicAdd(&open_n, 1);
-                        if (slot < KPP_OPEN) {
-                            open_pairs[slot] = (unsigned short)(((tid * 4 + a) << 4) | b);
-                            continue;
-                        }
-                        const double v = sqeuc_f64(x + row * d, x + cand[b] * d, d);
-                        r = v < m ? v : m;
+        if (tid == 0) list_n = rows;
+    } else {
+        for (int i0 = 0; i0 < rows; i0 += KPP_THREADS) {
+            const int i = i0 + tid;
+            bool open = false;
+            T m = T(0);
+            if (i < rows) {
+                m = mind[i];
+                int o = 0;
+                if (own_c >= 0) {
+                    if (m < prev[i]) {
+                        o = own_c;
+                        f.own[base + i] = o;
+                    } else {
+                        o = f.own[base + i];
                     }
-                    out[(long long)b * n + row] = r;
-                    psum[b] += r;
                 }
+                open = !below(m, f.thr[o]);
+                if (!open) skipped += est_of(m, esc);
+            }
+            __syncwarp();
+            if (i < rows && !open)
+                for (int t = 0; t < ntr; t++) out[(long long)t * n + i] = m;
+            const unsigned bm = __ballot_sync(0xffffffffu, open);
+            int at = 0;
+            if (lane == 0 && bm) at = atomicAdd(&list_n, __popc(bm));
+            at = __shfl_sync(0xffffffffu, at, 0);
+            if (open) list[at + __popc(bm & ((1u << lane) - 1u))] = (unsigned short)i;
+        }
+    }
+    __syncthreads();
+    const int nl = list_n;
+    const bool vec = (d & 3) == 0 && (reinterpret_cast<uintptr_t>(f.x32) & 15) == 0;
+    for (int l0 = 0; l0 < nl; l0 += KPP_THREADS) {
+        const int cnt = min(KPP_THREADS, nl - l0);
+        float acc[TT];
+#pragma unroll
+        for (int b = 0; b < TT; b++) acc[b] = 0.f;
+        if (!(F64 && INIT)) {
+            for (int j0 = 0; j0 < d; j0 += KPP_SLAB) {
+                const int jn = min(KPP_SLAB, d - j0), j4 = (jn + 3) / 4;
+                if (vec) {
+                    for (int e = tid; e < cnt * 16; e += KPP_THREADS) {
+                        const int r = e >> 4, q = e & 15;
+                        if (q < j4)
+                            cp_async16(xs + r * XS + 4 * q, f.x32 + (base + list[l0 + r]) * d + j0 + 4 * q, true);
+                    }
+                } else {
+                    for (int e = tid; e < cnt * KPP_SLAB; e += KPP_THREADS) {
+                        const int r = e >> 6, j = e & 63;
+                        if (j < 4 * j4)
+                            cp_async4(xs + r * XS + j, j < jn ? f.x32 + (base + list[l0 + r]) * d + j0 + j : f.x32,
+                                      j < jn);
+                    }
+                }
+                if (l0 == 0 || d > KPP_SLAB) {  // one slab: the candidates stay for every pass
+                    for (int e = tid; e < TT * KPP_SLAB; e += KPP_THREADS) {
+                        const int t = e >> 6, j = e & 63;
+                        if (j < 4 * j4) {
+                            const bool ok = t < ntr && j < jn;
+                            cp_async4(cs + t * W + j, ok ? f.x32 + cand[t] * d + j0 + j : f.x32, ok);
+                        }
+                    }
+                }
+                cp_async_wait_all();
+                __syncthreads();
+                if (tid < cnt) {
+                    const float4 *xr = reinterpret_cast<const float4 *>(xs + tid * XS);
+                    for (int q = 0; q < j4; q++) {
+                        const float4 xv = xr[q];
+#pragma unroll
+                        for (int b = 0; b < TT; b++) {
+                            const float4 cv = *reinterpret_cast<const float4 *>(cs + b * W + 4 * q);
+                            float t0 = __fsub_rn(xv.x, cv.x), t1 = __fsub_rn(xv.y, cv.y);
+                            float t2 = __fsub_rn(xv.z, cv.z), t3 = __fsub_rn(xv.w, cv.w);
+                            if (F64) {
+                                acc[b] = __fmaf_rn(t0, t0, acc[b]);
+                                acc[b] = __fmaf_rn(t1, t1, acc[b]);
+                                acc[b] = __fmaf_rn(t2, t2, acc[b]);
+                                acc[b] = __fmaf_rn(t3, t3, acc[b]);
+                            } else {  // a zero-padded feature adds +0: no change
+                                acc[b] = __fadd_rn(acc[b], __fmul_rn(t0, t0));
+                                acc[b] = __fadd_rn(acc[b], __fmul_rn(t1, t1));
+                                acc[b] = __fadd_rn(acc[b], __fmul_rn(t2, t2));
+                                acc[b] = __fadd_rn(acc[b], __fmul_rn(t3, t3));
+                            }
+                        }
+                    }
+                }
+                __syncthreads();  // the slab is refilled
             }
         }
+        if constexpr (!F64) {
+            if (tid < cnt) {
+                const int i = list[l0 + tid];
+                const T m = INIT ? T(0) : mind[i];
+#pragma unroll
+                for (int b = 0; b < TT; b++)
+                    if (b < ntr) {
+                        const T v = acc[b];
+                        const T r = INIT ? v : (v < m ? v : m);  // kmeans.rs:230-232
+                        out[(long long)b * n + i] = r;
+                        psum[b] += est_of(r, esc);
+                    }
+            }
+        } else {
+            // Pairs the FP32 bounds leave open -- rows the candidate may come
+            // closer to, non-finite values, values beyond the f32 range --
+            // are listed and formed in FP64 by the whole block, one pair a
+            // thread; the others keep D^2 (d32 - bound > D^2).
+            if (tid == 0) open_n = 0;
+            __syncthreads();
+            if (tid < cnt) {
+                const int i = list[l0 + tid];
+                const T m = INIT ? T(0) : mind[i];
+                const float mu = INIT ? 0.f : __double2float_ru(m);
+                const float er = INIT ? 0.f : f.xerr[base + i];
+#pragma unroll
+                for (int b = 0; b < TT; b++)
+                    if (b < ntr) {
+                        const float bnd = bound32(acc[b], __fadd_ru(er, cerr[b]), d);
+                        if (!INIT && __fsub_rd(acc[b], bnd) > mu) {
+                            out[(long long)b * n + i] = m;
+                            psum[b] += est_of(m, esc);
+                        } else {
+                            open_pairs[atomicAdd(&open_n, 1)] = (unsigned short)((tid << 4) | b);
+                        }
+                    }
+            }
+            __syncthreads();
+            const int no = open_n;
+            for (int q = tid; q < no; q += KPP_THREADS) {
+                const int e = open_pairs[q], b = e & 15, i = list[l0 + (e >> 4)];
+                const T v = sqeuc(f.x + (base + i) * d, f.x + cand[b] * d, d);
+                T r = v;
+                if (!INIT) {
+                    const T m = mind[i];
+                    r = v < m ? v : m;
+                }
+                out[(long long)b * n + i] = r;
+                // the summand's trial differs from thread to thread: one select per trial
+#pragma unroll
+                for (int t = 0; t < TT; t++) psum[t] += t == b ? est_of(r, esc) : 0.f;
+            }
+            __syncthreads();
+        }
     }
-    __syncthreads();  // the list is complete
-    for (int q = tid; q < min(open_n, KPP_OPEN); q += KPP_THREADS) {
-        const int e = open_pairs[q];
-        const int b = e & 15;
-        const long long row = base + (e >> 4);
-        const double m = mind[row];
-        const double v = sqeuc_f64(x + row * d, x + cand[b] * d, d);
-        const double r = v < m ? v : m;
-        out[(long long)b * n + row] = r;
-        atomicAdd(&open_sum[b], r);  // the chunk sums only steer the folds' windows
-    }
-    const int lane = tid & 31, w = tid >> 5;
 #pragma unroll
     for (int b = 0; b < TT; b++) {
-        double vv = psum[b];
+        float v = psum[b] + skipped;
 #pragma unroll
-        for (int off = 16; off >= 1; off >>= 1) vv += __shfl_xor_sync(0xffffffffu, vv, off);
-        if (lane == 0) red[b][w] = vv;
+        for (int o = 16; o >= 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane == 0) red[b][w] = v;
     }
     __syncthreads();
     if (tid < ntr) {
-        double vv = open_sum[tid];
-        for (int q = 0; q < KPP_THREADS / 32; q++) vv += red[tid][q];
-        csum[(long long)tid * nch + blockIdx.x] = vv;
+        float v = 0.f;
+        for (int q = 0; q < KPP_WARPS; q++) v += red[tid][q];
+        f.csum[(long long)tid * f.tiles + it.y] = v;
     }
 }
 
-// One warp per (chunk, trial): the maps of the chunk's 32 groups (lane g
-// folds group g) and of the whole chunk (ordered warp reduction), each for
-// the three binades around the chunk's estimated starting sum (an f64 sum of
-// the earlier chunks' sums: only which maps get built depends on it).
+// One CTA per (eight chunks, trial), one warp per chunk: the chunk's composed
+// map for the binade its estimated starting sum lies in, and for the one its
+// end lies in when that is the next. A chunk without exact halves is an
+// integer sum over coalesced loads (7 M values at n = 1M: bound by L2);
+// otherwise the lanes compose ordered runs of 32 values.
 template <typename T>
 __global__ void __launch_bounds__(KPP_THREADS)
-    kpp_compose_kernel(const T *__restrict__ chains, long long n, int tstride, const KppState *__restrict__ st,
-                       bool init, const double *__restrict__ csum, long long nch, FoldSlices fs) {
-    if (!init && st->direct) return;
-    const int lane = threadIdx.x & 31;
+    kpp_compose_kernel(const KppFit<T> *__restrict__ fits, const int2 *__restrict__ items, int scan, int c, bool init) {
+    const int2 it = item_at(items);
+    const KppFit<T> &f = fits[it.x];
+    const KppState *st = f.st;
     const int t = blockIdx.y;
-    const long long j = (long long)blockIdx.x * (KPP_THREADS / 32) + (threadIdx.x >> 5);
-    if (j >= nch) return;  // whole warps; no block-wide barrier below
-    const int wbuf = init ? 0 : 1 - st->cur;
-    const T *v = chains + ((long long)wbuf * tstride + t) * n + j * KPP_CH;
-    const long long off = ((long long)wbuf * tstride + t) * nch + j;
-    double e = 0.0;
-    for (long long q = lane; q < j; q += 32) e += csum[(long long)t * nch + q];
+    if (t >= (init ? 1 : f.trials) || (!init && st->direct[c & 1])) return;
+    __shared__ float red[KPP_WARPS];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int tpc = KPP_CH / scan;  // tiles per chunk
+    const float *cs = f.csum + (long long)t * f.tiles;
+    const long long t0 = (long long)it.y * KPP_WARPS * tpc;  // the group's first tile
+    float e = 0.f;
+    for (long long q = tid; q < t0; q += KPP_THREADS) e += cs[q];
 #pragma unroll
     for (int o = 16; o >= 1; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
-    const int be = normal_exp((T)e);
-    int lo = -1;
-    if (be > 0) {
-        lo = be > 1 ? be - 1 : 1;
-        if (lo + 2 >= Bits<T>::EXPM) lo = -1;
+    if (lane == 0) red[w] = e;
+    __syncthreads();
+    const long long j = (long long)it.y * KPP_WARPS + w;
+    if (j >= f.nch) return;
+    float s = 0.f;  // this chunk's sum
+    e = lane < KPP_WARPS ? red[lane] : 0.f;
+    for (int q = lane; q < (w + 1) * tpc; q += 32) {
+        const float v = t0 + q < f.tiles ? cs[t0 + q] : 0.f;
+        if (q < w * tpc) e += v;
+        else s += v;
     }
-    if (lane == 0) fs.elo[off] = lo;
-    if (lo < 0) return;
-    const int clen = (int)min((long long)KPP_CH, n - j * KPP_CH);
-    Step s0{0, 0}, s1{0, 0}, s2{0, 0};
-    const int g0 = lane * 32;
-    for (int q = 0; q < 32; q++) {
-        const int i = g0 + q;
-        if (i < clen) {
-            const T val = v[i];
-            s0 = compose(s0, step_of(val, lo));
-            s1 = compose(s1, step_of(val, lo + 1));
-            s2 = compose(s2, step_of(val, lo + 2));
-        }
-    }
-    Map3 gm;
-    gm.s[0] = s0;
-    gm.s[1] = s1;
-    gm.s[2] = s2;
-    fs.gmap[off * KPP_GROUPS + lane] = gm;
-    // ordered reduction: lane i (earlier groups) absorbs lane i + o (later)
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const Step r0 = shfl_down_step(s0, o), r1 = shfl_down_step(s1, o), r2 = shfl_down_step(s2, o);
-        if ((lane & (2 * o - 1)) == 0) {
-            s0 = compose(s0, r0);
-            s1 = compose(s1, r1);
-            s2 = compose(s2, r2);
+    for (int o = 16; o >= 1; o >>= 1) {
+        e += __shfl_xor_sync(0xffffffffu, e, o);
+        s += __shfl_xor_sync(0xffffffffu, s, o);
+    }
+    const int esc = init ? 0 : st->esc;
+    const int blo = est_exp(e * 0.9921875f, esc, T(0));
+    const int bhi = est_exp((e + s) * 1.0078125f, esc, T(0));
+    CMap<T> *cm = f.cmaps + (long long)t * f.nch + j;
+    if (blo == 0 || bhi == 0 || bhi - blo > 1) {
+        if (lane == 0) cm->elo = -1;
+        return;
+    }
+    using U = typename Bits<T>::U;
+    constexpr U OUT = (U)1 << (Bits<T>::MB + 1);
+    const int nb = bhi - blo + 1;
+    const int wbuf = init ? 0 : 1 - st->cur;
+    const T *v = f.chains + ((long long)wbuf * f.trials + t) * f.n + j * KPP_CH;
+    const int clen = (int)min((long long)KPP_CH, f.n - j * KPP_CH);
+    unsigned long long a0 = 0, a1 = 0;  // at most 1024 increments of 2^53: no overflow
+    bool tie = false;
+#pragma unroll 8
+    for (int q = 0; q < KPP_CH / 32; q++) {
+        const int i = q * 32 + lane;
+        const T val = i < clen ? v[i] : T(0);
+        a0 += inc_of(val, blo, tie);
+        if (nb == 2) a1 += inc_of(val, blo + 1, tie);
+    }
+    GMap<T> m0, m1;
+    if (!__any_sync(0xffffffffu, tie)) {
+#pragma unroll
+        for (int o = 16; o >= 1; o >>= 1) {
+            a0 += __shfl_xor_sync(0xffffffffu, a0, o);
+            a1 += __shfl_xor_sync(0xffffffffu, a1, o);
         }
+        m0.a0 = m0.a1 = (U)min(a0, (unsigned long long)OUT);
+        m1.a0 = m1.a1 = (U)min(a1, (unsigned long long)OUT);
+    } else {
+        // exact halves: the maps of the 32 groups, lane g keeping group g's
+        m0 = m1 = GMap<T>{0, 0};
+#pragma unroll 4
+        for (int g = 0; g < KPP_CH / 32; g++) {
+            const int i = g * 32 + lane;
+            const T val = i < clen ? v[i] : T(0);
+            const GMap<T> x0 = group_map(val, i < clen, blo);
+            if (lane == g) m0 = x0;
+            if (nb == 2) {
+                const GMap<T> x1 = group_map(val, i < clen, blo + 1);
+                if (lane == g) m1 = x1;
+            }
+        }
+        m0 = gscan(m0);
+        m1 = gscan(m1);
+        m0 = GMap<T>{min(__shfl_sync(0xffffffffu, m0.a0, 31), OUT), min(__shfl_sync(0xffffffffu, m0.a1, 31), OUT)};
+        m1 = GMap<T>{min(__shfl_sync(0xffffffffu, m1.a0, 31), OUT), min(__shfl_sync(0xffffffffu, m1.a1, 31), OUT)};
     }
     if (lane == 0) {
-        Map3 cm;
-        cm.s[0] = s0;
-        cm.s[1] = s1;
-        cm.s[2] = s2;
-        fs.cmap[off] = cm;
+        cm->elo = blo;
+        cm->cnt = nb;
+        cm->s[0] = m0;
+        cm->s[1] = m1;
     }
 }
 
-// One warp per fold (blockIdx.x = trial): the running sum over every chunk,
-// recorded at each chunk's end, and the whole fold (the trial's potential).
-// The chunk maps are scanned 32 chunks at a time; a chunk whose map does not
-// apply (the sum changes binade inside it, or has no map) is walked by its
-// groups (walk_chunk).
-template <typename T>
-__global__ void __launch_bounds__(32)
-    kpp_walk_kernel(const T *__restrict__ chains, long long n, int tstride, KppState *__restrict__ st, bool init,
-                    long long nch, FoldSlices fs) {
-    if (!init && st->direct) return;
-    const int t = blockIdx.x;
-    const int lane = threadIdx.x;
-    const int wbuf = init ? 0 : 1 - st->cur;
-    const long long slice = (long long)wbuf * tstride + t;
-    const T *v = chains + slice * n;
-    const int *elo = fs.elo + slice * nch;
-    const Map3 *cmap = fs.cmap + slice * nch;
-    const Map3 *gmap = fs.gmap + slice * nch * KPP_GROUPS;
-    T *sout = reinterpret_cast<T *>(fs.states) + slice * nch;
-    constexpr long long TOP = 1LL << (Bits<T>::MB + 1);
-    T p = T(0);
-    int e_cur = -1;
-    Map3 m_cur{};
-    if (lane < nch) {
-        e_cur = elo[lane];
-        if (e_cur >= 0) m_cur = cmap[lane];
-    }
-    for (long long jb = 0; jb < nch; jb += 32) {
-        // the next 32 chunks' maps load while these are scanned
-        int e_nxt = -1;
-        Map3 m_nxt{};
-        if (jb + 32 + lane < nch) {
-            e_nxt = elo[jb + 32 + lane];
-            if (e_nxt >= 0) m_nxt = cmap[jb + 32 + lane];
-        }
-        const int nb = (int)min(32LL, nch - jb);
-        int start = 0;
-        while (start < nb) {
-            const int be = normal_exp(p);
-            const bool live = lane >= start && lane < nb;
-            const int slot = be - e_cur;
-            const bool ok = be > 0 && e_cur >= 0 && slot >= 0 && slot < 3;
-            Step s = !live ? Step{0, 0} : (ok ? pick(m_cur, slot) : Step{KPP_SAT, KPP_SAT});
-#pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                const Step o = shfl_up_step(s, off);
-                if (lane >= off) s = compose(o, s);
-            }
-            const long long P = be > 0 ? significand(p) : 0;
-            const long long Pl = P + ((P & 1) ? s.a1 : s.a0);
-            const unsigned badm = __ballot_sync(0xffffffffu, live && !(be > 0 && Pl < TOP));
-            const int f0 = badm ? __ffs(badm) - 1 : nb;
-            if (live && lane < f0) sout[jb + lane] = from_parts<T>(be, Pl);
-            if (f0 > start) {
-                const long long Pb = (long long)__shfl_sync(0xffffffffu, (unsigned long long)Pl, f0 - 1);
-                p = from_parts<T>(be, Pb);
-            }
-            if (f0 >= nb) break;
-            const long long j = jb + f0;
-            const int ej = __shfl_sync(0xffffffffu, e_cur, f0);
-            const int clen = (int)min((long long)KPP_CH, n - j * KPP_CH);
-            int dummy;
-            p = walk_chunk<T, false>(p, v + j * KPP_CH, clen, gmap + j * KPP_GROUPS, ej, T(0), &dummy);
-            if (lane == 0) sout[j] = p;
-            start = f0 + 1;
-        }
-        e_cur = e_nxt;
-        m_cur = m_nxt;
-    }
-    if (lane == 0) st->pot[t] = (double)p;
-}
+// ------------------------------------------------- one fold by one CTA --
+constexpr int KPP_ROUND = 4 * KPP_THREADS;  // chunk maps scanned at a time
+static_assert(KPP_CH == 4 * KPP_THREADS && KPP_WARPS == 8, "a chunk is 32 groups, four a warp");
 
-// Single CTA, one warp per trial: resolve the pending trials into a centre,
-// then (centre c < k) the thresholds and candidates of centre c.
 template <typename T>
-__global__ void __launch_bounds__(MAX_TRIALS * 32)
-    kpp_select_kernel(const T *__restrict__ x, long long n, int d, const T *__restrict__ chains, int tstride,
-                      long long nch, FoldSlices fs, const double *__restrict__ draws, long long n_draws,
-                      int n_trials, int c, int k, KppState *__restrict__ st, T *__restrict__ centers) {
-    __shared__ long long copy_row;
-    __shared__ int copy_centre;
-    __shared__ int do_search;
-    __shared__ T thr_s[MAX_TRIALS];
+struct WalkShared {
+    unsigned long long pre[KPP_ROUND];     // prefix sums of the plain chunks' increments
+    GMap<T> map[2][KPP_ROUND];             // chunk maps
+    int elo[KPP_ROUND];                    // their binades (-1: none), and
+    unsigned char cnt[KPP_ROUND];          // how many
+    unsigned long long gtot[32];
+    unsigned special[32], words;           // chunks to look at one by one (words: the nonzero words)
+    GMap<T> gm[32];
+    T first[32], pb, vf;
+    int f0, last;
+};
+
+// The values of one chunk (clen of them) added to p in order, exactly as the
+// sequential fold, by the whole block: warp w holds groups 4 w .. 4 w + 3 of
+// 32 values. Per pass, the groups' maps for p's binade, their scan (by every
+// warp), and where the sum leaves the binade the group's own states and one
+// exact F addition: two barriers a pass. A fold's very first values (a binade
+// change at nearly each) are added one by one. gs (nullable): receives the
+// running sum after each group.
+template <typename T>
+__device__ T block_walk_chunk(T p, const T *__restrict__ cv, int clen, T *__restrict__ gs, WalkShared<T> &sh) {
+    using U = typename Bits<T>::U;
+    constexpr U TOP = (U)1 << (Bits<T>::MB + 1);
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    if (tid == 0) {
-        copy_row = -1;
-        copy_centre = -1;
-        do_search = 0;
-        if (st->pending) {
-            int best = 0;
-            for (int t = 1; t < st->ntr; t++)
-                if (st->pot[t] < st->pot[best]) best = t;  // strictly smaller: the first trial wins ties
-            st->cur = st->wbuf;
-            st->cur_trial = best;
-            st->total = st->pot[best];
-            if (st->pcentre >= 0) {
-                copy_row = st->cand[best];
-                copy_centre = st->pcentre;
+    T v[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        const int i = (4 * w + u) * 32 + lane;
+        v[u] = i < clen ? cv[i] : T(0);
+    }
+    int start = 0;
+    if (p == T(0)) {
+        if (w == 0) sh.first[lane] = v[0];
+        __syncthreads();
+        start = min(32, clen);
+        for (int i = 0; i < start; i++) p = kpp_add(p, sh.first[i]);
+        if (gs && tid == 0) gs[0] = p;
+    }
+    while (start < clen) {
+        const int be = normal_exp(p);
+        // the first group whose end state is not recorded yet
+        const int gfirst = max(0, start - 1) >> 5;
+        if (be == 0) {
+            // a NaN sum stays; +inf stays until a NaN value; a zero sum until a
+            // value other than zero; a subnormal sum takes the next value
+            const bool inf = is_inf_or_nan(p);
+            int first = INT32_MAX;
+            if (p == p) {
+#pragma unroll
+                for (int u = 3; u >= 0; u--) {
+                    const int i = (4 * w + u) * 32 + lane;
+                    const bool hit = inf ? v[u] != v[u] : (p == T(0) ? !(v[u] == T(0)) : true);
+                    if (i >= start && i < clen && hit) first = i;
+                }
             }
-            st->pending = 0;
+            first = __reduce_min_sync(0xffffffffu, first);
+            __syncthreads();  // the pass before is done with sh.f0
+            if (tid == 0) sh.f0 = INT32_MAX;
+            __syncthreads();
+            if (lane == 0 && first != INT32_MAX) atomicMin(&sh.f0, first);
+            __syncthreads();
+            const int f0 = min(sh.f0, clen);
+            if (gs && w == 0 && lane >= gfirst && lane < (f0 == clen ? 32 : f0 >> 5)) gs[lane] = p;
+            if (f0 == clen) return p;
+            if (w == f0 >> 7 && lane == (f0 & 31)) {
+                const int u = (f0 >> 5) & 3;
+                sh.vf = u == 0 ? v[0] : u == 1 ? v[1] : u == 2 ? v[2] : v[3];
+            }
+            __syncthreads();
+            p = kpp_add(p, sh.vf);
+            start = f0 + 1;
+            __syncthreads();
+            if (start >= clen && gs && w == 0 && lane >= (f0 >> 5)) gs[lane] = p;
+            continue;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int i = (4 * w + u) * 32 + lane;
+            const GMap<T> m = group_map(v[u], i >= start && i < clen, be);
+            if (lane == 0) sh.gm[4 * w + u] = m;
+        }
+        __syncthreads();
+        const GMap<T> m = gscan(sh.gm[lane]);
+        const U P = significand(p);
+        const U Pl = P + ((P & 1) ? m.a1 : m.a0);  // after group `lane`
+        const unsigned bad = __ballot_sync(0xffffffffu, Pl >= TOP);
+        const int gf = bad ? __ffs(bad) - 1 : 32;
+        if (gs && w == 0 && lane >= gfirst && lane < gf) gs[lane] = from_parts<T>(be, Pl);
+        if (gf == 32) return from_parts<T>(be, __shfl_sync(0xffffffffu, Pl, 31));
+        const U before = __shfl_sync(0xffffffffu, Pl, gf > 0 ? gf - 1 : 0);
+        const U Pg = gf > 0 ? before : P;
+        if (w == gf >> 2) {
+            const int u = gf & 3, i = gf * 32 + lane;
+            const T val = u == 0 ? v[0] : u == 1 ? v[1] : u == 2 ? v[2] : v[3];
+            const U S = group_states(val, i >= start && i < clen, be, Pg);
+            const int q = __ffs(__ballot_sync(0xffffffffu, S >= TOP)) - 1;  // the first value that leaves the binade
+            const U Sb = __shfl_sync(0xffffffffu, S, q > 0 ? q - 1 : 0);
+            if (lane == q) {
+                sh.pb = from_parts<T>(be, q > 0 ? Sb : Pg);
+                sh.vf = val;
+                sh.f0 = gf * 32 + q;
+            }
+        }
+        __syncthreads();
+        p = kpp_add(sh.pb, sh.vf);  // the one exact addition where the binade changes
+        start = sh.f0 + 1;
+        if (start >= clen && gs && w == 0 && lane >= gf) gs[lane] = p;
+    }
+    return p;
+}
+
+// The first value of a chunk whose inclusive running sum (from p) reaches thr,
+// or -1, by one warp. gs: the running sums after the chunk's groups, where they
+// are recorded (the first chunk): the group is found by them. Else the lanes'
+// runs of 32 values give the groups' maps for p's binade.
+template <typename T>
+__device__ int warp_search_chunk(T p, const T *__restrict__ cv, int clen, T thr, const T *__restrict__ gs) {
+    using U = typename Bits<T>::U;
+    constexpr U TOP = (U)1 << (Bits<T>::MB + 1);
+    const int lane = threadIdx.x & 31;
+    const int ng = (clen + 31) / 32;
+    int start = 0;  // the next group
+    if (gs) {
+        const T e = lane < ng ? __ldcg(gs + lane) : T(0);
+        const unsigned m = __ballot_sync(0xffffffffu, lane < ng && !(e < thr));
+        if (!m) return -1;
+        start = __ffs(m) - 1;
+        const T b = __shfl_sync(0xffffffffu, e, start > 0 ? start - 1 : 0);
+        if (start > 0) p = b;
+    }
+    while (start < ng) {
+        const int be = normal_exp(p);
+        int gsel = start;
+        if (be > 0 && !gs) {
+            GMap<T> m{0, 0};
+            if (lane >= start && lane < ng) {
+                // this lane's run in order, from an even and from an odd sum
+                const int gl = min(32, clen - lane * 32);
+#pragma unroll 8
+                for (int q = 0; q < gl; q++) {
+                    bool tie = false;
+                    const U inc = inc_of(cv[lane * 32 + q], be, tie);
+                    m.a0 += inc;
+                    m.a1 += inc;
+                    if (tie) {
+                        m.a0 += m.a0 & 1;
+                        m.a1 += 1 - (m.a1 & 1);
+                    }
+                }
+                m.a0 = min(m.a0, TOP);
+                m.a1 = min(m.a1, TOP);
+            }
+            __syncwarp();
+            m = gscan(m);
+            const U P = significand(p);
+            const U Pl = P + ((P & 1) ? m.a1 : m.a0);
+            const unsigned bad = __ballot_sync(0xffffffffu, lane >= start && lane < ng &&
+                                                                (Pl >= TOP || from_parts<T>(be, Pl) >= thr));
+            if (!bad) return -1;  // the chunk ends below thr
+            gsel = __ffs(bad) - 1;
+            const U Pb = __shfl_sync(0xffffffffu, Pl, gsel > 0 ? gsel - 1 : 0);
+            if (gsel > start) p = from_parts<T>(be, Pb);
+        }
+        // group gsel value by value
+        const int i0 = gsel * 32, len = min(32, clen - i0);
+        const T val = lane < len ? cv[i0 + lane] : T(0);
+        int at = 0;
+        while (at < len) {
+            const int b = normal_exp(p);
+            if (b > 0) {
+                const U S = group_states(val, lane >= at && lane < len, b, significand(p));
+                const unsigned bad = __ballot_sync(0xffffffffu, S >= TOP);
+                const int q = bad ? __ffs(bad) - 1 : len;
+                const unsigned hm = __ballot_sync(0xffffffffu,
+                                                  lane >= at && lane < q && from_parts<T>(b, S) >= thr);
+                if (hm) return i0 + __ffs(hm) - 1;
+                const U Sb = __shfl_sync(0xffffffffu, S, q > 0 ? q - 1 : 0);
+                if (q > at) p = from_parts<T>(b, Sb);
+                if (q >= len) break;
+                at = q;
+            }
+            p = kpp_add(p, __shfl_sync(0xffffffffu, val, at));
+            if (p >= thr) return i0 + at;
+            at++;
+        }
+        start = gsel + 1;
+    }
+    return -1;
+}
+
+// The pending trials resolved into centre c (init: the first D^2 array), then
+// the draws and candidates of centre c + 1 (init: 1), by one block. The folds'
+// results come from this launch's other CTAs: read past L1.
+template <typename T>
+__device__ void kpp_select(const KppFit<T> &f, int c, bool init) {
+    KppState *st = f.st;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int cn = init ? 1 : c + 1;
+    const int ntr = f.trials, d = f.d;
+    const long long n = f.n;
+    __shared__ long long copy_row, direct_row;
+    __shared__ long long draw0;
+    __shared__ T stotal;
+    __shared__ int scur, strial;
+    if (tid == 0) {
+        copy_row = direct_row = -1;
+        if (init) {
+            st->total = __ldcg(&st->pot[0]);
+        } else if (!st->direct[c & 1]) {
+            int best = 0;
+            double bp = __ldcg(&st->pot[0]);
+            for (int t = 1; t < ntr; t++) {
+                const double v = __ldcg(&st->pot[t]);
+                if (v < bp) {  // strictly smaller: the first trial wins ties
+                    bp = v;
+                    best = t;
+                }
+            }
+            st->prev_trial = st->cur_trial;
+            st->cur = 1 - st->cur;
+            st->cur_trial = best;
+            st->own_c = c;
+            st->total = bp;
+            copy_row = st->cand[best];
+            f.crow[c] = (int32_t)copy_row;
+        }
+        scur = st->cur;
+        strial = st->cur_trial;
+        if (cn < f.k) {
+            const T total = (T)st->total;
+            stotal = total;
+            long long cur = st->cursor;
+            if (sizeof(T) == 8) {
+                const unsigned long long b = (unsigned long long)__double_as_longlong(st->total);
+                const int e = (int)((b >> 52) & 0x7FFull);
+                st->esc = e > 0 && e < 0x7FF ? e - 1023 : 0;
+            }
+            // kmeans.rs:202-206: a uniform random row, the D^2 array unchanged
+            if (f.nan_direct ? !(total > T(0)) : total <= T(0)) {
+                direct_row = draw_to_range(draw_at(f, cur), n);
+                f.crow[cn] = (int32_t)direct_row;
+                st->direct[cn & 1] = 1;
+                cur += 1;
+            } else {
+                st->direct[cn & 1] = 0;
+                draw0 = cur;
+                cur += ntr;
+            }
+            st->cursor = cur;
         }
     }
     __syncthreads();
     if (copy_row >= 0)
-        for (int j = tid; j < d; j += blockDim.x) centers[(long long)copy_centre * d + j] = x[copy_row * d + j];
-    __syncthreads();
-    if (c >= k) return;
-    if (tid == 0) {
-        const T total = (T)st->total;
-        long long cur = st->cursor;
-        if (!(total > T(0))) {
-            // kmeans.rs:202-206: a uniform random row, the D^2 array unchanged
-            const double u = cur < n_draws ? draws[cur] : 0.0;
-            copy_row = draw_to_range(u, n);
-            copy_centre = c;
-            st->direct = 1;
-            cur += 1;
-        } else {
-            st->direct = 0;
-            for (int t = 0; t < n_trials; t++) {
-                const double u = cur < n_draws ? draws[cur] : 0.0;
-                thr_s[t] = kpp_mul((T)u, total);
-                st->thr[t] = (double)thr_s[t];
-                cur += 1;
-            }
-            st->pending = 1;
-            st->wbuf = 1 - st->cur;
-            st->ntr = n_trials;
-            st->pcentre = c;
-            do_search = 1;
-        }
-        st->cursor = cur;
-    }
-    __syncthreads();
-    if (!do_search) {
-        for (int j = tid; j < d; j += blockDim.x) centers[(long long)copy_centre * d + j] = x[copy_row * d + j];
+        for (int j = tid; j < d; j += KPP_THREADS) f.centers[(long long)c * d + j] = f.x[copy_row * d + j];
+    if (cn >= f.k) return;
+    if (direct_row >= 0) {
+        for (int j = tid; j < d; j += KPP_THREADS) f.centers[(long long)cn * d + j] = f.x[direct_row * d + j];
         return;
     }
-    if (w >= n_trials) return;
-    // trial w: the first row whose running sum reaches thr (kmeans.rs:215-223)
-    const T thr = thr_s[w];
-    const long long slice = (long long)st->cur * tstride + st->cur_trial;
-    const T *S = reinterpret_cast<const T *>(fs.states) + slice * nch;
-    const T *v = chains + slice * n;
-    // First chunk whose end state is not below thr: a 32-ary search (the
-    // states never decrease, and a NaN state stays NaN, so "not below" holds
-    // from one chunk on); that chunk is then walked with the exact test.
-    long long lo = 0, hi = nch;  // the answer lies in [lo, hi]; nch = none
-    while (lo < hi) {
-        const long long step = (hi - lo + 31) / 32;
-        const long long pos = lo + (long long)lane * step;
-        const unsigned m = __ballot_sync(0xffffffffu, pos < hi && !(S[pos] < thr));
-        if (!m) {
-            lo = lo + ((hi - 1 - lo) / step) * step + 1;  // past the last probe
-        } else {
-            const int f = __ffs(m) - 1;
-            const long long pf = lo + (long long)f * step;
-            if (f > 0) lo = lo + (long long)(f - 1) * step + 1;
-            hi = pf;
+    // each trial's first row whose running sum reaches its threshold (kmeans.rs:215-223)
+    const long long slice = (long long)scur * ntr + strial, nch = f.nch;
+    const T *S = f.states + slice * nch;
+    const T *v = f.chains + slice * n;
+    for (int t = w; t < ntr; t += KPP_WARPS) {
+        const T thr = kpp_mul((T)draw_at(f, draw0 + t), stotal);
+        // First chunk whose end state is not below thr: a 32-ary search (the
+        // states never decrease, and a NaN state stays NaN, so "not below"
+        // holds from one chunk on); that chunk is then walked with the exact test.
+        long long lo = 0, hi = nch;  // the answer lies in [lo, hi]; nch = none
+        while (lo < hi) {
+            const long long step = (hi - lo + 31) / 32;
+            const long long pos = lo + (long long)lane * step;
+            const unsigned m = __ballot_sync(0xffffffffu, pos < hi && !(__ldcg(S + pos) < thr));
+            if (!m) {
+                lo = lo + ((hi - 1 - lo) / step) * step + 1;  // past the last probe
+            } else {
+                const int q = __ffs(m) - 1;
+                const long long pf = lo + (long long)q * step;
+                if (q > 0) lo = lo + (long long)(q - 1) * step + 1;
+                hi = pf;
+            }
+        }
+        long long cand = n - 1;
+        if (lo < nch) {
+            const T p = lo > 0 ? __ldcg(S + lo - 1) : T(0);
+            const int hit = warp_search_chunk<T>(p, v + lo * KPP_CH, (int)min((long long)KPP_CH, n - lo * KPP_CH), thr,
+                                                 lo == 0 ? f.gstates + slice * 32 : nullptr);
+            if (hit >= 0) cand = lo * KPP_CH + hit;
+        }
+        if (lane == 0) st->cand[t] = cand;
+    }
+}
+
+// One CTA per (seeding, trial): the trial's fold over every chunk, the running
+// sum recorded at each chunk's end; the seeding's last CTA selects.
+//
+// Latency bound. Per round of 1024 chunks one scan forms the prefix sums of
+// the plain chunks' increments (one map, no exact half, the binade of the
+// chunk before): a run of them is then one addition and one comparison. The
+// others -- a second map, halves, a new binade -- are looked at one by one, and
+// a chunk in which the sum leaves its binade is walked (about one per binade).
+template <typename T>
+__global__ void __launch_bounds__(KPP_THREADS) kpp_walk_kernel(const KppFit<T> *__restrict__ fits, int c, bool init) {
+    using U = typename Bits<T>::U;
+    constexpr U TOP = (U)1 << (Bits<T>::MB + 1);
+    const KppFit<T> &f = fits[blockIdx.x];
+    KppState *st = f.st;
+    const int t = blockIdx.y, ntr = init ? 1 : f.trials;
+    if (t >= ntr) return;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    __shared__ WalkShared<T> sh;
+    if (!init && st->direct[c & 1]) {
+        // no trials to fold: the next centre's draws only
+        if (t == 0) kpp_select<T>(f, c, false);
+        return;
+    }
+    const int wbuf = init ? 0 : 1 - st->cur;
+    const long long slice = (long long)wbuf * f.trials + t, nch = f.nch, n = f.n;
+    const T *v = f.chains + slice * n;
+    const CMap<T> *cm = f.cmaps + (long long)t * nch;
+    T *sout = f.states + slice * nch;
+    T p = T(0);
+    for (long long jb = 0; jb < nch; jb += KPP_ROUND) {
+        const int nb = (int)min((long long)KPP_ROUND, nch - jb);
+        __syncthreads();  // the round before is done with sh
+        unsigned long long a[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int i = (4 * w + u) * 32 + lane;
+            CMap<T> m;
+            m.elo = -1;
+            m.cnt = 0;
+            m.s[0] = m.s[1] = GMap<T>{TOP, TOP};
+            if (i < nb) m = cm[jb + i];
+            sh.map[0][i] = m.s[0];
+            sh.map[1][i] = m.s[1];
+            sh.elo[i] = m.elo;
+            sh.cnt[i] = (unsigned char)m.cnt;
+            int before = __shfl_up_sync(0xffffffffu, m.elo, 1);
+            if (lane == 0) before = i > 0 && i < nb ? cm[jb + i - 1].elo : -1;
+            const bool plain = m.elo >= 0 && m.cnt == 1 && m.s[0].a0 == m.s[0].a1 && before == m.elo;
+            const unsigned sp = __ballot_sync(0xffffffffu, !plain && i < nb);
+            if (lane == 0) sh.special[4 * w + u] = sp;
+            a[u] = plain ? (unsigned long long)m.s[0].a0 : 0ull;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const unsigned long long o = __shfl_up_sync(0xffffffffu, a[u], off);
+                if (lane >= off) a[u] += o;
+            }
+            if (lane == 31) sh.gtot[4 * w + u] = a[u];
+        }
+        __syncthreads();
+        {
+            unsigned long long g = sh.gtot[lane];
+            const unsigned long long own = g;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const unsigned long long o = __shfl_up_sync(0xffffffffu, g, off);
+                if (lane >= off) g += o;
+            }
+            g -= own;  // the groups before
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                sh.pre[(4 * w + u) * 32 + lane] = a[u] + __shfl_sync(0xffffffffu, g, 4 * w + u);
+            const unsigned nz = __ballot_sync(0xffffffffu, sh.special[lane] != 0);
+            if (tid == 0) sh.words = nz;
+        }
+        __syncthreads();
+        int i = 0;
+        while (i < nb) {  // block-uniform
+            const int be = normal_exp(p);
+            const U P = be > 0 ? significand(p) : (U)0;
+            const int wd = i >> 5;
+            unsigned rest = sh.special[wd] >> (i & 31);
+            int s;  // the next chunk to look at by itself
+            if (rest) {
+                s = i + __ffs(rest) - 1;
+            } else {
+                const unsigned later = wd < 31 ? sh.words >> (wd + 1) << (wd + 1) : 0u;
+                const int q = later ? __ffs(later) - 1 : 32;
+                s = q < 32 ? q * 32 + __ffs(sh.special[q]) - 1 : nb;
+            }
+            bool slow = true;
+            if (s > i) {
+                if (be > 0 && sh.elo[i] == be) {
+                    const unsigned long long base = i > 0 ? sh.pre[i - 1] : 0ull;
+                    int e = s;
+                    if ((unsigned long long)P + (sh.pre[s - 1] - base) >= (unsigned long long)TOP) {
+                        int lo = i, hi = s - 1;  // the first chunk whose end leaves the binade
+                        while (lo < hi) {
+                            const int mid = (lo + hi) >> 1;
+                            if ((unsigned long long)P + (sh.pre[mid] - base) >= (unsigned long long)TOP) hi = mid;
+                            else lo = mid + 1;
+                        }
+                        e = lo;
+                    }
+                    for (int q = i + tid; q < e; q += KPP_THREADS)
+                        sout[jb + q] = from_parts<T>(be, (U)(P + (sh.pre[q] - base)));
+                    if (e > i) p = from_parts<T>(be, (U)(P + (sh.pre[e - 1] - base)));
+                    slow = e < s;
+                    i = e;
+                }
+            } else {
+                const int slot = be - sh.elo[i];
+                if (be > 0 && sh.elo[i] >= 0 && slot >= 0 && slot < sh.cnt[i]) {
+                    const GMap<T> m = sh.map[slot][i];
+                    const U Pn = P + ((P & 1) ? m.a1 : m.a0);
+                    if (Pn < TOP) {
+                        p = from_parts<T>(be, Pn);
+                        if (tid == 0) sout[jb + i] = p;
+                        i++;
+                        slow = false;
+                    }
+                }
+            }
+            if (slow) {
+                const long long j = jb + i;
+                p = block_walk_chunk<T>(p, v + j * KPP_CH, (int)min((long long)KPP_CH, n - j * KPP_CH),
+                                        j == 0 ? f.gstates + slice * 32 : nullptr, sh);
+                if (tid == 0) sout[j] = p;
+                i++;
+            }
         }
     }
-    long long cand = n - 1;
-    if (lo < nch) {
-        const long long j = lo;
-        const T p = j > 0 ? S[j - 1] : T(0);
-        const int clen = (int)min((long long)KPP_CH, n - j * KPP_CH);
-        int hit = -1;
-        walk_chunk<T, true>(p, v + j * KPP_CH, clen, fs.gmap + (slice * nch + j) * KPP_GROUPS, fs.elo[slice * nch + j],
-                            thr, &hit);
-        if (hit >= 0) cand = j * KPP_CH + hit;
+    __syncthreads();
+    if (tid == 0) {
+        st->pot[t] = (double)p;
+        __threadfence();  // the block's states and the potential, before the count
+        sh.last = atomicAdd(&st->done, 1) == ntr - 1;
+        if (sh.last) st->done = 0;
+        __threadfence();
     }
-    if (lane == 0) st->cand[w] = cand;
+    __syncthreads();
+    if (sh.last) kpp_select<T>(f, c, init);
 }
 
 template <typename T, int TT, bool INIT>
-void launch_trials(const T *x, long long n, int d, T *chains, int ts, const KppState *st, int ntr, double *csum,
-                   long long nch, cudaStream_t s) {
-    constexpr size_t smem = trial_smem<T, TT>();
-    static_assert(smem <= 227 * 1024, "two stages of the trial tile fit in shared memory");
+void launch_trials(const KppFit<T> *fits, const int2 *items, unsigned grid, int scan, int c, int dmax,
+                   cudaStream_t s) {
+    const size_t smem = trial_smem(dmax, TT);
     FK_CUDA(cudaFuncSetAttribute((const void *)kpp_trials_kernel<T, TT, INIT>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kpp_trials_kernel<T, TT, INIT><<<(unsigned)nch, KPP_THREADS, smem, s>>>(x, n, d, chains, ts, st, ntr, csum, nch);
+    kpp_trials_kernel<T, TT, INIT><<<grid, KPP_THREADS, smem, s>>>(fits, items, scan, c);
     FK_LAUNCH_CHECK();
-}
-
-template <int TT>
-void launch_trials_f64f(const double *x, const float *x32, const float *xerr, long long n, int d, double *chains,
-                        int ts, const KppState *st, int ntr, double *csum, long long nch, cudaStream_t s) {
-    constexpr size_t smem = trial_smem<float, TT>();
-    FK_CUDA(cudaFuncSetAttribute((const void *)kpp_trials_f64f_kernel<TT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
-    kpp_trials_f64f_kernel<TT><<<(unsigned)nch, KPP_THREADS, smem, s>>>(x, x32, xerr, n, d, chains, ts, st, ntr,
-                                                                        csum, nch);
-    FK_LAUNCH_CHECK();
-}
-
-void launch_trials_f64f_any(const double *x, const float *x32, const float *xerr, long long n, int d,
-                            double *chains, int ts, const KppState *st, int ntr, double *csum, long long nch,
-                            cudaStream_t s) {
-    switch (ntr) {
-        case 1: launch_trials_f64f<1>(x, x32, xerr, n, d, chains, ts, st, ntr, csum, nch, s); break;
-        case 2: launch_trials_f64f<2>(x, x32, xerr, n, d, chains, ts, st, ntr, csum, nch, s); break;
-        case 3: launch_trials_f64f<3>(x, x32, xerr, n, d, chains, ts, st, ntr, csum, nch, s); break;
-        case 4: launch_trials_f64f<4>(x, x32, xerr, n, d, chains, ts, st, ntr, csum, nch, s); break;
-        case 5: launch_trials_f64f<5>(x, x32, xerr, n, d, chains, ts, st, ntr, csum, nch, s); break;
-        case 6: launch_trials_f64f<6>(x, x32, xerr, n, d, chains, ts, st, ntr, csum, nch, s); break;
-        case 7: launch_trials_f64f<7>(x, x32, xerr, n, d, chains, ts, st, ntr, csum, nch, s); break;
-        case 8: launch_trials_f64f<8>(x, x32, xerr, n, d, chains, ts, st, ntr, csum, nch, s); break;
-        case 9: launch_trials_f64f<9>(x, x32, xerr, n, d, chains, ts, st, ntr, csum, nch, s); break;
-        case 10: launch_trials_f64f<10>(x, x32, xerr, n, d, chains, ts, st, ntr, csum, nch, s); break;
-        case 11: launch_trials_f64f<11>(x, x32, xerr, n, d, chains, ts, st, ntr, csum, nch, s); break;
-        case 12: launch_trials_f64f<12>(x, x32, xerr, n, d, chains, ts, st, ntr, csum, nch, s); break;
-        default: launch_trials_f64f<16>(x, x32, xerr, n, d, chains, ts, st, ntr, csum, nch, s); break;
-    }
 }
 
 // The trial pass with the smallest trial-slot count that holds ntr trials.
 template <typename T>
-void launch_trials_any(const T *x, long long n, int d, T *chains, int ts, const KppState *st, int ntr, double *csum,
-                       long long nch, cudaStream_t s) {
+void launch_trials_any(int ntr, const KppFit<T> *fits, const int2 *items, unsigned grid, int scan, int c, int dmax,
+                       cudaStream_t s) {
     switch (ntr) {
-        case 1: launch_trials<T, 1, false>(x, n, d, chains, ts, st, ntr, csum, nch, s); break;
-        case 2: launch_trials<T, 2, false>(x, n, d, chains, ts, st, ntr, csum, nch, s); break;
-        case 3: launch_trials<T, 3, false>(x, n, d, chains, ts, st, ntr, csum, nch, s); break;
-        case 4: launch_trials<T, 4, false>(x, n, d, chains, ts, st, ntr, csum, nch, s); break;
-        case 5: launch_trials<T, 5, false>(x, n, d, chains, ts, st, ntr, csum, nch, s); break;
-        case 6: launch_trials<T, 6, false>(x, n, d, chains, ts, st, ntr, csum, nch, s); break;
-        case 7: launch_trials<T, 7, false>(x, n, d, chains, ts, st, ntr, csum, nch, s); break;
-        case 8: launch_trials<T, 8, false>(x, n, d, chains, ts, st, ntr, csum, nch, s); break;
-        case 9: launch_trials<T, 9, false>(x, n, d, chains, ts, st, ntr, csum, nch, s); break;
-        case 10: launch_trials<T, 10, false>(x, n, d, chains, ts, st, ntr, csum, nch, s); break;
-        case 11: launch_trials<T, 11, false>(x, n, d, chains, ts, st, ntr, csum, nch, s); break;
-        case 12: launch_trials<T, 12, false>(x, n, d, chains, ts, st, ntr, csum, nch, s); break;
-        default: launch_trials<T, 16, false>(x, n, d, chains, ts, st, ntr, csum, nch, s); break;
+        case 1: case 2: launch_trials<T, 2, false>(fits, items, grid, scan, c, dmax, s); break;
+        case 3: launch_trials<T, 3, false>(fits, items, grid, scan, c, dmax, s); break;
+        case 4: launch_trials<T, 4, false>(fits, items, grid, scan, c, dmax, s); break;
+        case 5: launch_trials<T, 5, false>(fits, items, grid, scan, c, dmax, s); break;
+        case 6: launch_trials<T, 6, false>(fits, items, grid, scan, c, dmax, s); break;
+        case 7: launch_trials<T, 7, false>(fits, items, grid, scan, c, dmax, s); break;
+        case 8: launch_trials<T, 8, false>(fits, items, grid, scan, c, dmax, s); break;
+        case 9: launch_trials<T, 9, false>(fits, items, grid, scan, c, dmax, s); break;
+        case 10: launch_trials<T, 10, false>(fits, items, grid, scan, c, dmax, s); break;
+        case 11: case 12: launch_trials<T, 12, false>(fits, items, grid, scan, c, dmax, s); break;
+        default: launch_trials<T, 16, false>(fits, items, grid, scan, c, dmax, s); break;
     }
+}
+
+// Byte layout of one seeding's workspace (256-byte aligned parts).
+struct KppLayout {
+    size_t chains, states, gstates, cmaps, csum, thr, own, crow, st, total;
+};
+template <typename T>
+KppLayout kpp_layout(const KppJob &j, int trials, int scan) {
+    const size_t n = (size_t)j.n, nch = (n + KPP_CH - 1) / KPP_CH, tiles = (n + scan - 1) / scan;
+    KppLayout L{};
+    size_t at = 0;
+    auto part = [&](size_t bytes) {
+        const size_t p = at;
+        at += (bytes + 255) / 256 * 256;
+        return p;
+    };
+    L.chains = part(sizeof(T) * 2 * trials * n);
+    L.states = part(sizeof(T) * 2 * trials * nch);
+    L.gstates = part(sizeof(T) * 2 * trials * 32);
+    L.cmaps = part(sizeof(CMap<T>) * trials * nch);
+    L.csum = part(sizeof(float) * trials * tiles);
+    L.thr = part(sizeof(T) * (size_t)j.k);
+    L.own = part(sizeof(int32_t) * n);
+    L.crow = part(sizeof(int32_t) * (size_t)j.k);
+    L.st = part(sizeof(KppState));
+    L.total = at;
+    return L;
+}
+
+// Seedings [lo, hi) of the order (largest k first) together; false when their
+// workspace cannot be allocated and there are several.
+template <typename T>
+bool run_group(Ctx &ctx, const std::vector<KppJob> &jobs, const std::vector<int> &order, size_t lo, size_t hi, int scan,
+               int64_t *draws_used) {
+    cudaStream_t s = ctx.stream;
+    const size_t nf = hi - lo;
+    std::vector<KppFit<T>> fits(nf);
+    std::vector<size_t> off(nf);
+    size_t bytes = 0;
+    int dmax = 0, tmax = 1;
+    for (size_t q = 0; q < nf; q++) {
+        const KppJob &j = jobs[(size_t)order[lo + q]];
+        off[q] = bytes;
+        bytes += kpp_layout<T>(j, kpp_trials_host(j.k), scan).total;
+        dmax = std::max(dmax, j.d);
+        tmax = std::max(tmax, kpp_trials_host(j.k));
+    }
+    unsigned char *ws;
+    try {
+        ws = (unsigned char *)ctx.get(BUF_KPP1, bytes);
+    } catch (const Error &e) {
+        if (e.code != FK_ERR_OOM || nf == 1) throw;
+        return false;
+    }
+    // items of the trial pass (tiles) and of the composition (eight chunks), in
+    // seeding order: the seedings still running at a step are a prefix
+    std::vector<int2> items;
+    std::vector<unsigned> tile_end(nf), comp_end(nf);
+    unsigned nt = 0, ncg = 0;
+    for (size_t q = 0; q < nf; q++) {
+        const KppJob &j = jobs[(size_t)order[lo + q]];
+        KppFit<T> &f = fits[q];
+        const KppLayout L = kpp_layout<T>(j, kpp_trials_host(j.k), scan);
+        unsigned char *b = ws + off[q];
+        f.x = (const T *)j.x;
+        f.x32 = sizeof(T) == 8 ? j.x32 : (const float *)j.x;
+        f.xerr = sizeof(T) == 8 ? j.xerr : nullptr;
+        f.draws = j.draws;
+        f.centers = (T *)j.centers;
+        f.chains = (T *)(b + L.chains);
+        f.states = (T *)(b + L.states);
+        f.cmaps = (CMap<T> *)(b + L.cmaps);
+        f.gstates = (T *)(b + L.gstates);
+        f.csum = (float *)(b + L.csum);
+        f.thr = (T *)(b + L.thr);
+        f.own = (int32_t *)(b + L.own);
+        f.crow = (int32_t *)(b + L.crow);
+        f.st = (KppState *)(b + L.st);
+        f.n = j.n;
+        f.nch = (j.n + KPP_CH - 1) / KPP_CH;
+        f.tiles = (j.n + scan - 1) / scan;
+        f.n_draws = j.n_draws;
+        f.seed = j.seed;
+        f.d = j.d;
+        f.k = j.k;
+        f.trials = kpp_trials_host(j.k);
+        f.nan_direct = j.nan_direct ? 1 : 0;
+        nt += (unsigned)f.tiles;
+        ncg += (unsigned)((f.nch + KPP_WARPS - 1) / KPP_WARPS);
+        tile_end[q] = nt;
+        comp_end[q] = ncg;
+    }
+    KppFit<T> *dfits = (KppFit<T> *)ctx.get(BUF_KPP0, sizeof(KppFit<T>) * nf);
+    FK_CUDA(cudaMemcpyAsync(dfits, fits.data(), sizeof(KppFit<T>) * nf, cudaMemcpyHostToDevice, s));
+    const int2 *titems = nullptr, *citems = nullptr;
+    if (nf > 1) {
+        items.reserve((size_t)nt + ncg);
+        for (size_t q = 0; q < nf; q++)
+            for (int t = 0; t < (int)fits[q].tiles; t++) items.push_back(make_int2((int)q, t));
+        for (size_t q = 0; q < nf; q++)
+            for (long long t = 0; t * KPP_WARPS < fits[q].nch; t++) items.push_back(make_int2((int)q, (int)t));
+        int2 *di = (int2 *)ctx.get(BUF_KPP2, sizeof(int2) * items.size());
+        FK_CUDA(cudaMemcpyAsync(di, items.data(), sizeof(int2) * items.size(), cudaMemcpyHostToDevice, s));
+        titems = di;
+        citems = di + nt;
+    }
+    kpp_first_kernel<T><<<(unsigned)nf, 128, 0, s>>>(dfits);
+    FK_LAUNCH_CHECK();
+    for (int c = 0;; c++) {
+        // the seedings with a centre c to choose (c = 0: those with a second
+        // centre form the first D^2 array)
+        size_t na = 0;
+        while (na < nf && fits[na].k > std::max(c, 1)) na++;
+        if (na == 0) break;
+        const bool init = c == 0;
+        int nt_step = 1;
+        for (size_t q = 0; q < na; q++) nt_step = std::max(nt_step, fits[q].trials);
+        if (init) {
+            launch_trials<T, 1, true>(dfits, titems, tile_end[na - 1], scan, c, dmax, s);
+        } else {
+            kpp_pairs_kernel<T><<<(unsigned)(na * ((c + KPP_WARPS - 1) / KPP_WARPS)), KPP_THREADS, 0, s>>>(dfits, c);
+            FK_LAUNCH_CHECK();
+            launch_trials_any<T>(nt_step, dfits, titems, tile_end[na - 1], scan, c, dmax, s);
+        }
+        const unsigned gy = init ? 1u : (unsigned)nt_step;
+        kpp_compose_kernel<T><<<dim3(comp_end[na - 1], gy), KPP_THREADS, 0, s>>>(dfits, citems, scan, c, init);
+        FK_LAUNCH_CHECK();
+        kpp_walk_kernel<T><<<dim3((unsigned)na, gy), KPP_THREADS, 0, s>>>(dfits, c, init);
+        FK_LAUNCH_CHECK();
+    }
+    // the descriptors above are host stack memory, and the draws are read back
+    std::vector<long long> cur(nf);
+    if (draws_used)
+        for (size_t q = 0; q < nf; q++)
+            FK_CUDA(cudaMemcpyAsync(&cur[q], &fits[q].st->cursor, sizeof(long long), cudaMemcpyDeviceToHost, s));
+    FK_CUDA(cudaStreamSynchronize(s));
+    if (draws_used)
+        for (size_t q = 0; q < nf; q++) draws_used[order[lo + q]] = (int64_t)cur[q];
+    return true;
+}
+
+// A group that does not fit in memory runs as two halves.
+template <typename T>
+void run_split(Ctx &ctx, const std::vector<KppJob> &jobs, const std::vector<int> &order, size_t lo, size_t hi, int scan,
+               int64_t *draws_used) {
+    if (run_group<T>(ctx, jobs, order, lo, hi, scan, draws_used)) return;
+    run_split<T>(ctx, jobs, order, lo, (lo + hi) / 2, scan, draws_used);
+    run_split<T>(ctx, jobs, order, (lo + hi) / 2, hi, scan, draws_used);
 }
 
 }  // namespace
 
-int kpp_trials(int k) {
-    long long t = 2 + (long long)std::floor(std::log((double)k));
-    if (t < 1) t = 1;
-    return (int)t;
-}
+// Seedings run together while their workspaces stay within this many bytes
+// (one larger seeding runs alone).
+constexpr size_t KPP_GROUP_BYTES = (size_t)6 << 30;
 
 template <typename T>
-void run_kmeanspp(Ctx &ctx, const T *x, int64_t n, int d, int k, const double *draws_dev, int64_t n_draws,
-                  T *centers_out, int64_t *draws_used) {
-    cudaStream_t s = ctx.stream;
-    const int n_trials = kpp_trials(k);
-    if (n_trials > MAX_TRIALS) {
-        set_error("k-means++ with k=%d needs %d trials (max %d)", k, n_trials, MAX_TRIALS);
-        fail(FK_ERR_UNSUPPORTED);
+void run_kmeanspp(Ctx &ctx, std::vector<KppJob> &jobs, int64_t *draws_used) {
+    if (jobs.empty()) return;
+    long long rows = 0;
+    for (const KppJob &j : jobs) {
+        const int trials = kpp_trials_host(j.k);
+        if (trials > MAX_TRIALS) {
+            set_error("k-means++ with k=%d needs %d trials (max %d)", j.k, trials, MAX_TRIALS);
+            fail(FK_ERR_UNSUPPORTED);
+        }
+        rows += j.n;
     }
-    FK_CUDA(cudaMemsetAsync(centers_out, 0, sizeof(T) * (size_t)k * d, s));
-    const long long nch = (n + KPP_CH - 1) / KPP_CH;
-    const int ts = n_trials;  // trial slices per buffer
-    const size_t slices = 2 * (size_t)ts * (size_t)nch;  // per-chunk entries over both buffers
-    auto *st = (KppState *)ctx.get(BUF_KPP0, sizeof(KppState));
-    T *chains = (T *)ctx.get(BUF_KPP1, sizeof(T) * (size_t)n * ts * 2);
-    double *csum = (double *)ctx.get(BUF_KPP2, sizeof(double) * (size_t)nch * ts);
-    const size_t b_gmap = sizeof(Map3) * slices * KPP_GROUPS, b_cmap = sizeof(Map3) * slices,
-                 b_states = sizeof(T) * slices, b_elo = sizeof(int) * slices;
-    unsigned char *fold = (unsigned char *)ctx.get(BUF_KPP3, b_gmap + b_cmap + b_states + b_elo + 256);
-    FoldSlices fs;
-    fs.gmap = reinterpret_cast<Map3 *>(fold);
-    fs.cmap = reinterpret_cast<Map3 *>(fold + b_gmap);
-    fs.states = fold + b_gmap + b_cmap;
-    fs.elo = reinterpret_cast<int *>(fold + b_gmap + b_cmap + b_states);
-    FK_CUDA(cudaMemsetAsync(st, 0, sizeof(KppState), s));
-
-    kpp_first_kernel<T><<<1, 128, 0, s>>>(x, n, d, draws_dev, n_draws, st, centers_out);
-    FK_LAUNCH_CHECK();
-    // f64: the rows' f32 copies and rounding-error norms for the trials' FP32 bounds
-    float *x32 = nullptr, *xerr = nullptr;
     if constexpr (std::is_same<T, double>::value) {
-        if (k > 1) {
-            x32 = (float *)ctx.get(BUF_PF_X32, sizeof(float) * (size_t)n * d);
-            xerr = (float *)ctx.get(BUF_PF_XERR, sizeof(float) * (size_t)n);
-            launch_f32_copy(ctx, x, n, d, x32, xerr);
+        // f32 copies and rounding-error norms for the FP32 bounds (the f64
+        // callers' seedings are restarts on one matrix)
+        const KppJob &j0 = jobs[0];
+        if (j0.k > 1) {
+            float *x32 = (float *)ctx.get(BUF_PF_X32, sizeof(float) * (size_t)j0.n * j0.d);
+            float *xerr = (float *)ctx.get(BUF_PF_XERR, sizeof(float) * (size_t)j0.n);
+            launch_f32_copy(ctx, (const double *)j0.x, j0.n, j0.d, x32, xerr);
+            for (KppJob &j : jobs) {
+                j.x32 = x32;
+                j.xerr = xerr;
+            }
         }
     }
-    if (k == 1) {
-        if (draws_used) *draws_used = 1;
-        return;
-    }
-    const unsigned cgrid = (unsigned)((nch + KPP_THREADS / 32 - 1) / (KPP_THREADS / 32));
-    // the first D^2 array (distances to the first centre) and its fold
-    launch_trials<T, 1, true>(x, n, d, chains, ts, st, 1, csum, nch, s);
-    kpp_compose_kernel<T><<<dim3(cgrid, 1), KPP_THREADS, 0, s>>>(chains, n, ts, st, true, csum, nch, fs);
-    FK_LAUNCH_CHECK();
-    kpp_walk_kernel<T><<<1, 32, 0, s>>>(chains, n, ts, st, true, nch, fs);
-    FK_LAUNCH_CHECK();
-    for (int c = 1; c <= k; c++) {
-        kpp_select_kernel<T><<<1, MAX_TRIALS * 32, 0, s>>>(x, n, d, chains, ts, nch, fs, draws_dev, n_draws,
-                                                            n_trials, c, k, st, centers_out);
-        FK_LAUNCH_CHECK();
-        if (c == k) break;
-        if constexpr (std::is_same<T, double>::value)
-            launch_trials_f64f_any(x, x32, xerr, n, d, chains, ts, st, n_trials, csum, nch, s);
-        else
-            launch_trials_any<T>(x, n, d, chains, ts, st, n_trials, csum, nch, s);
-        kpp_compose_kernel<T><<<dim3(cgrid, (unsigned)n_trials), KPP_THREADS, 0, s>>>(chains, n, ts, st, false, csum,
-                                                                                     nch, fs);
-        FK_LAUNCH_CHECK();
-        kpp_walk_kernel<T><<<(unsigned)n_trials, 32, 0, s>>>(chains, n, ts, st, false, nch, fs);
-        FK_LAUNCH_CHECK();
-    }
-    if (draws_used) {
-        long long cur = 0;
-        FK_CUDA(cudaMemcpyAsync(&cur, &st->cursor, sizeof(cur), cudaMemcpyDeviceToHost, s));
-        FK_CUDA(cudaStreamSynchronize(s));
-        *draws_used = cur;
+    // Rows per trial-pass tile: 1024 (most room to gather listed rows into full
+    // warps), 256 while the larger tiles would leave SMs without one.
+    const int scan = rows / KPP_CH >= 4 * ctx.num_sms ? KPP_CH : KPP_THREADS;
+    std::vector<int> order(jobs.size());
+    for (size_t q = 0; q < jobs.size(); q++) order[q] = (int)q;
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return jobs[(size_t)a].k > jobs[(size_t)b].k; });
+    size_t lo = 0, bytes = 0;
+    for (size_t q = 0; q <= order.size(); q++) {
+        const size_t add = q < order.size()
+                               ? kpp_layout<T>(jobs[(size_t)order[q]], kpp_trials_host(jobs[(size_t)order[q]].k), scan).total
+                               : 0;
+        // (blockIdx.x counts the group's seedings too: far below its limit)
+        if (q > lo && (q == order.size() || bytes + add > KPP_GROUP_BYTES)) {
+            run_split<T>(ctx, jobs, order, lo, q, scan, draws_used);
+            lo = q;
+            bytes = 0;
+        }
+        bytes += add;
     }
 }
 
-template void run_kmeanspp<double>(Ctx &, const double *, int64_t, int, int, const double *, int64_t, double *,
-                                   int64_t *);
-template void run_kmeanspp<float>(Ctx &, const float *, int64_t, int, int, const double *, int64_t, float *,
-                                  int64_t *);
+template void run_kmeanspp<double>(Ctx &, std::vector<KppJob> &, int64_t *);
+template void run_kmeanspp<float>(Ctx &, std::vector<KppJob> &, int64_t *);
 
 }  // namespace fk
