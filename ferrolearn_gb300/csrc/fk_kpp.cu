@@ -35,16 +35,16 @@
 //                       formed in FP64 only where the candidate may come
 //                       closer.
 //   kpp_compose_kernel  per chunk of KPP_CH values the composed map for the
-//                       binade of the chunk's estimated starting sum (and the
-//                       next one, when the chunk may start or end there). The
+//                       binade of the chunk's estimated sums; where the sum may
+//                       change binade inside the chunk, the maps of its groups
+//                       of 32 values for both; the first chunk exactly. The
 //                       estimate, an f32 prefix of partial sums, steers speed,
 //                       never the result.
-//   kpp_walk_kernel     one CTA per fold scans the chunk maps, 1024 at a time;
-//                       a chunk whose map does not apply (the sum changes
-//                       binade in it, or is zero or not finite) is scanned
-//                       value by value, with one exact F addition where the
-//                       binade changes. Every state it records is bit for bit
-//                       the reference's running sum. The seeding's last CTA
+//   kpp_walk_kernel     one CTA per fold scans the chunk maps, 1024 at a time,
+//                       with one exact F addition where the binade changes; a
+//                       chunk whose maps do not apply is walked from its
+//                       values. Every state it records is bit for bit the
+//                       reference's running sum. The seeding's last CTA
 //                       then takes the strictly smallest potential (first
 //                       trial on ties: kmeans.rs:239-243), draws the next
 //                       thresholds u * total in F (:213-214) and finds each
@@ -76,7 +76,7 @@ constexpr int KPP_CH = 1024;      // values per fold chunk
 constexpr int KPP_THREADS = 256;  // every kernel's block
 constexpr int KPP_WARPS = KPP_THREADS / 32;
 constexpr int MAX_TRIALS = 16;
-constexpr int KPP_SLAB = 64;      // features staged at a time
+constexpr int KPP_SLAB = 32;      // features staged at a time
 
 // ---------------------------------------------------- binade arithmetic --
 template <typename T> struct Bits;
@@ -135,20 +135,19 @@ __device__ __forceinline__ typename Bits<T>::U inc_of(T v, int be, bool &tie) {
     using B = Bits<T>;
     using U = typename B::U;
     constexpr U OUT = (U)1 << (B::MB + 1);
+    // without branches: neighbouring values lie in many binades
     const U b = B::bits(v);
     const int ev = (int)(b >> B::MB);  // the sign bit makes it > EXPM
-    if (ev >= B::EXPM) return (U)(b << 1) == 0 ? (U)0 : OUT;  // negative (-0 is harmless), inf, NaN
-    const U mask = ((U)1 << B::MB) - 1;
-    const U m = (b & mask) | (ev ? (U)1 << B::MB : (U)0);
+    const U m = (b & (((U)1 << B::MB) - 1)) | (ev ? (U)1 << B::MB : (U)0);
     const int r = be - (ev ? ev : 1);
-    if (r < 0) return m == 0 ? (U)0 : OUT;
-    if (r > B::MB + 2) return (U)0;
-    if (r == 0) return m;
-    const U half = (U)1 << (r - 1);
+    const int sh = max(0, min(r, B::MB + 2));  // a shift of MB + 2 leaves nothing
+    const U half = ((U)1 << sh) >> 1;
     const U s = m + half;
-    const bool t = (s & ((half << 1) - 1)) == 0;
-    tie |= t;
-    return (s >> r) - (t ? (U)1 : (U)0);
+    const bool t = sh > 0 && (s & (((U)1 << sh) - 1)) == 0;
+    const U q = (s >> sh) - (t ? (U)1 : (U)0);
+    const bool out = (ev >= B::EXPM || r < 0) && (U)(b << 1) != 0;  // -0 is harmless
+    tie |= t && !out;
+    return out ? OUT : q;
 }
 
 // The map of 32 values, a lane each (dead lanes: increment 0), for binade be.
@@ -200,6 +199,18 @@ __device__ __forceinline__ GMap<T> group_map(T v, bool live, int be) {
     return GMap<T>{a0 < OUT ? a0 : OUT, a1 < OUT ? a1 : OUT};
 }
 
+// One more value at the end of a run held by one lane (at most 32 of them).
+template <typename T>
+__device__ __forceinline__ void run_add(GMap<T> &m, T v, int be) {
+    using U = typename Bits<T>::U;
+    bool tie = false;
+    const U inc = inc_of(v, be, tie);
+    m.a0 += inc;
+    m.a1 += inc;
+    m.a0 += tie ? m.a0 & 1 : (U)0;        // from an even sum: odd here rounds up
+    m.a1 += tie ? 1 - (m.a1 & 1) : (U)0;  // from an odd sum
+}
+
 // f then g
 template <typename T>
 __device__ __forceinline__ GMap<T> gcompose(const GMap<T> &f, const GMap<T> &g) {
@@ -241,13 +252,17 @@ __device__ __forceinline__ typename Bits<T>::U group_states(T v, bool live, int 
     return P + inc;
 }
 
-// Maps of one chunk for the binades elo and elo + 1 (elo < 0: none; cnt of
-// them built), saturated as GMap.
+// One chunk of a fold: its map for binade elo (KIND_MAP); the exact sum at its
+// end (KIND_END: the first chunk); or, where the sum may change from binade elo
+// to the next inside it, the slot of its groups' maps for both (KIND_SLOT).
+enum { KIND_NONE = 0, KIND_MAP = 1, KIND_END = 2, KIND_SLOT = 3 };
 template <typename T>
 struct CMap {
-    GMap<T> s[2];
-    int elo, cnt;
+    GMap<T> s;  // KIND_END: a0 = the sum's bits
+    int elo;
+    short kind, slot;
 };
+constexpr int KPP_SLOTS = 32;  // chunks of a fold with group maps (about one per binade)
 
 // A value as an f32 summand of the folds' estimates: F = f32 itself, F = f64
 // times 2^-esc by its bits (no FP64 conversion; out of range: 0 or inf).
@@ -291,6 +306,8 @@ struct KppFit {
     T *states;                // [2][trials][nch] running sum at each chunk's end
     CMap<T> *cmaps;           // [trials][nch]
     T *gstates;               // [2][trials][32] running sum after each 32 values of the first chunk
+    GMap<T> *slots;           // [trials][KPP_SLOTS][2][32] group maps of the chunks that have them
+    int *nslots;              // [trials]
     float *csum;              // [trials][tiles] estimates of the tiles' sums
     T *thr;                   // [k] skip threshold of each centre's rows at this step
     int32_t *own;             // [n] nearest centre so far
@@ -339,6 +356,7 @@ __global__ void kpp_first_kernel(const KppFit<T> *__restrict__ fits) {
         st->done = 0;
         st->esc = 0;
         st->cand[0] = first;
+        for (int t = 0; t < f.trials; t++) f.nslots[t] = 0;
         f.crow[0] = (int32_t)first;
     }
     __syncthreads();
@@ -481,27 +499,37 @@ __global__ void __launch_bounds__(KPP_THREADS)
         }
         if (tid == 0) list_n = rows;
     } else {
-        for (int i0 = 0; i0 < rows; i0 += KPP_THREADS) {
-            const int i = i0 + tid;
-            bool open = false;
-            T m = T(0);
+        // at most four rows a thread, their loads issued together
+        T m[KPP_CH / KPP_THREADS], pv[KPP_CH / KPP_THREADS];
+        int o[KPP_CH / KPP_THREADS];
+#pragma unroll
+        for (int a = 0; a < KPP_CH / KPP_THREADS; a++) {
+            const int i = a * KPP_THREADS + tid;
+            m[a] = pv[a] = T(0);
+            o[a] = 0;
             if (i < rows) {
-                m = mind[i];
-                int o = 0;
+                m[a] = mind[i];
                 if (own_c >= 0) {
-                    if (m < prev[i]) {
-                        o = own_c;
-                        f.own[base + i] = o;
-                    } else {
-                        o = f.own[base + i];
-                    }
+                    pv[a] = prev[i];
+                    o[a] = f.own[base + i];
                 }
-                open = !below(m, f.thr[o]);
-                if (!open) skipped += est_of(m, esc);
             }
-            __syncwarp();
-            if (i < rows && !open)
-                for (int t = 0; t < ntr; t++) out[(long long)t * n + i] = m;
+        }
+#pragma unroll
+        for (int a = 0; a < KPP_CH / KPP_THREADS; a++) {
+            const int i = a * KPP_THREADS + tid;
+            bool open = false;
+            if (i < rows) {
+                if (own_c >= 0 && m[a] < pv[a]) {
+                    o[a] = own_c;
+                    f.own[base + i] = own_c;
+                }
+                open = !below(m[a], f.thr[o[a]]);
+                if (!open) {
+                    skipped += est_of(m[a], esc);
+                    for (int t = 0; t < ntr; t++) out[(long long)t * n + i] = m[a];
+                }
+            }
             const unsigned bm = __ballot_sync(0xffffffffu, open);
             int at = 0;
             if (lane == 0 && bm) at = atomicAdd(&list_n, __popc(bm));
@@ -521,14 +549,14 @@ __global__ void __launch_bounds__(KPP_THREADS)
             for (int j0 = 0; j0 < d; j0 += KPP_SLAB) {
                 const int jn = min(KPP_SLAB, d - j0), j4 = (jn + 3) / 4;
                 if (vec) {
-                    for (int e = tid; e < cnt * 16; e += KPP_THREADS) {
-                        const int r = e >> 4, q = e & 15;
+                    for (int e = tid; e < cnt * (KPP_SLAB / 4); e += KPP_THREADS) {
+                        const int r = e / (KPP_SLAB / 4), q = e % (KPP_SLAB / 4);
                         if (q < j4)
                             cp_async16(xs + r * XS + 4 * q, f.x32 + (base + list[l0 + r]) * d + j0 + 4 * q, true);
                     }
                 } else {
                     for (int e = tid; e < cnt * KPP_SLAB; e += KPP_THREADS) {
-                        const int r = e >> 6, j = e & 63;
+                        const int r = e / KPP_SLAB, j = e % KPP_SLAB;
                         if (j < 4 * j4)
                             cp_async4(xs + r * XS + j, j < jn ? f.x32 + (base + list[l0 + r]) * d + j0 + j : f.x32,
                                       j < jn);
@@ -536,7 +564,7 @@ __global__ void __launch_bounds__(KPP_THREADS)
                 }
                 if (l0 == 0 || d > KPP_SLAB) {  // one slab: the candidates stay for every pass
                     for (int e = tid; e < TT * KPP_SLAB; e += KPP_THREADS) {
-                        const int t = e >> 6, j = e & 63;
+                        const int t = e / KPP_SLAB, j = e % KPP_SLAB;
                         if (j < 4 * j4) {
                             const bool ok = t < ntr && j < jn;
                             cp_async4(cs + t * W + j, ok ? f.x32 + cand[t] * d + j0 + j : f.x32, ok);
@@ -641,21 +669,118 @@ __global__ void __launch_bounds__(KPP_THREADS)
     }
 }
 
-// One CTA per (eight chunks, trial), one warp per chunk: the chunk's composed
-// map for the binade its estimated starting sum lies in, and for the one its
-// end lies in when that is the next. A chunk without exact halves is an
-// integer sum over coalesced loads (7 M values at n = 1M: bound by L2);
-// otherwise the lanes compose ordered runs of 32 values.
+// Rows of a staged chunk: value i at i + i / 32, so that reading a value a lane
+// and reading a run of 32 a lane both spread over the banks.
+__device__ __forceinline__ int staged(int i) { return i + (i >> 5); }
+constexpr int KPP_STAGED = KPP_CH + 32;
+template <typename T>
+__device__ __forceinline__ void cp_async_one(T *dst, const T *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+                 "n"((int)sizeof(T))
+                 : "memory");
+}
+
+// The first chunk of a fold exactly, by one warp: f32 value by value (a
+// dependent addition is four cycles); f64 (64 cycles) value by value for the
+// first group, then a group at a time, by its map where its estimated sums stay
+// in one binade (a run of 32 values a lane). gs[g] = the sum after group g.
+template <typename T>
+__device__ T first_chunk(const T *__restrict__ sv, int clen, int esc, T *__restrict__ gs) {
+    using U = typename Bits<T>::U;
+    constexpr U TOP = (U)1 << (Bits<T>::MB + 1);
+    const int lane = threadIdx.x & 31;
+    T p = T(0);
+    GMap<T> run{0, 0};
+    int run_be = 0;
+    if (sizeof(T) == 8) {
+        const int gl = max(0, min(32, clen - lane * 32));
+        float es = 0.f;
+#pragma unroll 4
+        for (int q = 0; q < gl; q++) es += est_of(sv[lane * 33 + q], esc);
+        float e = es;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const float o = __shfl_up_sync(0xffffffffu, e, off);
+            if (lane >= off) e += o;
+        }
+        const int blo = est_exp((e - es) * 0.9990234375f, esc, T(0));
+        if (blo > 0 && blo == est_exp(e * 1.0009765625f, esc, T(0))) {
+            run_be = blo;
+#pragma unroll 2
+            for (int q = 0; q < gl; q++) run_add(run, sv[lane * 33 + q], blo);
+        }
+        __syncwarp();
+        run = GMap<T>{min(run.a0, TOP), min(run.a1, TOP)};
+    }
+#pragma unroll 1
+    for (int g = 0; g * 32 < clen; g++) {
+        if (sizeof(T) == 8) {
+            const int be = normal_exp(p);
+            if (be > 0 && be == __shfl_sync(0xffffffffu, run_be, g)) {
+                const U P = significand(p);
+                const U Pn = P + __shfl_sync(0xffffffffu, (P & 1) ? run.a1 : run.a0, g);
+                if (Pn < TOP) {
+                    p = from_parts<T>(be, Pn);
+                    if (lane == 0) gs[g] = p;
+                    continue;
+                }
+            }
+        }
+        const int len = min(32, clen - g * 32);
+        const T val = lane < len ? sv[staged(g * 32 + lane)] : T(0);
+        int at = 0;
+        if (sizeof(T) == 4 || g == 0) {
+#pragma unroll 8
+            for (; at < len; at++) p = kpp_add(p, __shfl_sync(0xffffffffu, val, at));
+        }
+        while (at < len) {
+            const int be = normal_exp(p);
+            if (be > 0) {
+                const U S = group_states(val, lane >= at && lane < len, be, significand(p));
+                const unsigned bad = __ballot_sync(0xffffffffu, S >= TOP);
+                const int q = bad ? __ffs(bad) - 1 : 32;
+                const U Sb = __shfl_sync(0xffffffffu, S, q > 0 ? q - 1 : 0);
+                if (q > at) p = from_parts<T>(be, Sb);
+                if (q >= len) break;
+                at = q;
+            }
+            p = kpp_add(p, __shfl_sync(0xffffffffu, val, at));
+            at++;
+        }
+        if (lane == 0) gs[g] = p;
+    }
+    return p;
+}
+
+inline size_t compose_smem(size_t elem) { return elem * KPP_WARPS * KPP_STAGED; }
+
+// One CTA per (eight chunks, trial), one warp per chunk: the chunk's map for
+// the binade its estimated sums lie in -- an integer sum over a value a lane,
+// or, where exact halves occur, ordered runs of 32 a lane -- the group maps
+// for both binades where the estimate says that the sum may change binade, and
+// the first chunk exactly. The chunk's values are copied to shared memory
+// first: read in the loops, each load's latency was exposed (700 cycles a
+// value at n = 5,000).
 template <typename T>
 __global__ void __launch_bounds__(KPP_THREADS)
     kpp_compose_kernel(const KppFit<T> *__restrict__ fits, const int2 *__restrict__ items, int scan, int c, bool init) {
+    using U = typename Bits<T>::U;
+    constexpr U OUT = (U)1 << (Bits<T>::MB + 1);
     const int2 it = item_at(items);
     const KppFit<T> &f = fits[it.x];
     const KppState *st = f.st;
     const int t = blockIdx.y;
     if (t >= (init ? 1 : f.trials) || (!init && st->direct[c & 1])) return;
+    extern __shared__ __align__(16) unsigned char kpp_smem[];
     __shared__ float red[KPP_WARPS];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    T *sv = reinterpret_cast<T *>(kpp_smem) + w * KPP_STAGED;
+    const long long j = (long long)it.y * KPP_WARPS + w;
+    const int wbuf = init ? 0 : 1 - st->cur;
+    const T *v = f.chains + ((long long)wbuf * f.trials + t) * f.n + j * KPP_CH;
+    const int clen = j < f.nch ? (int)min((long long)KPP_CH, f.n - j * KPP_CH) : 0;
+#pragma unroll 8
+    for (int i = lane; i < clen; i += 32) cp_async_one(sv + staged(i), v + i);
     const int tpc = KPP_CH / scan;  // tiles per chunk
     const float *cs = f.csum + (long long)t * f.tiles;
     const long long t0 = (long long)it.y * KPP_WARPS * tpc;  // the group's first tile
@@ -665,77 +790,83 @@ __global__ void __launch_bounds__(KPP_THREADS)
     for (int o = 16; o >= 1; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
     if (lane == 0) red[w] = e;
     __syncthreads();
-    const long long j = (long long)it.y * KPP_WARPS + w;
     if (j >= f.nch) return;
     float s = 0.f;  // this chunk's sum
     e = lane < KPP_WARPS ? red[lane] : 0.f;
     for (int q = lane; q < (w + 1) * tpc; q += 32) {
-        const float v = t0 + q < f.tiles ? cs[t0 + q] : 0.f;
-        if (q < w * tpc) e += v;
-        else s += v;
+        const float x = t0 + q < f.tiles ? cs[t0 + q] : 0.f;
+        if (q < w * tpc) e += x;
+        else s += x;
     }
 #pragma unroll
     for (int o = 16; o >= 1; o >>= 1) {
         e += __shfl_xor_sync(0xffffffffu, e, o);
         s += __shfl_xor_sync(0xffffffffu, s, o);
     }
-    const int esc = init ? 0 : st->esc;
-    const int blo = est_exp(e * 0.9921875f, esc, T(0));
-    const int bhi = est_exp((e + s) * 1.0078125f, esc, T(0));
     CMap<T> *cm = f.cmaps + (long long)t * f.nch + j;
-    if (blo == 0 || bhi == 0 || bhi - blo > 1) {
-        if (lane == 0) cm->elo = -1;
+    cp_async_wait_all();
+    __syncwarp();
+    CMap<T> m;
+    m.s = GMap<T>{0, 0};
+    m.elo = -1;
+    m.kind = KIND_NONE;
+    m.slot = 0;
+    if (j == 0) {
+        m.s.a0 = Bits<T>::bits(first_chunk<T>(sv, clen, init ? 0 : st->esc, f.gstates + ((long long)wbuf * f.trials + t) * 32));
+        m.kind = KIND_END;
+        if (lane == 0) *cm = m;
         return;
     }
-    using U = typename Bits<T>::U;
-    constexpr U OUT = (U)1 << (Bits<T>::MB + 1);
-    const int nb = bhi - blo + 1;
-    const int wbuf = init ? 0 : 1 - st->cur;
-    const T *v = f.chains + ((long long)wbuf * f.trials + t) * f.n + j * KPP_CH;
-    const int clen = (int)min((long long)KPP_CH, f.n - j * KPP_CH);
-    unsigned long long a0 = 0, a1 = 0;  // at most 1024 increments of 2^53: no overflow
-    bool tie = false;
-#pragma unroll 8
-    for (int q = 0; q < KPP_CH / 32; q++) {
-        const int i = q * 32 + lane;
-        const T val = i < clen ? v[i] : T(0);
-        a0 += inc_of(val, blo, tie);
-        if (nb == 2) a1 += inc_of(val, blo + 1, tie);
+    // The f32 estimate's own error and the drift of a sequential f32 fold (a
+    // few 1e-5 at 10^6 values) lie inside the margins.
+    const int esc = init ? 0 : st->esc;
+    const int blo = est_exp(e * 0.9990234375f, esc, T(0));
+    const int bhi = est_exp((e + s) * 1.0009765625f, esc, T(0));
+    const int gl = max(0, min(32, clen - lane * 32));  // this lane's run
+    if (blo == 0 || bhi == 0 || bhi - blo > 1) {
+        if (lane == 0) *cm = m;
+        return;
     }
-    GMap<T> m0, m1;
+    m.elo = blo;
+    if (bhi > blo) {
+        int slot = 0;
+        if (lane == 0) slot = atomicAdd(f.nslots + t, 1);
+        slot = __shfl_sync(0xffffffffu, slot, 0);
+        if (slot < KPP_SLOTS) {
+            GMap<T> g0{0, 0}, g1{0, 0};
+#pragma unroll 2
+            for (int q = 0; q < gl; q++) {
+                const T x = sv[lane * 33 + q];
+                run_add(g0, x, blo);
+                run_add(g1, x, blo + 1);
+            }
+            GMap<T> *o = f.slots + ((long long)t * KPP_SLOTS + slot) * 64 + lane;
+            o[0] = GMap<T>{min(g0.a0, OUT), min(g0.a1, OUT)};
+            o[32] = GMap<T>{min(g1.a0, OUT), min(g1.a1, OUT)};
+            m.kind = KIND_SLOT;
+            m.slot = (short)slot;
+        }
+        if (lane == 0) *cm = m;
+        return;
+    }
+    unsigned long long a = 0;  // at most 1024 increments of 2^53: no overflow
+    bool tie = false;
+#pragma unroll 4
+    for (int i = lane; i < clen; i += 32) a += inc_of(sv[staged(i)], blo, tie);
     if (!__any_sync(0xffffffffu, tie)) {
 #pragma unroll
-        for (int o = 16; o >= 1; o >>= 1) {
-            a0 += __shfl_xor_sync(0xffffffffu, a0, o);
-            a1 += __shfl_xor_sync(0xffffffffu, a1, o);
-        }
-        m0.a0 = m0.a1 = (U)min(a0, (unsigned long long)OUT);
-        m1.a0 = m1.a1 = (U)min(a1, (unsigned long long)OUT);
+        for (int o = 16; o >= 1; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        m.s.a0 = m.s.a1 = (U)min(a, (unsigned long long)OUT);
     } else {
-        // exact halves: the maps of the 32 groups, lane g keeping group g's
-        m0 = m1 = GMap<T>{0, 0};
-#pragma unroll 4
-        for (int g = 0; g < KPP_CH / 32; g++) {
-            const int i = g * 32 + lane;
-            const T val = i < clen ? v[i] : T(0);
-            const GMap<T> x0 = group_map(val, i < clen, blo);
-            if (lane == g) m0 = x0;
-            if (nb == 2) {
-                const GMap<T> x1 = group_map(val, i < clen, blo + 1);
-                if (lane == g) m1 = x1;
-            }
-        }
-        m0 = gscan(m0);
-        m1 = gscan(m1);
-        m0 = GMap<T>{min(__shfl_sync(0xffffffffu, m0.a0, 31), OUT), min(__shfl_sync(0xffffffffu, m0.a1, 31), OUT)};
-        m1 = GMap<T>{min(__shfl_sync(0xffffffffu, m1.a0, 31), OUT), min(__shfl_sync(0xffffffffu, m1.a1, 31), OUT)};
+        GMap<T> g{0, 0};
+#pragma unroll 2
+        for (int q = 0; q < gl; q++) run_add(g, sv[lane * 33 + q], blo);
+        __syncwarp();
+        g = gscan(GMap<T>{min(g.a0, OUT), min(g.a1, OUT)});
+        m.s = GMap<T>{min(g.a0, OUT), min(g.a1, OUT)};
     }
-    if (lane == 0) {
-        cm->elo = blo;
-        cm->cnt = nb;
-        cm->s[0] = m0;
-        cm->s[1] = m1;
-    }
+    m.kind = KIND_MAP;
+    if (lane == 31) *cm = m;
 }
 
 // ------------------------------------------------- one fold by one CTA --
@@ -745,13 +876,12 @@ static_assert(KPP_CH == 4 * KPP_THREADS && KPP_WARPS == 8, "a chunk is 32 groups
 template <typename T>
 struct WalkShared {
     unsigned long long pre[KPP_ROUND];     // prefix sums of the plain chunks' increments
-    GMap<T> map[2][KPP_ROUND];             // chunk maps
-    int elo[KPP_ROUND];                    // their binades (-1: none), and
-    unsigned char cnt[KPP_ROUND];          // how many
+    CMap<T> map[KPP_ROUND];
     unsigned long long gtot[32];
     unsigned special[32], words;           // chunks to look at one by one (words: the nonzero words)
     GMap<T> gm[32];
-    T first[32], pb, vf;
+    T v[KPP_CH];                           // the values of a chunk walked by itself
+    T pb;
     int f0, last;
 };
 
@@ -759,42 +889,34 @@ struct WalkShared {
 // sequential fold, by the whole block: warp w holds groups 4 w .. 4 w + 3 of
 // 32 values. Per pass, the groups' maps for p's binade, their scan (by every
 // warp), and where the sum leaves the binade the group's own states and one
-// exact F addition: two barriers a pass. A fold's very first values (a binade
-// change at nearly each) are added one by one. gs (nullable): receives the
-// running sum after each group.
+// exact F addition: two barriers a pass.
 template <typename T>
-__device__ T block_walk_chunk(T p, const T *__restrict__ cv, int clen, T *__restrict__ gs, WalkShared<T> &sh) {
+__device__ T block_walk_chunk(T p, const T *__restrict__ cv, int clen, WalkShared<T> &sh) {
     using U = typename Bits<T>::U;
     constexpr U TOP = (U)1 << (Bits<T>::MB + 1);
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    T v[4];
+    __syncthreads();  // the chunk before is done with sh.v
 #pragma unroll
     for (int u = 0; u < 4; u++) {
-        const int i = (4 * w + u) * 32 + lane;
-        v[u] = i < clen ? cv[i] : T(0);
+        const int i = u * KPP_THREADS + tid;
+        sh.v[i] = i < clen ? cv[i] : T(0);
     }
+    __syncthreads();
     int start = 0;
-    if (p == T(0)) {
-        if (w == 0) sh.first[lane] = v[0];
-        __syncthreads();
-        start = min(32, clen);
-        for (int i = 0; i < start; i++) p = kpp_add(p, sh.first[i]);
-        if (gs && tid == 0) gs[0] = p;
-    }
+#pragma unroll 1
     while (start < clen) {
         const int be = normal_exp(p);
-        // the first group whose end state is not recorded yet
-        const int gfirst = max(0, start - 1) >> 5;
         if (be == 0) {
             // a NaN sum stays; +inf stays until a NaN value; a zero sum until a
             // value other than zero; a subnormal sum takes the next value
             const bool inf = is_inf_or_nan(p);
             int first = INT32_MAX;
             if (p == p) {
-#pragma unroll
+#pragma unroll 1
                 for (int u = 3; u >= 0; u--) {
                     const int i = (4 * w + u) * 32 + lane;
-                    const bool hit = inf ? v[u] != v[u] : (p == T(0) ? !(v[u] == T(0)) : true);
+                    const T x = sh.v[i];
+                    const bool hit = inf ? x != x : (p == T(0) ? !(x == T(0)) : true);
                     if (i >= start && i < clen && hit) first = i;
                 }
             }
@@ -805,23 +927,15 @@ __device__ T block_walk_chunk(T p, const T *__restrict__ cv, int clen, T *__rest
             if (lane == 0 && first != INT32_MAX) atomicMin(&sh.f0, first);
             __syncthreads();
             const int f0 = min(sh.f0, clen);
-            if (gs && w == 0 && lane >= gfirst && lane < (f0 == clen ? 32 : f0 >> 5)) gs[lane] = p;
             if (f0 == clen) return p;
-            if (w == f0 >> 7 && lane == (f0 & 31)) {
-                const int u = (f0 >> 5) & 3;
-                sh.vf = u == 0 ? v[0] : u == 1 ? v[1] : u == 2 ? v[2] : v[3];
-            }
-            __syncthreads();
-            p = kpp_add(p, sh.vf);
+            p = kpp_add(p, sh.v[f0]);
             start = f0 + 1;
-            __syncthreads();
-            if (start >= clen && gs && w == 0 && lane >= (f0 >> 5)) gs[lane] = p;
             continue;
         }
-#pragma unroll
+#pragma unroll 2
         for (int u = 0; u < 4; u++) {
             const int i = (4 * w + u) * 32 + lane;
-            const GMap<T> m = group_map(v[u], i >= start && i < clen, be);
+            const GMap<T> m = group_map(sh.v[i], i >= start && i < clen, be);
             if (lane == 0) sh.gm[4 * w + u] = m;
         }
         __syncthreads();
@@ -830,28 +944,74 @@ __device__ T block_walk_chunk(T p, const T *__restrict__ cv, int clen, T *__rest
         const U Pl = P + ((P & 1) ? m.a1 : m.a0);  // after group `lane`
         const unsigned bad = __ballot_sync(0xffffffffu, Pl >= TOP);
         const int gf = bad ? __ffs(bad) - 1 : 32;
-        if (gs && w == 0 && lane >= gfirst && lane < gf) gs[lane] = from_parts<T>(be, Pl);
         if (gf == 32) return from_parts<T>(be, __shfl_sync(0xffffffffu, Pl, 31));
         const U before = __shfl_sync(0xffffffffu, Pl, gf > 0 ? gf - 1 : 0);
         const U Pg = gf > 0 ? before : P;
         if (w == gf >> 2) {
-            const int u = gf & 3, i = gf * 32 + lane;
-            const T val = u == 0 ? v[0] : u == 1 ? v[1] : u == 2 ? v[2] : v[3];
-            const U S = group_states(val, i >= start && i < clen, be, Pg);
+            const int i = gf * 32 + lane;
+            const U S = group_states(sh.v[i], i >= start && i < clen, be, Pg);
             const int q = __ffs(__ballot_sync(0xffffffffu, S >= TOP)) - 1;  // the first value that leaves the binade
             const U Sb = __shfl_sync(0xffffffffu, S, q > 0 ? q - 1 : 0);
             if (lane == q) {
                 sh.pb = from_parts<T>(be, q > 0 ? Sb : Pg);
-                sh.vf = val;
                 sh.f0 = gf * 32 + q;
             }
         }
         __syncthreads();
-        p = kpp_add(sh.pb, sh.vf);  // the one exact addition where the binade changes
+        p = kpp_add(sh.pb, sh.v[sh.f0]);  // the one exact addition where the binade changes
         start = sh.f0 + 1;
-        if (start >= clen && gs && w == 0 && lane >= gf) gs[lane] = p;
     }
     return p;
+}
+
+// A chunk with group maps added to p, by every warp alike (no barrier): the
+// groups' maps for p's binade scanned, the group in which the sum leaves it by
+// its own states and one exact F addition, the groups after it by their maps
+// for the next binade. False where they do not apply.
+template <typename T>
+__device__ bool walk_slot_chunk(T &p, const T *__restrict__ cv, int clen, const GMap<T> *__restrict__ gm, int elo) {
+    using U = typename Bits<T>::U;
+    constexpr U TOP = (U)1 << (Bits<T>::MB + 1);
+    const int lane = threadIdx.x & 31;
+    const GMap<T> g0 = gm[lane], g1 = gm[32 + lane];
+    int be = normal_exp(p);
+    if (be != elo && be != elo + 1) return false;
+    int done = 0;  // groups added
+    T r = p;
+    if (be == elo) {
+        const U P = significand(r);
+        const GMap<T> m = gscan(g0);
+        const U Pl = P + ((P & 1) ? m.a1 : m.a0);
+        const unsigned bad = __ballot_sync(0xffffffffu, Pl >= TOP);
+        if (!bad) {
+            p = from_parts<T>(be, __shfl_sync(0xffffffffu, Pl, 31));
+            return true;
+        }
+        const int gf = __ffs(bad) - 1;
+        const int i = gf * 32 + lane;
+        const bool in = i < clen;
+        const T val = in ? cv[i] : T(0);
+        const U before = __shfl_sync(0xffffffffu, Pl, gf > 0 ? gf - 1 : 0);
+        const U Pg = gf > 0 ? before : P;
+        U S = group_states(val, in, be, Pg);
+        const int q = __ffs(__ballot_sync(0xffffffffu, S >= TOP)) - 1;  // the first value that leaves the binade
+        const U Sb = __shfl_sync(0xffffffffu, S, q > 0 ? q - 1 : 0);
+        r = kpp_add(from_parts<T>(be, q > 0 ? Sb : Pg), __shfl_sync(0xffffffffu, val, q));
+        be = normal_exp(r);
+        if (be != elo + 1) return false;
+        S = group_states(val, in && lane > q, be, significand(r));
+        S = __shfl_sync(0xffffffffu, S, 31);
+        if (S >= TOP) return false;
+        r = from_parts<T>(be, S);
+        done = gf + 1;
+    }
+    const U P = significand(r);
+    const GMap<T> m = gscan(lane < done ? GMap<T>{0, 0} : g1);
+    U Pl = P + ((P & 1) ? m.a1 : m.a0);
+    Pl = __shfl_sync(0xffffffffu, Pl, 31);
+    if (Pl >= TOP) return false;
+    p = from_parts<T>(be, Pl);
+    return true;
 }
 
 // The first value of a chunk whose inclusive running sum (from p) reaches thr,
@@ -881,16 +1041,9 @@ __device__ int warp_search_chunk(T p, const T *__restrict__ cv, int clen, T thr,
             if (lane >= start && lane < ng) {
                 // this lane's run in order, from an even and from an odd sum
                 const int gl = min(32, clen - lane * 32);
-#pragma unroll 8
+#pragma unroll 2
                 for (int q = 0; q < gl; q++) {
-                    bool tie = false;
-                    const U inc = inc_of(cv[lane * 32 + q], be, tie);
-                    m.a0 += inc;
-                    m.a1 += inc;
-                    if (tie) {
-                        m.a0 += m.a0 & 1;
-                        m.a1 += 1 - (m.a1 & 1);
-                    }
+                    run_add(m, cv[lane * 32 + q], be);
                 }
                 m.a0 = min(m.a0, TOP);
                 m.a1 = min(m.a1, TOP);
@@ -1042,8 +1195,9 @@ __device__ void kpp_select(const KppFit<T> &f, int c, bool init) {
 // Latency bound. Per round of 1024 chunks one scan forms the prefix sums of
 // the plain chunks' increments (one map, no exact half, the binade of the
 // chunk before): a run of them is then one addition and one comparison. The
-// others -- a second map, halves, a new binade -- are looked at one by one, and
-// a chunk in which the sum leaves its binade is walked (about one per binade).
+// others are looked at one by one: a chunk in which the sum changes binade
+// (about one per binade) through its group maps; one whose maps do not apply is
+// walked from its values.
 template <typename T>
 __global__ void __launch_bounds__(KPP_THREADS) kpp_walk_kernel(const KppFit<T> *__restrict__ fits, int c, bool init) {
     using U = typename Bits<T>::U;
@@ -1068,31 +1222,27 @@ __global__ void __launch_bounds__(KPP_THREADS) kpp_walk_kernel(const KppFit<T> *
     for (long long jb = 0; jb < nch; jb += KPP_ROUND) {
         const int nb = (int)min((long long)KPP_ROUND, nch - jb);
         __syncthreads();  // the round before is done with sh
-        unsigned long long a[4];
-#pragma unroll
+#pragma unroll 2
         for (int u = 0; u < 4; u++) {
             const int i = (4 * w + u) * 32 + lane;
             CMap<T> m;
             m.elo = -1;
-            m.cnt = 0;
-            m.s[0] = m.s[1] = GMap<T>{TOP, TOP};
+            m.kind = KIND_NONE;
             if (i < nb) m = cm[jb + i];
-            sh.map[0][i] = m.s[0];
-            sh.map[1][i] = m.s[1];
-            sh.elo[i] = m.elo;
-            sh.cnt[i] = (unsigned char)m.cnt;
+            sh.map[i] = m;
             int before = __shfl_up_sync(0xffffffffu, m.elo, 1);
             if (lane == 0) before = i > 0 && i < nb ? cm[jb + i - 1].elo : -1;
-            const bool plain = m.elo >= 0 && m.cnt == 1 && m.s[0].a0 == m.s[0].a1 && before == m.elo;
+            const bool plain = m.kind == KIND_MAP && m.s.a0 == m.s.a1 && before == m.elo;
             const unsigned sp = __ballot_sync(0xffffffffu, !plain && i < nb);
             if (lane == 0) sh.special[4 * w + u] = sp;
-            a[u] = plain ? (unsigned long long)m.s[0].a0 : 0ull;
+            unsigned long long a = plain ? (unsigned long long)m.s.a0 : 0ull;
 #pragma unroll
             for (int off = 1; off < 32; off <<= 1) {
-                const unsigned long long o = __shfl_up_sync(0xffffffffu, a[u], off);
-                if (lane >= off) a[u] += o;
+                const unsigned long long o = __shfl_up_sync(0xffffffffu, a, off);
+                if (lane >= off) a += o;
             }
-            if (lane == 31) sh.gtot[4 * w + u] = a[u];
+            sh.pre[i] = a;
+            if (lane == 31) sh.gtot[4 * w + u] = a;
         }
         __syncthreads();
         {
@@ -1105,8 +1255,7 @@ __global__ void __launch_bounds__(KPP_THREADS) kpp_walk_kernel(const KppFit<T> *
             }
             g -= own;  // the groups before
 #pragma unroll
-            for (int u = 0; u < 4; u++)
-                sh.pre[(4 * w + u) * 32 + lane] = a[u] + __shfl_sync(0xffffffffu, g, 4 * w + u);
+            for (int u = 0; u < 4; u++) sh.pre[(4 * w + u) * 32 + lane] += __shfl_sync(0xffffffffu, g, 4 * w + u);
             const unsigned nz = __ballot_sync(0xffffffffu, sh.special[lane] != 0);
             if (tid == 0) sh.words = nz;
         }
@@ -1127,7 +1276,7 @@ __global__ void __launch_bounds__(KPP_THREADS) kpp_walk_kernel(const KppFit<T> *
             }
             bool slow = true;
             if (s > i) {
-                if (be > 0 && sh.elo[i] == be) {
+                if (be > 0 && sh.map[i].elo == be) {
                     const unsigned long long base = i > 0 ? sh.pre[i - 1] : 0ull;
                     int e = s;
                     if ((unsigned long long)P + (sh.pre[s - 1] - base) >= (unsigned long long)TOP) {
@@ -1146,22 +1295,29 @@ __global__ void __launch_bounds__(KPP_THREADS) kpp_walk_kernel(const KppFit<T> *
                     i = e;
                 }
             } else {
-                const int slot = be - sh.elo[i];
-                if (be > 0 && sh.elo[i] >= 0 && slot >= 0 && slot < sh.cnt[i]) {
-                    const GMap<T> m = sh.map[slot][i];
-                    const U Pn = P + ((P & 1) ? m.a1 : m.a0);
+                const CMap<T> &m = sh.map[i];
+                if (m.kind == KIND_END) {
+                    p = Bits<T>::from(m.s.a0);
+                    slow = false;
+                } else if (m.kind == KIND_MAP && be > 0 && be == m.elo) {
+                    const U Pn = P + ((P & 1) ? m.s.a1 : m.s.a0);
                     if (Pn < TOP) {
                         p = from_parts<T>(be, Pn);
-                        if (tid == 0) sout[jb + i] = p;
-                        i++;
                         slow = false;
                     }
+                } else if (m.kind == KIND_SLOT) {
+                    const long long j = jb + i;
+                    slow = !walk_slot_chunk<T>(p, v + j * KPP_CH, (int)min((long long)KPP_CH, n - j * KPP_CH),
+                                               f.slots + ((long long)t * KPP_SLOTS + m.slot) * 64, m.elo);
+                }
+                if (!slow) {
+                    if (tid == 0) sout[jb + i] = p;
+                    i++;
                 }
             }
             if (slow) {
                 const long long j = jb + i;
-                p = block_walk_chunk<T>(p, v + j * KPP_CH, (int)min((long long)KPP_CH, n - j * KPP_CH),
-                                        j == 0 ? f.gstates + slice * 32 : nullptr, sh);
+                p = block_walk_chunk<T>(p, v + j * KPP_CH, (int)min((long long)KPP_CH, n - j * KPP_CH), sh);
                 if (tid == 0) sout[j] = p;
                 i++;
             }
@@ -1170,6 +1326,7 @@ __global__ void __launch_bounds__(KPP_THREADS) kpp_walk_kernel(const KppFit<T> *
     __syncthreads();
     if (tid == 0) {
         st->pot[t] = (double)p;
+        f.nslots[t] = 0;
         __threadfence();  // the block's states and the potential, before the count
         sh.last = atomicAdd(&st->done, 1) == ntr - 1;
         if (sh.last) st->done = 0;
@@ -1210,7 +1367,7 @@ void launch_trials_any(int ntr, const KppFit<T> *fits, const int2 *items, unsign
 
 // Byte layout of one seeding's workspace (256-byte aligned parts).
 struct KppLayout {
-    size_t chains, states, gstates, cmaps, csum, thr, own, crow, st, total;
+    size_t chains, states, gstates, slots, nslots, cmaps, csum, thr, own, crow, st, total;
 };
 template <typename T>
 KppLayout kpp_layout(const KppJob &j, int trials, int scan) {
@@ -1225,6 +1382,8 @@ KppLayout kpp_layout(const KppJob &j, int trials, int scan) {
     L.chains = part(sizeof(T) * 2 * trials * n);
     L.states = part(sizeof(T) * 2 * trials * nch);
     L.gstates = part(sizeof(T) * 2 * trials * 32);
+    L.slots = part(sizeof(GMap<T>) * trials * KPP_SLOTS * 2 * 32);
+    L.nslots = part(sizeof(int) * trials);
     L.cmaps = part(sizeof(CMap<T>) * trials * nch);
     L.csum = part(sizeof(float) * trials * tiles);
     L.thr = part(sizeof(T) * (size_t)j.k);
@@ -1279,6 +1438,8 @@ bool run_group(Ctx &ctx, const std::vector<KppJob> &jobs, const std::vector<int>
         f.states = (T *)(b + L.states);
         f.cmaps = (CMap<T> *)(b + L.cmaps);
         f.gstates = (T *)(b + L.gstates);
+        f.slots = (GMap<T> *)(b + L.slots);
+        f.nslots = (int *)(b + L.nslots);
         f.csum = (float *)(b + L.csum);
         f.thr = (T *)(b + L.thr);
         f.own = (int32_t *)(b + L.own);
@@ -1312,6 +1473,8 @@ bool run_group(Ctx &ctx, const std::vector<KppJob> &jobs, const std::vector<int>
         titems = di;
         citems = di + nt;
     }
+    FK_CUDA(cudaFuncSetAttribute((const void *)kpp_compose_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)compose_smem(sizeof(T))));
     kpp_first_kernel<T><<<(unsigned)nf, 128, 0, s>>>(dfits);
     FK_LAUNCH_CHECK();
     for (int c = 0;; c++) {
@@ -1331,7 +1494,8 @@ bool run_group(Ctx &ctx, const std::vector<KppJob> &jobs, const std::vector<int>
             launch_trials_any<T>(nt_step, dfits, titems, tile_end[na - 1], scan, c, dmax, s);
         }
         const unsigned gy = init ? 1u : (unsigned)nt_step;
-        kpp_compose_kernel<T><<<dim3(comp_end[na - 1], gy), KPP_THREADS, 0, s>>>(dfits, citems, scan, c, init);
+        kpp_compose_kernel<T><<<dim3(comp_end[na - 1], gy), KPP_THREADS, compose_smem(sizeof(T)), s>>>(dfits, citems,
+                                                                                                     scan, c, init);
         FK_LAUNCH_CHECK();
         kpp_walk_kernel<T><<<dim3((unsigned)na, gy), KPP_THREADS, 0, s>>>(dfits, c, init);
         FK_LAUNCH_CHECK();
