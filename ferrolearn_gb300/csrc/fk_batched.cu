@@ -16,15 +16,18 @@
 //                        per thread x centres per pass) is the autotuner's
 //                        choice for the bucket. Per item a fixed-tree f64
 //                        inertia partial.
-//   batch_update_kernel  per iteration, one persistent launch over the fits:
-//                        counting sort of the labels (stable, eight warps over
-//                        contiguous row ranges), then per (cluster, feature)
-//                        either the row-order f32 sum exactly like
-//                        recompute_centroids_into (kmeans.rs:358-401), or the
-//                        exact sum (integer, order-free) rounded once to f64
-//                        with the mean rounded once to f32; the empty cluster
-//                        rule, sqrt of the max squared shift, the tol test,
-//                        n_iter and the inertia (partials in item order).
+//   batch_accum_kernel   f64 reduction: the exact (integer, order-free) sums of
+//                        each (fit, row range) item added to its fit's;
+//   batch_means_kernel   then per fit each sum rounded once to f64 with the mean
+//                        rounded once to f32.
+//   batch_update_kernel  reference reduction, one persistent launch over the
+//                        fits: counting sort of the labels (stable, eight warps
+//                        over contiguous row ranges), then per (cluster,
+//                        feature) the row-order f32 sum exactly like
+//                        recompute_centroids_into (kmeans.rs:358-401).
+//                        Both end an iteration: the empty cluster rule, sqrt of
+//                        the max squared shift, the tol test, n_iter and the
+//                        inertia (partials in item order).
 // One iteration (counter reset + bucket launches + update) is captured once
 // in a CUDA graph and replayed until every fit has converged or reached
 // max_iter; converged fits are skipped inside the kernels.
@@ -50,6 +53,7 @@ struct BFit {
     float tol;
     int32_t first_item, n_items;
     int32_t prob, pad;
+    int64_t k_off;  // offset of this fit's k cluster counts
     uint64_t seed;
 };
 
@@ -285,15 +289,241 @@ __device__ double fixed128_to_double(uint64_t lo, uint64_t hi, int F) {
 
 __device__ __forceinline__ int bitlen64(long long v) { return 64 - __clzll(v > 0 ? v : 1); }
 
-template <bool WIDE>
+// The f64 reduction's running sums: per (cluster, feature) of every fit the two
+// integer sums, and the parts the grids cannot hold -- the 128-bit remainder in
+// four 32-bit limbs (added limb by limb, carries resolved at the end) and what
+// non-finite values occurred. The update kernel leaves all of it zero.
+struct BSums {
+    unsigned long long *a1, *a2;  // two's complement
+    unsigned long long *limb;     // [4] each
+    uint32_t *flags;              // FLAG_*
+    int *count;                   // per cluster
+};
+constexpr uint32_t FLAG_NAN = 1u, FLAG_PINF = 2u, FLAG_NINF = 4u, FLAG_LIMBS = 8u;
+
+// The constants of one problem's exact sums.
+struct ExactGrid {
+    bool grids;
+    int kb, F, b1, b2;
+    float C1, C2;
+    __device__ __forceinline__ ExactGrid(float amax, int n) {
+        const int ea = amax > 0.f ? (int)((__float_as_uint(amax) >> 23) & 0xFFu) - 127 : -126;
+        grids = ea >= -90 && ea <= 100;
+        kb = ea + 2;
+        F = 124 - bitlen64(n) - ea;
+        C1 = grids ? ldexpf(1.5f, kb) : 0.f;
+        C2 = grids ? ldexpf(1.5f, kb - 23) : 0.f;
+        b1 = __float_as_int(C1);
+        b2 = __float_as_int(C2);
+    }
+};
+
+constexpr int ACC_T = 256;
+constexpr int ACC_ROWS = 8192;  // rows of an item at most
+
+// The f64 reduction's sums of one (fit, row range) item: the item's rows
+// grouped by cluster in shared memory, then a thread per (cluster, feature)
+// over the cluster's rows (neighbouring threads read neighbouring features)
+// and one addition to the fit's sums. Integer sums are order-free, so any
+// number of CTAs can share a fit: 64 problems x 10 runs took 427 ms of 994
+// with one CTA a fit, its largest fits' sorts and chains last.
+__global__ void __launch_bounds__(ACC_T) batch_accum_kernel(const float *__restrict__ X, const BFit *__restrict__ fits,
+                                                            const BState *__restrict__ state,
+                                                            const BItem *__restrict__ items, int nitems, int *counter,
+                                                            const int *__restrict__ lab,
+                                                            const float *__restrict__ pamax, BSums S) {
+    __shared__ unsigned short ids[ACC_ROWS];
+    __shared__ int hist[MAX_K], off[MAX_K];
+    __shared__ int it_sh;
+    const int tid = threadIdx.x, lane = tid & 31;
+    while (true) {
+        if (tid == 0) it_sh = atomicAdd(counter, 1);
+        __syncthreads();
+        const int it = it_sh;
+        __syncthreads();
+        if (it >= nitems) break;
+        const BItem I = items[it];
+        if (state[I.fit].done) continue;
+        const BFit F = fits[I.fit];
+        const int d = F.d, k = F.k, rows = I.hi - I.lo;
+        const int *L = lab + F.s_off + I.lo;
+        for (int c = tid; c < k; c += ACC_T) hist[c] = 0;
+        __syncthreads();
+        for (int r = tid; r < rows; r += ACC_T) atomicAdd(&hist[L[r]], 1);
+        __syncthreads();
+        if (tid < 32) {
+            int base = 0;
+            for (int c0 = 0; c0 < k; c0 += 32) {
+                const int v = c0 + lane < k ? hist[c0 + lane] : 0;
+                int s = v;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int u = __shfl_up_sync(0xffffffffu, s, o);
+                    if (lane >= o) s += u;
+                }
+                if (c0 + lane < k) {
+                    off[c0 + lane] = base + s - v;
+                    if (v) atomicAdd(S.count + F.k_off + c0 + lane, v);
+                }
+                base += __shfl_sync(0xffffffffu, s, 31);
+            }
+        }
+        __syncthreads();
+        for (int r = tid; r < rows; r += ACC_T) ids[atomicAdd(&off[L[r]], 1)] = (unsigned short)r;
+        __syncthreads();  // off[c] is now the end of cluster c's rows
+        const ExactGrid g(pamax[F.prob], F.n);
+        const float *x = X + F.x_off + (int64_t)I.lo * d;
+        const int64_t a_off = F.c_off / 2;
+        // few clusters and features: several threads share one's rows
+        const int kd = k * d, nsub = max(1, ACC_T / kd);
+        for (int q = tid; q < kd * nsub; q += ACC_T) {
+            const int sub = q / kd, pr = q - sub * kd;
+            const int c = pr / d, j = pr - c * d;
+            const int cnt = hist[c], o = off[c] - cnt;
+            long long a1 = 0, a2 = 0;
+            uint64_t slo = 0, shi = 0;
+            uint32_t fl = 0;
+#pragma unroll 8
+            for (int m = sub; m < cnt; m += nsub) {
+                const float xv = x[(int64_t)ids[o + m] * d + j];
+                if (!(fabsf(xv) < INFINITY)) {
+                    fl |= xv != xv ? FLAG_NAN : (xv > 0.f ? FLAG_PINF : FLAG_NINF);
+                } else if (g.grids) {
+                    const float s1 = __fadd_rn(xv, g.C1);
+                    a1 += __float_as_int(s1) - g.b1;
+                    const float r = __fsub_rn(xv, __fsub_rn(s1, g.C1));
+                    const float s2 = __fadd_rn(r, g.C2);
+                    a2 += __float_as_int(s2) - g.b2;
+                    const float r2 = __fsub_rn(r, __fsub_rn(s2, g.C2));
+                    if (r2 != 0.f) fixed_add_small(slo, shi, r2, g.F);
+                } else {
+                    fixed_add_small(slo, shi, xv, g.F);
+                }
+            }
+            const int64_t e = a_off + pr;
+            if (a1) atomicAdd(S.a1 + e, (unsigned long long)a1);
+            if (a2) atomicAdd(S.a2 + e, (unsigned long long)a2);
+            if (slo | shi) {
+                fl |= FLAG_LIMBS;
+                atomicAdd(S.limb + 4 * e, slo & 0xFFFFFFFFull);
+                atomicAdd(S.limb + 4 * e + 1, slo >> 32);
+                atomicAdd(S.limb + 4 * e + 2, shi & 0xFFFFFFFFull);
+                atomicAdd(S.limb + 4 * e + 3, shi >> 32);
+            }
+            if (fl) atomicOr(S.flags + e, fl);
+        }
+        __syncthreads();  // ids and hist are refilled
+    }
+}
+
+// What ends an iteration of fit f, by thread 0: sqrt of the largest squared
+// shift against tol, the inertia's partials in item order, the state.
+__device__ __forceinline__ void finish_fit(const BFit &F, BState *state, int f, float m2,
+                                           const double *__restrict__ partial, int *active) {
+    const float shift = __fsqrt_rn(m2);
+    double in = 0.0;
+    for (int it = 0; it < F.n_items; it++) in += partial[F.first_item + it];
+    BState st = state[f];
+    st.inertia = in;
+    st.n_iter += 1;
+    st.cur = 1 - st.cur;
+    if (shift < F.tol || st.n_iter >= F.max_iter) {
+        st.done = 1;
+        atomicSub(active, 1);
+    }
+    state[f] = st;
+}
+
+// The f64 reduction's new centres from the sums (left zero for the next
+// iteration): each sum rounded once to f64, the mean once to f32.
+__global__ void __launch_bounds__(UPDATE_T) batch_means_kernel(const BFit *__restrict__ fits, BState *__restrict__ state,
+                                                               const int *__restrict__ order, int nf, int *counter,
+                                                               float *__restrict__ C, const double *__restrict__ partial,
+                                                               int *active, const float *__restrict__ pamax, BSums S) {
+    __shared__ int q_sh;
+    __shared__ float red[UPDATE_T / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    while (true) {
+        if (tid == 0) q_sh = atomicAdd(counter, 1);
+        __syncthreads();
+        const int q = q_sh;
+        __syncthreads();
+        if (q >= nf) break;
+        const int f = order[q];
+        if (state[f].done) continue;
+        const BFit F = fits[f];
+        const int d = F.d, k = F.k, cur = state[f].cur;
+        const float *oldc = C + F.c_off + (int64_t)cur * k * d;
+        float *newc = C + F.c_off + (int64_t)(1 - cur) * k * d;
+        const ExactGrid g(pamax[F.prob], F.n);
+        const int64_t a_off = F.c_off / 2;
+        for (int pr = tid; pr < k * d; pr += UPDATE_T) {
+            const int64_t e = a_off + pr;
+            const int cnt = S.count[F.k_off + pr / d];
+            if (cnt == 0) {
+                newc[pr] = oldc[pr];  // empty cluster keeps its centre
+                continue;
+            }
+            const uint32_t fl = S.flags[e];
+            double sum;
+            if (fl & (FLAG_NAN | FLAG_PINF | FLAG_NINF)) {  // IEEE f64 summation of the specials
+                sum = ((fl & FLAG_NAN) || (fl & (FLAG_PINF | FLAG_NINF)) == (FLAG_PINF | FLAG_NINF))
+                          ? __longlong_as_double(0x7FF8000000000000LL)
+                      : (fl & FLAG_PINF) ? __longlong_as_double(0x7FF0000000000000LL)
+                                         : __longlong_as_double((long long)0xFFF0000000000000ULL);
+            } else {
+                uint64_t slo = 0, shi = 0;
+                if (fl & FLAG_LIMBS) {
+                    for (int l = 0; l < 4; l++) {
+                        const unsigned __int128 v = (unsigned __int128)S.limb[4 * e + l] << (32 * l);
+                        add128u(slo, shi, (uint64_t)v, (uint64_t)(v >> 64));
+                    }
+                }
+                if (g.grids) {
+                    const __int128 v1 = (__int128)(long long)S.a1[e] << (g.kb - 23 + g.F);
+                    const __int128 v2 = (__int128)(long long)S.a2[e] << (g.kb - 46 + g.F);
+                    add128u(slo, shi, (uint64_t)v1, (uint64_t)((unsigned __int128)v1 >> 64));
+                    add128u(slo, shi, (uint64_t)v2, (uint64_t)((unsigned __int128)v2 >> 64));
+                }
+                sum = fixed128_to_double(slo, shi, g.F);
+            }
+            newc[pr] = __double2float_rn(__ddiv_rn(sum, (double)cnt));
+            S.a1[e] = 0;
+            S.a2[e] = 0;
+            if (fl) {
+                S.flags[e] = 0;
+                for (int l = 0; l < 4; l++) S.limb[4 * e + l] = 0;
+            }
+        }
+        __syncthreads();
+        // the largest squared shift (NaN shifts never raise it)
+        float ms = 0.f;
+        for (int c = tid; c < k; c += UPDATE_T) {
+            S.count[F.k_off + c] = 0;
+            const float sh = sqeuc_f32(newc + (int64_t)c * d, oldc + (int64_t)c * d, d);
+            if (sh > ms) ms = sh;
+        }
+#pragma unroll
+        for (int o = 16; o >= 1; o >>= 1) ms = fmaxf(ms, __shfl_xor_sync(0xffffffffu, ms, o));
+        if (lane == 0) red[warp] = ms;
+        __syncthreads();
+        if (tid == 0) {
+            float m2 = 0.f;
+            for (int w = 0; w < UPDATE_T / 32; w++) m2 = fmaxf(m2, red[w]);
+            finish_fit(F, state, f, m2, partial, active);
+        }
+        __syncthreads();
+    }
+}
+
+// The reference reduction: row-order f32 sums, one CTA a fit.
 __global__ void __launch_bounds__(UPDATE_T) batch_update_kernel(const float *__restrict__ X,
                                                                 const BFit *__restrict__ fits,
                                                                 BState *__restrict__ state,
                                                                 const int *__restrict__ order, int nf, int *counter,
                                                                 float *__restrict__ C, const int *__restrict__ lab,
                                                                 int *__restrict__ mem,
-                                                                const double *__restrict__ partial, int *active,
-                                                                const float *__restrict__ pamax) {
+                                                                const double *__restrict__ partial, int *active) {
     constexpr int NW = UPDATE_T / 32;
     __shared__ int wrun[NW][MAX_K];
     __shared__ int hist[MAX_K], off[MAX_K];
@@ -362,14 +592,6 @@ __global__ void __launch_bounds__(UPDATE_T) batch_update_kernel(const float *__r
         const float *oldc = C + F.c_off + (int64_t)cur * k * d;
         float *newc = C + F.c_off + (int64_t)(1 - cur) * k * d;
         const float *x = X + F.x_off;
-        // exact-sum constants (f64 reduction)
-        const float amax = WIDE ? pamax[F.prob] : 0.f;
-        const int ea = amax > 0.f ? (int)((__float_as_uint(amax) >> 23) & 0xFFu) - 127 : -126;
-        const bool grids = ea >= -90 && ea <= 100;
-        const int kb = ea + 2;
-        const int Fb = 124 - bitlen64(n) - ea;
-        const float C1 = grids ? ldexpf(1.5f, kb) : 0.f, C2 = grids ? ldexpf(1.5f, kb - 23) : 0.f;
-        const int b1 = __float_as_int(C1), b2 = __float_as_int(C2);
         for (int pr = tid; pr < k * d; pr += UPDATE_T) {
             const int c = pr / d, j = pr - c * d;
             const int cnt = hist[c], o = off[c];
@@ -381,65 +603,17 @@ __global__ void __launch_bounds__(UPDATE_T) batch_update_kernel(const float *__r
             float cur8[8], nxt8[8];
 #pragma unroll
             for (int u = 0; u < 8; u++) cur8[u] = u < cnt ? x[(int64_t)M[o + u] * d + j] : 0.f;
-            if (WIDE) {
-                long long a1 = 0, a2 = 0;
-                uint64_t slo = 0, shi = 0;
-                float probe = 0.f;
-                for (int m = 0; m < cnt; m += 8) {
+            float acc = 0.f;
+            for (int m = 0; m < cnt; m += 8) {
 #pragma unroll
-                    for (int u = 0; u < 8; u++) nxt8[u] = m + 8 + u < cnt ? x[(int64_t)M[o + m + 8 + u] * d + j] : 0.f;
+                for (int u = 0; u < 8; u++) nxt8[u] = m + 8 + u < cnt ? x[(int64_t)M[o + m + 8 + u] * d + j] : 0.f;
 #pragma unroll
-                    for (int u = 0; u < 8; u++) {
-                        const float xv = cur8[u];  // 0 past the end
-                        probe = __fmaf_rn(xv, 0.f, probe);
-                        if (grids) {
-                            const float s1 = __fadd_rn(xv, C1);
-                            a1 += __float_as_int(s1) - b1;
-                            const float r = __fsub_rn(xv, __fsub_rn(s1, C1));
-                            const float s2 = __fadd_rn(r, C2);
-                            a2 += __float_as_int(s2) - b2;
-                            const float r2 = __fsub_rn(r, __fsub_rn(s2, C2));
-                            if (r2 != 0.f) fixed_add_small(slo, shi, r2, Fb);
-                        } else {
-                            fixed_add_small(slo, shi, xv, Fb);
-                        }
-                    }
+                for (int u = 0; u < 8; u++)
+                    if (m + u < cnt) acc = __fadd_rn(acc, cur8[u]);
 #pragma unroll
-                    for (int u = 0; u < 8; u++) cur8[u] = nxt8[u];
-                }
-                double sum;
-                if (!(probe == 0.f)) {  // a non-finite value: IEEE f64 summation of the specials
-                    uint32_t fl = 0u;
-                    for (int m = 0; m < cnt; m++) {
-                        const uint32_t bb = __float_as_uint(x[(int64_t)M[o + m] * d + j]);
-                        if (((bb >> 23) & 0xFFu) == 0xFFu) fl |= (bb & 0x7FFFFFu) ? 1u : ((bb >> 31) ? 4u : 2u);
-                    }
-                    sum = ((fl & 1u) || (fl & 6u) == 6u) ? __longlong_as_double(0x7FF8000000000000LL)
-                          : (fl & 2u) ? __longlong_as_double(0x7FF0000000000000LL)
-                                      : __longlong_as_double((long long)0xFFF0000000000000ULL);
-                } else {
-                    if (grids) {
-                        const __int128 v1 = (__int128)a1 << (kb - 23 + Fb);
-                        const __int128 v2 = (__int128)a2 << (kb - 46 + Fb);
-                        add128u(slo, shi, (uint64_t)v1, (uint64_t)((unsigned __int128)v1 >> 64));
-                        add128u(slo, shi, (uint64_t)v2, (uint64_t)((unsigned __int128)v2 >> 64));
-                    }
-                    sum = fixed128_to_double(slo, shi, Fb);
-                }
-                newc[pr] = __double2float_rn(__ddiv_rn(sum, (double)cnt));
-            } else {
-                float acc = 0.f;
-                for (int m = 0; m < cnt; m += 8) {
-#pragma unroll
-                    for (int u = 0; u < 8; u++) nxt8[u] = m + 8 + u < cnt ? x[(int64_t)M[o + m + 8 + u] * d + j] : 0.f;
-#pragma unroll
-                    for (int u = 0; u < 8; u++)
-                        if (m + u < cnt) acc = __fadd_rn(acc, cur8[u]);
-#pragma unroll
-                    for (int u = 0; u < 8; u++) cur8[u] = nxt8[u];
-                }
-                newc[pr] = __fdiv_rn(acc, (float)cnt);  // counts as F are exact below 2^24
+                for (int u = 0; u < 8; u++) cur8[u] = nxt8[u];
             }
+            newc[pr] = __fdiv_rn(acc, (float)cnt);  // counts as F are exact below 2^24
         }
         __syncthreads();
         // sqrt of the largest squared shift (NaN shifts never raise it)
@@ -455,45 +629,27 @@ __global__ void __launch_bounds__(UPDATE_T) batch_update_kernel(const float *__r
         if (tid == 0) {
             float m2 = 0.f;
             for (int w = 0; w < NW; w++) m2 = fmaxf(m2, red[w]);
-            const float shift = __fsqrt_rn(m2);
-            double in = 0.0;
-            for (int it = 0; it < F.n_items; it++) in += partial[F.first_item + it];
-            BState st = state[f];
-            st.inertia = in;
-            st.n_iter += 1;
-            st.cur = 1 - cur;
-            if (shift < F.tol || st.n_iter >= F.max_iter) {
-                st.done = 1;
-                atomicSub(active, 1);
-            }
-            state[f] = st;
+            finish_fit(F, state, f, m2, partial, active);
         }
         __syncthreads();
     }
 }
 
-// max |x| over the finite values of each problem (the exact sums' scale)
+// max |x| over the finite values of each problem (the exact sums' scale);
+// amax starts at zero, and non-negative floats order as their bits.
+constexpr int AMAX_PARTS = 32;  // CTAs a problem
 __global__ void batch_amax_kernel(const float *__restrict__ X, const int64_t *__restrict__ xoff,
-                                  const int64_t *__restrict__ xlen, int np, float *__restrict__ amax) {
-    __shared__ float red[32];
-    for (int p = blockIdx.x; p < np; p += gridDim.x) {
-        const float *x = X + xoff[p];
-        float m = 0.f;
-        for (int64_t e = threadIdx.x; e < xlen[p]; e += blockDim.x) {
-            const float a = fabsf(x[e]);
-            if (a < INFINITY) m = fmaxf(m, a);
-        }
-#pragma unroll
-        for (int o = 16; o >= 1; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            float r = 0.f;
-            for (int w = 0; w < (int)(blockDim.x >> 5); w++) r = fmaxf(r, red[w]);
-            amax[p] = r;
-        }
-        __syncthreads();
+                                  const int64_t *__restrict__ xlen, float *__restrict__ amax) {
+    const int p = blockIdx.x / AMAX_PARTS, part = blockIdx.x % AMAX_PARTS;
+    const float *x = X + xoff[p];
+    float m = 0.f;
+    for (int64_t e = (int64_t)part * blockDim.x + threadIdx.x; e < xlen[p]; e += (int64_t)AMAX_PARTS * blockDim.x) {
+        const float a = fabsf(x[e]);
+        if (a < INFINITY) m = fmaxf(m, a);
     }
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<int *>(amax + p), __float_as_int(m));
 }
 
 __global__ void batch_labels_u64_kernel(const int *__restrict__ l, int n, uint64_t *__restrict__ out) {
@@ -600,7 +756,7 @@ fk_status batched_fit_impl(Ctx &ctx, fk_batch_problem *P, int64_t np, int reduct
     }
     std::vector<BFit> fits;
     std::vector<int> fit_prob, fit_run;
-    int64_t soff = 0, coff = 0;
+    int64_t soff = 0, coff = 0, koff = 0;
     for (int64_t p = 0; p < np; p++) {
         const fk_batch_problem &q = P[p];
         for (int64_t r = 0; r < q.n_init; r++) {
@@ -609,6 +765,7 @@ fk_status batched_fit_impl(Ctx &ctx, fk_batch_problem *P, int64_t np, int reduct
             F.x_off = xoff[p];
             F.s_off = soff;
             F.c_off = coff;
+            F.k_off = koff;
             F.n = (int32_t)q.n;
             F.d = (int32_t)q.d;
             F.k = (int32_t)q.n_clusters;
@@ -621,6 +778,7 @@ fk_status batched_fit_impl(Ctx &ctx, fk_batch_problem *P, int64_t np, int reduct
             fit_run.push_back((int)r);
             soff += q.n;
             coff += 2 * q.n_clusters * q.d;
+            koff += q.n_clusters;
         }
     }
     const int nf = (int)fits.size();
@@ -660,6 +818,17 @@ fk_status batched_fit_impl(Ctx &ctx, fk_batch_problem *P, int64_t np, int reduct
     float *dC = (float *)ctx.get(BUF_BCEN, sizeof(float) * (size_t)coff + 16);
     int64_t *dxo = (int64_t *)ctx.get(BUF_BXOFF, sizeof(int64_t) * (size_t)(2 * np) + sizeof(float) * (size_t)np + 64);
     float *damax = (float *)(dxo + 2 * np);
+    BSums sums{};
+    if (reduction == FK_REDUCE_F64) {
+        const size_t ne = (size_t)(coff / 2);
+        unsigned char *b = (unsigned char *)ctx.get(BUF_BSUMS, ne * 52 + sizeof(int) * (size_t)koff + 16);
+        sums.a1 = (unsigned long long *)b;
+        sums.a2 = sums.a1 + ne;
+        sums.limb = sums.a2 + ne;
+        sums.flags = (uint32_t *)(sums.limb + 4 * ne);
+        sums.count = (int *)(sums.flags + ne);
+        FK_CUDA(cudaMemsetAsync(b, 0, ne * 52 + sizeof(int) * (size_t)koff, s));
+    }
     for (int64_t p = 0; p < np; p++)
         FK_CUDA(cudaMemcpyAsync(X + xoff[p], P[p].x, sizeof(float) * (size_t)(P[p].n * P[p].d), cudaMemcpyDefault,
                                 s));
@@ -672,9 +841,11 @@ fk_status batched_fit_impl(Ctx &ctx, fk_batch_problem *P, int64_t np, int reduct
         }
         FK_CUDA(cudaMemcpyAsync(dxo, xol.data(), sizeof(int64_t) * xol.size(), cudaMemcpyHostToDevice, s));
         FK_CUDA(cudaStreamSynchronize(s));  // xol is host stack memory
-        batch_amax_kernel<<<(unsigned)std::min<int64_t>(np, ctx.num_sms * 4), 256, 0, s>>>(X, dxo, dxo + np, (int)np,
-                                                                                        damax);
-        FK_LAUNCH_CHECK();
+        if (reduction == FK_REDUCE_F64) {
+            FK_CUDA(cudaMemsetAsync(damax, 0, sizeof(float) * (size_t)np, s));
+            batch_amax_kernel<<<(unsigned)(np * AMAX_PARTS), 256, 0, s>>>(X, dxo, dxo + np, damax);
+            FK_LAUNCH_CHECK();
+        }
     }
     if (!items.empty())
         FK_CUDA(cudaMemcpyAsync(ditems, items.data(), sizeof(BItem) * items.size(), cudaMemcpyHostToDevice, s));
@@ -761,7 +932,7 @@ fk_status batched_fit_impl(Ctx &ctx, fk_batch_problem *P, int64_t np, int reduct
 
     // ---- Lloyd iterations: one captured iteration, replayed
     auto one_iteration = [&]() {
-        FK_CUDA(cudaMemsetAsync(dctr, 0, sizeof(int) * 21, s));
+        FK_CUDA(cudaMemsetAsync(dctr, 0, sizeof(int) * 22, s));
         for (int b = 0; b < NBUCKETS; b++) {
             const int cnt = bstart[b + 1] - bstart[b];
             if (cnt == 0) continue;
@@ -770,12 +941,15 @@ fk_status batched_fit_impl(Ctx &ctx, fk_batch_problem *P, int64_t np, int reduct
                 X, dfits, dstate, ditems + bstart[b], cnt, dctr + b, dC, dlab, dpart + bstart[b]);
         }
         const int ug = std::min(nf, ctx.num_sms * 4);
-        if (reduction == FK_REDUCE_F64)
-            batch_update_kernel<true><<<ug, UPDATE_T, 0, s>>>(X, dfits, dstate, dorder, nf, dctr + 20, dC, dlab,
-                                                              dmem, dpart, dctr + 31, damax);
-        else
-            batch_update_kernel<false><<<ug, UPDATE_T, 0, s>>>(X, dfits, dstate, dorder, nf, dctr + 20, dC, dlab,
-                                                               dmem, dpart, dctr + 31, damax);
+        if (reduction == FK_REDUCE_F64) {
+            batch_accum_kernel<<<(unsigned)std::min<size_t>(items.size(), (size_t)ctx.num_sms * 6), ACC_T, 0, s>>>(
+                X, dfits, dstate, ditems, (int)items.size(), dctr + 21, dlab, damax, sums);
+            batch_means_kernel<<<ug, UPDATE_T, 0, s>>>(dfits, dstate, dorder, nf, dctr + 20, dC, dpart, dctr + 31,
+                                                       damax, sums);
+        } else {
+            batch_update_kernel<<<ug, UPDATE_T, 0, s>>>(X, dfits, dstate, dorder, nf, dctr + 20, dC, dlab, dmem, dpart,
+                                                        dctr + 31);
+        }
     };
     int max_iter = 0;
     for (const BFit &F : fits) max_iter = std::max(max_iter, F.max_iter);
