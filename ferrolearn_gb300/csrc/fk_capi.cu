@@ -1133,7 +1133,7 @@ fk_status bisecting_impl(fk_ctx *ctxp, const T *x_in, int64_t n, int64_t d, cons
     T *fold = (T *)ctx.get(BUF_BK_FOLD, sizeof(T) * (size_t)std::max(runs, 2));
     // The reference's row-order sums (the 2-means centres and the SSEs) as
     // exact parallel folds (fk_fold.cu): chains [0, runs * 2 * d) are the
-    // centre sums of the current segment (rows gathered into xseg), the next
+    // centre sums of the current segment (gathered feature-major into xseg), the next
     // runs + 2 the SSE folds.
     T *xseg = (T *)ctx.get(BUF_BK_XSEG, sizeof(T) * (size_t)n * d);
     const size_t nsum = (size_t)runs * 2 * d;
@@ -1141,13 +1141,14 @@ fk_status bisecting_impl(fk_ctx *ctxp, const T *x_in, int64_t n, int64_t d, cons
     T *fres = (T *)ctx.get(BUF_BK_FRES, sizeof(T) * (nsum + 8));
     long long *fcnt = (long long *)ctx.get(BUF_BK_FCNT, sizeof(long long) * (nsum + runs + 8));
     std::vector<FoldChain> hchains;
-    auto upload_sum_chains = [&](const T *rows, int nr, bool gated) {
+    // feature j of the rows starts at rows + j * next, `stride` apart
+    auto upload_sum_chains = [&](const T *rows, int64_t next, int64_t stride, int nr, bool gated) {
         hchains.assign((size_t)nr * 2 * d, FoldChain{});
         for (int r = 0; r < nr; r++)
             for (int side = 0; side < 2; side++)
                 for (int64_t j = 0; j < d; j++)
                     hchains[((size_t)r * 2 + side) * d + j] =
-                        FoldChain{rows + j, d, lab + (size_t)r * n, side, gated ? r : -1};
+                        FoldChain{rows + j * next, stride, lab + (size_t)r * n, side, gated ? r : -1};
         FK_CUDA(cudaMemcpyAsync(dchains, hchains.data(), sizeof(FoldChain) * hchains.size(), cudaMemcpyHostToDevice,
                                 s));
     };
@@ -1170,7 +1171,7 @@ fk_status bisecting_impl(fk_ctx *ctxp, const T *x_in, int64_t n, int64_t d, cons
     // compute_cluster_stats of every row (:192-222): the centre (sums / F::from(n)) and the SSE
     std::vector<T> hfold((size_t)std::max(runs, 2));
     FK_CUDA(cudaMemsetAsync(lab, 0, (size_t)n, s));
-    upload_sum_chains(x, 1, false);  // every row, in row order (the permutation is the identity)
+    upload_sum_chains(x, 1, d, 1, false);  // every row, in row order (the permutation is the identity)
     run_exact_folds<T>(ctx, dchains, (int)(2 * d), n, nullptr, fres, fcnt);
     launch_bk_centres<T>(fres, fcnt, 1, (int)d, nullptr, true, n, cen, s);
     launch_bk_dist<T>(x, (int)d, perm, n, cen, lab, n, dist, n, 1, s);
@@ -1220,8 +1221,8 @@ fk_status bisecting_impl(fk_ctx *ctxp, const T *x_in, int64_t n, int64_t d, cons
         FK_CUDA(cudaMemcpyAsync(picks, hpicks.data(), sizeof(int) * 2 * (size_t)runs, cudaMemcpyHostToDevice, s));
         FK_CUDA(cudaMemcpyAsync(active, hact.data(), sizeof(int) * (size_t)runs, cudaMemcpyHostToDevice, s));
         launch_bk_pick<T>(x, (int)d, segp, picks, runs, cen, s);
-        launch_gather_rows<T>(x, (int)d, segp, m, xseg, s);
-        upload_sum_chains(xseg, runs, true);
+        launch_gather_columns<T>(x, (int)d, segp, m, xseg, s);
+        upload_sum_chains(xseg, m, 1, runs, true);
         FK_CUDA(cudaMemset2DAsync(lab, (size_t)n, 0, (size_t)m, (size_t)runs, s));
         int nact = runs;
         for (int64_t it = 0; it < p->max_iter && nact > 0; it++) {

@@ -367,6 +367,9 @@ void launch_labels_to_u64(const int32_t *l, int64_t n, uint64_t *out, cudaStream
 // counts = the running per-centre counts, shift_bits = max_c ||c - old||^2.
 template <typename T>
 void launch_gather_rows(const T *x, int d, const int32_t *idx, int64_t m, T *out, cudaStream_t s);
+// The same rows feature-major (out[j m + i]).
+template <typename T>
+void launch_gather_columns(const T *x, int d, const int32_t *idx, int64_t m, T *out, cudaStream_t s);
 template <typename T>
 void launch_minibatch_update(const T *xb, const int32_t *labels, int64_t m, int d, int k, T *centres, T *old,
                              long long *counts, unsigned long long *shift_bits, cudaStream_t s);

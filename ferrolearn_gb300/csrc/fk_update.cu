@@ -1177,6 +1177,26 @@ __global__ void gather_rows_kernel(const T *__restrict__ x, int d, const int32_t
     }
 }
 
+// The rows idx[0 .. m) of x feature-major: out[j m + i] = x[idx[i] d + j], a
+// 32 x 32 tile a block (the folds of a segment's features read them in row
+// order: adjacent here, d values apart in x).
+template <typename T>
+__global__ void gather_columns_kernel(const T *__restrict__ x, int d, const int32_t *__restrict__ idx, int64_t m,
+                                      T *__restrict__ out) {
+    __shared__ T tile[32][33];
+    const int64_t i0 = (int64_t)blockIdx.x * 32;
+    const int j0 = (int)blockIdx.y * 32;
+    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
+        const int j = j0 + (int)threadIdx.x;
+        if (i0 + r < m && j < d) tile[r][threadIdx.x] = x[(int64_t)idx[i0 + r] * d + j];
+    }
+    __syncthreads();
+    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
+        const int64_t i = i0 + threadIdx.x;
+        if (i < m && j0 + r < d) out[(int64_t)(j0 + r) * m + i] = tile[threadIdx.x][r];
+    }
+}
+
 // update_centers_mini_batch (mini_batch_kmeans.rs:410-447): one block per
 // centre. Every thread walks the whole batch in order (the labels staged in
 // shared memory, so the test is uniform across the block) and owns fixed
@@ -1346,6 +1366,14 @@ void launch_gather_rows(const T *x, int d, const int32_t *idx, int64_t m, T *out
 }
 
 template <typename T>
+void launch_gather_columns(const T *x, int d, const int32_t *idx, int64_t m, T *out, cudaStream_t s) {
+    if (m == 0 || d == 0) return;
+    gather_columns_kernel<T><<<dim3((unsigned)((m + 31) / 32), (unsigned)((d + 31) / 32)), dim3(32, 8), 0, s>>>(x, d, idx,
+                                                                                                            m, out);
+    FK_LAUNCH_CHECK();
+}
+
+template <typename T>
 void launch_minibatch_update(const T *xb, const int32_t *labels, int64_t m, int d, int k, T *centres, T *old,
                              long long *counts, unsigned long long *shift_bits, cudaStream_t s) {
     FK_CUDA(cudaMemsetAsync(shift_bits, 0, sizeof(unsigned long long), s));
@@ -1437,6 +1465,8 @@ template void launch_bk_dist<float>(const float *, int, const int32_t *, int64_t
                                     int64_t, float *, int64_t, int, cudaStream_t);
 
 template void launch_gather_rows<double>(const double *, int, const int32_t *, int64_t, double *, cudaStream_t);
+template void launch_gather_columns<double>(const double *, int, const int32_t *, int64_t, double *, cudaStream_t);
+template void launch_gather_columns<float>(const float *, int, const int32_t *, int64_t, float *, cudaStream_t);
 template void launch_gather_rows<float>(const float *, int, const int32_t *, int64_t, float *, cudaStream_t);
 template void launch_minibatch_update<double>(const double *, const int32_t *, int64_t, int, int, double *, double *,
                                               long long *, unsigned long long *, cudaStream_t);
