@@ -278,7 +278,7 @@ template <typename TX, typename TC>
 void lloyd_iteration(Ctx &ctx, const TX *x, int64_t n, int d, const TC *c, int k, int prec, TC *nc,
                      int32_t *labels, DevScalars *sc, const SortPlan &plan, bool x_changed, fk_fit_report *rep,
                      bool timing, int mode = UPDATE_FULL, const int32_t *prev_labels = nullptr,
-                     const TC *prev_c = nullptr) {
+                     const TC *prev_c = nullptr, bool pruned = false) {
     cudaStream_t s = ctx.stream;
     int32_t *members = (int32_t *)ctx.get(BUF_MEMBERS, sizeof(int32_t) * (size_t)n);
     int32_t *seg = (int32_t *)ctx.get(BUF_SEGHIST, sizeof(int32_t) * (size_t)plan.k * plan.nseg);
@@ -289,7 +289,11 @@ void lloyd_iteration(Ctx &ctx, const TX *x, int64_t n, int d, const TC *c, int k
     ctx.count_acc = (timing && rep) ? &rep->ms_count_pass : nullptr;
     {
         Timer t(timing, ctx, rep ? &rep->ms_assign : nullptr);
-        if (prec == FK_PRECISION_PLAIN) {
+        if (pruned) {
+            // a fit's labels alone: its inertia is formed once, at its end
+            if constexpr (std::is_same<TX, TC>::value)
+                launch_assign_pruned<TC>(ctx, x, n, d, c, prev_c, k, prev_labels, labels, x_changed);
+        } else if (prec == FK_PRECISION_PLAIN) {
             TC *mind = (TC *)ctx.get(BUF_MIND, sizeof(TC) * (size_t)n);
             double *part = (double *)ctx.get(BUF_PARTIAL, sizeof(double) * (size_t)sum_fixed_partials(n));
             if constexpr (std::is_same<TX, double>::value && std::is_same<TC, double>::value)
@@ -490,6 +494,8 @@ fk_status fit_impl(fk_ctx *ctxp, const TX *x_in, int64_t n, int64_t d, const fk_
     // are updated from the rows whose label changed. Decided once the first
     // preparation has shown X finite and inside the split's exponent range.
     bool inc_candidate = false, incremental = false;
+    // Plain forms of some size: centres that cannot win are left out
+    const bool prune = std::is_same<TX, TC>::value && p->precision == FK_PRECISION_PLAIN && prune_shape_ok(n, (int)d, (int)k);
     if constexpr (std::is_same<TX, float>::value && std::is_same<TC, double>::value)
         inc_candidate = p->precision != FK_PRECISION_PLAIN && incremental_shape_ok((const float *)x, (int)d);
     for (int64_t run = 0; run < p->n_init; run++) {
@@ -569,7 +575,8 @@ fk_status fit_impl(fk_ctx *ctxp, const TX *x_in, int64_t n, int64_t d, const fk_
             auto iteration = [&] {
                 lloyd_iteration<TX, TC>(ctx, x, n, (int)d, cb3[it % 3], (int)k, p->precision, cb3[(it + 1) % 3],
                                         labels2 + (size_t)par * n, sc, plan, x_changed, rep, timing, mode,
-                                        labels2 + (size_t)(par ^ 1) * n, count ? cb3[(it + 2) % 3] : nullptr);
+                                        labels2 + (size_t)(par ^ 1) * n,
+                                        count || (prune && it > 0) ? cb3[(it + 2) % 3] : nullptr, prune);
             };
             if (!timing && !x_changed && it >= 2) {
                 // steady state: the memset, the iteration and the scalars' copy as one graph
@@ -614,6 +621,16 @@ fk_status fit_impl(fk_ctx *ctxp, const TX *x_in, int64_t n, int64_t d, const fk_
             // the kept assignment, against its centres cb3[(n_iter - 1) % 3]
             if constexpr (std::is_same<TX, float>::value && std::is_same<TC, double>::value) {
                 launch_row_inertia(ctx, x, n, (int)d, labels, cb3[(n_iter - 1) % 3], (int)k, sc);
+                read_scalars(ctx, sc);
+                inertia = (TC)ctx.host_scalars->inertia;
+            }
+        }
+        if constexpr (std::is_same<TX, TC>::value) {
+            if (prune && n_iter > 0) {
+                TC *mind = (TC *)ctx.get(BUF_MIND, sizeof(TC) * (size_t)n);
+                double *part = (double *)ctx.get(BUF_PARTIAL, sizeof(double) * (size_t)sum_fixed_partials(n));
+                launch_label_dist<TC>(ctx, x, n, (int)d, cb3[(n_iter - 1) % 3], labels, mind);
+                launch_sum_fixed<TC>(mind, n, part, &sc->inertia, s);
                 read_scalars(ctx, sc);
                 inertia = (TC)ctx.host_scalars->inertia;
             }

@@ -159,7 +159,7 @@ enum BufSlot {
     BUF_FOLD_MAP, BUF_MASKS, BUF_THRESH, BUF_FLOORS, BUF_SHIFT, BUF_THMAIN, BUF_TH2, BUF_CNT2, BUF_LIST3,
     BUF_SLOT3, BUF_TH3, BUF_XB3,
     BUF_BX, BUF_BFITS, BUF_BSTATE, BUF_BITEMS, BUF_BPART, BUF_BORDER, BUF_BCTR, BUF_BLAB, BUF_BMEM, BUF_BCEN, BUF_BXOFF, BUF_BSUMS,
-    BUF_KPPC,
+    BUF_KPPC, BUF_PR_UB, BUF_PR_SHIFT, BUF_PR_NEAR, BUF_PR_LIST,
     BUF_PF_X32, BUF_PF_XERR, BUF_PF_C32, BUF_PF_CERR, BUF_PF_LIST, BUF_PF_CNT,
     BUF_COUNT
 };
@@ -304,6 +304,20 @@ void launch_transform_direct(const T *x, int64_t n, int d, const T *c, int k, T 
 // (its f32 copy is rebuilt).
 void launch_assign_f64_filtered(Ctx &ctx, const double *x, int64_t n, int d, const double *c, int k,
                                 int32_t *labels, double *mind, bool fresh_x);
+// The plain assignment of a fit's iteration (fk_prune.cu): the labels of
+// launch_assign_direct<F, F>, without the distances. c_prev null: the first
+// iteration, every centre for every row; else prev are the labels against
+// c_prev, and the context's bounds are those the call before left.
+bool prune_shape_ok(int64_t n, int d, int k);
+template <typename F>
+void launch_assign_pruned(Ctx &ctx, const F *x, int64_t n, int d, const F *c, const F *c_prev, int k,
+                          const int32_t *prev, int32_t *labels, bool fresh_x);
+// Each row's direct-form distance to its label, F::MAX where it is not below.
+template <typename F>
+void launch_label_dist(Ctx &ctx, const F *x, int64_t n, int d, const F *c, const int32_t *labels, F *mind);
+// The FP64 direct form over every centre for the listed rows (fk_prefilter.cu).
+void launch_f64_open_rows(Ctx &ctx, const double *x, int d, const double *c, int k, const int32_t *list,
+                          const unsigned long long *count, int32_t *labels);
 // f32 copies of f64 rows and an upper bound of the norm of each row's
 // rounding error (the inputs of the FP32 bounds).
 void launch_f32_copy(Ctx &ctx, const double *x, int64_t n, int d, float *x32, float *err);

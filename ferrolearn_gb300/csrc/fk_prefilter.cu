@@ -270,6 +270,12 @@ void launch_f32_copy(Ctx &ctx, const double *x, int64_t n, int d, float *x32, fl
     FK_LAUNCH_CHECK();
 }
 
+void launch_f64_open_rows(Ctx &ctx, const double *x, int d, const double *c, int k, const int32_t *list,
+                          const unsigned long long *count, int32_t *labels) {
+    f64_open_rows_kernel<<<ctx.num_sms * 8, 256, 0, ctx.stream>>>(x, d, c, k, list, count, labels, nullptr);
+    FK_LAUNCH_CHECK();
+}
+
 void launch_assign_f64_filtered(Ctx &ctx, const double *x, int64_t n, int d, const double *c, int k,
                                 int32_t *labels, double *mind, bool fresh_x) {
     if (n == 0) return;
@@ -279,7 +285,7 @@ void launch_assign_f64_filtered(Ctx &ctx, const double *x, int64_t n, int d, con
     float *c32 = (float *)ctx.get(BUF_PF_C32, sizeof(float) * (size_t)k * d);
     float *cerr = (float *)ctx.get(BUF_PF_CERR, sizeof(float) * (size_t)k);
     int32_t *open_list = (int32_t *)ctx.get(BUF_PF_LIST, sizeof(int32_t) * (size_t)n);
-    unsigned long long *open_count = (unsigned long long *)ctx.get(BUF_PF_CNT, sizeof(unsigned long long));
+    unsigned long long *open_count = (unsigned long long *)ctx.get(BUF_PF_CNT, sizeof(unsigned long long) * 4);
     const int grid_rows = ctx.num_sms * 8;
     if (fresh_x) {
         f32_copy_rows_kernel<<<grid_rows, 256, 0, s>>>(x, n, d, x32, xerr);
