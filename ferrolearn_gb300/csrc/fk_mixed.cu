@@ -85,10 +85,14 @@ __global__ void col_mean_partial_kernel(const TX *__restrict__ x, int64_t n, int
 
 __global__ void col_mean_final_kernel(const double *__restrict__ part, int nparts, int64_t rows, int d,
                                       double *__restrict__ mu, float *__restrict__ mu32) {
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
+    // one warp per column: the lanes' sums side by side (1,024 dependent FP64
+    // additions a column took 128 us)
+    const int j = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (j >= d) return;
     double s = 0.0;
-    for (int p = 0; p < nparts; p++) s += part[(int64_t)p * d + j];
+    for (int p = lane; p < nparts; p += 32) s += part[(int64_t)p * d + j];
+    s = warp_sum_d(s);
+    if (lane != 0) return;
     float m = (float)(s / (double)rows);
     if (!isfinite(m)) m = 0.f;
     mu32[j] = m;
@@ -101,15 +105,17 @@ template <typename TX>
 __global__ void sample_tmax_kernel(const TX *__restrict__ x, int64_t n, int d, int64_t stride, int64_t rows,
                                    const float *__restrict__ mu32, MixedStats *stats) {
     float m = 0.f;
-    const int64_t total = rows * (int64_t)d;
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t i = (e / d) * stride;
-        const int j = (int)(e % d);
-        if (i < n) {
-            const float t = fabsf(__fsub_rn((float)x[i * d + j], mu32[j]));
+    // a warp per row
+    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows && r * stride < n; r += nw) {
+        const TX *row = x + r * stride * d;
+#pragma unroll 4
+        for (int j = threadIdx.x & 31; j < d; j += 32) {
+            const float t = fabsf(__fsub_rn((float)row[j], mu32[j]));
             if (t < INFINITY) m = fmaxf(m, t);
         }
     }
+    __syncwarp();
 #pragma unroll
     for (int off = 16; off >= 1; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
     if ((threadIdx.x & 31) == 0 && m > 0.f) atomicMax((unsigned int *)&stats->tmax, __float_as_uint(m));
@@ -1569,88 +1575,81 @@ __global__ void gather_xq_rows_kernel(const uint4 *__restrict__ xq, int pieces, 
     }
 }
 
-// The FP64 decisions: one warp per queued row stages the widened row and its
-// candidate centres (rows padded by one double) in shared memory, then lane
-// j < m sums candidate j in the oracle's order (sqeuc64's arithmetic from
-// shared memory, so the dependent FP64 additions are the only wait); the
-// lowest distance below F::MAX wins, the lowest index on ties, else label 0,
-// exactly as nearest_center.
+// The FP64 decisions: a warp takes 32 queued rows, forms their (row, candidate)
+// pairs -- two a row mostly -- and sums 32 pairs at a time, one a lane, in the
+// oracle's order; then each row's lowest distance below F::MAX wins, the lowest
+// index on ties, else label 0, exactly as nearest_center. An FP64 addition
+// takes 64 cycles for one lane or for 32: with a warp a row, two of its lanes at
+// work, 200,000 rows of 256 features took 3.4 ms.
 constexpr int F64_WARPS = 4;
-size_t f64_smem_bytes(int d) { return sizeof(double) * (size_t)F64_WARPS * ((size_t)d + 8 * ((size_t)d + 1)); }
+constexpr int F64_ITEMS = 32;  // rows a warp takes at a time
 
 template <typename TX>
 __global__ void __launch_bounds__(F64_WARPS * 32)
     f64_decide_kernel(const TX *__restrict__ x, int d, const double *__restrict__ c, const Oct *__restrict__ items,
                       DevScalars *sc, int32_t *__restrict__ labels) {
-    extern __shared__ double f64_smem[];
+    __shared__ int first_s[F64_WARPS][F64_ITEMS + 1];  // a row's first pair
+    __shared__ double dist_s[F64_WARPS][F64_ITEMS * 8];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    double *xs = f64_smem + (size_t)w * ((size_t)d + 8 * ((size_t)d + 1)), *cs = xs + d;
+    int *first = first_s[w];
+    double *dist = dist_s[w];
     const unsigned long long cnt = sc->f64_count;
+    // few rows: fewer to a warp, so that every SM gets some
     const unsigned long long nw = (unsigned long long)gridDim.x * F64_WARPS;
-    for (unsigned long long q = (unsigned long long)blockIdx.x * F64_WARPS + w; q < cnt; q += nw) {
-        const Oct it = items[q];
-        for (int j = lane; j < d; j += 32) xs[j] = (double)x[(int64_t)it.row * d + j];
-        int my_id = INT32_MAX;
+    const int per = (int)min((unsigned long long)F64_ITEMS, max(1ull, (cnt + nw - 1) / nw));
+    for (unsigned long long q0 = ((unsigned long long)blockIdx.x * F64_WARPS + w) * per; q0 < cnt; q0 += nw * per) {
+        const int rows = (int)min((unsigned long long)per, cnt - q0);
+        int m = lane < rows ? items[q0 + lane].m : 0;
+        int incl = m;
 #pragma unroll
-        for (int t = 0; t < 8; t++)
-            if (t < it.m && t == lane) my_id = it.ids[t];
-        // the candidates' rows as one flat index space, so every load of the
-        // staging is independent of the others
-        const int md = it.m * d;
-        for (int e = lane; e < md; e += 32) {
-            const int t = e / d, j = e - t * d;
-            int id = it.ids[0];
+        for (int off = 1; off < 32; off <<= 1) {
+            const int o = __shfl_up_sync(0xffffffffu, incl, off);
+            if (lane >= off) incl += o;
+        }
+        first[lane + 1] = incl;
+        if (lane == 0) first[0] = 0;
+        const int pairs = __shfl_sync(0xffffffffu, incl, 31);
+        __syncwarp();
+        for (int p0 = 0; p0 < pairs; p0 += 32) {
+            const int p = p0 + lane;
+            if (p < pairs) {
+                int r = 0;  // the row of pair p
 #pragma unroll
-            for (int u = 1; u < 8; u++)
-                if (u == t) id = it.ids[u];
-            cs[(size_t)t * (d + 1) + j] = c[(int64_t)id * d + j];
+                for (int step = 16; step >= 1; step >>= 1)
+                    if (first[r + step] <= p) r += step;
+                const Oct &it = items[q0 + r];
+                dist[p] = sqeuc64<TX>(x + (int64_t)it.row * d, c + (int64_t)it.ids[p - first[r]] * d, d);
+            }
         }
         __syncwarp();
-        double v = DBL_MAX;
-        int id = INT32_MAX;
-        if (lane < it.m) {
-            const double *cr = cs + (size_t)lane * (d + 1);
-            double acc = 0.0;
-#pragma unroll 8
-            for (int j = 0; j < d; j++) {  // unrolled: the loads and squares run ahead of the add chain
-                const double t = __dsub_rn(xs[j], cr[j]);
-                acc = __dadd_rn(acc, __dmul_rn(t, t));
+        if (lane < rows) {
+            const Oct &it = items[q0 + lane];
+            double v = DBL_MAX, b2 = DBL_MAX;
+            int id = INT32_MAX;
+            for (int t = 0; t < m; t++) {
+                const double ov = dist[first[lane] + t];
+                const int oi = it.ids[t];
+                if (!(ov < DBL_MAX)) continue;  // not below F::MAX (or NaN): never chosen
+                if (ov < v || (ov == v && oi < id)) {
+                    b2 = v;
+                    v = ov;
+                    id = oi;
+                } else if (ov < b2) {
+                    b2 = ov;
+                }
             }
-            if (acc < DBL_MAX) {  // not below F::MAX (or NaN): never chosen
-                v = acc;
-                id = my_id;
-            }
-        }
-        double b2 = DBL_MAX;
-#pragma unroll
-        for (int off = 16; off >= 1; off >>= 1) {
-            const double ov = __shfl_xor_sync(0xffffffffu, v, off);
-            const int oi = __shfl_xor_sync(0xffffffffu, id, off);
-            const double ob2 = __shfl_xor_sync(0xffffffffu, b2, off);
-            if (ov < v || (ov == v && oi < id)) {
-                b2 = fmin(v, ob2);
-                v = ov;
-                id = oi;
-            } else {
-                b2 = fmin(b2, ov);
-            }
-        }
-        if (lane == 0) {
             labels[it.row] = id == INT32_MAX ? 0 : id;
-            atomicAdd(&sc->recheck_rows, 1ULL);
             if (id != INT32_MAX && b2 < DBL_MAX && near_tie(v, b2)) atomicAdd(&sc->near_tie_rows, 1ULL);
         }
-        __syncwarp();  // the staging area is reused for the next row
+        if (lane == 0) atomicAdd(&sc->recheck_rows, (unsigned long long)rows);
+        __syncwarp();  // the pairs' space is reused
     }
 }
 
 template <typename TX>
 void launch_f64_decide(Ctx &ctx, const TX *x, int d, const double *c, const Oct *items, DevScalars *sc,
                        int32_t *labels) {
-    const size_t smem = f64_smem_bytes(d);
-    FK_CUDA(cudaFuncSetAttribute((const void *)f64_decide_kernel<TX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
-    f64_decide_kernel<TX><<<ctx.num_sms * 2, F64_WARPS * 32, smem, ctx.stream>>>(x, d, c, items, sc, labels);
+    f64_decide_kernel<TX><<<ctx.num_sms * 4, F64_WARPS * 32, 0, ctx.stream>>>(x, d, c, items, sc, labels);
     FK_LAUNCH_CHECK();
 }
 
@@ -1746,10 +1745,10 @@ MixedBufs prepare_mixed(Ctx &ctx, const TX *x, int64_t n, int d, const double *c
         dim3 g1(nparts, (d + 127) / 128);
         col_mean_partial_kernel<TX><<<g1, 128, 0, s>>>(x, n, d, rows_per, stride, part);
         FK_LAUNCH_CHECK();
-        col_mean_final_kernel<<<(d + 127) / 128, 128, 0, s>>>(part, nparts, rows, d, B.mu, B.mu32);
+        col_mean_final_kernel<<<(d + 3) / 4, 128, 0, s>>>(part, nparts, rows, d, B.mu, B.mu32);
         FK_LAUNCH_CHECK();
         if (fp8) {
-            sample_tmax_kernel<TX><<<ctx.num_sms * 2, 256, 0, s>>>(x, n, d, stride, rows, B.mu32, B.stats);
+            sample_tmax_kernel<TX><<<ctx.num_sms * 8, 256, 0, s>>>(x, n, d, stride, rows, B.mu32, B.stats);
             FK_LAUNCH_CHECK();
         }
         if (fp8)
