@@ -964,8 +964,8 @@ fk_status minibatch_impl(fk_ctx *ctxp, const T *x_in, int64_t n, int64_t d, cons
     int32_t *didx = (int32_t *)ctx.get(BUF_MB_IDX, sizeof(int32_t) * (size_t)std::max(m * chunk, k));
     T *xb = (T *)ctx.get(BUF_MB_XB, sizeof(T) * (size_t)m * d);
     int32_t *blab = (int32_t *)ctx.get(BUF_MB_LAB, sizeof(int32_t) * (size_t)m);
-    // a batch is too few rows to fill the GPU by row tiles: split the centres too
-    const int splits = assign_splits<T>(m, (int)k, ctx.num_sms);
+    // f32: a batch is too few rows to fill the GPU by row tiles, so the centres are split too
+    const int splits = std::is_same<T, float>::value ? assign_splits<T>(m, (int)k, ctx.num_sms) : 1;
     T *part_v = splits > 1 ? (T *)ctx.get(BUF_MB_PARTV, sizeof(T) * (size_t)splits * m) : nullptr;
     int32_t *part_i = splits > 1 ? (int32_t *)ctx.get(BUF_MB_PARTI, sizeof(int32_t) * (size_t)splits * m) : nullptr;
     std::vector<int32_t> hidx;
@@ -1023,8 +1023,13 @@ fk_status minibatch_impl(fk_ctx *ctxp, const T *x_in, int64_t n, int64_t d, cons
             FK_CUDA(cudaMemcpyAsync(didx, hidx.data(), sizeof(int32_t) * (size_t)(ci * m), cudaMemcpyHostToDevice, s));
             for (int64_t q = 0; q < ci; q++) {
                 launch_gather_rows<T>(x, (int)d, didx + q * m, m, xb, s);
-                launch_assign_direct_split<T, T>(xb, m, (int)d, c, (int)k, blab, nullptr, splits, part_v, part_i, s);
-                launch_minibatch_update<T>(xb, blab, m, (int)d, (int)k, c, old, counts, &sc->shift_bits, s);
+                if constexpr (std::is_same<T, double>::value)
+                    launch_assign_f64_filtered(ctx, xb, m, (int)d, c, (int)k, blab, nullptr, true);
+                else
+                    launch_assign_direct_split<T, T>(xb, m, (int)d, c, (int)k, blab, nullptr, splits, part_v, part_i, s);
+                // the shift is formed where the early stop reads it
+                launch_minibatch_update<T>(xb, blab, m, (int)d, (int)k, c, old, counts,
+                                           tol > T(0) ? &sc->shift_bits : nullptr, s);
                 n_iter += 1;
                 if (tol > T(0)) {
                     FK_CUDA(cudaMemcpyAsync(&ctx.host_scalars->shift_bits, &sc->shift_bits, sizeof(unsigned long long),

@@ -378,7 +378,8 @@ void launch_labels_to_u64(const int32_t *l, int64_t n, uint64_t *out, cudaStream
 // MiniBatchKMeans (mini_batch_kmeans.rs): rows idx[0..m) of x into out
 // (m x d), and update_centers_mini_batch (:410-447) for one batch -- the
 // centres updated in place in batch order, old = the centres before it,
-// counts = the running per-centre counts, shift_bits = max_c ||c - old||^2.
+// counts = the running per-centre counts, shift_bits (nullable) = max_c ||c -
+// old||^2.
 template <typename T>
 void launch_gather_rows(const T *x, int d, const int32_t *idx, int64_t m, T *out, cudaStream_t s);
 // The same rows feature-major (out[j m + i]).

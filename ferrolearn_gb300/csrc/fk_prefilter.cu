@@ -203,6 +203,95 @@ __global__ void __launch_bounds__(PNT)
     }
 }
 
+// The same decisions for few rows: 16 rows a block (1,024 rows are 64 blocks
+// where 128-row tiles are 8), a thread four rows and one centre of a 64-centre
+// tile, 32 features staged at a time.
+constexpr int FBM = 16;  // rows per block
+constexpr int FBN = 64;  // centres per tile
+constexpr int FDJ = 32;  // features staged
+
+__global__ void __launch_bounds__(PNT)
+    f32_filter_few_kernel(const float *__restrict__ x32, const float *__restrict__ xerr, int64_t n, int d,
+                          const float *__restrict__ c32, const float *__restrict__ cerr, int k,
+                          int32_t *__restrict__ labels, int32_t *__restrict__ open_list,
+                          unsigned long long *__restrict__ open_count) {
+    constexpr int RPT = FBM * FBN / PNT;  // rows per thread
+    __shared__ float xs[FDJ][FBM];
+    __shared__ float cs[FDJ][FBN + 1];
+    __shared__ RowBound part[2][FBM];
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int tc = tid % FBN, tr = tid / FBN;  // a warp: 32 centres, one row group
+    const int64_t row0 = (int64_t)blockIdx.x * FBM;
+    RowBound rb[RPT];
+    float ex[RPT];
+#pragma unroll
+    for (int a = 0; a < RPT; a++) {
+        rb[a] = RowBound{INFINITY, INFINITY, INFINITY, -1, false};
+        const int64_t gr = row0 + tr * RPT + a;
+        ex[a] = gr < n ? xerr[gr] : 0.f;
+    }
+    for (int ct = 0; ct < k; ct += FBN) {
+        float acc[RPT];
+#pragma unroll
+        for (int a = 0; a < RPT; a++) acc[a] = 0.f;
+        for (int j0 = 0; j0 < d; j0 += FDJ) {
+            for (int e = tid; e < FBM * FDJ; e += PNT) {
+                const int r = e / FDJ, j = e % FDJ;
+                xs[j][r] = row0 + r < n && j0 + j < d ? x32[(row0 + r) * d + j0 + j] : 0.f;
+            }
+#pragma unroll
+            for (int e = tid; e < FBN * FDJ; e += PNT) {
+                const int r = e / FDJ, j = e % FDJ;
+                cs[j][r] = ct + r < k && j0 + j < d ? c32[(int64_t)(ct + r) * d + j0 + j] : 0.f;
+            }
+            __syncthreads();
+            const int jn = min(FDJ, d - j0);
+#pragma unroll 8
+            for (int j = 0; j < jn; j++) {
+                const float cv = cs[j][tc];
+#pragma unroll
+                for (int a = 0; a < RPT; a++) {
+                    const float t = xs[j][tr * RPT + a] - cv;
+                    acc[a] = fmaf(t, t, acc[a]);
+                }
+            }
+            __syncthreads();
+        }
+        const int gc = ct + tc;
+        if (gc < k) {
+            const float ec = cerr[gc];
+#pragma unroll
+            for (int a = 0; a < RPT; a++) {
+                const float bnd = bound32(acc[a], __fadd_ru(ex[a], ec), d);
+                rb_add(rb[a], __fsub_rd(acc[a], bnd), __fadd_ru(acc[a], bnd), gc);
+            }
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < RPT; a++) {
+        RowBound r = rb[a];
+#pragma unroll
+        for (int off = 16; off >= 1; off >>= 1) {
+            RowBound o;
+            o.ua = __shfl_xor_sync(0xffffffffu, r.ua, off);
+            o.la = __shfl_xor_sync(0xffffffffu, r.la, off);
+            o.lb2 = __shfl_xor_sync(0xffffffffu, r.lb2, off);
+            o.ia = __shfl_xor_sync(0xffffffffu, r.ia, off);
+            o.bad = __shfl_xor_sync(0xffffffffu, (int)r.bad, off) != 0;
+            rb_merge(r, o);
+        }
+        if (lane == 0) part[tc / 32][tr * RPT + a] = r;
+    }
+    __syncthreads();
+    if (tid < FBM && row0 + tid < n) {
+        RowBound r = part[0][tid];
+        rb_merge(r, part[1][tid]);
+        const bool decided = !r.bad && r.ia >= 0 && r.lb2 > r.ua;
+        labels[row0 + tid] = decided ? r.ia : -1;
+        if (!decided) open_list[atomicAdd(open_count, 1ULL)] = (int32_t)(row0 + tid);
+    }
+}
+
 // FP64 direct form of row x against centre c, in the reference's order.
 __device__ __forceinline__ double sqeuc64_rn(const double *__restrict__ x, const double *__restrict__ c, int d) {
     double acc = 0.0;
@@ -294,8 +383,14 @@ void launch_assign_f64_filtered(Ctx &ctx, const double *x, int64_t n, int d, con
     f32_copy_rows_kernel<<<(unsigned)std::min<int64_t>((k + 7) / 8, grid_rows), 256, 0, s>>>(c, k, d, c32, cerr);
     FK_LAUNCH_CHECK();
     FK_CUDA(cudaMemsetAsync(open_count, 0, sizeof(unsigned long long), s));
-    f32_filter_kernel<<<(unsigned)((n + PBM - 1) / PBM), PNT, 0, s>>>(x32, xerr, n, d, c32, cerr, k, labels,
-                                                                      open_list, open_count);
+    // 128-row tiles read the centres least often; below one tile an SM the small
+    // ones fill the chip (1,024 rows, k = 256, d = 64)
+    if ((n + PBM - 1) / PBM < ctx.num_sms)
+        f32_filter_few_kernel<<<(unsigned)((n + FBM - 1) / FBM), PNT, 0, s>>>(x32, xerr, n, d, c32, cerr, k, labels,
+                                                                              open_list, open_count);
+    else
+        f32_filter_kernel<<<(unsigned)((n + PBM - 1) / PBM), PNT, 0, s>>>(x32, xerr, n, d, c32, cerr, k, labels,
+                                                                          open_list, open_count);
     FK_LAUNCH_CHECK();
     if (mind) {
         f64_label_dist_kernel<<<grid_rows, 256, 0, s>>>(x, n, d, c, labels, mind);

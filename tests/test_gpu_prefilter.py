@@ -74,3 +74,13 @@ def test_prefilter_dirichlet_shape_steps_and_fit():
     assert np.array_equal(g.cluster_centers(), o["centers"])
     assert abs(g.inertia() - o["inertia"]) <= 1e-12 * o["inertia"]
     assert gl.shape[0] == x.shape[0]
+
+
+@pytest.mark.parametrize("n,d,k", [(1, 1, 1), (15, 33, 63), (16, 32, 64), (17, 31, 65), (1023, 64, 129), (4000, 100, 8)])
+def test_few_rows_match_oracle(n, d, k):
+    # fewer 128-row tiles than SMs: the 16-row kernel, at the edges of its tiles; a grid makes exact ties
+    rng = np.random.default_rng(n + d + k)
+    for x, c in ((rng.normal(size=(n, d)), rng.normal(size=(k, d))),
+                 (rng.integers(-1, 2, size=(n, d)) * 1.0, rng.integers(-1, 2, size=(k, d)) * 1.0)):
+        model = F.FittedKMeans(c, None, 0.0, 0, "f64")
+        assert np.array_equal(model.predict(x), O.predict(c, x))
