@@ -278,7 +278,7 @@ template <typename TX, typename TC>
 void lloyd_iteration(Ctx &ctx, const TX *x, int64_t n, int d, const TC *c, int k, int prec, TC *nc,
                      int32_t *labels, DevScalars *sc, const SortPlan &plan, bool x_changed, fk_fit_report *rep,
                      bool timing, int mode = UPDATE_FULL, const int32_t *prev_labels = nullptr,
-                     const TC *prev_c = nullptr, bool pruned = false) {
+                     const TC *prev_c = nullptr, bool pruned = false, int main = MAIN_TOP2) {
     cudaStream_t s = ctx.stream;
     int32_t *members = (int32_t *)ctx.get(BUF_MEMBERS, sizeof(int32_t) * (size_t)n);
     int32_t *seg = (int32_t *)ctx.get(BUF_SEGHIST, sizeof(int32_t) * (size_t)plan.k * plan.nseg);
@@ -303,7 +303,7 @@ void lloyd_iteration(Ctx &ctx, const TX *x, int64_t n, int d, const TC *c, int k
             launch_sum_fixed<TC>(mind, n, part, &sc->inertia, s);
         } else {
             if constexpr (std::is_same<TX, float>::value && std::is_same<TC, double>::value) {
-                run_assign_mixed(ctx, x, n, d, c, k, prec, labels, nullptr, sc, x_changed, prev_c,
+                run_assign_mixed(ctx, x, n, d, c, k, prec, labels, nullptr, sc, x_changed, main, prev_c,
                                  prev_c ? prev_labels : nullptr);
             }
         }
@@ -539,9 +539,18 @@ fk_status fit_impl(fk_ctx *ctxp, const TX *x_in, int64_t n, int64_t d, const fk_
         // second pass, or 0.2% to the exhaustive re-score, holds it off for
         // the next two iterations (the centres still move too much for the
         // carried bound).
+        // Larger fits keep row bounds from the top-2 pass instead, counting from
+        // the second iteration on how many rows they would keep; from the fourth
+        // on, once that is a sixth, the main pass is over the other rows. Where
+        // it is less by then, the fit goes on with the count pass.
         bool count_ok = false, calm = false;
         if constexpr (std::is_same<TX, float>::value && std::is_same<TC, double>::value)
             count_ok = p->precision == FK_PRECISION_MIXED_BF16 || p->precision == FK_PRECISION_MIXED_FP8;
+        bool bounds = false;  // this run's top-2 passes leave row bounds
+        if constexpr (std::is_same<TX, float>::value && std::is_same<TC, double>::value)
+            bounds = count_ok && mixed_bounds_ok(n, (int)d, (int)k);
+        bool was_listed = false;
+        int64_t kept = 0;  // rows kept, of the last iteration read
         bool was_count[2] = {false, false};
         int64_t count_from = FK_COUNT_FROM;
         auto finish = [&](int64_t r) {
@@ -552,6 +561,7 @@ fk_status fit_impl(fk_ctx *ctxp, const TX *x_in, int64_t n, int64_t d, const fk_
                 fail(FK_ERR_TIMEOUT);
             }
             calm = (int64_t)(h.flag_count + h.full_count) <= n / 4;
+            kept = (int64_t)h.kept_rows;
             if (was_count[r & 1] && ((int64_t)h.full_count > n / 10 || (int64_t)h.ex_count > n / 500))
                 count_from = std::max(count_from, r + 3);
             accumulate_report(rep, h, n);
@@ -560,30 +570,48 @@ fk_status fit_impl(fk_ctx *ctxp, const TX *x_in, int64_t n, int64_t d, const fk_
             return shift_from_bits<TC>(h.shift_bits) < (TC)p->tol;
         };
         bool stop = false;
-        int64_t launched = 0;
+        int64_t launched = 0, finished = 0;
+        auto finish_next = [&] {
+            if (finished < launched && !stop) stop = finish(finished++);
+        };
         for (int64_t it = 0; it < p->max_iter && !stop; it++) {
+            if (bounds && it == FK_COUNT_FROM) {
+                // the one choice that waits for the iteration before: whether its
+                // bounds keep enough rows
+                finish_next();
+                if (stop) break;
+            }
             const int par = (int)(it & 1);
             // the first two iterations move many rows (a third of them is
             // common in the second): the full pass is cheaper there
             const int mode = !inc_candidate ? UPDATE_FULL
                              : (it < 2 || !incremental) ? UPDATE_FULL_STATE
                                                         : UPDATE_INCREMENTAL;
-            const bool count = count_ok && calm && it >= count_from;
+            const bool pays = kept >= n / 6;
+            if (bounds && it >= FK_COUNT_FROM && (!pays || !reserve_listed(ctx, n, (int)d, p->precision))) bounds = false;
+            // (the count pass carries every row's floor: a pass over listed rows left the others' behind)
+            const bool count = count_ok && calm && it >= count_from && !bounds && !was_listed;
+            const int main = bounds ? (it >= FK_COUNT_FROM ? MAIN_LISTED : MAIN_TOP2_BOUNDS)
+                             : count ? MAIN_COUNT
+                                     : MAIN_TOP2;
+            const bool with_prev = main == MAIN_COUNT || main == MAIN_LISTED || (main == MAIN_TOP2_BOUNDS && it > 0) ||
+                                   (prune && it > 0);
             was_count[par] = count;
+            was_listed = main == MAIN_LISTED;
             if (count && rep) rep->count_iterations++;
             // iteration it - 1 read cb3[(it + 2) % 3]; it is not overwritten before iteration it + 1
             auto iteration = [&] {
                 lloyd_iteration<TX, TC>(ctx, x, n, (int)d, cb3[it % 3], (int)k, p->precision, cb3[(it + 1) % 3],
                                         labels2 + (size_t)par * n, sc, plan, x_changed, rep, timing, mode,
                                         labels2 + (size_t)(par ^ 1) * n,
-                                        count || (prune && it > 0) ? cb3[(it + 2) % 3] : nullptr, prune);
+                                        with_prev ? cb3[(it + 2) % 3] : nullptr, prune, main);
             };
             if (!timing && !x_changed && it >= 2) {
                 // steady state: the memset, the iteration and the scalars' copy as one graph
                 // (phase timers record events, so timed fits run without graphs)
                 const uint64_t key[10] = {(uint64_t)(uintptr_t)x, (uint64_t)n, (uint64_t)d, (uint64_t)k,
                                           (uint64_t)p->precision, (uint64_t)(it % 6), (uint64_t)mode,
-                                          (uint64_t)count, (uint64_t)(uintptr_t)sc, sizeof(TX) * 16 + sizeof(TC)};
+                                          (uint64_t)main, (uint64_t)(uintptr_t)sc, sizeof(TX) * 16 + sizeof(TC)};
                 run_graphed(ctx, key, [&] {
                     FK_CUDA(cudaMemsetAsync(sc, 0, sizeof(DevScalars), s));
                     iteration();
@@ -592,7 +620,7 @@ fk_status fit_impl(fk_ctx *ctxp, const TX *x_in, int64_t n, int64_t d, const fk_
                 });
                 FK_CUDA(cudaEventRecord(iter_done[par], s));
                 launched = it + 1;
-                if (it > 0) stop = finish(it - 1);
+                if (finished < it) finish_next();
                 continue;
             }
             FK_CUDA(cudaMemsetAsync(sc, 0, sizeof(DevScalars), s));
@@ -610,7 +638,7 @@ fk_status fit_impl(fk_ctx *ctxp, const TX *x_in, int64_t n, int64_t d, const fk_
             FK_CUDA(cudaMemcpyAsync(&ctx.host_scalars[1 + par], sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, s));
             FK_CUDA(cudaEventRecord(iter_done[par], s));
             launched = it + 1;
-            if (it > 0) stop = finish(it - 1);
+            if (finished < it) finish_next();
         }
         if (!stop && launched > 0) finish(launched - 1);
         // the result of iteration n_iter - 1: centres in cb3[n_iter % 3]

@@ -65,6 +65,8 @@ struct DevScalars {
     unsigned long long moved_rows;  // incremental update: rows whose label changed
     unsigned long long incremental; // 1: this iteration's update was incremental
     unsigned long long mask_count;  // FP8 second pass: rows left to its mask pass
+    unsigned long long kept_rows;   // rows whose bounds keep their label (fits of some size)
+    unsigned long long listed_rows; // rows listed for the main pass
 };
 
 // --------------------------------------------------- mixed precision --
@@ -159,6 +161,7 @@ enum BufSlot {
     BUF_FOLD_MAP, BUF_MASKS, BUF_THRESH, BUF_FLOORS, BUF_SHIFT, BUF_THMAIN, BUF_TH2, BUF_CNT2, BUF_LIST3,
     BUF_SLOT3, BUF_TH3, BUF_XB3,
     BUF_BX, BUF_BFITS, BUF_BSTATE, BUF_BITEMS, BUF_BPART, BUF_BORDER, BUF_BCTR, BUF_BLAB, BUF_BMEM, BUF_BCEN, BUF_BXOFF, BUF_BSUMS,
+    BUF_XSQ, BUF_MX_UB, BUF_MX_NEAR, BUF_LROWS, BUF_LXB, BUF_LXAUG, BUF_LSCALE,
     BUF_KPPC, BUF_PR_UB, BUF_PR_SHIFT, BUF_PR_NEAR, BUF_PR_LIST,
     BUF_PF_X32, BUF_PF_XERR, BUF_PF_C32, BUF_PF_CERR, BUF_PF_LIST, BUF_PF_CNT,
     BUF_COUNT
@@ -185,6 +188,7 @@ struct Ctx {
     MixedPlan mixedm2; // its mask pass (BF16, the slicing of mixed2)
     MixedPlan mixedm;  // second pass (BF16, candidate masks) over the rows a BF16 main pass left open
     MixedPlan mixedc;  // count pass (main pass from the fourth iteration of a fit)
+    MixedPlan mixedl;  // top-2 pass over listed rows
     // Captured steady-state fit iterations (fk_capi.cu), keyed by what the
     // iteration's launches depend on; a buffer (re)allocation bumps buf_gen,
     // which retires them all (their pointers would be stale).
@@ -452,13 +456,21 @@ void run_kmeanspp(Ctx &ctx, std::vector<KppJob> &jobs, int64_t *draws_used);
 // Mixed-precision assignment (BF16 / FP8 tcgen05 approximate pass, FP32 and
 // FP64 exact re-check) of X stored as f32. Results identical to the FP64
 // direct form.
-// With c_prev and labels_prev (the previous iteration's centres and labels,
-// and this context's row floors from that iteration's pass), the main pass is
-// the count pass.
+// The main pass of an iteration: a top-2 ranking of every row (with bounds for
+// the next iteration where the fit keeps them, and a count of the rows that
+// the bounds of the last one would keep), the count pass against thresholds
+// carried from the last iteration, or a top-2 ranking of the rows that the
+// bounds do not keep. The last two, and the count, need the previous
+// iteration's centres and labels.
+enum MainPass { MAIN_TOP2 = 0, MAIN_TOP2_BOUNDS = 1, MAIN_COUNT = 2, MAIN_LISTED = 3 };
+bool mixed_bounds_ok(int64_t n, int d, int k);
+// The buffers of a listed pass; false when they cannot be allocated.
+bool reserve_listed(Ctx &ctx, int64_t n, int d, int precision);
 template <typename TX>
 void run_assign_mixed(Ctx &ctx, const TX *x, int64_t n, int d, const double *c, int k,
                       int precision, int32_t *labels, double *mind, DevScalars *scalars,
-                      bool x_changed, const double *c_prev = nullptr, const int32_t *labels_prev = nullptr);
+                      bool x_changed, int main = MAIN_TOP2, const double *c_prev = nullptr,
+                      const int32_t *labels_prev = nullptr);
 // Inertia of the mixed precisions: the per-(cluster, feature) partials of
 // the update pass folded in f64 (relative error about 1e-7).
 void launch_mixed_inertia(Ctx &ctx, const double *part, int64_t m, DevScalars *scalars);

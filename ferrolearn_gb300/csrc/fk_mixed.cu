@@ -194,8 +194,8 @@ template <typename TX, bool FP8>
 __global__ void prep_rows_kernel(const TX *__restrict__ x, int64_t n, int d, int d_pad,
                                  const float *__restrict__ mu32, void *__restrict__ xq_out,
                                  __nv_bfloat16 *__restrict__ xaug, float4 *__restrict__ rowinfo, MixedStats *stats,
-                                 const int32_t *__restrict__ list = nullptr,
-                                 const unsigned long long *count = nullptr) {
+                                 const int32_t *__restrict__ list, const unsigned long long *count,
+                                 float *__restrict__ xsq) {
     __shared__ float sh_xn[32], sh_am[32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
@@ -257,6 +257,7 @@ __global__ void prep_rows_kernel(const TX *__restrict__ x, int64_t n, int d, int
         float ex = __fadd_ru(__fsqrt_ru(__fmul_ru(ex2, up)), __fmul_ru(__fsqrt_ru(__fmul_ru(tn2, up)), 5.9604645e-08f));
         float xo = __fsqrt_ru(__fmul_ru(xo2, up));
         if (lane == 0) rowinfo[slot] = make_float4(xn, ex, xo, inv);
+        if (lane == 0 && xsq) xsq[slot] = tn2;
         if (FP8 && lane < 16)
             xaug[slot * 16 + lane] = lane < 3 ? __float2bfloat16_rn(inv) : __float2bfloat16_rn(0.f);
         if (xn < INFINITY) xn_hi = fmaxf(xn_hi, xn);  // NaN / inf rows are re-scored in full
@@ -305,7 +306,8 @@ template <bool FP8, int LPR>
 __global__ void prep_rows4_kernel(const float *__restrict__ x, int64_t n, int d, int d_pad,
                                   const float *__restrict__ mu32, void *__restrict__ xq_out,
                                   __nv_bfloat16 *__restrict__ xaug, float4 *__restrict__ rowinfo, MixedStats *stats,
-                                  const int32_t *__restrict__ list, const unsigned long long *count) {
+                                  const int32_t *__restrict__ list, const unsigned long long *count,
+                                  float *__restrict__ xsq) {
     constexpr int RPW = 32 / LPR;  // rows a warp
     constexpr int NPL = 4;         // 4-feature pieces a lane
     __shared__ float sh_xn[32], sh_am[32];
@@ -422,6 +424,7 @@ __global__ void prep_rows4_kernel(const float *__restrict__ x, int64_t n, int d,
         const float xo = __fsqrt_ru(__fmul_ru(xo2, up));
         if (ok) {
             if (sl == 0) rowinfo[slot] = make_float4(xn, ex, xo, inv);
+            if (sl == 0 && xsq) xsq[slot] = tn2;
             if (FP8) {
 #pragma unroll
                 for (int j = sl; j < 16; j += LPR)
@@ -458,21 +461,21 @@ __global__ void prep_rows4_kernel(const float *__restrict__ x, int64_t n, int d,
 template <typename TX, bool FP8>
 void launch_prep_rows(Ctx &ctx, const TX *x, int64_t n, int d, int d_pad, const float *mu32, void *xq,
                       __nv_bfloat16 *xaug, float4 *rowinfo, MixedStats *stats, const int32_t *list = nullptr,
-                      const unsigned long long *count = nullptr) {
+                      const unsigned long long *count = nullptr, float *xsq = nullptr) {
     const int64_t pblocks = std::min<int64_t>((n + 7) / 8, (int64_t)ctx.num_sms * 16);
     if (std::is_same<TX, float>::value && (d & 3) == 0 && d_pad <= 256 && ((uintptr_t)x & 15u) == 0) {
         // 8 lanes a row up to 128 features (4 rows a warp), else 16 (2 rows a warp)
         if (d_pad <= 128)
             prep_rows4_kernel<FP8, 8><<<(unsigned)std::min<int64_t>((n + 31) / 32, (int64_t)ctx.num_sms * 16), 256,
                                         0, ctx.stream>>>((const float *)x, n, d, d_pad, mu32, xq, xaug, rowinfo,
-                                                         stats, list, count);
+                                                         stats, list, count, xsq);
         else
             prep_rows4_kernel<FP8, 16><<<(unsigned)std::min<int64_t>((n + 15) / 16, (int64_t)ctx.num_sms * 16),
                                          256, 0, ctx.stream>>>((const float *)x, n, d, d_pad, mu32, xq, xaug, rowinfo,
-                                                               stats, list, count);
+                                                               stats, list, count, xsq);
     } else {
         prep_rows_kernel<TX, FP8><<<(unsigned)pblocks, 256, 0, ctx.stream>>>(x, n, d, d_pad, mu32, xq, xaug,
-                                                                             rowinfo, stats, list, count);
+                                                                             rowinfo, stats, list, count, xsq);
     }
     FK_LAUNCH_CHECK();
 }
@@ -653,6 +656,200 @@ __device__ __forceinline__ float row_floor(float v1, float key_slack, const floa
     return __fsub_rd(f, stats->big);
 }
 
+// ------------------------------------------------------ row bounds --
+// A fit of some size keeps, per row, ub >= d(x, c_label) and lb <= d(x, c) for
+// every other centre (exact distances). The next iteration's centres have
+// moved by at most their shifts D, so ub + D(label) and lb - max D of the others
+// bound the new distances; where they still separate, the label is the FP64
+// oracle's again and the row needs no pass.
+struct RowBounds {
+    const float *xsq;  // ||x'||^2, f32 sums of the rounded x'
+    float *ub, *lb;
+};
+
+// Relative error of xsq: the sum's roundings, and twice that of x' itself.
+__device__ __forceinline__ float xsq_rel(int d) { return (float)(d + 64) * 2.4e-7f; }
+
+// d(x, c) from the exact score S = BIG + (||x'||^2 - d^2) / 2: an upper bound
+// from a lower bound of S, and a lower bound from an upper bound of S.
+__device__ __forceinline__ float score_dist_up(float s_lo, float x2, float big, int d) {
+    const float sq = __fadd_ru(__fmul_ru(x2, 1.f + xsq_rel(d)), __fmul_ru(2.f, __fsub_ru(big, s_lo)));
+    return sq >= 0.f ? __fadd_ru(__fsqrt_ru(sq), 1e-20f) : (sq < 0.f ? 1e-20f : INFINITY);
+}
+__device__ __forceinline__ float score_dist_down(float s_hi, float x2, float big, int d) {
+    const float sq = __fadd_rd(__fmul_rd(x2, 1.f - xsq_rel(d)), __fmul_rd(2.f, __fsub_rd(big, s_hi)));
+    return sq > 0.f && sq < INFINITY ? __fsqrt_rd(sq) : 0.f;
+}
+
+// The same from FP32 distances with their bounds (pair re-score).
+__device__ __forceinline__ float pair_dist_up(float d32, float e) {
+    return __fadd_ru(__fsqrt_ru(__fadd_ru(d32, e)), 1e-20f);
+}
+__device__ __forceinline__ float pair_dist_down(float d32, float e) {
+    const float sq = __fsub_rd(d32, e);
+    return sq > 0.f && sq < INFINITY ? __fsqrt_rd(sq) : 0.f;
+}
+
+// A lower bound of each centre's squared distance to its nearest other centre
+// (near2, set to a large value before): 64 x 64 tiles of the upper triangle in
+// FP32 with the bound of the f32 copies' distances, 4 x 4 pairs a thread. 2 k^2 d / 2
+// operations: 0.1 ms at k = 4096, d = 256, less than 1% of a full pass.
+constexpr int NT_ = 64, NDJ = 16;
+__global__ void __launch_bounds__(256)
+    centre_near_kernel(const float *__restrict__ c32, const float *__restrict__ ec32, int k, int d,
+                       float *__restrict__ near2) {
+    if (blockIdx.y < blockIdx.x) return;
+    __shared__ __align__(16) float as[NDJ][NT_], bs[NDJ][NT_];
+    __shared__ unsigned rmin[NT_], cmin[NT_];
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int r0 = blockIdx.x * NT_, c0 = blockIdx.y * NT_;
+    if (tid < NT_) rmin[tid] = cmin[tid] = 0x7F7FFFFFu;
+    float acc[4][4];
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+        for (int b = 0; b < 4; b++) acc[a][b] = 0.f;
+    for (int j0 = 0; j0 < d; j0 += NDJ) {
+#pragma unroll
+        for (int e = tid; e < NT_ * NDJ; e += 256) {
+            const int r = e / NDJ, jj = e % NDJ, j = j0 + jj;
+            as[jj][r] = r0 + r < k && j < d ? c32[(int64_t)(r0 + r) * d + j] : 0.f;
+            bs[jj][r] = c0 + r < k && j < d ? c32[(int64_t)(c0 + r) * d + j] : 0.f;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int jj = 0; jj < NDJ; jj++) {  // features past d are zero in both
+            const float4 av = *reinterpret_cast<const float4 *>(&as[jj][4 * ty]);
+            const float4 bv = *reinterpret_cast<const float4 *>(&bs[jj][4 * tx]);
+            const float a4[4] = {av.x, av.y, av.z, av.w}, b4[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll
+            for (int a = 0; a < 4; a++)
+#pragma unroll
+                for (int b = 0; b < 4; b++) {
+                    const float t = a4[a] - b4[b];
+                    acc[a][b] = fmaf(t, t, acc[a][b]);
+                }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int a = 0; a < 4; a++) {
+        const int i = r0 + 4 * ty + a;
+        unsigned rm = 0x7F7FFFFFu;
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
+            const int q = c0 + 4 * tx + b;
+            if (i >= k || q >= k || i == q) continue;
+            const float e = bound32(acc[a][b], __fadd_ru(ec32[i], ec32[q]), d);
+            const float lo = __fsub_rd(acc[a][b], e);
+            const unsigned v = lo > 0.f ? min(__float_as_uint(lo), 0x7F7FFFFFu) : 0u;  // NaN: 0
+            rm = min(rm, v);
+            atomicMin(&cmin[4 * tx + b], v);
+        }
+        atomicMin(&rmin[4 * ty + a], rm);
+    }
+    __syncthreads();
+    if (tid < NT_) {
+        if (r0 + tid < k) atomicMin(reinterpret_cast<unsigned *>(near2) + r0 + tid, rmin[tid]);
+        if (c0 + tid < k) atomicMin(reinterpret_cast<unsigned *>(near2) + c0 + tid, cmin[tid]);
+    }
+}
+
+// Rows whose bounds keep their label, and the list of the others (rows null:
+// only the count of the kept ones). Besides the carried bound of the other
+// centres stands half the distance from the label's centre to its nearest
+// other one (near2): d(x, c) >= d(c_label, c) - d(x, c_label). Blocks of 256 threads, eight rows each and
+// one atomic per 2,048 rows: a list entry a row from warp atomics waited on the
+// counter (4M rows: 32 bytes a row otherwise).
+constexpr int MBT = 256, MB_ROWS = 8;
+__global__ void __launch_bounds__(MBT)
+    mixed_bound_kernel(int64_t n, int k, const int32_t *__restrict__ prev, int32_t *__restrict__ labels,
+                       float *__restrict__ ub, float *__restrict__ lb, const float2 *__restrict__ shift,
+                       const float *__restrict__ near2, int32_t *__restrict__ rows, DevScalars *sc) {
+    __shared__ float m1s[MBT / 32], m2s[MBT / 32];
+    __shared__ int a1s[MBT / 32], wsum[MBT / 32];
+    __shared__ unsigned long long base_s;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    // the largest shift, its centre, and the largest of the others
+    float m1 = -1.f, m2 = -1.f;
+    int a1 = -1;
+    auto merge = [&](float v1, int i1, float v2) {
+        if (v1 > m1) {
+            m2 = fmaxf(m1, v2);
+            m1 = v1;
+            a1 = i1;
+        } else {
+            m2 = fmaxf(m2, v1);
+        }
+    };
+    for (int q = tid; q < k; q += MBT) merge(shift[q].x, q, -1.f);
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) {
+        const float v1 = __shfl_xor_sync(0xffffffffu, m1, o), v2 = __shfl_xor_sync(0xffffffffu, m2, o);
+        const int i1 = __shfl_xor_sync(0xffffffffu, a1, o);
+        if (i1 != a1) merge(v1, i1, v2);
+    }
+    if (lane == 0) {
+        m1s[w] = m1;
+        m2s[w] = m2;
+        a1s[w] = a1;
+    }
+    __syncthreads();
+    m1 = m2 = -1.f;
+    a1 = -1;
+    for (int q = 0; q < MBT / 32; q++)
+        if (a1s[q] >= 0) merge(m1s[q], a1s[q], m2s[q]);
+    m2 = fmaxf(m2, 0.f);
+    unsigned kept = 0;
+    const int64_t chunk = (int64_t)MBT * MB_ROWS;
+    for (int64_t c0 = (int64_t)blockIdx.x * chunk; c0 < n; c0 += (int64_t)gridDim.x * chunk) {
+        unsigned listed = 0;
+#pragma unroll
+        for (int e = 0; e < MB_ROWS; e++) {
+            const int64_t i = c0 + e * MBT + tid;
+            if (i >= n) continue;
+            const int a = prev[i];
+            const float u = __fadd_ru(ub[i], shift[a].x);
+            const float gap = __fsqrt_rd(near2[a]);  // to the nearest other centre
+            const float l = fmaxf(__fsub_rd(lb[i], a == a1 ? m2 : m1), __fsub_rd(gap, u));
+            if (__fmul_ru(u, 1.000001f) < l && l > 1e-15f) {
+                kept++;
+                if (rows) {
+                    labels[i] = a;
+                    ub[i] = u;
+                    lb[i] = l;
+                }
+            } else {
+                listed |= 1u << e;
+            }
+        }
+        if (!rows) continue;
+        const int mine = __popc(listed);
+        int incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        if (lane == 31) wsum[w] = incl;
+        __syncthreads();
+        int at = incl - mine, total = 0;
+        for (int q = 0; q < MBT / 32; q++) {
+            if (q < w) at += wsum[q];
+            total += wsum[q];
+        }
+        if (tid == 0) base_s = total ? atomicAdd(&sc->listed_rows, (unsigned long long)total) : 0ull;
+        __syncthreads();
+        const unsigned long long base = base_s;
+#pragma unroll
+        for (int e = 0; e < MB_ROWS; e++)
+            if (listed >> e & 1u) rows[base + at++] = (int32_t)(c0 + e * MBT + tid);
+        __syncthreads();  // wsum and base_s are rewritten
+    }
+    const unsigned k32 = __reduce_add_sync(0xffffffffu, kept);
+    if (lane == 0 && k32) atomicAdd(&sc->kept_rows, (unsigned long long)k32);
+}
+
 // Merge of two slice records: (v1 >= v2, i1, i2) with u3 bounding the rest,
 // and the same for the other slice.
 __device__ __forceinline__ void merge_top2(float &v1, int &i1, float &v2, int &i2, float &u3, float w1, int j1,
@@ -701,6 +898,8 @@ constexpr int FINALIZE_THREADS = 512;
 struct RowClass {
     int cls, a, b;
     float th;
+    float rest;      // a pair: lower bound of the distance to every other centre
+    int64_t row;     // the row (of the pass's record i)
 };
 
 // Persistent finalize loop: each block takes chunks of FINALIZE_THREADS rows
@@ -724,17 +923,17 @@ __device__ __forceinline__ void finalize_rows(int64_t n, Load load, Classify cla
     if (ch < chunks && ch * FINALIZE_THREADS + threadIdx.x < n) cur = load(ch * FINALIZE_THREADS + threadIdx.x);
     // the previous chunk's entry of this thread, its warp's ballots, and
     // (thread 0) the atomics' pending results
-    RowClass pc{-1, -1, -1, 0.f};
-    int64_t pi = -1;
+    RowClass pc{-1, -1, -1, 0.f, 0.f, -1};
     unsigned pba = 0u, pbb = 0u;
     unsigned long long pend_a = 0ull, pend_b = 0ull;
     int buf = 0;
     bool have_prev = false;
     auto write_prev = [&](int pbuf) {
-        if (pc.cls == 1) pair_list[base_a + wa[pbuf][w] + (unsigned)__popc(pba & below)] = make_int4((int)pi, pc.a, pc.b, 0);
+        if (pc.cls == 1) pair_list[base_a + wa[pbuf][w] + (unsigned)__popc(pba & below)] =
+                make_int4((int)pc.row, pc.a, pc.b, __float_as_int(pc.rest));
         if (pc.cls == 2) {
             const unsigned long long q = base_b + wb[pbuf][w] + (unsigned)__popc(pbb & below);
-            full_list[q] = (int32_t)pi;
+            full_list[q] = (int32_t)pc.row;
             if (full_thresh) full_thresh[q] = pc.th;
         }
     };
@@ -742,7 +941,7 @@ __device__ __forceinline__ void finalize_rows(int64_t n, Load load, Classify cla
         const int64_t nrow = (ch + gridDim.x) * FINALIZE_THREADS + threadIdx.x;
         if (ch + gridDim.x < chunks && nrow < n) nxt = load(nrow);
         const int64_t i = ch * FINALIZE_THREADS + threadIdx.x;
-        RowClass c{-1, -1, -1, 0.f};
+        RowClass c{-1, -1, -1, 0.f, 0.f, -1};
         if (i < n) c = classify(i, cur);
         const unsigned ba = __ballot_sync(0xffffffffu, c.cls == 1), bb = __ballot_sync(0xffffffffu, c.cls == 2);
         if (lane == 0) {
@@ -768,7 +967,6 @@ __device__ __forceinline__ void finalize_rows(int64_t n, Load load, Classify cla
         __syncthreads();
         if (have_prev) write_prev(buf ^ 1);
         pc = c;
-        pi = i;
         pba = ba;
         pbb = bb;
         have_prev = true;
@@ -790,20 +988,27 @@ __global__ void __launch_bounds__(FINALIZE_THREADS, 2)
     finalize_kernel(const SliceTop2 *__restrict__ parts, int nparts, int kp, int64_t n, int k, int d,
                     const float4 *__restrict__ rowinfo, const MixedStats *stats, float acc_rel, float mu_norm,
                     int32_t *__restrict__ labels, int4 *__restrict__ pair_list, int32_t *__restrict__ full_list,
-                    float *__restrict__ full_thresh, float *__restrict__ floor_out, DevScalars *sc) {
+                    float *__restrict__ full_thresh, float *__restrict__ floor_out, DevScalars *sc, RowBounds rb,
+                    const int32_t *__restrict__ rows) {
+    // rows: record i is row rows[i], sc->listed_rows of them (records of slice p
+    // from p * n on either way)
     struct Rec {
         float4 ri;
         SliceTop2 t, o1;
+        float x2;
+        int row;
     };
     auto load = [&](int64_t i) {
         Rec r;
-        r.ri = rowinfo[i];
+        r.row = rows ? rows[i] : (int)i;
+        r.ri = rowinfo[r.row];
+        r.x2 = rb.ub ? rb.xsq[r.row] : 0.f;
         r.t = parts[i];
         r.o1 = nparts > 1 ? parts[(int64_t)n + i] : r.t;
         return r;
     };
     auto classify = [&](int64_t i, const Rec &rec) {
-        RowClass c{-1, -1, -1, -INFINITY};
+        RowClass c{-1, -1, -1, -INFINITY, 0.f, rec.row};
         const float4 ri = rec.ri;
         const SliceTop2 t = rec.t, o1 = rec.o1;
         float v1 = t.v1, v2 = t.v2, u3 = t.u3;
@@ -824,16 +1029,23 @@ __global__ void __launch_bounds__(FINALIZE_THREADS, 2)
             u3 *= unit;
         }
         const float thr = row_threshold(ri, stats, acc_rel, mu_norm, d, v1);
-        if (floor_out) floor_out[i] = row_floor(v1, 192.f * stats->ulp, ri, stats, acc_rel, mu_norm, d);
+        if (floor_out) floor_out[c.row] = row_floor(v1, 192.f * stats->ulp, ri, stats, acc_rel, mu_norm, d);
+        // a key is within 192 ulp of its score, a score within E of the exact one
+        const float off = __fadd_ru(192.f * stats->ulp, row_error(ri, stats, acc_rel));
         const float m12 = __fsub_rd(v1, v2);  // lower bounds of the margins
         const float m13 = __fsub_rd(v1, u3);
         c.a = i1;
         c.b = i2;
         if (i1 >= 0 && i1 < k && m12 > thr) {
             c.cls = 0;
-            labels[i] = i1;
+            labels[c.row] = i1;
+            if (rb.ub) {
+                rb.ub[c.row] = score_dist_up(__fsub_rd(v1, off), rec.x2, stats->big, d);
+                rb.lb[c.row] = score_dist_down(__fadd_ru(fmaxf(v2, u3), off), rec.x2, stats->big, d);
+            }
         } else if (i1 >= 0 && i1 < k && i2 >= 0 && i2 < k && i1 != i2 && m13 > thr) {
             c.cls = 1;
+            if (rb.ub) c.rest = score_dist_down(__fadd_ru(u3, off), rec.x2, stats->big, d);
         } else {
             c.cls = 2;
             // Mask pass threshold (BF16 main pass, whose scores the mask pass
@@ -846,9 +1058,13 @@ __global__ void __launch_bounds__(FINALIZE_THREADS, 2)
             const float t2 = __fsub_rd(v1, __fmul_ru(2.f, thr));
             c.th = t2 >= stats->ulp * 2097152.f ? t2 : -INFINITY;
         }
+        if (rb.ub && c.cls != 0) {  // no bound unless a re-score leaves one
+            rb.ub[c.row] = INFINITY;
+            rb.lb[c.row] = 0.f;
+        }
         return c;
     };
-    finalize_rows(n, load, classify, pair_list, full_list, full_thresh, sc);
+    finalize_rows(rows ? (int64_t)sc->listed_rows : n, load, classify, pair_list, full_list, full_thresh, sc);
 }
 
 // ------------------------------------------------------------ count pass --
@@ -952,7 +1168,7 @@ __global__ void __launch_bounds__(FINALIZE_THREADS, 2)  // two blocks an SM: 64 
         return r;
     };
     auto classify = [&](int64_t i, const Rec &rec) {
-        RowClass c{-1, -1, -1, 0.f};
+        RowClass c{-1, -1, -1, 0.f, 0.f, i};
         float vmax = 0.f;
         uint32_t cnt = 0, w1 = 0, w2 = 0;
         int b1 = 0, b2 = 0;  // the words' first centre
@@ -1056,6 +1272,17 @@ __device__ __forceinline__ bool below(float da, float ea, float db, float eb) {
     return __fadd_ru(da, ea) < __fsub_rd(db, eb);
 }
 
+// A pair decided by its FP32 intervals: the label, and the row's bounds from
+// both distances and the bound of every other centre that came with the pair.
+__device__ __forceinline__ void pair_decided(const int4 &e, int label, float near, float e_near, float far, float e_far,
+                                             int32_t *__restrict__ labels, const RowBounds &rb) {
+    labels[e.x] = label;
+    if (rb.ub) {
+        rb.ub[e.x] = pair_dist_up(near, e_near);
+        rb.lb[e.x] = fminf(pair_dist_down(far, e_far), __int_as_float(e.w));
+    }
+}
+
 // One warp per listed row (coalesced over the features): FP32 distances to
 // the two candidates decide the row when their bounded intervals do not
 // overlap; otherwise lanes 0 and 1 score the two exactly in FP64 (direct
@@ -1064,7 +1291,7 @@ template <typename TX>
 __global__ void pair_rescore_kernel(const TX *__restrict__ x, int d, const double *__restrict__ c,
                                     const float *__restrict__ c32, const float *__restrict__ ec32,
                                     const int4 *__restrict__ list, DevScalars *sc, int32_t *__restrict__ labels,
-                                    Oct *__restrict__ f64_items) {
+                                    Oct *__restrict__ f64_items, RowBounds rb) {
     const unsigned long long cnt = sc->flag_count;
     const int lane = threadIdx.x & 31;
     const unsigned long long wid = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1081,11 +1308,11 @@ __global__ void pair_rescore_kernel(const TX *__restrict__ x, int d, const doubl
             const float sa = __shfl_sync(0xffffffffu, acc, 0), sb = __shfl_sync(0xffffffffu, acc, 16);
             const float ea = bound32(sa, ec32[a], d), eb = bound32(sb, ec32[b], d);
             if (below(sa, ea, sb, eb)) {
-                if (lane == 0) labels[e.x] = a;
+                if (lane == 0) pair_decided(e, a, sa, ea, sb, eb, labels, rb);
                 continue;
             }
             if (below(sb, eb, sa, ea)) {
-                if (lane == 0) labels[e.x] = b;
+                if (lane == 0) pair_decided(e, b, sb, eb, sa, ea, labels, rb);
                 continue;
             }
         }
@@ -1103,7 +1330,7 @@ __global__ void __launch_bounds__(256)
     pair_rescore4_kernel(const float *__restrict__ x, int d, const double *__restrict__ c,
                          const float *__restrict__ c32, const float *__restrict__ ec32,
                          const int4 *__restrict__ list, DevScalars *sc, int32_t *__restrict__ labels,
-                         Oct *__restrict__ f64_items) {
+                         Oct *__restrict__ f64_items, RowBounds rb) {
     const unsigned long long cnt = sc->flag_count;
     const int lane = threadIdx.x & 31, hl = lane & 15;
     const unsigned long long nw = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
@@ -1151,9 +1378,9 @@ __global__ void __launch_bounds__(256)
         const float ea = bound32(sa, __shfl_sync(0xffffffffu, eca, 0), d),
                     eb = bound32(sb, __shfl_sync(0xffffffffu, eca, 16), d);
         if (below(sa, ea, sb, eb)) {
-            if (lane == 0) labels[e0.x] = a;
+            if (lane == 0) pair_decided(e0, a, sa, ea, sb, eb, labels, rb);
         } else if (below(sb, eb, sa, ea)) {
-            if (lane == 0) labels[e0.x] = b;
+            if (lane == 0) pair_decided(e0, b, sb, eb, sa, ea, labels, rb);
         } else {
             const int ids[8] = {a, b, 0, 0, 0, 0, 0, 0};
             queue_f64(f64_items, sc, e0.x, 2, ids);
@@ -1527,7 +1754,8 @@ __global__ void second_finalize_kernel(const SliceCount *__restrict__ parts, int
                                        const float4 *__restrict__ rowinfo2, const MixedStats *st2, float acc_rel2,
                                        float mu_norm, const float *__restrict__ th, int32_t *__restrict__ labels,
                                        int32_t *__restrict__ ex_list, int32_t *__restrict__ list3,
-                                       int32_t *__restrict__ slot3, float *__restrict__ th3, DevScalars *sc) {
+                                       int32_t *__restrict__ slot3, float *__restrict__ th3, DevScalars *sc,
+                                       RowBounds rb) {
     const unsigned long long cnt = *count;
     for (unsigned long long s = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; s < cnt;
          s += (unsigned long long)gridDim.x * blockDim.x) {
@@ -1548,7 +1776,15 @@ __global__ void second_finalize_kernel(const SliceCount *__restrict__ parts, int
         const bool decided = marks == 1 && a >= 0 && a < k;
         const bool to_ex = !decided && marks == 0;
         const bool to_mask = !decided && !to_ex;
-        if (decided) labels[row] = a;
+        if (decided) {
+            labels[row] = a;
+            if (rb.ub) {  // every other centre scores at most the threshold here
+                const float4 ri = rowinfo2[s];
+                const float e2 = row_error(ri, st2, acc_rel2), x2 = rb.xsq[row];
+                rb.ub[row] = score_dist_up(__fsub_rd(vmax, e2), x2, st2->big, d);
+                rb.lb[row] = score_dist_down(__fadd_ru(th[s], e2), x2, st2->big, d);
+            }
+        }
         const unsigned long long es = warp_reserve(&sc->ex_count, to_ex);
         const unsigned long long ms = warp_reserve(&sc->mask_count, to_mask);
         if (to_ex) ex_list[es] = row;
@@ -1572,6 +1808,19 @@ __global__ void gather_xq_rows_kernel(const uint4 *__restrict__ xq, int pieces, 
         const unsigned long long s = e / (unsigned)pieces;
         const int q = (int)(e - s * (unsigned)pieces);
         out[e] = xq[(int64_t)list[s] * pieces + q];
+    }
+}
+
+// FP8: the listed rows' augmentation rows (32 bytes) and scales.
+__global__ void gather_row_scales_kernel(const uint4 *__restrict__ xaug, const float *__restrict__ scale,
+                                         const int32_t *__restrict__ list, const unsigned long long *count,
+                                         uint4 *__restrict__ out, float *__restrict__ scale_out) {
+    const unsigned long long total = *count * 2ull;
+    for (unsigned long long e = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
+         e += (unsigned long long)gridDim.x * blockDim.x) {
+        const int64_t row = list[e >> 1];
+        out[e] = xaug[row * 2 + (int64_t)(e & 1)];
+        if (!(e & 1)) scale_out[e >> 1] = scale[row];
     }
 }
 
@@ -1711,6 +1960,7 @@ struct MixedBufs {
     void *xq;               // BF16 or E4M3 rows, n x d_pad
     __nv_bfloat16 *xaug;    // FP8: per-row augmentation rows, n x 16
     float4 *rowinfo;
+    float *xsq;             // ||x'||^2 of each row, f32 sums
     void *cq;               // BF16 or E4M3 centres, k_pad x d_pad
     __nv_bfloat16 *caug;    // k_pad x 16
     double *half_norm;
@@ -1733,6 +1983,7 @@ MixedBufs prepare_mixed(Ctx &ctx, const TX *x, int64_t n, int d, const double *c
     B.xq = ctx.get(BUF_XB, es * (size_t)n * mp.d_pad);
     B.xaug = fp8 ? (__nv_bfloat16 *)ctx.get(BUF_XAUG, sizeof(__nv_bfloat16) * 16 * (size_t)n) : nullptr;
     B.rowinfo = (float4 *)ctx.get(BUF_XNORM, sizeof(float4) * (size_t)n);
+    B.xsq = (float *)ctx.get(BUF_XSQ, sizeof(float) * (size_t)n);
     if (replan) {
         FK_CUDA(cudaMemsetAsync(B.stats, 0, sizeof(MixedStats), s));
         // the centring vector only needs to be finite: a strided sample of at
@@ -1752,9 +2003,11 @@ MixedBufs prepare_mixed(Ctx &ctx, const TX *x, int64_t n, int d, const double *c
             FK_LAUNCH_CHECK();
         }
         if (fp8)
-            launch_prep_rows<TX, true>(ctx, x, n, d, mp.d_pad, B.mu32, B.xq, B.xaug, B.rowinfo, B.stats);
+            launch_prep_rows<TX, true>(ctx, x, n, d, mp.d_pad, B.mu32, B.xq, B.xaug, B.rowinfo, B.stats, nullptr,
+                                       nullptr, B.xsq);
         else
-            launch_prep_rows<TX, false>(ctx, x, n, d, mp.d_pad, B.mu32, B.xq, nullptr, B.rowinfo, B.stats);
+            launch_prep_rows<TX, false>(ctx, x, n, d, mp.d_pad, B.mu32, B.xq, nullptr, B.rowinfo, B.stats, nullptr,
+                                        nullptr, B.xsq);
         // ||mu|| for the bound on ||x|| (host side, tiny)
         std::vector<double> hmu(d);
         FK_CUDA(cudaMemcpyAsync(hmu.data(), B.mu, sizeof(double) * d, cudaMemcpyDeviceToHost, s));
@@ -1816,7 +2069,7 @@ float mu_norm_up(double v) {
 // over the rows it leaves open, then the same re-score.
 void second_pass(Ctx &ctx, const float *x, int64_t n, int d, const double *c, int k, const MixedBufs &B,
                  double mu_norm, const int32_t *full, const float *full_thresh, int32_t *labels, DevScalars *sc,
-                 Oct *f64_items) {
+                 Oct *f64_items, const RowBounds &rb) {
     cudaStream_t s = ctx.stream;
     const int grid = ctx.num_sms * 4;
     int32_t *ex = (int32_t *)ctx.get(BUF_EX, sizeof(int32_t) * (size_t)n);
@@ -1898,7 +2151,7 @@ void second_pass(Ctx &ctx, const float *x, int64_t n, int d, const double *c, in
     launch_tc_assign(ctx, m2, xb2, cb2, caug2, nullptr, sc, st2, nullptr, &sc->full_count, nullptr, nullptr,
                      nullptr, th2, cnt2);
     second_finalize_kernel<<<grid, 256, 0, s>>>(cnt2, m2.parts, m2.kp, n, k, d, full, &sc->full_count, ri2, st2,
-                                                acc_rel2, mun, th2, labels, ex, list3, slot3, th3, sc);
+                                                acc_rel2, mun, th2, labels, ex, list3, slot3, th3, sc, rb);
     FK_LAUNCH_CHECK();
     const int pieces = m2.d_pad * 2 / 16;
     gather_xq_rows_kernel<<<ctx.num_sms * 8, 256, 0, s>>>((const uint4 *)xb2, pieces, slot3, &sc->mask_count,
@@ -1923,9 +2176,30 @@ void second_pass(Ctx &ctx, const float *x, int64_t n, int d, const double *c, in
 
 }  // namespace
 
+// Fits whose main pass is long against the bounds' few launches (2e10: about 20
+// us of BF16 contraction) keep them.
+bool mixed_bounds_ok(int64_t n, int d, int k) { return (double)n * k * d >= 2e10; }
+
+bool reserve_listed(Ctx &ctx, int64_t n, int d, int precision) {
+    const bool fp8 = precision == FK_PRECISION_MIXED_FP8;
+    const int per = fp8 ? 128 : 64;
+    try {
+        ctx.get(BUF_LROWS, sizeof(int32_t) * (size_t)n);
+        ctx.get(BUF_LXB, (fp8 ? 1 : 2) * (size_t)((d + per - 1) / per * per) * (size_t)n);
+        if (fp8) {
+            ctx.get(BUF_LXAUG, sizeof(__nv_bfloat16) * 16 * (size_t)n);
+            ctx.get(BUF_LSCALE, sizeof(float) * (size_t)n);
+        }
+    } catch (const Error &e) {
+        if (e.code != FK_ERR_OOM) throw;
+        return false;
+    }
+    return true;
+}
+
 template <typename TX>
 void run_assign_mixed(Ctx &ctx, const TX *x, int64_t n, int d, const double *c, int k, int precision,
-                      int32_t *labels, double *, DevScalars *sc, bool x_changed, const double *c_prev,
+                      int32_t *labels, double *, DevScalars *sc, bool x_changed, int main, const double *c_prev,
                       const int32_t *labels_prev) {
     cudaStream_t s = ctx.stream;
     MixedPlan &mp = ctx.mixed;
@@ -1957,7 +2231,68 @@ void run_assign_mixed(Ctx &ctx, const TX *x, int64_t n, int d, const double *c, 
     static const int fin_top2 = resident_blocks((const void *)finalize_kernel, FINALIZE_THREADS);
     static const int fin_count = resident_blocks((const void *)finalize_count_kernel, FINALIZE_THREADS);
     const int64_t fin_chunks = (n + FINALIZE_THREADS - 1) / FINALIZE_THREADS;
-    if (c_prev && labels_prev) {
+    RowBounds rb{nullptr, nullptr, nullptr};
+    float2 *shift = nullptr;
+    if (c_prev) {
+        shift = (float2 *)ctx.get(BUF_SHIFT, sizeof(float2) * (size_t)k);
+        centre_shift_kernel<<<(unsigned)(((int64_t)k * 32 + 255) / 256), 256, 0, s>>>(c, c_prev, B.mu, k, d, shift);
+        FK_LAUNCH_CHECK();
+    }
+    float *near2 = nullptr;
+    if (c_prev && (main == MAIN_TOP2_BOUNDS || main == MAIN_LISTED)) {
+        near2 = (float *)ctx.get(BUF_MX_NEAR, sizeof(float) * (size_t)k);
+        FK_CUDA(cudaMemsetAsync(near2, 0x7F, sizeof(float) * (size_t)k, s));
+        const unsigned t = (unsigned)((k + NT_ - 1) / NT_);
+        centre_near_kernel<<<dim3(t, t), 256, 0, s>>>(B.c32, B.ec32, k, d, near2);
+        FK_LAUNCH_CHECK();
+    }
+    const unsigned bound_grid =
+        (unsigned)std::min<int64_t>((n + MBT * MB_ROWS - 1) / (MBT * MB_ROWS), (int64_t)ctx.num_sms * 6);
+    if (main == MAIN_TOP2_BOUNDS || main == MAIN_LISTED) {
+        rb.xsq = B.xsq;
+        rb.ub = (float *)ctx.get(BUF_MX_UB, sizeof(float) * 2 * (size_t)n);
+        rb.lb = rb.ub + n;
+    }
+    if (main == MAIN_LISTED) {
+        // the rows that the bounds do not keep: their operands gathered, ranked
+        // and finalized as the full pass does, by their own row numbers
+        MixedPlan &ml = ctx.mixedl;
+        if (ml.n != n || ml.d != d || ml.k != k || ml.kp != mp.kp || ml.fp8 != fp8)
+            plan_tc(ctx, ml, n, d, k, fp8, 2, mp.kp);
+        if (ml.k_pad != mp.k_pad || ml.d_pad != mp.d_pad) {
+            set_error("listed pass plan (k_pad %d, d_pad %d) differs from the main pass (%d, %d)", ml.k_pad, ml.d_pad,
+                      mp.k_pad, mp.d_pad);
+            fail(FK_ERR_CUDA);
+        }
+        const size_t row_bytes = (fp8 ? 1 : 2) * (size_t)mp.d_pad;
+        int32_t *rows = (int32_t *)ctx.get(BUF_LROWS, sizeof(int32_t) * (size_t)n);
+        void *lxb = ctx.get(BUF_LXB, row_bytes * (size_t)n);
+        __nv_bfloat16 *lxaug = nullptr;
+        float *lscale = nullptr;
+        if (fp8) {
+            lxaug = (__nv_bfloat16 *)ctx.get(BUF_LXAUG, sizeof(__nv_bfloat16) * 16 * (size_t)n);
+            lscale = (float *)ctx.get(BUF_LSCALE, sizeof(float) * (size_t)n);
+        }
+        mixed_bound_kernel<<<bound_grid, MBT, 0, s>>>(n, k, labels_prev, labels, rb.ub, rb.lb, shift, near2, rows, sc);
+        FK_LAUNCH_CHECK();
+        gather_xq_rows_kernel<<<ctx.num_sms * 8, 256, 0, s>>>((const uint4 *)B.xq, (int)(row_bytes / 16), rows,
+                                                              &sc->listed_rows, (uint4 *)lxb);
+        FK_LAUNCH_CHECK();
+        if (fp8) {
+            gather_row_scales_kernel<<<ctx.num_sms * 8, 256, 0, s>>>((const uint4 *)B.xaug, rowscale, rows,
+                                                                     &sc->listed_rows, (uint4 *)lxaug, lscale);
+            FK_LAUNCH_CHECK();
+        }
+        SliceTop2 *top = (SliceTop2 *)ctx.get(BUF_TOP2, sizeof(SliceTop2) * (size_t)n * mp.parts);
+        {
+            Timer t(ctx.contract_acc != nullptr, ctx, ctx.contract_acc);
+            launch_tc_assign(ctx, ml, lxb, B.cq, B.caug, top, sc, B.stats, nullptr, &sc->listed_rows, lxaug, lscale);
+        }
+        finalize_kernel<<<(unsigned)std::min<int64_t>(fin_chunks, (int64_t)ctx.num_sms * fin_top2), FINALIZE_THREADS,
+                          0, s>>>(top, mp.parts, mp.kp, n, k, d, B.rowinfo, B.stats, acc_rel, mun, labels, pairs, full,
+                                  full_thresh, floors, sc, rb, rows);
+        FK_LAUNCH_CHECK();
+    } else if (main == MAIN_COUNT) {
         // count pass, against thresholds carried from the previous iteration
         MixedPlan &mc = ctx.mixedc;
         if (mc.n != n || mc.d != d || mc.k != k || mc.kp != mp.kp || mc.fp8 != fp8)
@@ -1967,9 +2302,6 @@ void run_assign_mixed(Ctx &ctx, const TX *x, int64_t n, int d, const double *c, 
                       mp.k_pad, mp.d_pad);
             fail(FK_ERR_CUDA);
         }
-        float2 *shift = (float2 *)ctx.get(BUF_SHIFT, sizeof(float2) * (size_t)k);
-        centre_shift_kernel<<<(unsigned)(((int64_t)k * 32 + 255) / 256), 256, 0, s>>>(c, c_prev, B.mu, k, d, shift);
-        FK_LAUNCH_CHECK();
         float *th = (float *)ctx.get(BUF_THMAIN, sizeof(float) * (size_t)n);
         count_thresh_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, k, d, floors, labels_prev, B.rowinfo,
                                                                       shift, B.stats, acc_rel, mun, th);
@@ -1987,6 +2319,12 @@ void run_assign_mixed(Ctx &ctx, const TX *x, int64_t n, int d, const double *c, 
                                                                       full_thresh, floors, sc);
         FK_LAUNCH_CHECK();
     } else {
+        if (rb.ub && c_prev) {
+            // how many rows the bounds would have kept: the fit lists rows once it pays
+            mixed_bound_kernel<<<bound_grid, MBT, 0, s>>>(n, k, labels_prev, nullptr, rb.ub, rb.lb, shift, near2, nullptr,
+                                                        sc);
+            FK_LAUNCH_CHECK();
+        }
         SliceTop2 *top = (SliceTop2 *)ctx.get(BUF_TOP2, sizeof(SliceTop2) * (size_t)n * mp.parts);
         {
             Timer t(ctx.contract_acc != nullptr, ctx, ctx.contract_acc);
@@ -1996,7 +2334,7 @@ void run_assign_mixed(Ctx &ctx, const TX *x, int64_t n, int d, const double *c, 
         finalize_kernel<<<(unsigned)std::min<int64_t>(fin_chunks, (int64_t)ctx.num_sms * fin_top2), FINALIZE_THREADS,
                           0, s>>>(top, mp.parts, mp.kp, n, k, d, B.rowinfo, B.stats,
                                                                 acc_rel, mun, labels, pairs, full, full_thresh,
-                                                                floors, sc);
+                                                                floors, sc, rb, nullptr);
         FK_LAUNCH_CHECK();
     }
     const int grid = ctx.num_sms * 4;
@@ -2004,11 +2342,11 @@ void run_assign_mixed(Ctx &ctx, const TX *x, int64_t n, int d, const double *c, 
     if (std::is_same<TX, float>::value && d % 4 == 0 && d <= 128 && ((uintptr_t)x & 15u) == 0) {
         static const int pair_blocks = resident_blocks((const void *)pair_rescore4_kernel, 256);
         pair_rescore4_kernel<<<ctx.num_sms * pair_blocks, 256, 0, s>>>((const float *)x, d, c, B.c32, B.ec32, pairs,
-                                                                       sc, labels, f64_items);
+                                                                       sc, labels, f64_items, rb);
     } else
-        pair_rescore_kernel<TX><<<grid, 256, 0, s>>>(x, d, c, B.c32, B.ec32, pairs, sc, labels, f64_items);
+        pair_rescore_kernel<TX><<<grid, 256, 0, s>>>(x, d, c, B.c32, B.ec32, pairs, sc, labels, f64_items, rb);
     FK_LAUNCH_CHECK();
-    second_pass(ctx, x, n, d, c, k, B, mp.mu_norm, full, full_thresh, labels, sc, f64_items);
+    second_pass(ctx, x, n, d, c, k, B, mp.mu_norm, full, full_thresh, labels, sc, f64_items, rb);
     launch_f64_decide<TX>(ctx, x, d, c, f64_items, sc, labels);
 }
 
@@ -2021,7 +2359,7 @@ void launch_mixed_inertia(Ctx &ctx, const double *part, int64_t m, DevScalars *s
 }
 
 template void run_assign_mixed<float>(Ctx &, const float *, int64_t, int, const double *, int, int, int32_t *,
-                                      double *, DevScalars *, bool, const double *, const int32_t *);
+                                      double *, DevScalars *, bool, int, const double *, const int32_t *);
 
 // Diagnostics for the tests: one tensor-core pass over x (f32, on the device)
 // against c (f64), returning the raw accumulators of CTA 0's first tile and

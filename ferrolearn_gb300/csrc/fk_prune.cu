@@ -203,7 +203,10 @@ __global__ void __launch_bounds__(PT)
     for (int64_t i = (int64_t)blockIdx.x * PT + tid; i < n; i += stride) {
         const int a = prev[i];
         const float u = __fadd_ru(ub[i], shift[a]);
-        const float l = __fsub_rd(lb[i], a == a1 ? m2 : m1);
+        // every other centre is at least twice the root of the nearest one's
+        // threshold away from this one
+        const float gap = __fmul_rd(2.f, __fsqrt_rd(nthr[(int64_t)a * NROW]));
+        const float l = fmaxf(__fsub_rd(lb[i], a == a1 ? m2 : m1), __fsub_rd(gap, u));
         const bool keep = __fmul_ru(u, rel) < l && l > 1e-15f;
         bool near = false;
         if (keep) {
