@@ -65,6 +65,7 @@ struct DevScalars {
     unsigned long long moved_rows;  // incremental update: rows whose label changed
     unsigned long long incremental; // 1: this iteration's update was incremental
     unsigned long long mask_count;  // FP8 second pass: rows left to its mask pass
+    unsigned long long pair2_count; // FP8 second pass: pairs its count pass left
     unsigned long long kept_rows;   // rows whose bounds keep their label (fits of some size)
     unsigned long long listed_rows; // rows listed for the main pass
 };

@@ -1290,14 +1290,15 @@ __device__ __forceinline__ void pair_decided(const int4 &e, int label, float nea
 template <typename TX>
 __global__ void pair_rescore_kernel(const TX *__restrict__ x, int d, const double *__restrict__ c,
                                     const float *__restrict__ c32, const float *__restrict__ ec32,
-                                    const int4 *__restrict__ list, DevScalars *sc, int32_t *__restrict__ labels,
-                                    Oct *__restrict__ f64_items, RowBounds rb) {
-    const unsigned long long cnt = sc->flag_count;
+                                    const int4 *__restrict__ list, int step, const unsigned long long *count,
+                                    DevScalars *sc, int32_t *__restrict__ labels, Oct *__restrict__ f64_items,
+                                    RowBounds rb) {
+    const unsigned long long cnt = *count;
     const int lane = threadIdx.x & 31;
     const unsigned long long wid = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const unsigned long long nw = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
     for (unsigned long long s = wid; s < cnt; s += nw) {
-        const int4 e = list[s];
+        const int4 e = list[(int64_t)s * step];
         const TX *row = x + (int64_t)e.x * d;
         const int a = e.y < e.z ? e.y : e.z, b = e.y < e.z ? e.z : e.y;
         if constexpr (std::is_same<TX, float>::value) {
@@ -1321,28 +1322,29 @@ __global__ void pair_rescore_kernel(const TX *__restrict__ x, int d, const doubl
     }
 }
 
-// pair_rescore_kernel for f32 rows with d % 4 == 0 and d <= 128: the same
+// pair_rescore_kernel for f32 rows with d % 4 == 0 and d <= 64 NP: the same
 // decisions, software-pipelined -- the list entry two rows ahead and the
 // feature and centre pieces (and the centres' rounding errors) one row ahead
 // load while this row is decided.
-// Lanes 0-15 hold centre a, lanes 16-31 centre b, 16-byte pieces hl, hl + 16.
+// Lanes 0-15 hold centre a, lanes 16-31 centre b, 16-byte pieces hl + 16 i.
+template <int NP>
 __global__ void __launch_bounds__(256)
     pair_rescore4_kernel(const float *__restrict__ x, int d, const double *__restrict__ c,
                          const float *__restrict__ c32, const float *__restrict__ ec32,
-                         const int4 *__restrict__ list, DevScalars *sc, int32_t *__restrict__ labels,
-                         Oct *__restrict__ f64_items, RowBounds rb) {
-    const unsigned long long cnt = sc->flag_count;
+                         const int4 *__restrict__ list, int step, const unsigned long long *count, DevScalars *sc,
+                         int32_t *__restrict__ labels, Oct *__restrict__ f64_items, RowBounds rb) {
+    const unsigned long long cnt = *count;
     const int lane = threadIdx.x & 31, hl = lane & 15;
     const unsigned long long nw = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
     const int d4 = d >> 2;
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    auto entry = [&](unsigned long long q) { return q < cnt ? list[q] : make_int4(-1, 0, 0, 0); };
+    auto entry = [&](unsigned long long q) { return q < cnt ? list[(int64_t)q * step] : make_int4(-1, 0, 0, 0); };
     // this lane's pieces of the row and of its centre (a for lanes 0-15, b for
     // 16-31), and that centre's rounding error
-    auto pieces = [&](const int4 &e, float4 (&xv)[2], float4 (&cv)[2], float &ec) {
+    auto pieces = [&](const int4 &e, float4 (&xv)[NP], float4 (&cv)[NP], float &ec) {
         const int a = min(e.y, e.z), b = max(e.y, e.z);
 #pragma unroll
-        for (int i = 0; i < 2; i++) {
+        for (int i = 0; i < NP; i++) {
             const int q = hl + 16 * i;
             const bool ok = e.x >= 0 && q < d4;
             xv[i] = ok ? reinterpret_cast<const float4 *>(x + (int64_t)e.x * d)[q] : z4;
@@ -1352,17 +1354,17 @@ __global__ void __launch_bounds__(256)
     };
     unsigned long long s = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int4 e0 = entry(s), e1 = entry(s + nw);
-    float4 xa[2], ca[2];
+    float4 xa[NP], ca[NP];
     float eca;
     pieces(e0, xa, ca, eca);
     for (; s < cnt; s += nw) {
         const int4 e2 = entry(s + 2 * nw);
-        float4 xb[2], cb[2];
+        float4 xb[NP], cb[NP];
         float ecb;
         pieces(e1, xb, cb, ecb);
         float acc = 0.f;  // padding pieces are zero on both sides
 #pragma unroll
-        for (int i = 0; i < 2; i++) {
+        for (int i = 0; i < NP; i++) {
             float t = xa[i].x - ca[i].x;
             acc = fmaf(t, t, acc);
             t = xa[i].y - ca[i].y;
@@ -1389,7 +1391,7 @@ __global__ void __launch_bounds__(256)
         e1 = e2;
         eca = ecb;
 #pragma unroll
-        for (int i = 0; i < 2; i++) {
+        for (int i = 0; i < NP; i++) {
             xa[i] = xb[i];
             ca[i] = cb[i];
         }
@@ -1615,12 +1617,25 @@ __device__ __forceinline__ float cand_dists(const float *__restrict__ xrow, cons
     return my;
 }
 
+// What a row decided among its marked centres leaves as bounds: every other
+// centre scored at most the row's threshold th in the marking pass (statistics
+// st, row ingredients info at slot[s], or at the row itself).
+struct MaskBounds {
+    RowBounds rb;
+    const float *th;
+    const float4 *info;
+    const int32_t *slot;
+    const MixedStats *st;
+    float acc_rel;
+};
+
 template <bool FAST>
 __global__ void __launch_bounds__(MASK_WARPS * 32)
     mask_rescore_kernel(const float *__restrict__ x, int d, const float *__restrict__ c32,
                         const float *__restrict__ ec32, int k, const uint32_t *__restrict__ masks, int wpr,
                         const int32_t *__restrict__ list, const unsigned long long *count, DevScalars *sc,
-                        int32_t *__restrict__ labels, Oct *__restrict__ f64_items, int32_t *__restrict__ ex_list) {
+                        int32_t *__restrict__ labels, Oct *__restrict__ f64_items, int32_t *__restrict__ ex_list,
+                        MaskBounds mb) {
     __shared__ int cand_sm[MASK_WARPS][MASK_CANDS];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     int *cand = cand_sm[wid];
@@ -1691,9 +1706,21 @@ __global__ void __launch_bounds__(MASK_WARPS * 32)
             const int nsurv = __popc(surv);
             if (nsurv == 1) {
                 const int only = __shfl_sync(0xffffffffu, my_id, __ffs(surv) - 1);
+                float other = is_cand && my_id != only ? pair_dist_down(my_dist, my_err) : INFINITY;
+                if (mb.rb.ub) {  // uniform
+#pragma unroll
+                    for (int off = 16; off >= 1; off >>= 1)
+                        other = fminf(other, __shfl_xor_sync(0xffffffffu, other, off));
+                }
                 if (lane == 0) {
                     labels[row] = only;
                     decided++;
+                    if (mb.rb.ub) {
+                        const float4 ri = mb.info[mb.slot ? mb.slot[s] : row];
+                        const float hi = __fadd_ru(mb.th[s], row_error(ri, mb.st, mb.acc_rel));
+                        mb.rb.ub[row] = __fadd_ru(__fsqrt_ru(ub), 1e-20f);  // the one survivor has the smallest
+                        mb.rb.lb[row] = fminf(other, score_dist_down(hi, mb.rb.xsq[row], mb.st->big, d));
+                    }
                 }
             } else {
                 // the survivors (all candidates if no FP32 value was finite)
@@ -1745,8 +1772,10 @@ __global__ void second_thresh_kernel(const int32_t *__restrict__ list, const uns
     }
 }
 
-// After that count pass: one mark is the label; none (a NaN row) the
-// exhaustive re-score; more go to the mask pass with max(th, vmax - thr),
+// After that count pass: one mark is the label; two a pair for the exact
+// re-score (listed from pair_end downwards: the main pass's pairs and these are
+// different rows, together at most n); none (a NaN row) the exhaustive
+// re-score; more go to the mask pass with max(th, vmax - thr),
 // vmax the pass's exact best score (the winner scores at least vmax - 2 E2 -
 // FP64 slack there). list3 / slot3 hold the row and its slot here.
 __global__ void second_finalize_kernel(const SliceCount *__restrict__ parts, int nparts, int kp, int64_t cap, int k,
@@ -1755,27 +1784,42 @@ __global__ void second_finalize_kernel(const SliceCount *__restrict__ parts, int
                                        float mu_norm, const float *__restrict__ th, int32_t *__restrict__ labels,
                                        int32_t *__restrict__ ex_list, int32_t *__restrict__ list3,
                                        int32_t *__restrict__ slot3, float *__restrict__ th3, DevScalars *sc,
-                                       RowBounds rb) {
+                                       RowBounds rb, int4 *__restrict__ pair_end) {
     const unsigned long long cnt = *count;
     for (unsigned long long s = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; s < cnt;
          s += (unsigned long long)gridDim.x * blockDim.x) {
         float vmax = 0.f;
-        uint32_t marks = 0, w1 = 0;
-        int b1 = 0;
+        uint32_t marks = 0, w1 = 0, w2 = 0;
+        int b1 = 0, b2 = 0;  // the words' first centre
         for (int p = 0; p < nparts; p++) {
             const SliceCount o = parts[(int64_t)p * cap + s];
             vmax = fmaxf(vmax, o.vmax);
             marks += o.meta & 0xFFFFu;
-            if (!w1 && o.w1) {
-                w1 = o.w1;
-                b1 = p * kp + 32 * (int)((o.meta >> 16) & 0xFFu);
+            const uint32_t ow[2] = {o.w1, o.w2};
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                if (!ow[u]) continue;
+                const int first = p * kp + 32 * (int)((o.meta >> (16 + 8 * u)) & 0xFFu);
+                if (!w1) {
+                    w1 = ow[u];
+                    b1 = first;
+                } else if (!w2) {
+                    w2 = ow[u];
+                    b2 = first;
+                }
             }
         }
         const int row = list[s];
-        const int a = (marks == 1 && w1) ? count_column(b1, 0, __ffs(w1) - 1) : -1;
+        const int a = (marks >= 1 && marks <= 2 && w1) ? count_column(b1, 0, __ffs(w1) - 1) : -1;
+        const uint32_t w1_rest = w1 & (w1 - 1u);
+        const int b = marks != 2  ? -1
+                      : w1_rest   ? count_column(b1, 0, __ffs(w1_rest) - 1)
+                      : w2        ? count_column(b2, 0, __ffs(w2) - 1)
+                                  : -1;
         const bool decided = marks == 1 && a >= 0 && a < k;
+        const bool pair = marks == 2 && a >= 0 && a < k && b >= 0 && b < k && a != b;
         const bool to_ex = !decided && marks == 0;
-        const bool to_mask = !decided && !to_ex;
+        const bool to_mask = !decided && !pair && !to_ex;
         if (decided) {
             labels[row] = a;
             if (rb.ub) {  // every other centre scores at most the threshold here
@@ -1784,6 +1828,12 @@ __global__ void second_finalize_kernel(const SliceCount *__restrict__ parts, int
                 rb.ub[row] = score_dist_up(__fsub_rd(vmax, e2), x2, st2->big, d);
                 rb.lb[row] = score_dist_down(__fadd_ru(th[s], e2), x2, st2->big, d);
             }
+        }
+        const unsigned long long ps = warp_reserve(&sc->pair2_count, pair);
+        if (pair) {
+            const float hi = __fadd_ru(th[s], row_error(rowinfo2[s], st2, acc_rel2));
+            const float rest = rb.ub ? score_dist_down(hi, rb.xsq[row], st2->big, d) : 0.f;
+            pair_end[-(int64_t)ps] = make_int4(row, a, b, __float_as_int(rest));
         }
         const unsigned long long es = warp_reserve(&sc->ex_count, to_ex);
         const unsigned long long ms = warp_reserve(&sc->mask_count, to_mask);
@@ -2060,6 +2110,26 @@ float mu_norm_up(double v) {
     return (double)f >= v ? f : std::nextafter(f, INFINITY);
 }
 
+// The exact re-score of listed pairs (entry q at list + q * step).
+template <typename TX>
+void launch_pairs(Ctx &ctx, const TX *x, int d, const double *c, const MixedBufs &B, const int4 *list, int step,
+                  const unsigned long long *count, DevScalars *sc, int32_t *labels, Oct *f64_items, const RowBounds &rb) {
+    if (std::is_same<TX, float>::value && d % 4 == 0 && d <= 256 && ((uintptr_t)x & 15u) == 0) {
+        static const int blocks2 = resident_blocks((const void *)pair_rescore4_kernel<2>, 256);
+        static const int blocks4 = resident_blocks((const void *)pair_rescore4_kernel<4>, 256);
+        if (d <= 128)
+            pair_rescore4_kernel<2><<<ctx.num_sms * blocks2, 256, 0, ctx.stream>>>((const float *)x, d, c, B.c32, B.ec32, list,
+                                                                                  step, count, sc, labels, f64_items, rb);
+        else
+            pair_rescore4_kernel<4><<<ctx.num_sms * blocks4, 256, 0, ctx.stream>>>((const float *)x, d, c, B.c32, B.ec32, list,
+                                                                                  step, count, sc, labels, f64_items, rb);
+    } else {
+        pair_rescore_kernel<TX><<<ctx.num_sms * 4, 256, 0, ctx.stream>>>(x, d, c, B.c32, B.ec32, list, step, count, sc, labels,
+                                                                         f64_items, rb);
+    }
+    FK_LAUNCH_CHECK();
+}
+
 // Second pass over the rows listed in full (count sc->full_count). After a
 // BF16 main pass: the rows' BF16 operands gathered from the main pass's
 // copy, a tensor pass that marks every centre scoring above the row's
@@ -2069,7 +2139,7 @@ float mu_norm_up(double v) {
 // over the rows it leaves open, then the same re-score.
 void second_pass(Ctx &ctx, const float *x, int64_t n, int d, const double *c, int k, const MixedBufs &B,
                  double mu_norm, const int32_t *full, const float *full_thresh, int32_t *labels, DevScalars *sc,
-                 Oct *f64_items, const RowBounds &rb) {
+                 Oct *f64_items, const RowBounds &rb, int4 *pairs) {
     cudaStream_t s = ctx.stream;
     const int grid = ctx.num_sms * 4;
     int32_t *ex = (int32_t *)ctx.get(BUF_EX, sizeof(int32_t) * (size_t)n);
@@ -2093,15 +2163,17 @@ void second_pass(Ctx &ctx, const float *x, int64_t n, int d, const double *c, in
         FK_LAUNCH_CHECK();
         launch_tc_assign(ctx, mm, xb2, B.cq, B.caug, nullptr, sc, B.stats, nullptr, &sc->full_count,
                          nullptr, nullptr, masks, full_thresh);
+        const float acc_rel = (float)((double)((size_t)mm.d_pad + 32) * ACC_REL_PER_K);  // exact: integer * 2^-22
+        const MaskBounds mb{rb, full_thresh, B.rowinfo, nullptr, B.stats, acc_rel};
         // latency-bound (a few dependent loads per row): as many warps as the SMs hold
         if (d % 4 == 0 && d <= 256 && (((uintptr_t)x | (uintptr_t)B.c32) & 15u) == 0) {
             static const int mask_blocks = resident_blocks((const void *)mask_rescore_kernel<true>, MASK_WARPS * 32);
             mask_rescore_kernel<true><<<ctx.num_sms * mask_blocks, MASK_WARPS * 32, 0, s>>>(
-                x, d, B.c32, B.ec32, k, masks, wpr, full, &sc->full_count, sc, labels, f64_items, ex);
+                x, d, B.c32, B.ec32, k, masks, wpr, full, &sc->full_count, sc, labels, f64_items, ex, mb);
         } else {
             static const int mask_blocks = resident_blocks((const void *)mask_rescore_kernel<false>, MASK_WARPS * 32);
             mask_rescore_kernel<false><<<ctx.num_sms * mask_blocks, MASK_WARPS * 32, 0, s>>>(
-                x, d, B.c32, B.ec32, k, masks, wpr, full, &sc->full_count, sc, labels, f64_items, ex);
+                x, d, B.c32, B.ec32, k, masks, wpr, full, &sc->full_count, sc, labels, f64_items, ex, mb);
         }
         FK_LAUNCH_CHECK();
         exhaustive_rescore_kernel<<<ctx.num_sms * 2, EX_THREADS, exhaustive_smem_bytes(d, k), s>>>(
@@ -2151,22 +2223,24 @@ void second_pass(Ctx &ctx, const float *x, int64_t n, int d, const double *c, in
     launch_tc_assign(ctx, m2, xb2, cb2, caug2, nullptr, sc, st2, nullptr, &sc->full_count, nullptr, nullptr,
                      nullptr, th2, cnt2);
     second_finalize_kernel<<<grid, 256, 0, s>>>(cnt2, m2.parts, m2.kp, n, k, d, full, &sc->full_count, ri2, st2,
-                                                acc_rel2, mun, th2, labels, ex, list3, slot3, th3, sc, rb);
+                                                acc_rel2, mun, th2, labels, ex, list3, slot3, th3, sc, rb, pairs + n - 1);
     FK_LAUNCH_CHECK();
+    launch_pairs<float>(ctx, x, d, c, B, pairs + n - 1, -1, &sc->pair2_count, sc, labels, f64_items, rb);
     const int pieces = m2.d_pad * 2 / 16;
     gather_xq_rows_kernel<<<ctx.num_sms * 8, 256, 0, s>>>((const uint4 *)xb2, pieces, slot3, &sc->mask_count,
                                                           (uint4 *)xb3);
     FK_LAUNCH_CHECK();
     launch_tc_assign(ctx, mm, xb3, cb2, caug2, nullptr, sc, st2, nullptr, &sc->mask_count, nullptr,
                      nullptr, masks, th3);
+    const MaskBounds mb{rb, th3, ri2, slot3, st2, acc_rel2};
     if (d % 4 == 0 && d <= 256 && (((uintptr_t)x | (uintptr_t)B.c32) & 15u) == 0) {
         static const int mask_blocks = resident_blocks((const void *)mask_rescore_kernel<true>, MASK_WARPS * 32);
         mask_rescore_kernel<true><<<ctx.num_sms * mask_blocks, MASK_WARPS * 32, 0, s>>>(
-            x, d, B.c32, B.ec32, k, masks, wpr, list3, &sc->mask_count, sc, labels, f64_items, ex);
+            x, d, B.c32, B.ec32, k, masks, wpr, list3, &sc->mask_count, sc, labels, f64_items, ex, mb);
     } else {
         static const int mask_blocks = resident_blocks((const void *)mask_rescore_kernel<false>, MASK_WARPS * 32);
         mask_rescore_kernel<false><<<ctx.num_sms * mask_blocks, MASK_WARPS * 32, 0, s>>>(
-            x, d, B.c32, B.ec32, k, masks, wpr, list3, &sc->mask_count, sc, labels, f64_items, ex);
+            x, d, B.c32, B.ec32, k, masks, wpr, list3, &sc->mask_count, sc, labels, f64_items, ex, mb);
     }
     FK_LAUNCH_CHECK();
     exhaustive_rescore_kernel<<<ctx.num_sms * 2, EX_THREADS, exhaustive_smem_bytes(d, k), s>>>(
@@ -2337,16 +2411,9 @@ void run_assign_mixed(Ctx &ctx, const TX *x, int64_t n, int d, const double *c, 
                                                                 floors, sc, rb, nullptr);
         FK_LAUNCH_CHECK();
     }
-    const int grid = ctx.num_sms * 4;
     Oct *f64_items = (Oct *)ctx.get(BUF_F64ITEMS, sizeof(Oct) * (size_t)n);
-    if (std::is_same<TX, float>::value && d % 4 == 0 && d <= 128 && ((uintptr_t)x & 15u) == 0) {
-        static const int pair_blocks = resident_blocks((const void *)pair_rescore4_kernel, 256);
-        pair_rescore4_kernel<<<ctx.num_sms * pair_blocks, 256, 0, s>>>((const float *)x, d, c, B.c32, B.ec32, pairs,
-                                                                       sc, labels, f64_items, rb);
-    } else
-        pair_rescore_kernel<TX><<<grid, 256, 0, s>>>(x, d, c, B.c32, B.ec32, pairs, sc, labels, f64_items, rb);
-    FK_LAUNCH_CHECK();
-    second_pass(ctx, x, n, d, c, k, B, mp.mu_norm, full, full_thresh, labels, sc, f64_items, rb);
+    launch_pairs<TX>(ctx, x, d, c, B, pairs, 1, &sc->flag_count, sc, labels, f64_items, rb);
+    second_pass(ctx, x, n, d, c, k, B, mp.mu_norm, full, full_thresh, labels, sc, f64_items, rb, pairs);
     launch_f64_decide<TX>(ctx, x, d, c, f64_items, sc, labels);
 }
 
