@@ -168,6 +168,17 @@ enum BufSlot {
     BUF_COUNT
 };
 
+// Workers that carry a large result into pageable host memory (fk_capi.cu):
+// each has a stream and two pinned pieces. Made at the first such copy.
+struct HostCopy {
+    static constexpr int WORKERS = 8;
+    static constexpr size_t PIECE = (size_t)1 << 20;
+    cudaStream_t stream[WORKERS] = {};
+    cudaEvent_t ready = nullptr, done[WORKERS][2] = {};
+    unsigned char *pinned = nullptr;  // WORKERS x 2 pieces
+    bool made = false, failed = false;
+};
+
 struct Ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -184,6 +195,7 @@ struct Ctx {
         double *acc;
     };
     std::vector<PendingTimer> pending;  // phase timers read after the loop
+    HostCopy host_copy;
     MixedPlan mixed;   // main pass
     MixedPlan mixed2;  // second pass (BF16 count pass) over the rows an FP8 main pass left open
     MixedPlan mixedm2; // its mask pass (BF16, the slicing of mixed2)
