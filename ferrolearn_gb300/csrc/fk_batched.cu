@@ -11,11 +11,14 @@
 //   batch_assign_kernel  per Lloyd iteration, one persistent launch per
 //                        (d, k) bucket over a queue of (fit, row range) items,
 //                        largest fits first; the fit's centres in shared
-//                        memory, rows in registers; direct-form f32 distances
+//                        memory; rows that cannot have changed their label
+//                        score one centre, the others every centre, rows in
+//                        registers; direct-form f32 distances
 //                        (no FMA), strict < from F::MAX. The tile shape (rows
 //                        per thread x centres per pass) is the autotuner's
 //                        choice for the bucket. Per item a fixed-tree f64
 //                        inertia partial.
+//   batch_near_kernel    the thresholds of that test for the next iteration.
 //   batch_accum_kernel   f64 reduction: the exact (integer, order-free) sums of
 //                        each (fit, row range) item added to its fit's;
 //   batch_means_kernel   then per fit each sum rounded once to f64 with the mean
@@ -52,8 +55,9 @@ struct BFit {
     int32_t n, d, k, max_iter;
     float tol;
     int32_t first_item, n_items;
-    int32_t prob, pad;
-    int64_t k_off;  // offset of this fit's k cluster counts
+    int32_t prob;
+    int32_t bounded;  // rows are tested against their last label's centre first
+    int64_t k_off;    // offset of this fit's k cluster counts and row thresholds
     uint64_t seed;
 };
 
@@ -70,6 +74,7 @@ constexpr int ASSIGN_T = 128;
 constexpr int UPDATE_T = 256;
 constexpr int NBUCKETS = 20;  // d in {8, 16, 32, 64, other} x k in {<=16, <=32, <=64, >64}
 constexpr int NVARIANTS = 5;  // (rows per thread, centres per pass): (1,1) (2,1) (1,2) (2,2) (4,1)
+constexpr int BOUND_K = 128;  // clusters of a bounded fit at most
 constexpr int MAX_K = 1024, MAX_D = 256, MAX_KD = 32768;
 
 // squared_euclidean (kmeans.rs:159-163) in f32: left fold, no FMA.
@@ -96,18 +101,63 @@ __device__ __forceinline__ double block_sum_f64(double v, double *sh) {
     return r;
 }
 
-// D > 0: rows of exactly D features in registers (TR per thread), CP centres
-// per pass; D = 0: any d, one row and one centre at a time.
+// Rows of an item at most, features staged at a time, stages.
+constexpr int ITEM_ROWS = 1024, ROW_SLAB = 32, ROW_STAGES = 2;
+__host__ __device__ constexpr int row_slab(int d) { return d < ROW_SLAB ? d : ROW_SLAB; }
+// Row stride in shared memory: an odd number of 16-byte units, so that eight
+// lanes reading 16 bytes of eight rows meet no bank conflict (d = 8, 16, 32, 64).
+__host__ __device__ constexpr int row_stride(int d) { return d + 4; }
+// Rows of up to 16 features are read straight into registers.
+__host__ __device__ constexpr bool rows_staged(int d) { return d > 16; }
+size_t assign_smem(int d, int k) {
+    const size_t stages = rows_staged(d) ? (size_t)ROW_STAGES * ASSIGN_T * row_stride(row_slab(d)) : 0;
+    return sizeof(float) * ((size_t)k * row_stride(d) + stages + ITEM_ROWS) + sizeof(uint16_t) * ITEM_ROWS;
+}
+
+__device__ __forceinline__ void copy16_async(float *dst, const float *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+
+// acc + (a - b)^2 over four features in order, no FMA.
+__device__ __forceinline__ float add_sq4(float acc, const float4 &a, const float4 &b) {
+    const float t0 = __fsub_rn(a.x, b.x), t1 = __fsub_rn(a.y, b.y), t2 = __fsub_rn(a.z, b.z), t3 = __fsub_rn(a.w, b.w);
+    acc = __fadd_rn(acc, __fmul_rn(t0, t0));
+    acc = __fadd_rn(acc, __fmul_rn(t1, t1));
+    acc = __fadd_rn(acc, __fmul_rn(t2, t2));
+    return __fadd_rn(acc, __fmul_rn(t3, t3));
+}
+
+// D > 0: rows of exactly D features; D = 0: any d, one row and one centre at a
+// time.
+//
+// From a fit's second iteration on, a row is first scored against the centre
+// of its last label only: a distance below thr,
+// a quarter of the centre's squared distance to its nearest other centre with
+// room for every rounding (batch_near_kernel), leaves every other centre
+// strictly farther, so the label stays and the distance is its term of the
+// inertia. The other rows are listed and scored against every centre: rows in
+// registers (TR per thread), CP centres per pass, shared-memory reads of the
+// centres against 3 FP32 operations each. The inertia's terms meet in shared
+// memory and are added in row order, whichever way they came.
+//
+// 64 problems x 10 runs (d 8 to 64, k 4 to 64, 2,000 to 200,000 rows): 108 ms in
+// these kernels with every row scored against every centre, 51 ms like this
+// (whole call 142 -> 115 ms). Items of 8,192 rows, as few centres and features
+// once had, made a CTA's 64 passes in turn the length of an iteration (104 us at
+// d = 8; 15 us with 1,024); rows of 8 or 16 features cost less read directly.
 template <int D, int TR, int CP>
 __global__ void __launch_bounds__(ASSIGN_T) batch_assign_kernel(const float *__restrict__ X,
                                                                 const BFit *__restrict__ fits,
                                                                 const BState *__restrict__ state,
                                                                 const BItem *__restrict__ items, int nitems,
                                                                 int *counter, const float *__restrict__ C,
-                                                                int *__restrict__ lab, double *__restrict__ partial) {
-    extern __shared__ float cs[];
-    __shared__ int it_sh;
+                                                                const float *__restrict__ thr, int *__restrict__ lab,
+                                                                double *__restrict__ partial) {
+    extern __shared__ __align__(16) float cs[];
+    __shared__ int it_sh, list_n;
     __shared__ double red[ASSIGN_T / 32];
+    constexpr int CS = D > 0 ? row_stride(D) : 0, W = row_slab(D), XS = row_stride(W);
     const int tid = threadIdx.x;
     int loaded = -1;
     while (true) {
@@ -123,7 +173,7 @@ __global__ void __launch_bounds__(ASSIGN_T) batch_assign_kernel(const float *__r
         const int d = D > 0 ? D : F.d, k = F.k;
         if (f != loaded) {
             const float *src = C + F.c_off + (int64_t)state[f].cur * k * d;
-            for (int e = tid; e < k * d; e += ASSIGN_T) cs[e] = src[e];
+            for (int e = tid; e < k * d; e += ASSIGN_T) cs[D > 0 ? e / D * CS + e % D : e] = src[e];
             __syncthreads();
             loaded = f;
         }
@@ -131,16 +181,107 @@ __global__ void __launch_bounds__(ASSIGN_T) batch_assign_kernel(const float *__r
         int *L = lab + F.s_off;
         double s = 0.0;
         if constexpr (D > 0) {
-            for (int base = I.lo; base < I.hi; base += ASSIGN_T * TR) {
+            float *const xs = cs + k * CS;  // [ROW_STAGES][ASSIGN_T][XS]
+            float *const vals = xs + (rows_staged(D) ? ROW_STAGES * ASSIGN_T * XS : 0);  // [ITEM_ROWS] distances
+            uint16_t *const list = reinterpret_cast<uint16_t *>(vals + ITEM_ROWS);       // [ITEM_ROWS] rows to score
+            const bool bounded = F.bounded && state[f].n_iter > 0;
+            const int rows = I.hi - I.lo;
+            const float *const xi = x + (int64_t)I.lo * D;
+            int nl = rows;
+            if (bounded) {
+                if (tid == 0) list_n = 0;
+                // row i (live: it exists) at distance v from its label's centre
+                auto settle = [&](int i, bool live, float v, float th) {
+                    const bool open = live && !(v < th);  // NaN: open
+                    if (live && !open) vals[i] = v;
+                    const unsigned bm = __ballot_sync(0xffffffffu, open);
+                    int at = 0;
+                    if ((tid & 31) == 0 && bm) at = atomicAdd(&list_n, __popc(bm));
+                    at = __shfl_sync(0xffffffffu, at, 0);
+                    if (open) list[at + __popc(bm & ((1u << (tid & 31)) - 1u))] = (uint16_t)i;
+                };
+                if constexpr (!rows_staged(D)) {
+                    __syncthreads();
+                    constexpr int U = 4;  // rows a thread at a time, their loads in flight together
+                    for (int st = 0; st < rows; st += U * ASSIGN_T) {
+                        float4 xv[U][D / 4];
+                        float th[U];
+                        int l[U];
+#pragma unroll
+                        for (int u = 0; u < U; u++) {
+                            const int i = st + u * ASSIGN_T + tid;
+                            l[u] = i < rows ? L[I.lo + i] : 0;
+#pragma unroll
+                            for (int q = 0; q < D / 4; q++)
+                                xv[u][q] = i < rows ? reinterpret_cast<const float4 *>(xi + (int64_t)i * D)[q]
+                                                    : make_float4(0.f, 0.f, 0.f, 0.f);
+                        }
+#pragma unroll
+                        for (int u = 0; u < U; u++) th[u] = thr[F.k_off + l[u]];
+#pragma unroll
+                        for (int u = 0; u < U; u++) {
+                            const int i = st + u * ASSIGN_T + tid;
+                            const float4 *cv = reinterpret_cast<const float4 *>(cs + l[u] * CS);
+                            float acc = 0.f;
+#pragma unroll
+                            for (int q = 0; q < D / 4; q++) acc = add_sq4(acc, xv[u][q], cv[q]);
+                            settle(i, i < rows, acc, th[u]);
+                        }
+                    }
+                } else {
+                    // slab by slab (W features of ASSIGN_T rows), the next one's copies in flight
+                    constexpr int SL = D / W;
+                    const int ns = (rows + ASSIGN_T - 1) / ASSIGN_T * SL;
+                    auto fetch = [&](int g) {
+                        const int st = g / SL * ASSIGN_T, j0 = g % SL * W, cnt = min(ASSIGN_T, rows - st);
+                        float *dst = xs + g % ROW_STAGES * ASSIGN_T * XS;
+                        for (int e = tid; e < cnt * (W / 4); e += ASSIGN_T) {
+                            const int r = e / (W / 4), q = e % (W / 4);
+                            copy16_async(dst + r * XS + 4 * q, xi + (int64_t)(st + r) * D + j0 + 4 * q);
+                        }
+                        asm volatile("cp.async.commit_group;" ::: "memory");
+                    };
+                    fetch(0);
+                    float acc = 0.f, th = 0.f;
+                    int l = 0;
+                    for (int g = 0; g < ns; g++) {
+                        const int i = g / SL * ASSIGN_T + tid;
+                        if (g % SL == 0) {
+                            l = i < rows ? L[I.lo + i] : 0;
+                            th = thr[F.k_off + l];
+                            acc = 0.f;
+                        }
+                        if (g + 1 < ns) {
+                            fetch(g + 1);
+                            asm volatile("cp.async.wait_group 1;" ::: "memory");
+                        } else {
+                            asm volatile("cp.async.wait_group 0;" ::: "memory");
+                        }
+                        __syncthreads();
+                        if (i < rows) {
+                            const float4 *xv = reinterpret_cast<const float4 *>(xs + (g % ROW_STAGES * ASSIGN_T + tid) * XS);
+                            const float4 *cv = reinterpret_cast<const float4 *>(cs + l * CS + g % SL * W);
+#pragma unroll
+                            for (int q = 0; q < W / 4; q++) acc = add_sq4(acc, xv[q], cv[q]);
+                        }
+                        if (g % SL == SL - 1) settle(i, i < rows, acc, th);
+                        __syncthreads();  // the stage is free for the fetch after next
+                    }
+                }
+                __syncthreads();
+                nl = list_n;
+            }
+            for (int base = 0; base < nl; base += ASSIGN_T * TR) {
                 float xr[TR][D];
-                int rr[TR];
+                int rr[TR];  // row of the item, -1: none
 #pragma unroll
                 for (int u = 0; u < TR; u++) {
-                    rr[u] = base + tid + u * ASSIGN_T;
-                    const bool ok = rr[u] < I.hi;
+                    const int i = base + tid + u * ASSIGN_T;
+                    const bool ok = i < nl;
+                    rr[u] = ok ? (bounded ? (int)list[i] : i) : -1;
 #pragma unroll
                     for (int j4 = 0; j4 < D / 4; j4++) {
-                        const float4 v = ok ? reinterpret_cast<const float4 *>(x + (int64_t)rr[u] * D)[j4]
+                        const float4 v = ok ? reinterpret_cast<const float4 *>(x + (int64_t)(I.lo + rr[u]) * D)[j4]
                                             : make_float4(0.f, 0.f, 0.f, 0.f);
                         xr[u][4 * j4] = v.x;
                         xr[u][4 * j4 + 1] = v.y;
@@ -165,7 +306,7 @@ __global__ void __launch_bounds__(ASSIGN_T) batch_assign_kernel(const float *__r
                     for (int j = 0; j < D; j++) {
 #pragma unroll
                         for (int p = 0; p < CP; p++) {
-                            const float cv = c + p < k ? cs[(c + p) * D + j] : 0.f;
+                            const float cv = c + p < k ? cs[(c + p) * CS + j] : 0.f;
 #pragma unroll
                             for (int u = 0; u < TR; u++) {
                                 const float t = __fsub_rn(xr[u][j], cv);
@@ -185,11 +326,13 @@ __global__ void __launch_bounds__(ASSIGN_T) batch_assign_kernel(const float *__r
                 }
 #pragma unroll
                 for (int u = 0; u < TR; u++)
-                    if (rr[u] < I.hi) {
-                        L[rr[u]] = bi[u];
-                        s += (double)best[u];
+                    if (rr[u] >= 0) {
+                        L[I.lo + rr[u]] = bi[u];
+                        vals[rr[u]] = best[u];
                     }
             }
+            __syncthreads();
+            for (int i = tid; i < rows; i += ASSIGN_T) s += (double)vals[i];
         } else {
             for (int r = I.lo + tid; r < I.hi; r += ASSIGN_T) {
                 const float *xr = x + (int64_t)r * d;
@@ -209,6 +352,50 @@ __global__ void __launch_bounds__(ASSIGN_T) batch_assign_kernel(const float *__r
         const double tot = block_sum_f64(s, red);
         if (tid == 0) partial[it] = tot;
         __syncthreads();
+    }
+}
+
+constexpr int NEAR_T = 256, NEAR_PARTS = 4;
+
+// Row thresholds of a bounded fit's next iteration, one per centre (CTA
+// (fit, part): every NEAR_PARTS-th group of centres, a warp a centre, lanes over
+// the others, all of the fit's centres in shared memory). thr[q] = (1 - rho) / 4
+// of a lower bound of the smallest squared distance from centre q to another:
+// a row whose computed distance m to q is below it is at least m (1 + 2 rho - 8g)
+// > m from every other centre, in computed distances too, with g = (d + 4) u
+// the relative error of a direct form and rho = (d + 8) 1e-6 (the triangle
+// inequality: D(x, q) <= m (1 + 2g), so sqrt D(x, c) >= sqrt D(q, c) -
+// sqrt D(x, q) >= sqrt D(x, q) (1 + rho - 2g)). Distances below 1e-30, where
+// underflow would count, and NaN give 0: no row is below it.
+__global__ void __launch_bounds__(NEAR_T)
+    batch_near_kernel(const BFit *__restrict__ fits, const BState *__restrict__ state, const int *__restrict__ order,
+                      const float *__restrict__ C, float *__restrict__ thr) {
+    const int f = order[blockIdx.x];
+    const BFit F = fits[f];
+    if (!F.bounded || state[f].done) return;
+    extern __shared__ __align__(16) float cs[];
+    const int d = F.d, k = F.k, stride = d + 1;  // odd: lanes over rows meet no bank conflict
+    const int tid = threadIdx.x, lane = tid & 31;
+    if ((int)blockIdx.y * (NEAR_T / 32) >= k) return;
+    const float *src = C + F.c_off + (int64_t)state[f].cur * k * d;
+    for (int e = tid; e < k * d; e += NEAR_T) cs[e / d * stride + e % d] = src[e];
+    __syncthreads();
+    const float rho = (float)(d + 8) * 1e-6f;
+    for (int q = (int)blockIdx.y * (NEAR_T / 32) + (tid >> 5); q < k; q += NEAR_PARTS * (NEAR_T / 32)) {
+        float th = FLT_MAX;
+        for (int c = lane; c < k; c += 32) {
+            float v = 0.f;
+#pragma unroll 8
+            for (int j = 0; j < d; j++) {
+                const float t = __fsub_rn(cs[c * stride + j], cs[q * stride + j]);
+                v = __fmaf_rn(t, t, v);
+            }
+            const float b = 0.25f * __fsub_rd(v, bound32(v, 0.f, d)) * (1.0f - rho);
+            if (c != q) th = b < th ? b : (b >= th ? th : 0.f);  // NaN: 0
+        }
+#pragma unroll
+        for (int o = 16; o >= 1; o >>= 1) th = fminf(th, __shfl_xor_sync(0xffffffffu, th, o));
+        if (lane == 0) thr[F.k_off + q] = th > 1e-30f ? th : 0.f;
     }
 }
 
@@ -663,7 +850,7 @@ int kbucket(int k) { return k <= 16 ? 0 : k <= 32 ? 1 : k <= 64 ? 2 : 3; }
 int bucket_d(int b) { static const int v[5] = {8, 16, 32, 64, 0}; return v[b / 4]; }
 
 using AssignFn = void (*)(const float *, const BFit *, const BState *, const BItem *, int, int *, const float *,
-                          int *, double *);
+                          const float *, int *, double *);
 
 template <int D>
 AssignFn pick_variant(int v) {
@@ -773,6 +960,8 @@ fk_status batched_fit_impl(Ctx &ctx, fk_batch_problem *P, int64_t np, int reduct
             F.tol = (float)q.tol;
             F.seed = q.random_state + (uint64_t)r;
             F.prob = (int32_t)p;
+            // the thresholds cost k^2 d in one CTA group a fit: little beside n k d
+            F.bounded = dbucket(F.d) < 4 && F.k <= BOUND_K && (int64_t)F.n >= 16 * (int64_t)F.k;
             fits.push_back(F);
             fit_prob.push_back((int)p);
             fit_run.push_back((int)r);
@@ -794,7 +983,7 @@ fk_status batched_fit_impl(Ctx &ctx, fk_batch_problem *P, int64_t np, int reduct
         for (int f : byc) {
             BFit &F = fits[f];
             if (dbucket(F.d) * 4 + kbucket(F.k) != b) continue;
-            const int ch = std::max(128, std::min(8192, (int)(4194304.0 / ((double)F.k * F.d * 3.0)) / 128 * 128));
+            const int ch = std::max(128, std::min(ITEM_ROWS, (int)(4194304.0 / ((double)F.k * F.d * 3.0)) / 128 * 128));
             F.first_item = (int)items.size();
             for (int lo = 0; lo < F.n; lo += ch) items.push_back(BItem{f, lo, std::min(F.n, lo + ch), 0});
             F.n_items = (int)items.size() - F.first_item;
@@ -821,6 +1010,7 @@ fk_status batched_fit_impl(Ctx &ctx, fk_batch_problem *P, int64_t np, int reduct
     int *dctr = (int *)ctx.get(BUF_BCTR, sizeof(int) * 32);
     int *dlab = (int *)ctx.get(BUF_BLAB, sizeof(int) * (size_t)soff + 16);
     int *dmem = (int *)ctx.get(BUF_BMEM, sizeof(int) * (size_t)soff + 16);
+    float *dthr = (float *)ctx.get(BUF_BTHR, sizeof(float) * (size_t)koff + 16);
     float *dC = (float *)ctx.get(BUF_BCEN, sizeof(float) * (size_t)coff + 16);
     int64_t *dxo = (int64_t *)ctx.get(BUF_BXOFF, sizeof(int64_t) * (size_t)(2 * np) + sizeof(float) * (size_t)np + 64);
     float *damax = (float *)(dxo + 2 * np);
@@ -899,16 +1089,21 @@ fk_status batched_fit_impl(Ctx &ctx, fk_batch_problem *P, int64_t np, int reduct
     FK_CUDA(cudaEventRecord(ev[2], s));
 
     // ---- autotuner: time every variant of each new (d, k) bucket on its items
-    int bmaxkd[NBUCKETS] = {0};
+    size_t bsmem[NBUCKETS] = {0};
+    size_t near_smem = 0;
     for (const BFit &F : fits) {
         const int b = dbucket(F.d) * 4 + kbucket(F.k);
-        bmaxkd[b] = std::max(bmaxkd[b], F.k * F.d);
+        bsmem[b] = std::max(bsmem[b], bucket_d(b) ? assign_smem(F.d, F.k) : sizeof(float) * (size_t)(F.k * F.d));
+        if (F.bounded) near_smem = std::max(near_smem, sizeof(float) * (size_t)F.k * (size_t)(F.d + 1));
     }
+    if (near_smem)
+        FK_CUDA(cudaFuncSetAttribute((const void *)batch_near_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)near_smem));
     int64_t tuned = 0;
     for (int b = 0; b < NBUCKETS; b++) {
         const int cnt = bstart[b + 1] - bstart[b];
         if (cnt == 0) continue;
-        const size_t smem = sizeof(float) * (size_t)bmaxkd[b];
+        const size_t smem = bsmem[b];
         for (int v = 0; v < n_variants(b); v++)
             FK_CUDA(cudaFuncSetAttribute((const void *)assign_fn(b, v), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)std::max<size_t>(smem, 1)));
@@ -920,7 +1115,7 @@ fk_status batched_fit_impl(Ctx &ctx, fk_batch_problem *P, int64_t np, int reduct
             FK_CUDA(cudaMemsetAsync(dctr + b, 0, sizeof(int), s));
             FK_CUDA(cudaEventRecord(ev[4], s));
             assign_fn(b, v)<<<grid, ASSIGN_T, smem, s>>>(X, dfits, dstate, ditems + bstart[b], cnt, dctr + b, dC,
-                                                          dlab, dpart + bstart[b]);
+                                                          dthr, dlab, dpart + bstart[b]);
             FK_LAUNCH_CHECK();
             FK_CUDA(cudaEventRecord(ev[5], s));
             FK_CUDA(cudaEventSynchronize(ev[5]));
@@ -943,8 +1138,8 @@ fk_status batched_fit_impl(Ctx &ctx, fk_batch_problem *P, int64_t np, int reduct
             const int cnt = bstart[b + 1] - bstart[b];
             if (cnt == 0) continue;
             const int grid = std::min(cnt, ctx.num_sms * 8);
-            assign_fn(b, ctx.batch_variant[b])<<<grid, ASSIGN_T, sizeof(float) * (size_t)bmaxkd[b], s>>>(
-                X, dfits, dstate, ditems + bstart[b], cnt, dctr + b, dC, dlab, dpart + bstart[b]);
+            assign_fn(b, ctx.batch_variant[b])<<<grid, ASSIGN_T, bsmem[b], s>>>(
+                X, dfits, dstate, ditems + bstart[b], cnt, dctr + b, dC, dthr, dlab, dpart + bstart[b]);
         }
         const int ug = std::min(nf, ctx.num_sms * 4);
         if (reduction == FK_REDUCE_F64) {
@@ -956,6 +1151,8 @@ fk_status batched_fit_impl(Ctx &ctx, fk_batch_problem *P, int64_t np, int reduct
             batch_update_kernel<<<ug, UPDATE_T, 0, s>>>(X, dfits, dstate, dorder, nf, dctr + 20, dC, dlab, dmem, dpart,
                                                         dctr + 31);
         }
+        if (near_smem)
+            batch_near_kernel<<<dim3((unsigned)nf, NEAR_PARTS), NEAR_T, near_smem, s>>>(dfits, dstate, dorder, dC, dthr);
     };
     int max_iter = 0;
     for (const BFit &F : fits) max_iter = std::max(max_iter, F.max_iter);
