@@ -873,6 +873,37 @@ AssignFn assign_fn(int bucket, int v) {
     }
 }
 
+// Streams that a capture forks to (nothing runs on them outside it).
+struct Branches {
+    static constexpr int N = 4;
+    cudaStream_t stream[N] = {};
+    cudaEvent_t fork = nullptr, join[N] = {};
+    Branches() {
+        try {
+            FK_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+            for (int q = 0; q < N; q++) {
+                FK_CUDA(cudaStreamCreateWithFlags(&stream[q], cudaStreamNonBlocking));
+                FK_CUDA(cudaEventCreateWithFlags(&join[q], cudaEventDisableTiming));
+            }
+        } catch (...) {
+            release();
+            throw;
+        }
+    }
+    Branches(const Branches &) = delete;
+    Branches &operator=(const Branches &) = delete;
+    ~Branches() { release(); }
+
+  private:
+    void release() {
+        for (int q = 0; q < N; q++) {
+            if (join[q]) cudaEventDestroy(join[q]);
+            if (stream[q]) cudaStreamDestroy(stream[q]);
+        }
+        if (fork) cudaEventDestroy(fork);
+    }
+};
+
 int n_variants(int bucket) {
     const int d = bucket_d(bucket);
     return d == 0 ? 1 : d == 64 ? 3 : NVARIANTS;
@@ -1131,15 +1162,24 @@ fk_status batched_fit_impl(Ctx &ctx, fk_batch_problem *P, int64_t np, int reduct
     }
     FK_CUDA(cudaEventRecord(ev[3], s));
 
-    // ---- Lloyd iterations: one captured iteration, replayed
+    // ---- Lloyd iterations: one captured iteration, replayed. The buckets'
+    // assignments are independent: branches of the graph.
+    Branches side;
     auto one_iteration = [&]() {
         FK_CUDA(cudaMemsetAsync(dctr, 0, sizeof(int) * 22, s));
+        FK_CUDA(cudaEventRecord(side.fork, s));
+        for (int q = 0; q < Branches::N; q++) FK_CUDA(cudaStreamWaitEvent(side.stream[q], side.fork, 0));
+        int at = 0;
         for (int b = 0; b < NBUCKETS; b++) {
             const int cnt = bstart[b + 1] - bstart[b];
             if (cnt == 0) continue;
             const int grid = std::min(cnt, ctx.num_sms * 8);
-            assign_fn(b, ctx.batch_variant[b])<<<grid, ASSIGN_T, bsmem[b], s>>>(
+            assign_fn(b, ctx.batch_variant[b])<<<grid, ASSIGN_T, bsmem[b], side.stream[at++ % Branches::N]>>>(
                 X, dfits, dstate, ditems + bstart[b], cnt, dctr + b, dC, dthr, dlab, dpart + bstart[b]);
+        }
+        for (int q = 0; q < Branches::N; q++) {
+            FK_CUDA(cudaEventRecord(side.join[q], side.stream[q]));
+            FK_CUDA(cudaStreamWaitEvent(s, side.join[q], 0));
         }
         const int ug = std::min(nf, ctx.num_sms * 4);
         if (reduction == FK_REDUCE_F64) {
