@@ -55,15 +55,17 @@ struct BFit {
     int32_t n, d, k, max_iter;
     float tol;
     int32_t first_item, n_items;
-    int32_t prob;
-    int32_t bounded;  // rows are tested against their last label's centre first
+    int32_t prob, pad;
+    int32_t keep_sums;  // f64 reduction: the sums carry over to the next iteration
+    int32_t bounded;    // rows are tested against their last label's centre first
     int64_t k_off;    // offset of this fit's k cluster counts and row thresholds
     uint64_t seed;
 };
 
 struct BState {
     double inertia;
-    int32_t cur, n_iter, done, pad;
+    int32_t cur, n_iter, done;
+    int32_t full;  // f64 reduction: the sums are zero, every row is to be added
 };
 
 struct BItem {
@@ -479,7 +481,10 @@ __device__ __forceinline__ int bitlen64(long long v) { return 64 - __clzll(v > 0
 // The f64 reduction's running sums: per (cluster, feature) of every fit the two
 // integer sums, and the parts the grids cannot hold -- the 128-bit remainder in
 // four 32-bit limbs (added limb by limb, carries resolved at the end) and what
-// non-finite values occurred. The update kernel leaves all of it zero.
+// non-finite values occurred. Integer sums can be undone exactly: they carry
+// over, and an iteration only moves the rows whose label changed. A fit with
+// non-finite values, or one so long that the limbs could overflow (2^32
+// additions of 32 bits), starts from zero each time instead.
 struct BSums {
     unsigned long long *a1, *a2;  // two's complement
     unsigned long long *limb;     // [4] each
@@ -506,100 +511,141 @@ struct ExactGrid {
 };
 
 constexpr int ACC_T = 256;
+constexpr unsigned LEAVES = 0x8000u;
 constexpr int ACC_ROWS = 1024;  // rows of an item at most: with 5,000, the last fits' few items ran 130 us (1,024: 33 us)
 
-// The f64 reduction's sums of one (fit, row range) item: the item's rows
-// grouped by cluster in shared memory, then a thread per (cluster, feature)
-// over the cluster's rows (neighbouring threads read neighbouring features)
-// and one addition to the fit's sums. Integer sums are order-free, so any
+// The f64 reduction's sums of one (fit, row range) item: the item's rows whose
+// label changed, once for the cluster they join and once for the one they
+// leave, grouped by cluster in shared memory; then a thread per (cluster,
+// feature) over the cluster's entries (neighbouring threads read neighbouring
+// features) and one addition to the fit's sums. Integer sums are order-free, so any
 // number of CTAs can share a fit: 64 problems x 10 runs took 427 ms of 994
-// with one CTA a fit, its largest fits' sorts and chains last.
+// with one CTA a fit, its largest fits' sorts and chains last; 28 of 107 with
+// every row added in every iteration.
 __global__ void __launch_bounds__(ACC_T) batch_accum_kernel(const float *__restrict__ X, const BFit *__restrict__ fits,
                                                             const BState *__restrict__ state,
-                                                            const BItem *__restrict__ items, int nitems, int *counter,
-                                                            const int *__restrict__ lab,
+                                                            const BItem *__restrict__ items, int nitems,
+                                                            const int *__restrict__ lab, int *__restrict__ prev,
                                                             const float *__restrict__ pamax, BSums S) {
-    __shared__ unsigned short ids[ACC_ROWS];
-    __shared__ int hist[MAX_K], off[MAX_K];
-    __shared__ int it_sh;
+    __shared__ unsigned short ids[2 * ACC_ROWS];  // row, LEAVES: subtracted
+    __shared__ int hist[MAX_K], off[MAX_K], net[MAX_K];
+    __shared__ int todo[ACC_T], todo_n;
     const int tid = threadIdx.x, lane = tid & 31;
-    while (true) {
-        if (tid == 0) it_sh = atomicAdd(counter, 1);
+    // ACC_T of the block's items (every gridDim.x-th) looked at together: most
+    // belong to converged fits (30 us an iteration one by one)
+    for (int it0 = blockIdx.x; it0 < nitems; it0 += ACC_T * gridDim.x) {
+        if (tid == 0) todo_n = 0;
         __syncthreads();
-        const int it = it_sh;
+        const int64_t mine = it0 + (int64_t)tid * gridDim.x;
+        if (mine < nitems && !state[items[mine].fit].done) todo[atomicAdd(&todo_n, 1)] = (int)mine;
         __syncthreads();
-        if (it >= nitems) break;
-        const BItem I = items[it];
-        if (state[I.fit].done) continue;
-        const BFit F = fits[I.fit];
-        const int d = F.d, k = F.k, rows = I.hi - I.lo;
-        const int *L = lab + F.s_off + I.lo;
-        for (int c = tid; c < k; c += ACC_T) hist[c] = 0;
-        __syncthreads();
-        for (int r = tid; r < rows; r += ACC_T) atomicAdd(&hist[L[r]], 1);
-        __syncthreads();
-        if (tid < 32) {
-            int base = 0;
-            for (int c0 = 0; c0 < k; c0 += 32) {
-                const int v = c0 + lane < k ? hist[c0 + lane] : 0;
-                int s = v;
+        for (int q = 0; q < todo_n; q++) {
+            const BItem I = items[todo[q]];
+            const BFit F = fits[I.fit];
+            const int d = F.d, k = F.k, rows = I.hi - I.lo;
+            const bool full = state[I.fit].full != 0;
+            int nw[ACC_ROWS / ACC_T], old[ACC_ROWS / ACC_T];  // a row without a change: equal
+            bool any = false;
 #pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int u = __shfl_up_sync(0xffffffffu, s, o);
-                    if (lane >= o) s += u;
+            for (int u = 0; u < ACC_ROWS / ACC_T; u++) {
+                const int r = u * ACC_T + tid;
+                nw[u] = old[u] = -1;
+                if (r < rows) {
+                    const int64_t at = F.s_off + I.lo + r;
+                    nw[u] = lab[at];
+                    if (!full) old[u] = prev[at];
+                    if (nw[u] != old[u]) {
+                        prev[at] = nw[u];
+                        any = true;
+                    }
                 }
-                if (c0 + lane < k) {
-                    off[c0 + lane] = base + s - v;
-                    if (v) atomicAdd(S.count + F.k_off + c0 + lane, v);
-                }
-                base += __shfl_sync(0xffffffffu, s, 31);
             }
-        }
-        __syncthreads();
-        for (int r = tid; r < rows; r += ACC_T) ids[atomicAdd(&off[L[r]], 1)] = (unsigned short)r;
-        __syncthreads();  // off[c] is now the end of cluster c's rows
-        const ExactGrid g(pamax[F.prob], F.n);
-        const float *x = X + F.x_off + (int64_t)I.lo * d;
-        const int64_t a_off = F.c_off / 2;
-        // few clusters and features: several threads share one's rows
-        const int kd = k * d, nsub = max(1, ACC_T / kd);
-        for (int q = tid; q < kd * nsub; q += ACC_T) {
-            const int sub = q / kd, pr = q - sub * kd;
-            const int c = pr / d, j = pr - c * d;
-            const int cnt = hist[c], o = off[c] - cnt;
-            long long a1 = 0, a2 = 0;
-            uint64_t slo = 0, shi = 0;
-            uint32_t fl = 0;
+            if (!__syncthreads_or(any)) continue;
+            for (int c = tid; c < k; c += ACC_T) hist[c] = net[c] = 0;
+            __syncthreads();
+#pragma unroll
+            for (int u = 0; u < ACC_ROWS / ACC_T; u++) {
+                if (nw[u] == old[u]) continue;
+                atomicAdd(&hist[nw[u]], 1);
+                atomicAdd(&net[nw[u]], 1);
+                if (old[u] >= 0) {
+                    atomicAdd(&hist[old[u]], 1);
+                    atomicSub(&net[old[u]], 1);
+                }
+            }
+            __syncthreads();
+            if (tid < 32) {
+                int base = 0;
+                for (int c0 = 0; c0 < k; c0 += 32) {
+                    const int v = c0 + lane < k ? hist[c0 + lane] : 0;
+                    int s = v;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int u = __shfl_up_sync(0xffffffffu, s, o);
+                        if (lane >= o) s += u;
+                    }
+                    if (c0 + lane < k) {
+                        off[c0 + lane] = base + s - v;
+                        if (net[c0 + lane]) atomicAdd(S.count + F.k_off + c0 + lane, net[c0 + lane]);
+                    }
+                    base += __shfl_sync(0xffffffffu, s, 31);
+                }
+            }
+            __syncthreads();
+#pragma unroll
+            for (int u = 0; u < ACC_ROWS / ACC_T; u++) {
+                if (nw[u] == old[u]) continue;
+                const unsigned short r = (unsigned short)(u * ACC_T + tid);
+                ids[atomicAdd(&off[nw[u]], 1)] = r;
+                if (old[u] >= 0) ids[atomicAdd(&off[old[u]], 1)] = (unsigned short)(r | LEAVES);
+            }
+            __syncthreads();  // off[c] is now the end of cluster c's entries
+            const ExactGrid g(pamax[F.prob], F.n);
+            const float *x = X + F.x_off + (int64_t)I.lo * d;
+            const int64_t a_off = F.c_off / 2;
+            // few clusters and features: several threads share one's rows
+            const int kd = k * d, nsub = max(1, ACC_T / kd);
+            for (int q = tid; q < kd * nsub; q += ACC_T) {
+                const int sub = q / kd, pr = q - sub * kd;
+                const int c = pr / d, j = pr - c * d;
+                const int cnt = hist[c], o = off[c] - cnt;
+                long long a1 = 0, a2 = 0;
+                uint64_t slo = 0, shi = 0;
+                uint32_t fl = 0;
 #pragma unroll 8
-            for (int m = sub; m < cnt; m += nsub) {
-                const float xv = x[(int64_t)ids[o + m] * d + j];
-                if (!(fabsf(xv) < INFINITY)) {
-                    fl |= xv != xv ? FLAG_NAN : (xv > 0.f ? FLAG_PINF : FLAG_NINF);
-                } else if (g.grids) {
-                    const float s1 = __fadd_rn(xv, g.C1);
-                    a1 += __float_as_int(s1) - g.b1;
-                    const float r = __fsub_rn(xv, __fsub_rn(s1, g.C1));
-                    const float s2 = __fadd_rn(r, g.C2);
-                    a2 += __float_as_int(s2) - g.b2;
-                    const float r2 = __fsub_rn(r, __fsub_rn(s2, g.C2));
-                    if (r2 != 0.f) fixed_add_small(slo, shi, r2, g.F);
-                } else {
-                    fixed_add_small(slo, shi, xv, g.F);
+                for (int m = sub; m < cnt; m += nsub) {
+                    const unsigned id = ids[o + m];
+                    const float xr = x[(int64_t)(id & (LEAVES - 1u)) * d + j];
+                    const float xv = id & LEAVES ? -xr : xr;  // every step below is odd in xv
+                    if (!(fabsf(xv) < INFINITY)) {
+                        fl |= xv != xv ? FLAG_NAN : (xv > 0.f ? FLAG_PINF : FLAG_NINF);
+                    } else if (g.grids) {
+                        const float s1 = __fadd_rn(xv, g.C1);
+                        a1 += __float_as_int(s1) - g.b1;
+                        const float r = __fsub_rn(xv, __fsub_rn(s1, g.C1));
+                        const float s2 = __fadd_rn(r, g.C2);
+                        a2 += __float_as_int(s2) - g.b2;
+                        const float r2 = __fsub_rn(r, __fsub_rn(s2, g.C2));
+                        if (r2 != 0.f) fixed_add_small(slo, shi, r2, g.F);
+                    } else {
+                        fixed_add_small(slo, shi, xv, g.F);
+                    }
                 }
+                const int64_t e = a_off + pr;
+                if (a1) atomicAdd(S.a1 + e, (unsigned long long)a1);
+                if (a2) atomicAdd(S.a2 + e, (unsigned long long)a2);
+                if (slo | shi) {
+                    fl |= FLAG_LIMBS;
+                    atomicAdd(S.limb + 4 * e, slo & 0xFFFFFFFFull);
+                    atomicAdd(S.limb + 4 * e + 1, slo >> 32);
+                    atomicAdd(S.limb + 4 * e + 2, shi & 0xFFFFFFFFull);
+                    atomicAdd(S.limb + 4 * e + 3, shi >> 32);
+                }
+                if (fl) atomicOr(S.flags + e, fl);
             }
-            const int64_t e = a_off + pr;
-            if (a1) atomicAdd(S.a1 + e, (unsigned long long)a1);
-            if (a2) atomicAdd(S.a2 + e, (unsigned long long)a2);
-            if (slo | shi) {
-                fl |= FLAG_LIMBS;
-                atomicAdd(S.limb + 4 * e, slo & 0xFFFFFFFFull);
-                atomicAdd(S.limb + 4 * e + 1, slo >> 32);
-                atomicAdd(S.limb + 4 * e + 2, shi & 0xFFFFFFFFull);
-                atomicAdd(S.limb + 4 * e + 3, shi >> 32);
-            }
-            if (fl) atomicOr(S.flags + e, fl);
+            __syncthreads();  // ids and hist are refilled
         }
-        __syncthreads();  // ids and hist are refilled
+        __syncthreads();  // and todo
     }
 }
 
@@ -608,21 +654,22 @@ __global__ void __launch_bounds__(ACC_T) batch_accum_kernel(const float *__restr
 __device__ __forceinline__ void finish_fit(const BFit &F, BState *state, int f, float m2,
                                            const double *__restrict__ partial, int *active) {
     const float shift = __fsqrt_rn(m2);
-    double in = 0.0;
-    for (int it = 0; it < F.n_items; it++) in += partial[F.first_item + it];
     BState st = state[f];
-    st.inertia = in;
     st.n_iter += 1;
     st.cur = 1 - st.cur;
     if (shift < F.tol || st.n_iter >= F.max_iter) {
+        // a serial chain of FP64 additions (10 us for 312 items): the last iteration's only
+        double in = 0.0;
+        for (int it = 0; it < F.n_items; it++) in += partial[F.first_item + it];
+        st.inertia = in;
         st.done = 1;
         atomicSub(active, 1);
     }
     state[f] = st;
 }
 
-// The f64 reduction's new centres from the sums (left zero for the next
-// iteration): each sum rounded once to f64, the mean once to f32.
+// The f64 reduction's new centres from the sums (kept for the next iteration,
+// or left zero): each sum rounded once to f64, the mean once to f32.
 __global__ void __launch_bounds__(UPDATE_T) batch_means_kernel(const BFit *__restrict__ fits, BState *__restrict__ state,
                                                                const int *__restrict__ order, int nf, int *counter,
                                                                float *__restrict__ C, const double *__restrict__ partial,
@@ -642,6 +689,7 @@ __global__ void __launch_bounds__(UPDATE_T) batch_means_kernel(const BFit *__res
         const int d = F.d, k = F.k, cur = state[f].cur;
         const float *oldc = C + F.c_off + (int64_t)cur * k * d;
         float *newc = C + F.c_off + (int64_t)(1 - cur) * k * d;
+        bool full = !F.keep_sums;  // the next iteration starts from zero sums
         const ExactGrid g(pamax[F.prob], F.n);
         const int64_t a_off = F.c_off / 2;
         for (int pr = tid; pr < k * d; pr += UPDATE_T) {
@@ -653,6 +701,7 @@ __global__ void __launch_bounds__(UPDATE_T) batch_means_kernel(const BFit *__res
             }
             const uint32_t fl = S.flags[e];
             double sum;
+            full |= (fl & (FLAG_NAN | FLAG_PINF | FLAG_NINF)) != 0;
             if (fl & (FLAG_NAN | FLAG_PINF | FLAG_NINF)) {  // IEEE f64 summation of the specials
                 sum = ((fl & FLAG_NAN) || (fl & (FLAG_PINF | FLAG_NINF)) == (FLAG_PINF | FLAG_NINF))
                           ? __longlong_as_double(0x7FF8000000000000LL)
@@ -675,18 +724,21 @@ __global__ void __launch_bounds__(UPDATE_T) batch_means_kernel(const BFit *__res
                 sum = fixed128_to_double(slo, shi, g.F);
             }
             newc[pr] = __double2float_rn(__ddiv_rn(sum, (double)cnt));
-            S.a1[e] = 0;
-            S.a2[e] = 0;
-            if (fl) {
+        }
+        full = __syncthreads_or(full);
+        if (full) {
+            for (int pr = tid; pr < k * d; pr += UPDATE_T) {
+                const int64_t e = a_off + pr;
+                S.a1[e] = S.a2[e] = 0;
                 S.flags[e] = 0;
                 for (int l = 0; l < 4; l++) S.limb[4 * e + l] = 0;
             }
+            for (int c = tid; c < k; c += UPDATE_T) S.count[F.k_off + c] = 0;
         }
-        __syncthreads();
+        if (tid == 0) state[f].full = full;
         // the largest squared shift (NaN shifts never raise it)
         float ms = 0.f;
         for (int c = tid; c < k; c += UPDATE_T) {
-            S.count[F.k_off + c] = 0;
             const float sh = sqeuc_f32(newc + (int64_t)c * d, oldc + (int64_t)c * d, d);
             if (sh > ms) ms = sh;
         }
@@ -992,6 +1044,7 @@ fk_status batched_fit_impl(Ctx &ctx, fk_batch_problem *P, int64_t np, int reduct
             F.seed = q.random_state + (uint64_t)r;
             F.prob = (int32_t)p;
             // the thresholds cost k^2 d in one CTA group a fit: little beside n k d
+            F.keep_sums = q.n * std::max<int64_t>(q.max_iter, 1) <= ((int64_t)1 << 30);
             F.bounded = dbucket(F.d) < 4 && F.k <= BOUND_K && (int64_t)F.n >= 16 * (int64_t)F.k;
             fits.push_back(F);
             fit_prob.push_back((int)p);
@@ -1084,7 +1137,7 @@ fk_status batched_fit_impl(Ctx &ctx, fk_batch_problem *P, int64_t np, int reduct
         st0[f].cur = 0;
         st0[f].n_iter = 0;
         st0[f].done = fits[f].max_iter == 0 ? 1 : 0;
-        st0[f].pad = 0;
+        st0[f].full = 1;
         active += st0[f].done ? 0 : 1;
     }
     FK_CUDA(cudaMemcpyAsync(dstate, st0.data(), sizeof(BState) * (size_t)nf, cudaMemcpyHostToDevice, s));
@@ -1184,7 +1237,7 @@ fk_status batched_fit_impl(Ctx &ctx, fk_batch_problem *P, int64_t np, int reduct
         const int ug = std::min(nf, ctx.num_sms * 4);
         if (reduction == FK_REDUCE_F64) {
             batch_accum_kernel<<<(unsigned)std::min<size_t>(n_sums, (size_t)ctx.num_sms * 8), ACC_T, 0, s>>>(
-                X, dfits, dstate, ditems + n_assign, (int)n_sums, dctr + 21, dlab, damax, sums);
+                X, dfits, dstate, ditems + n_assign, (int)n_sums, dlab, dmem, damax, sums);
             batch_means_kernel<<<ug, UPDATE_T, 0, s>>>(dfits, dstate, dorder, nf, dctr + 20, dC, dpart, dctr + 31,
                                                        damax, sums);
         } else {

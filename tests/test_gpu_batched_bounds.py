@@ -47,3 +47,18 @@ def test_bounded_rows(kind):
         assert f.n_iter() == o["n_iter"][0], shape
         assert np.array_equal(f.labels(), o["labels"][0]), shape
         assert np.array_equal(f.cluster_centers(), o["centers"][0], equal_nan=True), shape
+
+
+@pytest.mark.parametrize("max_iter", [40, 1 << 20])
+def test_sums_carried_over_and_rebuilt(max_iter):
+    """To convergence, with the sums kept between iterations and (too many
+    iterations for that) rebuilt in each."""
+    rng = np.random.default_rng(4)
+    x = rng.normal(size=(3000, 16)).astype(np.float32)
+    x[::5] *= np.float32(1e-7)  # remainders below the grids
+    init = x[rng.choice(3000, size=6, replace=False)][None].copy()
+    fitted, _ = F.fit_batched([dict(x=x, k=6, n_init=1, init=init, max_iter=max_iter, tol=0.02)], reduction="f64")
+    o = O.fit_runs(x, 6, max_iter=max_iter, tol=0.02, n_init=1, init=init, wide_sums=True)
+    assert fitted[0].n_iter() == o["n_iter"][0]
+    assert np.array_equal(fitted[0].labels(), o["labels"][0])
+    assert np.array_equal(fitted[0].cluster_centers(), o["centers"][0])
