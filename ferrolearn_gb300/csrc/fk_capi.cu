@@ -360,6 +360,22 @@ void run_graphed(Ctx &ctx, const uint64_t (&key)[10], Body &&body) {
     FK_CUDA(cudaGraphLaunch(exec, ctx.stream));
 }
 
+// The labels of the direct form (no FP64 centres on FP64 rows).
+template <typename TX, typename TC>
+void assign_direct_labels(Ctx &ctx, const TX *x, int64_t n, int d, const TC *c, int k, int32_t *labels) {
+    if constexpr (std::is_same<TX, float>::value && std::is_same<TC, float>::value) {
+        if (f32_scores_pay(n, d, k)) {
+            try {
+                launch_assign_f32_scored(ctx, x, n, d, c, k, labels);
+                return;
+            } catch (const Error &e) {
+                if (e.code != FK_ERR_OOM) throw;  // no room for its list of open rows
+            }
+        }
+    }
+    launch_assign_direct<TX, TC>(x, n, d, c, k, labels, nullptr, ctx.stream);
+}
+
 // Assignment against c (labels, inertia into scalars), then the update into
 // nc (+ shift bits). Mixed precisions fold the inertia into the update pass.
 template <typename TX, typename TC>
@@ -870,7 +886,7 @@ fk_status predict_impl(fk_ctx *ctxp, const TC *c_in, int64_t k, int64_t d_fit, c
         if constexpr (std::is_same<TX, double>::value && std::is_same<TC, double>::value)
             launch_assign_f64_filtered(ctx, x, n, (int)d, c, (int)k, labels, nullptr, true);
         else
-            launch_assign_direct<TX, TC>(x, n, (int)d, c, (int)k, labels, nullptr, s);
+            assign_direct_labels<TX, TC>(ctx, x, n, (int)d, c, (int)k, labels);
     } else {
         if constexpr (std::is_same<TX, float>::value && std::is_same<TC, double>::value) {
             DevScalars *sc = (DevScalars *)ctx.get(BUF_SCALARS, sizeof(DevScalars));

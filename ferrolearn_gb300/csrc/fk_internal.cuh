@@ -162,6 +162,7 @@ enum BufSlot {
     BUF_FOLD_MAP, BUF_MASKS, BUF_THRESH, BUF_FLOORS, BUF_SHIFT, BUF_THMAIN, BUF_TH2, BUF_CNT2, BUF_LIST3,
     BUF_SLOT3, BUF_TH3, BUF_XB3,
     BUF_BX, BUF_BFITS, BUF_BSTATE, BUF_BITEMS, BUF_BPART, BUF_BORDER, BUF_BCTR, BUF_BLAB, BUF_BMEM, BUF_BCEN, BUF_BXOFF, BUF_BSUMS, BUF_BTHR,
+    BUF_SC_C,
     BUF_XSQ, BUF_MX_UB, BUF_MX_NEAR, BUF_LROWS, BUF_LXB, BUF_LXAUG, BUF_LSCALE,
     BUF_KPPC, BUF_PR_UB, BUF_PR_SHIFT, BUF_PR_NEAR, BUF_PR_LIST,
     BUF_PF_X32, BUF_PF_XERR, BUF_PF_C32, BUF_PF_CERR, BUF_PF_LIST, BUF_PF_CNT,
@@ -321,6 +322,11 @@ void launch_transform_direct(const T *x, int64_t n, int d, const T *c, int k, T 
 // (its f32 copy is rebuilt).
 void launch_assign_f64_filtered(Ctx &ctx, const double *x, int64_t n, int d, const double *c, int k,
                                 int32_t *labels, double *mind, bool fresh_x);
+// The plain f32 labels -- launch_assign_direct<float, float>'s -- through FMA
+// scores with rigorous bounds (fk_score.cu): the direct form only for the rows
+// they cannot decide. Where it pays: f32_scores_pay.
+bool f32_scores_pay(int64_t n, int d, int k);
+void launch_assign_f32_scored(Ctx &ctx, const float *x, int64_t n, int d, const float *c, int k, int32_t *labels);
 // The plain assignment of a fit's iteration (fk_prune.cu): the labels of
 // launch_assign_direct<F, F>, without the distances. c_prev null: the first
 // iteration, every centre for every row; else prev are the labels against
