@@ -222,20 +222,28 @@ __global__ void centroid_sum_kernel(const TX *__restrict__ x, int d, int k, int6
 // Plain update (KMeans<f32> and KMeans<f64>): the same row-order chain in F
 // per (cluster, feature), fed from shared memory. A block takes one cluster and
 // a slab of 32 features; its threads copy pages of CH_ROWS member rows straight
-// to shared memory (asynchronous 16-byte copies where the rows allow, CH_STAGES
-// pages in flight, the rows' indices one page further ahead) while warp 0 adds
-// the page that has landed, one lane per feature (a row's 32 features are
+// to shared memory (asynchronous 16-byte copies where the rows allow, several
+// pages in flight, the rows' indices copied as far ahead of those) while warp 0
+// adds the page that has landed, one lane per feature (a row's 32 features are
 // adjacent: no bank conflicts).
 //
 // Bound by the dependent additions of the largest cluster's chain: 4 cycles a
-// row in f32, 64 in f64. Through registers, one page ahead, a page of 512 rows
-// took 21 cycles a row in f32 (247 us at n = 1M, d = 64, k = 256).
+// row in f32, 64 in f64. At n = 1M, d = 64, k = 256 (f32; the largest cluster has
+// about 24,000 rows) 91 us: 176 with pages of 64 rows whose indices were read
+// one page before their copies (the wait for them set the pace), 117 with the
+// indices further ahead; the rest from pages of 128 and an adding warp that
+// copies nothing. f64 at n = 333,337, d = 50, k = 200: 263 -> 230 us.
 constexpr int CH_THREADS = 256;
 constexpr int CH_SW = 32;    // features per block
-constexpr int CH_ROWS = 64;  // rows per page
-constexpr int CH_STAGES = 6;
+constexpr int CH_ROWS = 128;  // rows per page
+constexpr int CH_COPIERS = CH_THREADS - 32;  // every warp but the one that adds
+template <typename T> struct ChStages { static constexpr int N = 5; };  // pages in flight: 80 KB, 96 KB
+template <> struct ChStages<double> { static constexpr int N = 3; };
+constexpr int CH_IDS = 9;  // pages of row indices in shared memory: those in flight and as many ahead
 template <typename T>
-size_t chain_smem_bytes() { return sizeof(T) * (size_t)CH_STAGES * CH_ROWS * CH_SW; }
+size_t chain_smem_bytes() {
+    return sizeof(T) * (size_t)ChStages<T>::N * CH_ROWS * CH_SW + sizeof(int32_t) * (size_t)CH_IDS * CH_ROWS;
+}
 
 __device__ __forceinline__ void ch_copy16(void *dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
@@ -256,10 +264,11 @@ __global__ void __launch_bounds__(CH_THREADS)
     using A = UArith<T>;
     constexpr int VW = 16 / (int)sizeof(T);                   // values per 16-byte copy
     constexpr int PIECES = CH_SW / VW;                        // copies per row
-    constexpr int CPT = CH_ROWS * PIECES / CH_THREADS;        // copies per thread and page
-    static_assert(CH_ROWS * PIECES % CH_THREADS == 0, "a page is whole copies per thread");
     extern __shared__ __align__(16) unsigned char ch_raw[];
+    constexpr int CH_STAGES = ChStages<T>::N;
+    static_assert(2 * CH_STAGES - 1 <= CH_IDS, "a page's indices are replaced after its copies");
     T *pages = reinterpret_cast<T *>(ch_raw);
+    int32_t *const ids = reinterpret_cast<int32_t *>(pages + (size_t)CH_STAGES * CH_ROWS * CH_SW);
     const int c = blockIdx.x;
     const int j0 = blockIdx.y * CH_SW;
     const int sw = min(CH_SW, d - j0);
@@ -269,22 +278,19 @@ __global__ void __launch_bounds__(CH_THREADS)
     // j0 is a multiple of 32: the slab starts on a 16-byte boundary when the rows do
     const bool vec = sw == CH_SW && (d % VW) == 0 && (((uintptr_t)x) & 15u) == 0;
     const int64_t np = (end - start + CH_ROWS - 1) / CH_ROWS;
-    int ids[CPT];  // the rows of this thread's copies of the next page
     auto load_ids = [&](int64_t pg) {
-#pragma unroll
-        for (int u = 0; u < CPT; u++) {
-            const int64_t r = start + pg * CH_ROWS + (tid + u * CH_THREADS) / PIECES;
-            ids[u] = r < end ? members[r] : -1;
-        }
+        const int64_t r = start + pg * CH_ROWS + tid - 32;
+        if (tid >= 32 && tid < 32 + CH_ROWS && r < end) ch_copy_one(ids + pg % CH_IDS * CH_ROWS + tid - 32, members + r);
     };
     auto copy_page = [&](int64_t pg) {
         T *dst = pages + (pg % CH_STAGES) * (CH_ROWS * CH_SW);
-        if (pg < np) {
-#pragma unroll
-            for (int u = 0; u < CPT; u++) {
-                const int e = tid + u * CH_THREADS, r = e / PIECES, q = e % PIECES;
-                if (ids[u] < 0) continue;
-                const T *src = x + (int64_t)ids[u] * d + j0 + VW * q;
+        if (pg < np && tid >= 32) {
+            const int32_t *id = ids + pg % CH_IDS * CH_ROWS;
+            const int rows = (int)min((int64_t)CH_ROWS, end - start - pg * CH_ROWS);
+#pragma unroll 4
+            for (int e = tid - 32; e < rows * PIECES; e += CH_COPIERS) {
+                const int r = e / PIECES, q = e % PIECES;
+                const T *src = x + (int64_t)id[r] * d + j0 + VW * q;
                 T *to = dst + r * CH_SW + VW * q;
                 if (vec) {
                     ch_copy16(to, src);
@@ -295,20 +301,26 @@ __global__ void __launch_bounds__(CH_THREADS)
                 }
             }
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");  // also an empty one: the count of groups stays the pages'
     };
-    load_ids(0);
-#pragma unroll
+    // a group of copies per page, also an empty one; with page pg go the indices
+    // of page pg + CH_STAGES - 1, which the wait for page pg completes too
+    auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
+    for (int pg = 0; pg < CH_STAGES - 1; pg++) load_ids(pg);
+    commit();
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
     for (int pg = 0; pg < CH_STAGES - 1; pg++) {
         copy_page(pg);
-        load_ids(pg + 1);
+        load_ids(pg + CH_STAGES - 1);
+        commit();
     }
     T s = T(0);
     for (int64_t pg = 0; pg < np; pg++) {
         asm volatile("cp.async.wait_group %0;" ::"n"(CH_STAGES - 2) : "memory");
         __syncthreads();  // page pg has landed, and the page before it has been added
         copy_page(pg + CH_STAGES - 1);  // into the stage of the page before
-        load_ids(pg + CH_STAGES);
+        load_ids(pg + 2 * (CH_STAGES - 1));
+        commit();
         if (tid < 32 && lane < sw) {
             const T *col = pages + (pg % CH_STAGES) * (CH_ROWS * CH_SW) + lane;
             const int cnt = (int)min((int64_t)CH_ROWS, end - start - pg * CH_ROWS);
