@@ -56,3 +56,23 @@ def test_batched_seedings_of_uneven_sizes():
     fitted, _ = F.fit_batched(probs)
     for f, p in zip(fitted, probs):  # no iteration: run 0 is kept, its centres are its seeds
         assert np.array_equal(f.cluster_centers(), O.kmeanspp(p["x"], p["k"], seed=p["random_state"])[0])
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("scale", [1.0, 1e-19, 1e17])
+@pytest.mark.parametrize("kind", ["few points", "near ties"])
+def test_trials_of_nearly_equal_potential(kind, scale, dt):
+    """Equal and nearly equal trials (the first of the smallest wins), and sums at
+    the ends of the estimates' range."""
+    rng = np.random.default_rng(8)
+    if kind == "few points":  # 12 places, many rows each: trials repeat
+        x = rng.normal(size=(12, 4))[rng.integers(0, 12, size=5000)]
+    else:  # mirror images: potentials equal but for their roundings
+        h = rng.normal(size=(2500, 4))
+        x = np.concatenate([h, -h])
+    x = np.ascontiguousarray(x * scale, dtype=dt)
+    name = "f32" if dt == np.float32 else "f64"
+    for seed in range(4):
+        oc, _ = O.kmeanspp(x, 20, seed=seed)
+        gc, _ = F.kmeans_plus_plus(x, 20, seed=seed, dtype=name)
+        assert np.array_equal(gc, oc), seed
