@@ -34,6 +34,8 @@
 //                       no FMA; in f64 they are bounded in FP32 first and
 //                       formed in FP64 only where the candidate may come
 //                       closer.
+//                       In f64 with many rows FP32 estimates come first and
+//                       only the trials that can win are formed (kpp_contenders_kernel).
 //                       Trials whose estimated potential is too far above the
 //                       smallest (rounding bounds included) end here.
 //   kpp_compose_kernel  per chunk of KPP_CH values the composed map for the
@@ -78,6 +80,7 @@ constexpr int KPP_CH = 1024;      // values per fold chunk
 constexpr int KPP_THREADS = 256;  // every kernel's block
 constexpr int KPP_WARPS = KPP_THREADS / 32;
 constexpr int MAX_TRIALS = 16;
+constexpr long long KPP_SPLIT_ROWS = 100000;  // f64: rows of a step from which it takes two passes
 constexpr int KPP_SLAB = 32;      // features staged at a time
 
 // ---------------------------------------------------- binade arithmetic --
@@ -295,7 +298,8 @@ struct KppState {
     long long cand[MAX_TRIALS];
     double pot[MAX_TRIALS];  // fold of each trial's array (F, widened)
     double total;            // fold of the current D^2 array
-    double est[2][MAX_TRIALS];  // estimate of each trial's fold (centre c: slot c & 1)
+    double est[2][MAX_TRIALS];  // estimate of each trial's fold (centre c: slot c & 1), in 2^esc
+    double err[2];              // and a bound of what FP32 distances in it are off by
 };
 
 // One seeding (device copy of a KppJob and its workspace).
@@ -314,6 +318,7 @@ struct KppFit {
     float *csum;              // [trials][tiles] estimates of the tiles' sums
     T *thr;                   // [k] skip threshold of each centre's rows at this step
     int32_t *own;             // [n] nearest centre so far
+    unsigned short *closer;   // [n] F = f64: trials whose candidate may come closer to the row (split steps)
     int32_t *crow;            // [k] rows chosen
     KppState *st;
     long long n, nch, tiles, n_draws;
@@ -361,6 +366,7 @@ __global__ void kpp_first_kernel(const KppFit<T> *__restrict__ fits) {
         st->cand[0] = first;
         for (int t = 0; t < f.trials; t++) f.nslots[t] = 0;
         for (int t = 0; t < MAX_TRIALS; t++) st->est[0][t] = st->est[1][t] = 0.0;
+        st->err[0] = st->err[1] = 0.0;
         f.crow[0] = (int32_t)first;
     }
     __syncthreads();
@@ -450,6 +456,29 @@ inline size_t trial_smem(int dmax, int tt) {
     return sizeof(float) * ((size_t)KPP_THREADS * slab_stride(w) + (size_t)tt * w);
 }
 
+// Whether trial t's fold can be the smallest of the step's (by a whole warp).
+// An estimate differs from the exact sum by less than 1e-5 of it (truncated to
+// 24 bits, fewer than 100 f32 additions in a row) and err, and a fold in F by n u: a
+// trial whose estimate is further above the smallest one than both allow has a
+// strictly larger fold, which then need not be formed. Estimates that are not
+// finite, or that values below the estimates' range could move, exclude no one.
+// Three seedings of 1M x 64 in f64, k = 256: compose 77 -> 29 us a step, walk 54
+// -> 47 (a MiniBatchKMeans fit 154 -> 142 ms); in f32 the folds' own rounding
+// (n u = 6% at 1M rows) leaves more trials in.
+template <typename T>
+__device__ __forceinline__ bool contends(const KppFit<T> &f, int c, int t) {
+    const int lane = threadIdx.x & 31;
+    const float e = lane < f.trials ? (float)__ldcg(&f.st->est[c & 1][lane]) : INFINITY;
+    float lo = e;
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    const float eps = 1.1e-5f + 1.01f * (float)f.n * (sizeof(T) == 8 ? 1.2e-16f : 6.0e-8f);
+    const float mine = __shfl_sync(0xffffffffu, e, t);
+    const float err = 1.001f * (float)__ldcg(&f.st->err[c & 1]);
+    if (!(lo >= 1e-18f && lo <= 1e37f) || eps > 0.2f) return true;
+    return !(mine * (1.f - eps) - err > lo * (1.f + eps) + err);
+}
+
 // One CTA per tile of `scan` rows (a divisor of KPP_CH, a multiple of 256):
 // every trial's min(D^2, d(x, candidate)) (INIT: d(x, first row), the first
 // D^2 array; kmeans.rs:188-195, 225-233), and estimates of the tile's sums.
@@ -460,10 +489,19 @@ inline size_t trial_smem(int dmax, int tt) {
 //
 // Bound at n = 1M, d = 64, 7 trials in f32: the FP32 pipe for the listed rows
 // (3 d operations a pair), L2 for the values (8 bytes a pair).
-template <typename T, int TT, bool INIT>
+//
+// In f64 with many rows the step takes two passes: PASS_EST forms FP32 distances
+// only, for estimates of the trials' sums with a bound of what they are off by,
+// and marks the rows each candidate may come closer to; kpp_contenders_kernel
+// then forms the arrays of the trials that can win, nearly always one. Three
+// seedings of 1M x 64, k = 256, 7 trials: 273 us a
+// step in one pass (FP64 distances and arrays of every trial), 100 + 61 in two.
+enum { PASS_INIT, PASS_ALL, PASS_EST };
+template <typename T, int TT, int PASS>
 __global__ void __launch_bounds__(KPP_THREADS)
     kpp_trials_kernel(const KppFit<T> *__restrict__ fits, const int2 *__restrict__ items, int scan, int c) {
-    constexpr bool F64 = sizeof(T) == 8;
+    constexpr bool F64 = sizeof(T) == 8, INIT = PASS == PASS_INIT, EST = PASS == PASS_EST;
+    static_assert(F64 || !EST, "FP32 estimates are of FP64 distances");
     const int2 it = item_at(items);
     const KppFit<T> &f = fits[it.x];
     const KppState *st = f.st;
@@ -492,7 +530,9 @@ __global__ void __launch_bounds__(KPP_THREADS)
     T *out = f.chains + (long long)(INIT ? 0 : 1 - cur) * f.trials * n + base;
     const int rows = (int)min((long long)scan, n - base);
     const int own_c = st->own_c;
-    float psum[TT], skipped = 0.f;
+    // a power of two; far from 1 the estimates are not used
+    const float unit = EST ? (esc >= -100 && esc <= 100 ? __int_as_float((127 - esc) << 23) : NAN) : 1.f;
+    float psum[TT], skipped = 0.f, err = 0.f;
 #pragma unroll
     for (int b = 0; b < TT; b++) psum[b] = 0.f;
     __syncthreads();
@@ -531,7 +571,9 @@ __global__ void __launch_bounds__(KPP_THREADS)
                 open = !below(m[a], f.thr[o[a]]);
                 if (!open) {
                     skipped += est_of(m[a], esc);
-                    for (int t = 0; t < ntr; t++) out[(long long)t * n + i] = m[a];
+                    if (EST) f.closer[base + i] = 0;
+                    else
+                        for (int t = 0; t < ntr; t++) out[(long long)t * n + i] = m[a];
                 }
             }
             const unsigned bm = __ballot_sync(0xffffffffu, open);
@@ -616,6 +658,28 @@ __global__ void __launch_bounds__(KPP_THREADS)
                         psum[b] += est_of(r, esc);
                     }
             }
+        } else if constexpr (EST) {
+            if (tid < cnt) {
+                const int i = list[l0 + tid];
+                const T m = mind[i];
+                const float mu = __double2float_ru(m), me = est_of(m, esc), er = f.xerr[base + i];
+                float worst = 0.f;
+                unsigned closer = 0;
+#pragma unroll
+                for (int b = 0; b < TT; b++)
+                    if (b < ntr) {
+                        const float bnd = bound32(acc[b], __fadd_ru(er, cerr[b]), d);
+                        float e = me;
+                        if (!(__fsub_rd(acc[b], bnd) > mu)) {
+                            closer |= 1u << b;
+                            e = fminf(acc[b] * unit, me);
+                            worst = bnd < FLT_MAX ? fmaxf(worst, bnd) : INFINITY;  // NaN: INFINITY
+                        }
+                        psum[b] += e;
+                    }
+                f.closer[base + i] = (unsigned short)closer;
+                err = __fmaf_rn(worst, unit, err);
+            }
         } else {
             // Pairs the FP32 bounds leave open -- rows the candidate may come
             // closer to, non-finite values, values beyond the f32 range --
@@ -665,35 +729,79 @@ __global__ void __launch_bounds__(KPP_THREADS)
         for (int o = 16; o >= 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
         if (lane == 0) red[b][w] = v;
     }
+    if (EST) {
+#pragma unroll
+        for (int o = 16; o >= 1; o >>= 1) err += __shfl_xor_sync(0xffffffffu, err, o);
+        if (lane == 0 && err != 0.f) atomicAdd(&f.st->err[c & 1], (double)err);  // NaN too
+    }
     __syncthreads();
     if (tid < ntr) {
         float v = 0.f;
         for (int q = 0; q < KPP_WARPS; q++) v += red[tid][q];
-        f.csum[(long long)tid * f.tiles + it.y] = v;
-        if (!INIT) atomicAdd(&f.st->est[c & 1][tid], (double)v);
+        if (!EST) f.csum[(long long)tid * f.tiles + it.y] = v;
+        if (EST || PASS == PASS_ALL) atomicAdd(&f.st->est[c & 1][tid], (double)v);
     }
 }
 
-// Whether trial t's fold can be the smallest of the step's (by a whole warp).
-// An estimate differs from the exact sum by less than 1e-5 of it (truncated to
-// 24 bits, fewer than 100 f32 additions in a row), and a fold in F by n u: a
-// trial whose estimate is further above the smallest one than both allow has a
-// strictly larger fold, which then need not be formed. Estimates that are not
-// finite, or that values below the estimates' range could move, exclude no one.
-// Three seedings of 1M x 64 in f64, k = 256: compose 77 -> 29 us a step, walk 54
-// -> 47 (a MiniBatchKMeans fit 154 -> 142 ms); in f32 the folds' own rounding
-// (n u = 6% at 1M rows) leaves more trials in.
+// The second pass of a split step: min(D^2, d(x, candidate)) of the trials that
+// can win, `per` rows a CTA (2,048 or 4,096). Rows the candidate cannot come
+// closer to keep their value; the others are listed and formed in FP64, a
+// thread a row. Bound by the arrays' traffic (18 bytes a row) and by FP64, which
+// takes a warp with one listed row as long as a full one: hence the many rows
+// of a CTA (with 1,024, 104 us a step for three seedings of 1M x 64).
+constexpr int CONT_ROWS = 4096;
 template <typename T>
-__device__ __forceinline__ bool contends(const KppFit<T> &f, int c, int t) {
-    const int lane = threadIdx.x & 31;
-    const float e = lane < f.trials ? (float)__ldcg(&f.st->est[c & 1][lane]) : INFINITY;
-    float lo = e;
+__global__ void __launch_bounds__(KPP_THREADS)
+    kpp_contenders_kernel(const KppFit<T> *__restrict__ fits, const int2 *__restrict__ items, int scan, int per, int c) {
+    const int2 it = item_at(items);
+    const KppFit<T> &f = fits[it.x];
+    const KppState *st = f.st;
+    if (st->direct[c & 1]) return;
+    const long long n = f.n, base = (long long)it.y * per;
+    __shared__ unsigned short list[CONT_ROWS];
+    __shared__ float sums[CONT_ROWS / KPP_THREADS];  // of the tiles of `scan` rows
+    __shared__ int list_n;
+    const int tid = threadIdx.x, lane = tid & 31, esc = st->esc, d = f.d;
+    const T *mind = f.chains + ((long long)st->cur * f.trials + st->cur_trial) * n + base;
+    const int rows = (int)min((long long)per, n - base);
+    for (int t = 0; t < f.trials; t++) {
+        if (!contends(f, c, t)) continue;
+        T *out = f.chains + ((long long)(1 - st->cur) * f.trials + t) * n + base;
+        if (tid == 0) list_n = 0;
+        if (tid < CONT_ROWS / KPP_THREADS) sums[tid] = 0.f;
+        __syncthreads();
+#pragma unroll 8
+        for (int i0 = 0; i0 < rows; i0 += KPP_THREADS) {
+            const int i = i0 + tid;
+            const bool live = i < rows;
+            const T m = live ? mind[i] : T(0);
+            const bool open = live && ((f.closer[base + i] >> t) & 1u);
+            if (live && !open) out[i] = m;
+            float v = live && !open ? est_of(m, esc) : 0.f;
 #pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-    const float eps = 1.1e-5f + 1.01f * (float)f.n * (sizeof(T) == 8 ? 1.2e-16f : 6.0e-8f);
-    const float mine = __shfl_sync(0xffffffffu, e, t);
-    if (!(lo >= 1e-18f && lo <= 1e37f) || eps > 0.2f) return true;
-    return !(mine * (1.f - eps) > lo * (1.f + eps));
+            for (int o = 16; o >= 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            const unsigned bm = __ballot_sync(0xffffffffu, open);
+            int at = 0;
+            if (lane == 0) {
+                atomicAdd(&sums[i0 / scan], v);
+                if (bm) at = atomicAdd(&list_n, __popc(bm));
+            }
+            at = __shfl_sync(0xffffffffu, at, 0);
+            if (open) list[at + __popc(bm & ((1u << lane) - 1u))] = (unsigned short)i;
+        }
+        __syncthreads();
+        const T *cand = f.x + st->cand[t] * d;
+        for (int q = tid; q < list_n; q += KPP_THREADS) {
+            const int i = list[q];
+            const T v = sqeuc(f.x + (base + i) * d, cand, d), old = mind[i];
+            const T r = v < old ? v : old;  // kmeans.rs:230-232
+            out[i] = r;
+            atomicAdd(&sums[i / scan], est_of(r, esc));
+        }
+        __syncthreads();
+        if (tid * scan < rows) f.csum[(long long)t * f.tiles + base / scan + tid] = sums[tid];
+        __syncthreads();
+    }
 }
 
 // Rows of a staged chunk: value i at i + i / 32, so that reading a value a lane
@@ -1129,6 +1237,7 @@ __device__ void kpp_select(const KppFit<T> &f, int c, bool init) {
     __shared__ T stotal;
     __shared__ int scur, strial;
     if (tid < MAX_TRIALS) st->est[cn & 1][tid] = 0.0;
+    if (tid == 0) st->err[cn & 1] = 0.0;
     if (tid == 0) {
         copy_row = direct_row = -1;
         if (init) {
@@ -1366,38 +1475,38 @@ __global__ void __launch_bounds__(KPP_THREADS) kpp_walk_kernel(const KppFit<T> *
     if (sh.last) kpp_select<T>(f, c, init);
 }
 
-template <typename T, int TT, bool INIT>
+template <typename T, int TT, int PASS>
 void launch_trials(const KppFit<T> *fits, const int2 *items, unsigned grid, int scan, int c, int dmax,
                    cudaStream_t s) {
     const size_t smem = trial_smem(dmax, TT);
-    FK_CUDA(cudaFuncSetAttribute((const void *)kpp_trials_kernel<T, TT, INIT>,
+    FK_CUDA(cudaFuncSetAttribute((const void *)kpp_trials_kernel<T, TT, PASS>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kpp_trials_kernel<T, TT, INIT><<<grid, KPP_THREADS, smem, s>>>(fits, items, scan, c);
+    kpp_trials_kernel<T, TT, PASS><<<grid, KPP_THREADS, smem, s>>>(fits, items, scan, c);
     FK_LAUNCH_CHECK();
 }
 
 // The trial pass with the smallest trial-slot count that holds ntr trials.
-template <typename T>
+template <typename T, int PASS>
 void launch_trials_any(int ntr, const KppFit<T> *fits, const int2 *items, unsigned grid, int scan, int c, int dmax,
                        cudaStream_t s) {
     switch (ntr) {
-        case 1: case 2: launch_trials<T, 2, false>(fits, items, grid, scan, c, dmax, s); break;
-        case 3: launch_trials<T, 3, false>(fits, items, grid, scan, c, dmax, s); break;
-        case 4: launch_trials<T, 4, false>(fits, items, grid, scan, c, dmax, s); break;
-        case 5: launch_trials<T, 5, false>(fits, items, grid, scan, c, dmax, s); break;
-        case 6: launch_trials<T, 6, false>(fits, items, grid, scan, c, dmax, s); break;
-        case 7: launch_trials<T, 7, false>(fits, items, grid, scan, c, dmax, s); break;
-        case 8: launch_trials<T, 8, false>(fits, items, grid, scan, c, dmax, s); break;
-        case 9: launch_trials<T, 9, false>(fits, items, grid, scan, c, dmax, s); break;
-        case 10: launch_trials<T, 10, false>(fits, items, grid, scan, c, dmax, s); break;
-        case 11: case 12: launch_trials<T, 12, false>(fits, items, grid, scan, c, dmax, s); break;
-        default: launch_trials<T, 16, false>(fits, items, grid, scan, c, dmax, s); break;
+        case 1: case 2: launch_trials<T, 2, PASS>(fits, items, grid, scan, c, dmax, s); break;
+        case 3: launch_trials<T, 3, PASS>(fits, items, grid, scan, c, dmax, s); break;
+        case 4: launch_trials<T, 4, PASS>(fits, items, grid, scan, c, dmax, s); break;
+        case 5: launch_trials<T, 5, PASS>(fits, items, grid, scan, c, dmax, s); break;
+        case 6: launch_trials<T, 6, PASS>(fits, items, grid, scan, c, dmax, s); break;
+        case 7: launch_trials<T, 7, PASS>(fits, items, grid, scan, c, dmax, s); break;
+        case 8: launch_trials<T, 8, PASS>(fits, items, grid, scan, c, dmax, s); break;
+        case 9: launch_trials<T, 9, PASS>(fits, items, grid, scan, c, dmax, s); break;
+        case 10: launch_trials<T, 10, PASS>(fits, items, grid, scan, c, dmax, s); break;
+        case 11: case 12: launch_trials<T, 12, PASS>(fits, items, grid, scan, c, dmax, s); break;
+        default: launch_trials<T, 16, PASS>(fits, items, grid, scan, c, dmax, s); break;
     }
 }
 
 // Byte layout of one seeding's workspace (256-byte aligned parts).
 struct KppLayout {
-    size_t chains, states, gstates, slots, nslots, cmaps, csum, thr, own, crow, st, total;
+    size_t chains, states, gstates, slots, nslots, cmaps, csum, thr, own, closer, crow, st, total;
 };
 template <typename T>
 KppLayout kpp_layout(const KppJob &j, int trials, int scan) {
@@ -1418,6 +1527,7 @@ KppLayout kpp_layout(const KppJob &j, int trials, int scan) {
     L.csum = part(sizeof(float) * trials * tiles);
     L.thr = part(sizeof(T) * (size_t)j.k);
     L.own = part(sizeof(int32_t) * n);
+    L.closer = part(sizeof(T) == 8 ? sizeof(unsigned short) * n : 0);
     L.crow = part(sizeof(int32_t) * (size_t)j.k);
     L.st = part(sizeof(KppState));
     L.total = at;
@@ -1452,8 +1562,11 @@ bool run_group(Ctx &ctx, const std::vector<KppJob> &jobs, const std::vector<int>
     // items of the trial pass (tiles) and of the composition (eight chunks), in
     // seeding order: the seedings still running at a step are a prefix
     std::vector<int2> items;
-    std::vector<unsigned> tile_end(nf), comp_end(nf);
-    unsigned nt = 0, ncg = 0;
+    std::vector<unsigned> tile_end(nf), comp_end(nf), cont_end(nf);
+    unsigned nt = 0, ncg = 0, ncp = 0;
+    long long rows = 0;
+    for (size_t q = 0; q < nf; q++) rows += jobs[(size_t)order[lo + q]].n;
+    const int per = rows >= 2ll * CONT_ROWS * ctx.num_sms ? CONT_ROWS : CONT_ROWS / 2;
     for (size_t q = 0; q < nf; q++) {
         const KppJob &j = jobs[(size_t)order[lo + q]];
         KppFit<T> &f = fits[q];
@@ -1473,6 +1586,7 @@ bool run_group(Ctx &ctx, const std::vector<KppJob> &jobs, const std::vector<int>
         f.csum = (float *)(b + L.csum);
         f.thr = (T *)(b + L.thr);
         f.own = (int32_t *)(b + L.own);
+        f.closer = (unsigned short *)(b + L.closer);
         f.crow = (int32_t *)(b + L.crow);
         f.st = (KppState *)(b + L.st);
         f.n = j.n;
@@ -1486,22 +1600,27 @@ bool run_group(Ctx &ctx, const std::vector<KppJob> &jobs, const std::vector<int>
         f.nan_direct = j.nan_direct ? 1 : 0;
         nt += (unsigned)f.tiles;
         ncg += (unsigned)((f.nch + KPP_WARPS - 1) / KPP_WARPS);
+        ncp += (unsigned)((j.n + per - 1) / per);
+        cont_end[q] = ncp;
         tile_end[q] = nt;
         comp_end[q] = ncg;
     }
     KppFit<T> *dfits = (KppFit<T> *)ctx.get(BUF_KPP0, sizeof(KppFit<T>) * nf);
     FK_CUDA(cudaMemcpyAsync(dfits, fits.data(), sizeof(KppFit<T>) * nf, cudaMemcpyHostToDevice, s));
-    const int2 *titems = nullptr, *citems = nullptr;
+    const int2 *titems = nullptr, *citems = nullptr, *pitems = nullptr;
     if (nf > 1) {
-        items.reserve((size_t)nt + ncg);
+        items.reserve((size_t)nt + ncg + ncp);
         for (size_t q = 0; q < nf; q++)
             for (int t = 0; t < (int)fits[q].tiles; t++) items.push_back(make_int2((int)q, t));
         for (size_t q = 0; q < nf; q++)
             for (long long t = 0; t * KPP_WARPS < fits[q].nch; t++) items.push_back(make_int2((int)q, (int)t));
+        for (size_t q = 0; q < nf; q++)
+            for (long long t = 0; t * per < fits[q].n; t++) items.push_back(make_int2((int)q, (int)t));
         int2 *di = (int2 *)ctx.get(BUF_KPP2, sizeof(int2) * items.size());
         FK_CUDA(cudaMemcpyAsync(di, items.data(), sizeof(int2) * items.size(), cudaMemcpyHostToDevice, s));
         titems = di;
         citems = di + nt;
+        pitems = citems + ncg;
     }
     FK_CUDA(cudaFuncSetAttribute((const void *)kpp_compose_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)compose_smem(sizeof(T))));
@@ -1517,11 +1636,20 @@ bool run_group(Ctx &ctx, const std::vector<KppJob> &jobs, const std::vector<int>
         int nt_step = 1;
         for (size_t q = 0; q < na; q++) nt_step = std::max(nt_step, fits[q].trials);
         if (init) {
-            launch_trials<T, 1, true>(dfits, titems, tile_end[na - 1], scan, c, dmax, s);
+            launch_trials<T, 1, PASS_INIT>(dfits, titems, tile_end[na - 1], scan, c, dmax, s);
         } else {
             kpp_pairs_kernel<T><<<(unsigned)(na * ((c + KPP_WARPS - 1) / KPP_WARPS)), KPP_THREADS, 0, s>>>(dfits, c);
             FK_LAUNCH_CHECK();
-            launch_trials_any<T>(nt_step, dfits, titems, tile_end[na - 1], scan, c, dmax, s);
+            bool split = false;
+            if constexpr (sizeof(T) == 8) {
+                split = (long long)tile_end[na - 1] * scan >= KPP_SPLIT_ROWS;
+                if (split) {
+                    launch_trials_any<T, PASS_EST>(nt_step, dfits, titems, tile_end[na - 1], scan, c, dmax, s);
+                    kpp_contenders_kernel<T><<<cont_end[na - 1], KPP_THREADS, 0, s>>>(dfits, pitems, scan, per, c);
+                    FK_LAUNCH_CHECK();
+                }
+            }
+            if (!split) launch_trials_any<T, PASS_ALL>(nt_step, dfits, titems, tile_end[na - 1], scan, c, dmax, s);
         }
         const unsigned gy = init ? 1u : (unsigned)nt_step;
         kpp_compose_kernel<T><<<dim3(comp_end[na - 1], gy), KPP_THREADS, compose_smem(sizeof(T)), s>>>(dfits, citems,

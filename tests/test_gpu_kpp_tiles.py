@@ -76,3 +76,22 @@ def test_trials_of_nearly_equal_potential(kind, scale, dt):
         oc, _ = O.kmeanspp(x, 20, seed=seed)
         gc, _ = F.kmeans_plus_plus(x, 20, seed=seed, dtype=name)
         assert np.array_equal(gc, oc), seed
+
+
+@pytest.mark.parametrize("kind", ["blobs", "grid", "outlier"])
+@pytest.mark.parametrize("n,d,k,runs", [(100001, 5, 9, 1), (102401, 37, 6, 1), (50009, 4, 8, 2), (26000, 16, 12, 5),
+                                        (1300001, 3, 5, 1)])
+def test_split_steps(n, d, k, runs, kind):
+    """f64 steps of 100,000 rows and more: estimates first, then the arrays of the
+    trials that can win (n at the edges of both passes' tiles)."""
+    x = _rows(n, d, kind, n + d, np.float64)
+    if runs == 1:
+        x[::9] = x[1]  # equal rows
+        oc, _ = O.kmeanspp(x, k, seed=n)
+        gc, _ = F.kmeans_plus_plus(x, k, seed=n, dtype="f64")
+        assert np.array_equal(gc, oc)
+    else:
+        g = F.KMeans(k, dtype="f64").with_n_init(runs).with_random_state(n).with_max_iter(2).fit(x)
+        o = O.fit(x, k, max_iter=2, n_init=runs, seed=n)
+        assert np.array_equal(g.cluster_centers(), o["centers"]) and np.array_equal(g.labels(), o["labels"])
+        assert g.report["best_run"] == o["best_run"]
