@@ -338,9 +338,11 @@ void launch_assign_pruned(Ctx &ctx, const F *x, int64_t n, int d, const F *c, co
 // Each row's direct-form distance to its label, F::MAX where it is not below.
 template <typename F>
 void launch_label_dist(Ctx &ctx, const F *x, int64_t n, int d, const F *c, const int32_t *labels, F *mind);
-// The FP64 direct form over every centre for the listed rows (fk_prefilter.cu).
-void launch_f64_open_rows(Ctx &ctx, const double *x, int d, const double *c, int k, const int32_t *list,
-                          const unsigned long long *count, int32_t *labels);
+// The labels (and distances, when mind is set) of the listed rows by the FP64
+// direct form (fk_prefilter.cu).
+void launch_f64_open_rows(Ctx &ctx, const double *x, const float *x32, const float *xerr, int d, const double *c,
+                          const float *c32, const float *cerr, int k, const int32_t *list,
+                          const unsigned long long *count, int32_t *labels, double *mind);
 // f32 copies of f64 rows and an upper bound of the norm of each row's
 // rounding error (the inputs of the FP32 bounds).
 void launch_f32_copy(Ctx &ctx, const double *x, int64_t n, int d, float *x32, float *err);

@@ -612,7 +612,8 @@ void launch_assign_pruned(Ctx &ctx, const F *x, int64_t n, int d, const F *c, co
         prune_scan_kernel<F><<<tiles, PT, 0, s>>>(x32, xerr, n, d, c32, cerr, k, L.scan_rows, labels, ub, lb, L);
         FK_LAUNCH_CHECK();
     }
-    if constexpr (!S) launch_f64_open_rows(ctx, x, d, c, k, L.open_rows, L.count + 2, labels);
+    if constexpr (!S) 
+        launch_f64_open_rows(ctx, x, x32, xerr, d, c, c32, cerr, k, L.open_rows, L.count + 2, labels, nullptr);
 }
 
 template <typename F>
