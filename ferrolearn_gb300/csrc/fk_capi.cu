@@ -881,6 +881,16 @@ fk_status predict_impl(fk_ctx *ctxp, const TC *c_in, int64_t k, int64_t d_fit, c
     cudaStream_t s = ctx.stream;
     const TX *x = stage_in<TX>(ctx, BUF_X, x_in, (size_t)n * d);
     const TC *c = stage_in<TC>(ctx, BUF_C0, c_in, (size_t)k * d);
+    if constexpr (std::is_same<TX, TC>::value) {
+        if (prec == FK_PRECISION_PLAIN && assign_small_ok(n, (int)d, (int)k)) {
+            const bool dev = is_device_ptr(labels_out);
+            uint64_t *l64 = dev ? labels_out : (uint64_t *)ctx.get(BUF_OUT, sizeof(uint64_t) * (size_t)n);
+            launch_assign_small<TC>(x, n, (int)d, c, (int)k, l64, s);
+            if (!dev) copy_out<uint64_t>(ctx, labels_out, l64, (size_t)n);
+            FK_CUDA(cudaStreamSynchronize(s));
+            return FK_OK;
+        }
+    }
     int32_t *labels = (int32_t *)ctx.get(BUF_LABELS, sizeof(int32_t) * (size_t)n);
     if (prec == FK_PRECISION_PLAIN) {
         if constexpr (std::is_same<TX, double>::value && std::is_same<TC, double>::value)

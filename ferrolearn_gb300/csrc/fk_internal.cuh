@@ -285,6 +285,10 @@ inline void flush_timers(Ctx &ctx) {
 template <typename TX, typename TC>
 void launch_assign_direct(const TX *x, int64_t n, int d, const TC *c, int k, int32_t *labels,
                           TC *mind, cudaStream_t s);
+// The direct-form labels of a small call in one launch (assign_small_ok).
+bool assign_small_ok(int64_t n, int d, int k);
+template <typename T>
+void launch_assign_small(const T *x, int64_t n, int d, const T *c, int k, uint64_t *labels, cudaStream_t s);
 // Transform (kmeans.rs:568-617): out[i*k+c] = sqrt(direct distance).
 // The assignment with the centres split over `splits` CTA columns (for row
 // counts too small to fill the GPU), then an ordered combine: the same labels
