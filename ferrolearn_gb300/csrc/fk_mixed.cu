@@ -124,7 +124,8 @@ __global__ void sample_tmax_kernel(const TX *__restrict__ x, int64_t n, int d, i
 // Exponent of the FP8 centre scale t = 2^sh_t: max |t| / t in [128, 256).
 __device__ __forceinline__ int fp8_scale_exp(float tmax) {
     int sh = 0;
-    if (tmax > 0.f && tmax < INFINITY) sh = ilogbf(tmax) - 7;
+    // the exponent field: a subnormal's clamps like its own exponent would
+    if (tmax > 0.f && tmax < INFINITY) sh = (int)(__float_as_uint(tmax) >> 23) - 127 - 7;
     return sh < -120 ? -120 : (sh > 120 ? 120 : sh);
 }
 constexpr int FP8_ROW_BELOW = 40;  // per-row scales stay within [2^(sh_t-40), 2^(sh_t+60)]
@@ -302,12 +303,17 @@ __device__ __forceinline__ float group_max_f(float v) {
     return v;
 }
 
+// LPR lanes a row, 16 bytes a lane and step, the next rows' loads in flight. BF16 is
+// bound by memory (4M x 128: 3 GB in 0.56 ms); FP8 by its instructions:
+// 2M x 256 (2.6 GB) took 878 us with a conversion each way per value, the
+// finite tests of the maxima per value and a root per norm and lane; 648 with
+// conversions in pairs, the tests once per row and a root per lane.
 template <bool FP8, int LPR>
-__global__ void prep_rows4_kernel(const float *__restrict__ x, int64_t n, int d, int d_pad,
-                                  const float *__restrict__ mu32, void *__restrict__ xq_out,
-                                  __nv_bfloat16 *__restrict__ xaug, float4 *__restrict__ rowinfo, MixedStats *stats,
-                                  const int32_t *__restrict__ list, const unsigned long long *count,
-                                  float *__restrict__ xsq) {
+__global__ void __launch_bounds__(256, 3)
+    prep_rows4_kernel(const float *__restrict__ x, int64_t n, int d, int d_pad, const float *__restrict__ mu32,
+                      void *__restrict__ xq_out, __nv_bfloat16 *__restrict__ xaug, float4 *__restrict__ rowinfo,
+                      MixedStats *stats, const int32_t *__restrict__ list, const unsigned long long *count,
+                      float *__restrict__ xsq) {
     constexpr int RPW = 32 / LPR;  // rows a warp
     constexpr int NPL = 4;         // 4-feature pieces a lane
     __shared__ float sh_xn[32], sh_am[32];
@@ -335,6 +341,7 @@ __global__ void prep_rows4_kernel(const float *__restrict__ x, int64_t n, int d,
         }
     };
     float xn_hi = 0.f, am_hi = 0.f, nonfin = 0.f;
+    const int sh_t = FP8 ? fp8_scale_exp(stats->tmax) : 0;
     int64_t base = ((int64_t)blockIdx.x * (blockDim.x >> 5) + w) * RPW;  // warp-uniform
     float4 cur[NPL];
 #pragma unroll
@@ -357,18 +364,27 @@ __global__ void prep_rows4_kernel(const float *__restrict__ x, int64_t n, int d,
                 const float xs[4] = {cur[i].x, cur[i].y, cur[i].z, cur[i].w};
                 const float ms[4] = {m4[i].x, m4[i].y, m4[i].z, m4[i].w};
 #pragma unroll
-                for (int c = 0; c < 4; c++) {
-                    const float tv = fabsf(__fsub_rn(xs[c], ms[c]));
-                    if (tv < INFINITY) tmax = fmaxf(tmax, tv);
-                }
+                for (int c = 0; c < 4; c++) tmax = fmaxf(tmax, fabsf(__fsub_rn(xs[c], ms[c])));  // NaN: left out
             }
             tmax = group_max_f<LPR>(tmax);
-            const int sh_t = fp8_scale_exp(stats->tmax);
+            if (__any_sync(0xffffffffu, tmax == INFINITY)) {  // the finite ones only
+                tmax = 0.f;
+                for (int i = 0; i < NPL; i++) {
+                    if (sl + LPR * i >= d4) continue;
+                    const float xs[4] = {cur[i].x, cur[i].y, cur[i].z, cur[i].w};
+                    const float ms[4] = {m4[i].x, m4[i].y, m4[i].z, m4[i].w};
+                    for (int c = 0; c < 4; c++) {
+                        const float tv = fabsf(__fsub_rn(xs[c], ms[c]));
+                        if (tv < INFINITY) tmax = fmaxf(tmax, tv);
+                    }
+                }
+                tmax = group_max_f<LPR>(tmax);
+            }
             int sh = tmax > 0.f ? fp8_scale_exp(tmax) : sh_t;
             sh = max(min(sh, sh_t + FP8_ROW_ABOVE), sh_t - FP8_ROW_BELOW);
             sh = max(min(sh, 120), -120);
-            scale = ldexpf(1.f, sh);
-            inv = ldexpf(1.f, -sh);
+            scale = __int_as_float((127 + sh) << 23);
+            inv = __int_as_float((127 - sh) << 23);
         }
 #pragma unroll
         for (int i = 0; i < NPL; i++) {
@@ -378,15 +394,26 @@ __global__ void prep_rows4_kernel(const float *__restrict__ x, int64_t n, int d,
                 const float xs[4] = {cur[i].x, cur[i].y, cur[i].z, cur[i].w};
                 const float ms[4] = {m4[i].x, m4[i].y, m4[i].z, m4[i].w};
                 uint32_t packed[2] = {0u, 0u};
+                float h8[4];  // FP8: the rounded values, converted in pairs
+                if (FP8) {
+#pragma unroll
+                    for (int c = 0; c < 4; c += 2) {
+                        const float2 s2 = make_float2(__fmul_rn(__fsub_rn(xs[c], ms[c]), inv),
+                                                      __fmul_rn(__fsub_rn(xs[c + 1], ms[c + 1]), inv));
+                        const __nv_fp8x2_storage_t q2 = __nv_cvt_float2_to_fp8x2(s2, __NV_SATFINITE, __NV_E4M3);
+                        packed[0] |= (uint32_t)q2 << (8 * c);
+                        const float2 f2 = __half22float2(__half2(__nv_cvt_fp8x2_to_halfraw2(q2, __NV_E4M3)));
+                        h8[c] = f2.x;
+                        h8[c + 1] = f2.y;
+                    }
+                }
 #pragma unroll
                 for (int c = 0; c < 4; c++) {
                     const float xv = xs[c];
                     const float t = __fsub_rn(xv, ms[c]);
                     float hv;
                     if (FP8) {
-                        const __nv_fp8_e4m3 q8(__fmul_rn(t, inv));
-                        packed[0] |= (uint32_t)q8.__x << (8 * c);
-                        hv = __fmul_rn((float)q8, scale);
+                        hv = __fmul_rn(h8[c], scale);
                     } else {
                         const __nv_bfloat16 h = __float2bfloat16_rn(t);
                         packed[c >> 1] |= (uint32_t)__bfloat16_as_ushort(h) << (16 * (c & 1));
@@ -397,7 +424,7 @@ __global__ void prep_rows4_kernel(const float *__restrict__ x, int64_t n, int d,
                     ex2 = __fmaf_rn(e, e, ex2);
                     tn2 = __fmaf_rn(t, t, tn2);
                     xo2 = __fmaf_rn(xv, xv, xo2);
-                    if (fabsf(xv) < INFINITY) amax = fmaxf(amax, fabsf(xv));  // finite values only
+                    amax = fmaxf(amax, fabsf(xv));  // NaN: left out
                 }
                 if (ok) {
                     if (FP8)
@@ -417,11 +444,24 @@ __global__ void prep_rows4_kernel(const float *__restrict__ x, int64_t n, int d,
         tn2 = group_sum_f<LPR>(tn2);
         xo2 = group_sum_f<LPR>(xo2);
         amax = group_max_f<LPR>(amax);
+        if (__any_sync(0xffffffffu, amax == INFINITY)) {  // the finite ones only
+            amax = 0.f;
+            for (int i = 0; i < NPL; i++) {
+                if (sl + LPR * i >= d4) continue;
+                const float xs[4] = {cur[i].x, cur[i].y, cur[i].z, cur[i].w};
+                for (int c = 0; c < 4; c++)
+                    if (fabsf(xs[c]) < INFINITY) amax = fmaxf(amax, fabsf(xs[c]));
+            }
+            amax = group_max_f<LPR>(amax);
+        }
+        // one root a lane: four lanes of the row hold the four norms
         const float up = 1.0f + (float)(d + 64) * 1.1920929e-07f;
-        const float xn = __fsqrt_ru(__fmul_ru(xn2, up));
-        const float ex =
-            __fadd_ru(__fsqrt_ru(__fmul_ru(ex2, up)), __fmul_ru(__fsqrt_ru(__fmul_ru(tn2, up)), 5.9604645e-08f));
-        const float xo = __fsqrt_ru(__fmul_ru(xo2, up));
+        const float sq = (sl & 3) == 0 ? xn2 : (sl & 3) == 1 ? ex2 : (sl & 3) == 2 ? tn2 : xo2;
+        const float root = __fsqrt_ru(__fmul_ru(sq, up));
+        const float xn = __shfl_sync(0xffffffffu, root, 0, LPR);
+        const float ex = __fadd_ru(__shfl_sync(0xffffffffu, root, 1, LPR),
+                                   __fmul_ru(__shfl_sync(0xffffffffu, root, 2, LPR), 5.9604645e-08f));
+        const float xo = __shfl_sync(0xffffffffu, root, 3, LPR);
         if (ok) {
             if (sl == 0) rowinfo[slot] = make_float4(xn, ex, xo, inv);
             if (sl == 0 && xsq) xsq[slot] = tn2;
