@@ -225,6 +225,17 @@ __global__ void assign_combine_kernel(const TC *__restrict__ part_v, const int32
     if (mind) mind[r] = v;
 }
 
+// A warp a row, a value a lane.
+template <typename T>
+__global__ void __launch_bounds__(NT)
+    repitch_kernel(const T *__restrict__ src, int64_t n, int d, T *__restrict__ dst, int dp) {
+    const int64_t nw = (int64_t)gridDim.x * (NT / 32);
+    for (int64_t r = (int64_t)blockIdx.x * (NT / 32) + (threadIdx.x >> 5); r < n; r += nw) {
+#pragma unroll 4
+        for (int j = threadIdx.x & 31; j < dp; j += 32) dst[r * dp + j] = j < d ? src[r * d + j] : T(0);
+    }
+}
+
 // ---------------------------------------------------------- fixed sums --
 constexpr int SUM_THREADS = 256;
 
@@ -308,6 +319,16 @@ void launch_assign_small(const T *x, int64_t n, int d, const T *c, int k, uint64
 }
 template void launch_assign_small<float>(const float *, int64_t, int, const float *, int, uint64_t *, cudaStream_t);
 template void launch_assign_small<double>(const double *, int64_t, int, const double *, int, uint64_t *, cudaStream_t);
+
+template <typename T>
+void launch_repitch(const T *src, int64_t n, int d, T *dst, int dp, cudaStream_t s) {
+    if (n == 0 || dp == 0) return;
+    const int64_t blocks = std::min<int64_t>((n + NT / 32 - 1) / (NT / 32), 1 << 16);
+    repitch_kernel<T><<<(unsigned)blocks, NT, 0, s>>>(src, n, d, dst, dp);
+    FK_LAUNCH_CHECK();
+}
+template void launch_repitch<float>(const float *, int64_t, int, float *, int, cudaStream_t);
+template void launch_repitch<double>(const double *, int64_t, int, double *, int, cudaStream_t);
 
 template <typename TC>
 int assign_splits(int64_t n, int k, int num_sms) {

@@ -360,6 +360,28 @@ void run_graphed(Ctx &ctx, const uint64_t (&key)[10], Body &&body) {
     FK_CUDA(cudaGraphLaunch(exec, ctx.stream));
 }
 
+// The mixed forms' kernels read rows in 16-byte pieces; rows whose length or start
+// does not allow that are copied once into rows of dp = the next multiple of
+// four, zeros behind. A zero feature adds exactly +0 to every distance and sum,
+// so nothing else changes. Fits of 20 iterations, one value at a time / copied:
+// 1M x 127 against 1,000 centres 30.0 / 8.1 ms in BF16 and 43.4 / 11.9 in FP8,
+// 300,000 x 250 against 500 23.1 / 6.6 and 33.1 / 7.9 (d = 128 and 252 as they are:
+// 7.9, 11.6, 6.3, 7.4). nullptr: not needed, d beyond these forms, or no memory
+// for the copy (the kernels for single values run then).
+const float *pad_rows(Ctx &ctx, const float *x, int64_t n, int64_t d, int64_t &dp) {
+    dp = (d + 3) / 4 * 4;
+    if (dp > 256 || d == 0 || (dp == d && ((uintptr_t)x & 15u) == 0)) return nullptr;
+    float *xp;
+    try {
+        xp = (float *)ctx.get(BUF_XPAD, sizeof(float) * (size_t)n * dp);
+    } catch (const Error &e) {
+        if (e.code != FK_ERR_OOM) throw;
+        return nullptr;
+    }
+    launch_repitch<float>(x, n, (int)d, xp, (int)dp, ctx.stream);
+    return xp;
+}
+
 // The labels of the direct form (no FP64 centres on FP64 rows).
 template <typename TX, typename TC>
 void assign_direct_labels(Ctx &ctx, const TX *x, int64_t n, int d, const TC *c, int k, int32_t *labels) {
@@ -532,8 +554,17 @@ fk_status fit_impl(fk_ctx *ctxp, const TX *x_in, int64_t n, int64_t d, const fk_
         tev.reset(new Events<2>());
         FK_CUDA(cudaEventRecord((*tev)[0], s));
     }
-    const size_t kd = (size_t)k * d;
     const TX *x = stage_in<TX>(ctx, BUF_X, x_in, (size_t)n * d);
+    const int64_t d_in = d;
+    if constexpr (std::is_same<TX, float>::value && std::is_same<TC, double>::value) {
+        int64_t dp = d;
+        if (p->precision != FK_PRECISION_PLAIN)
+            if (const float *xp = pad_rows(ctx, x, n, d, dp)) {
+                x = xp;
+                d = dp;
+            }
+    }
+    const size_t kd = (size_t)k * d;
     // Three rotating centre buffers: iteration it reads cb3[it % 3] and writes
     // cb3[(it + 1) % 3], so neither the kept iteration's input nor its output
     // is overwritten by the successor queued before the convergence test.
@@ -552,7 +583,12 @@ fk_status fit_impl(fk_ctx *ctxp, const TX *x_in, int64_t n, int64_t d, const fk_
 
     // a slot of its own: the runs after the first read it while the mixed
     // updates use their own scratch (which may grow and move)
-    const TC *init = init_in ? stage_in<TC>(ctx, BUF_INIT, init_in, kd * (size_t)p->n_init) : nullptr;
+    const TC *init = init_in ? stage_in<TC>(ctx, BUF_INIT, init_in, (size_t)k * d_in * (size_t)p->n_init) : nullptr;
+    if (init && d != d_in) {
+        TC *ip = (TC *)ctx.get(BUF_IPAD, sizeof(TC) * kd * (size_t)p->n_init);
+        launch_repitch<TC>(init, k * p->n_init, (int)d_in, ip, (int)d, s);
+        init = ip;
+    }
     const double *draws_dev = nullptr;
     int64_t n_draws = 0;
     if (!init && p->draws) {
@@ -777,7 +813,11 @@ fk_status fit_impl(fk_ctx *ctxp, const TX *x_in, int64_t n, int64_t d, const fk_
             FK_CUDA(cudaMemcpyAsync(lbest, labels, sizeof(int32_t) * (size_t)n, cudaMemcpyDeviceToDevice, s));
         }
     }
-    copy_out<TC>(ctx, centers_out, cbest, kd);
+    if (d != d_in) {
+        launch_repitch<TC>(cbest, k, (int)d, cb3[0], (int)d_in, s);
+        cbest = cb3[0];
+    }
+    copy_out<TC>(ctx, centers_out, cbest, (size_t)k * d_in);
     if (is_device_ptr(labels_out)) {
         launch_labels_to_u64(lbest, n, labels_out, s);
     } else {
@@ -901,7 +941,14 @@ fk_status predict_impl(fk_ctx *ctxp, const TC *c_in, int64_t k, int64_t d_fit, c
         if constexpr (std::is_same<TX, float>::value && std::is_same<TC, double>::value) {
             DevScalars *sc = (DevScalars *)ctx.get(BUF_SCALARS, sizeof(DevScalars));
             FK_CUDA(cudaMemsetAsync(sc, 0, sizeof(DevScalars), s));
-            run_assign_mixed(ctx, x, n, (int)d, c, (int)k, prec, labels, nullptr, sc, true);
+            int64_t dp = d;
+            const float *xp = pad_rows(ctx, x, n, d, dp);
+            if (xp && dp != d) {
+                double *cp = (double *)ctx.get(BUF_IPAD, sizeof(double) * (size_t)k * dp);
+                launch_repitch<double>(c, k, (int)d, cp, (int)dp, s);
+                c = cp;
+            }
+            run_assign_mixed(ctx, xp ? xp : x, n, (int)(xp ? dp : d), c, (int)k, prec, labels, nullptr, sc, true);
         }
     }
     if (is_device_ptr(labels_out)) {

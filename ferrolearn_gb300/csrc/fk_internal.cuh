@@ -161,7 +161,7 @@ enum BufSlot {
     BUF_BK_FOLD, BUF_BK_LABELS, BUF_BK_XSEG, BUF_BK_CHAINS, BUF_BK_FRES, BUF_BK_FCNT, BUF_FOLD_SUM, BUF_FOLD_CNT,
     BUF_FOLD_MAP, BUF_MASKS, BUF_THRESH, BUF_FLOORS, BUF_SHIFT, BUF_THMAIN, BUF_TH2, BUF_CNT2, BUF_LIST3,
     BUF_SLOT3, BUF_TH3, BUF_XB3,
-    BUF_BX, BUF_BFITS, BUF_BSTATE, BUF_BITEMS, BUF_BPART, BUF_BORDER, BUF_BCTR, BUF_BLAB, BUF_BMEM, BUF_BCEN, BUF_BXOFF, BUF_BSUMS, BUF_BTHR,
+    BUF_BX, BUF_BFITS, BUF_BSTATE, BUF_BITEMS, BUF_BPART, BUF_BORDER, BUF_BCTR, BUF_BLAB, BUF_BMEM, BUF_BCEN, BUF_BXOFF, BUF_BSUMS, BUF_BTHR, BUF_XPAD, BUF_IPAD,
     BUF_SC_C,
     BUF_XSQ, BUF_MX_UB, BUF_MX_NEAR, BUF_LROWS, BUF_LXB, BUF_LXAUG, BUF_LSCALE,
     BUF_KPPC, BUF_PR_UB, BUF_PR_SHIFT, BUF_PR_NEAR, BUF_PR_LIST,
@@ -285,6 +285,9 @@ inline void flush_timers(Ctx &ctx) {
 template <typename TX, typename TC>
 void launch_assign_direct(const TX *x, int64_t n, int d, const TC *c, int k, int32_t *labels,
                           TC *mind, cudaStream_t s);
+// Rows of d values as rows of dp >= d, zeros behind (dp < d: the first dp values).
+template <typename T>
+void launch_repitch(const T *src, int64_t n, int d, T *dst, int dp, cudaStream_t s);
 // The direct-form labels of a small call in one launch (assign_small_ok).
 bool assign_small_ok(int64_t n, int d, int k);
 template <typename T>
