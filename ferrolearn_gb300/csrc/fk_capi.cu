@@ -130,7 +130,10 @@ const T *stage_in(Ctx &ctx, BufSlot slot, const T *p, size_t count) {
 // buffer with one host thread, which also takes the page faults of a fresh
 // array: a transform with a 102 MB result took 4.4 ms, with eight threads 3.0
 // (four 4.0, six 3.2, twelve 2.8; pieces of 2 and 4 MB no faster). A 16 MB result,
-// whose array the allocator mostly reuses, was slower with threads.
+// whose array the allocator mostly reuses, was slower with threads. So was an f64
+// transform (160 MB 17.9 -> 19.8 ms): its 16 ms of FP64 leave the driver the time
+// to prepare the pages. Only f32 transforms, whose kernels are short beside
+// their results' copies, take the threads.
 constexpr size_t HOST_COPY_MIN = (size_t)48 << 20;
 
 bool make_host_copy(Ctx &ctx) {
@@ -213,7 +216,6 @@ bool copy_out_threads(Ctx &ctx, void *dst, const void *dev_src, size_t bytes) {
 template <typename T>
 void copy_out(Ctx &ctx, T *dst, const T *dev_src, size_t count) {
     if (!count || !dst) return;
-    if (copy_out_threads(ctx, dst, dev_src, sizeof(T) * count)) return;
     FK_CUDA(cudaMemcpyAsync(dst, dev_src, sizeof(T) * count, cudaMemcpyDefault, ctx.stream));
 }
 
@@ -987,7 +989,8 @@ fk_status transform_impl(fk_ctx *ctxp, const T *c_in, int64_t k, int64_t d_fit, 
     const T *c = stage_in<T>(ctx, BUF_C0, c_in, (size_t)k * d);
     T *o = is_device_ptr(out) ? out : (T *)ctx.get(BUF_OUT, sizeof(T) * (size_t)n * k);
     launch_transform_direct<T>(x, n, (int)d, c, (int)k, o, s);
-    if (o != out) copy_out<T>(ctx, out, o, (size_t)n * k);
+    if (o != out && !(sizeof(T) == 4 && copy_out_threads(ctx, out, o, sizeof(T) * (size_t)n * k)))
+        copy_out<T>(ctx, out, o, (size_t)n * k);
     FK_CUDA(cudaStreamSynchronize(s));
     return FK_OK;
 }

@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(SNT)
         for (int c0 = 0; c0 < k; c0 += 128) {
             float acc[4] = {0.f, 0.f, 0.f, 0.f};
             const float *cp = ct + c0 + lane;
-#pragma unroll 4
+#pragma unroll 8
             for (int j = 0; j < d; j++) {
                 const float xv = xr[j];
 #pragma unroll
@@ -323,9 +323,12 @@ void launch_rows(const float *x, int64_t n, int d, int k, const ScorePlan &p, bo
 // the two operations saved per feature; below 2e8 products the direct pass (18 us
 // at 1e8) costs little more than the two launches around the tiled one (7 us).
 // Predict calls at the line, direct / scored: 1,000,000 x 16, 24 centres 382 /
-// 184 us, 400,000 x 16, 32: 179 / 109, 2,000 x 256, 500: 383 / 257.
+// 184 us, 400,000 x 16, 32: 179 / 109, 2,000 x 256, 500: 383 / 257. Where the
+// direct pass's 128-row tiles fill the SMs about once it needs 3e8: 30,000 x 80, 100
+// (2.4e8) 92 / 81 us when few rows stay open, 92 / 97 when many do.
 bool f32_scores_pay(int64_t n, int d, int k) {
-    return d >= 16 && d <= 1024 && k >= 24 && n < INT32_MAX && (double)n * d * k >= 2e8;
+    const double w = (double)n * d * k;
+    return d >= 16 && d <= 1024 && k >= 24 && n < INT32_MAX && w >= 2e8 && (w >= 3e8 || n < 16384 || n >= 38912);
 }
 
 void launch_assign_f32_scored(Ctx &ctx, const float *x, int64_t n, int d, const float *c, int k, int32_t *labels) {

@@ -23,12 +23,12 @@ def test_transform_into_host_memory(n):
 
 def test_two_threads_carry_results_at_once():
     rng = np.random.default_rng(1)
-    x, c = rng.normal(size=(100003, 4)), rng.normal(size=(64, 4))
+    x, c = rng.normal(size=(200003, 4)).astype(np.float32), rng.normal(size=(64, 4)).astype(np.float32)
     want = O.transform(c, x)
     got = {}
 
     def work(i):
-        model = F.FittedKMeans(c, None, 0.0, 0, "f64")
+        model = F.FittedKMeans(c, None, 0.0, 0, "f32")
         got[i] = [model.transform(x) for _ in range(3)]  # a context a thread
 
     threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
