@@ -28,10 +28,13 @@ struct Error {
     fk_status code;
 };
 
+// The runtime also keeps the error of a refused call until it is asked for; the
+// next launch check would take it for its own.
 #define FK_CUDA(call)                                                                   \
     do {                                                                                \
         cudaError_t _e = (call);                                                        \
         if (_e != cudaSuccess) {                                                        \
+            (void)cudaGetLastError();                                                   \
             ::fk::set_error("%s failed: %s (%s:%d)", #call, cudaGetErrorString(_e),    \
                             __FILE__, __LINE__);                                        \
             throw ::fk::Error{_e == cudaErrorMemoryAllocation ? FK_ERR_OOM : FK_ERR_CUDA}; \
