@@ -80,6 +80,7 @@ struct MixedStats {
     float amax;    // max |x_ij| over finite entries (set once per X)
     float tmax;    // max |x_ij - mu_j| over finite entries (set once per X)
     float nonfinite;  // 1 if some row of X holds a non-finite value or overflows ||x|| (set once per X)
+    float mu_norm;    // ||mu||, the norm of the centring vector (set once per X; here, as captured launches outlive X)
     float cn_max;  // max_c ||c' ||            (per iteration from here on)
     float ec_max;  // max_c ||c' - ch||
     float ch_max;  // max_c ||ch||
@@ -139,7 +140,6 @@ struct MixedPlan {
     int slots = 3;        // rotating tile-merge slots of the top-2 pass
     size_t smem = 0;
     const void *x = nullptr;
-    double mu_norm = 0.0;
     const void *tm_x_ptr = nullptr, *tm_c_ptr = nullptr, *tm_aug_ptr = nullptr, *tm_xaug_ptr = nullptr;
     bool fp8 = false;
     alignas(64) unsigned char tm_xaug[128];

@@ -1026,10 +1026,11 @@ __device__ __forceinline__ void finalize_rows(int64_t n, Load load, Classify cla
 
 __global__ void __launch_bounds__(FINALIZE_THREADS, 2)
     finalize_kernel(const SliceTop2 *__restrict__ parts, int nparts, int kp, int64_t n, int k, int d,
-                    const float4 *__restrict__ rowinfo, const MixedStats *stats, float acc_rel, float mu_norm,
+                    const float4 *__restrict__ rowinfo, const MixedStats *stats, float acc_rel,
                     int32_t *__restrict__ labels, int4 *__restrict__ pair_list, int32_t *__restrict__ full_list,
                     float *__restrict__ full_thresh, float *__restrict__ floor_out, DevScalars *sc, RowBounds rb,
                     const int32_t *__restrict__ rows) {
+    const float mu_norm = stats->mu_norm;
     // rows: record i is row rows[i], sc->listed_rows of them (records of slice p
     // from p * n on either way)
     struct Rec {
@@ -1159,7 +1160,8 @@ __global__ void centre_shift_kernel(const double *__restrict__ c, const double *
 __global__ void count_thresh_kernel(int64_t n, int k, int d, const float *__restrict__ floor_prev,
                                     const int32_t *__restrict__ labels_prev, const float4 *__restrict__ rowinfo,
                                     const float2 *__restrict__ shift, const MixedStats *stats, float acc_rel,
-                                    float mu_norm, float *__restrict__ th_out) {
+                                    float *__restrict__ th_out) {
+    const float mu_norm = stats->mu_norm;
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int l = labels_prev[i];
@@ -1190,10 +1192,11 @@ __device__ __forceinline__ int count_column(int base, int w, int b) {
 // iteration (the largest score is a raw accumulator: no key slack).
 __global__ void __launch_bounds__(FINALIZE_THREADS, 2)  // two blocks an SM: 64 registers a thread
     finalize_count_kernel(const SliceCount *__restrict__ parts, int nparts, int kp, int64_t n, int k, int d,
-                          const float4 *__restrict__ rowinfo, const MixedStats *stats, float acc_rel, float mu_norm,
+                          const float4 *__restrict__ rowinfo, const MixedStats *stats, float acc_rel,
                           const float *__restrict__ thresh, int32_t *__restrict__ labels,
                           int4 *__restrict__ pair_list, int32_t *__restrict__ full_list,
                           float *__restrict__ full_thresh, float *__restrict__ floor_out, DevScalars *sc) {
+    const float mu_norm = stats->mu_norm;
     struct Rec {
         float4 ri;
         SliceCount o0, o1;
@@ -1799,8 +1802,9 @@ __global__ void __launch_bounds__(MASK_WARPS * 32)
 // mark is the label.
 __global__ void second_thresh_kernel(const int32_t *__restrict__ list, const unsigned long long *count,
                                      const float *__restrict__ floors, const float4 *__restrict__ rowinfo2,
-                                     const MixedStats *st2, float acc_rel2, float mu_norm, int d,
+                                     const MixedStats *st2, float acc_rel2, const float *mu_norm_p, int d,
                                      float *__restrict__ th) {
+    const float mu_norm = *mu_norm_p;
     const unsigned long long cnt = *count;
     for (unsigned long long s = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; s < cnt;
          s += (unsigned long long)gridDim.x * blockDim.x) {
@@ -1821,10 +1825,12 @@ __global__ void second_thresh_kernel(const int32_t *__restrict__ list, const uns
 __global__ void second_finalize_kernel(const SliceCount *__restrict__ parts, int nparts, int kp, int64_t cap, int k,
                                        int d, const int32_t *__restrict__ list, const unsigned long long *count,
                                        const float4 *__restrict__ rowinfo2, const MixedStats *st2, float acc_rel2,
-                                       float mu_norm, const float *__restrict__ th, int32_t *__restrict__ labels,
-                                       int32_t *__restrict__ ex_list, int32_t *__restrict__ list3,
+                                       const float *mu_norm_p, const float *__restrict__ th,
+                                       int32_t *__restrict__ labels, int32_t *__restrict__ ex_list,
+                                       int32_t *__restrict__ list3,
                                        int32_t *__restrict__ slot3, float *__restrict__ th3, DevScalars *sc,
                                        RowBounds rb, int4 *__restrict__ pair_end) {
+    const float mu_norm = *mu_norm_p;
     const unsigned long long cnt = *count;
     for (unsigned long long s = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; s < cnt;
          s += (unsigned long long)gridDim.x * blockDim.x) {
@@ -2057,6 +2063,12 @@ struct MixedBufs {
     float *c32, *ec32, *c32t;
 };
 
+// ||mu|| as an f32 upper bound.
+float mu_norm_up(double v) {
+    const float f = (float)v;
+    return (double)f >= v ? f : std::nextafter(f, INFINITY);
+}
+
 // Plans the launch and prepares the rows (when X changed) and the centres.
 template <typename TX>
 MixedBufs prepare_mixed(Ctx &ctx, const TX *x, int64_t n, int d, const double *c, int k, bool fp8, bool x_changed) {
@@ -2104,7 +2116,8 @@ MixedBufs prepare_mixed(Ctx &ctx, const TX *x, int64_t n, int d, const double *c
         FK_CUDA(cudaStreamSynchronize(s));
         double m2 = 0.0;
         for (double v : hmu) m2 += v * v;
-        mp.mu_norm = std::sqrt(m2) * (1.0 + 1e-12);
+        const float mu_norm = mu_norm_up(std::sqrt(m2) * (1.0 + 1e-12));
+        FK_CUDA(cudaMemcpyAsync(&B.stats->mu_norm, &mu_norm, sizeof(float), cudaMemcpyHostToDevice, s));
     } else {
         // centre statistics are per iteration; the row maxima stay
         FK_CUDA(cudaMemsetAsync((char *)B.stats + offsetof(MixedStats, cn_max), 0,
@@ -2144,12 +2157,6 @@ __global__ void rowscale_kernel(const float4 *__restrict__ rowinfo, int64_t n, c
     if (i < n) rowscale[i] = rowinfo[i].w * stats->inv_t;
 }
 
-// ||mu|| as an f32 upper bound.
-float mu_norm_up(double v) {
-    const float f = (float)v;
-    return (double)f >= v ? f : std::nextafter(f, INFINITY);
-}
-
 // The exact re-score of listed pairs (entry q at list + q * step).
 template <typename TX>
 void launch_pairs(Ctx &ctx, const TX *x, int d, const double *c, const MixedBufs &B, const int4 *list, int step,
@@ -2178,7 +2185,7 @@ void launch_pairs(Ctx &ctx, const TX *x, int d, const double *c, const MixedBufs
 // BF16 count pass against thresholds from the rows' floors, the mask pass
 // over the rows it leaves open, then the same re-score.
 void second_pass(Ctx &ctx, const float *x, int64_t n, int d, const double *c, int k, const MixedBufs &B,
-                 double mu_norm, const int32_t *full, const float *full_thresh, int32_t *labels, DevScalars *sc,
+                 const int32_t *full, const float *full_thresh, int32_t *labels, DevScalars *sc,
                  Oct *f64_items, const RowBounds &rb, int4 *pairs) {
     cudaStream_t s = ctx.stream;
     const int grid = ctx.num_sms * 4;
@@ -2250,7 +2257,7 @@ void second_pass(Ctx &ctx, const float *x, int64_t n, int d, const double *c, in
     uint32_t *masks = (uint32_t *)ctx.get(BUF_MASKS, sizeof(uint32_t) * (size_t)n * wpr);
     const float *floors = (const float *)ctx.get(BUF_FLOORS, sizeof(float) * (size_t)n);
     const float acc_rel2 = (float)((double)((size_t)m2.d_pad + 32) * ACC_REL_PER_K);  // exact: integer * 2^-22
-    const float mun = mu_norm_up(mu_norm);
+    const float *mun = &B.stats->mu_norm;
     FK_CUDA(cudaMemsetAsync(st2, 0, sizeof(MixedStats), s));
     launch_prep_rows<float, false>(ctx, x, n, d, m2.d_pad, B.mu32, xb2, nullptr, ri2, st2, full, &sc->full_count);
     prep_centres_kernel<false><<<(m2.k_pad + 7) / 8, 256, 0, s>>>(c, k, m2.k_pad, d, m2.d_pad, B.mu, cb2, hn2,
@@ -2341,7 +2348,6 @@ void run_assign_mixed(Ctx &ctx, const TX *x, int64_t n, int d, const double *c, 
     // every pass leaves each row's floor for a count pass in the next iteration
     float *floors = (float *)ctx.get(BUF_FLOORS, sizeof(float) * (size_t)n);
     const float acc_rel = (float)((double)((size_t)mp.d_pad + 32) * ACC_REL_PER_K);  // exact: integer * 2^-22
-    const float mun = mu_norm_up(mp.mu_norm);
     static const int fin_top2 = resident_blocks((const void *)finalize_kernel, FINALIZE_THREADS);
     static const int fin_count = resident_blocks((const void *)finalize_count_kernel, FINALIZE_THREADS);
     const int64_t fin_chunks = (n + FINALIZE_THREADS - 1) / FINALIZE_THREADS;
@@ -2403,7 +2409,7 @@ void run_assign_mixed(Ctx &ctx, const TX *x, int64_t n, int d, const double *c, 
             launch_tc_assign(ctx, ml, lxb, B.cq, B.caug, top, sc, B.stats, nullptr, &sc->listed_rows, lxaug, lscale);
         }
         finalize_kernel<<<(unsigned)std::min<int64_t>(fin_chunks, (int64_t)ctx.num_sms * fin_top2), FINALIZE_THREADS,
-                          0, s>>>(top, mp.parts, mp.kp, n, k, d, B.rowinfo, B.stats, acc_rel, mun, labels, pairs, full,
+                          0, s>>>(top, mp.parts, mp.kp, n, k, d, B.rowinfo, B.stats, acc_rel, labels, pairs, full,
                                   full_thresh, floors, sc, rb, rows);
         FK_LAUNCH_CHECK();
     } else if (main == MAIN_COUNT) {
@@ -2418,7 +2424,7 @@ void run_assign_mixed(Ctx &ctx, const TX *x, int64_t n, int d, const double *c, 
         }
         float *th = (float *)ctx.get(BUF_THMAIN, sizeof(float) * (size_t)n);
         count_thresh_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, k, d, floors, labels_prev, B.rowinfo,
-                                                                      shift, B.stats, acc_rel, mun, th);
+                                                                      shift, B.stats, acc_rel, th);
         FK_LAUNCH_CHECK();
         SliceCount *cnt = (SliceCount *)ctx.get(BUF_TOP2, sizeof(SliceCount) * (size_t)n * mc.parts);
         {
@@ -2429,7 +2435,7 @@ void run_assign_mixed(Ctx &ctx, const TX *x, int64_t n, int d, const double *c, 
         }
         finalize_count_kernel<<<(unsigned)std::min<int64_t>(fin_chunks, (int64_t)ctx.num_sms * fin_count),
                                 FINALIZE_THREADS, 0, s>>>(cnt, mc.parts, mc.kp, n, k, d, B.rowinfo,
-                                                                      B.stats, acc_rel, mun, th, labels, pairs, full,
+                                                                      B.stats, acc_rel, th, labels, pairs, full,
                                                                       full_thresh, floors, sc);
         FK_LAUNCH_CHECK();
     } else {
@@ -2447,13 +2453,13 @@ void run_assign_mixed(Ctx &ctx, const TX *x, int64_t n, int d, const double *c, 
         }
         finalize_kernel<<<(unsigned)std::min<int64_t>(fin_chunks, (int64_t)ctx.num_sms * fin_top2), FINALIZE_THREADS,
                           0, s>>>(top, mp.parts, mp.kp, n, k, d, B.rowinfo, B.stats,
-                                                                acc_rel, mun, labels, pairs, full, full_thresh,
+                                                                acc_rel, labels, pairs, full, full_thresh,
                                                                 floors, sc, rb, nullptr);
         FK_LAUNCH_CHECK();
     }
     Oct *f64_items = (Oct *)ctx.get(BUF_F64ITEMS, sizeof(Oct) * (size_t)n);
     launch_pairs<TX>(ctx, x, d, c, B, pairs, 1, &sc->flag_count, sc, labels, f64_items, rb);
-    second_pass(ctx, x, n, d, c, k, B, mp.mu_norm, full, full_thresh, labels, sc, f64_items, rb, pairs);
+    second_pass(ctx, x, n, d, c, k, B, full, full_thresh, labels, sc, f64_items, rb, pairs);
     launch_f64_decide<TX>(ctx, x, d, c, f64_items, sc, labels);
 }
 
