@@ -16,7 +16,7 @@ _lib = None
 
 # Every symbol declared in include/ferrokmeans.h.
 EXPORTS = [
-    "fk_ctx_create", "fk_ctx_destroy", "fk_last_error_message", "fk_version", "fk_debug_launch_count",
+    "fk_ctx_create", "fk_ctx_destroy", "fk_last_error_message", "fk_version", "fk_debug_launch_count", "fk_debug_memory",
     "fk_kmeans_params_default", "fk_draws_f64",
     "fk_kmeans_fit_f64", "fk_kmeans_fit_f32", "fk_kmeans_fit_f32x64",
     "fk_lloyd_step_f64", "fk_lloyd_step_f32", "fk_lloyd_step_f32x64",
@@ -152,6 +152,8 @@ def _declare(lib):
     lib.fk_version.restype = C.c_char_p
     lib.fk_debug_launch_count.argtypes = []
     lib.fk_debug_launch_count.restype = C.c_uint64
+    lib.fk_debug_memory.argtypes = [p, u64, C.POINTER(C.c_uint64)]
+    lib.fk_debug_memory.restype = st
     lib.fk_kmeans_params_default.argtypes = [C.POINTER(KMeansParams), i64]
     lib.fk_kmeans_params_default.restype = None
     lib.fk_draws_f64.argtypes = [u64, i64, p]

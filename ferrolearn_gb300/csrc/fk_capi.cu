@@ -55,29 +55,44 @@ void Ctx::bind() {
 void *Ctx::get(BufSlot s, size_t bytes) {
     if (bytes == 0) bytes = 16;
     if (cap[s] >= bytes) return buf[s];
-    if (buf[s]) {
-        FK_CUDA(cudaStreamSynchronize(stream));
-        FK_CUDA(cudaFree(buf[s]));
-        buf[s] = nullptr;
-        cap[s] = 0;
-    }
-    size_t want = bytes + bytes / 8;  // headroom for slightly larger calls
-    void *p = nullptr;
+    drop(s);
     buf_gen++;  // captured iterations that used the old buffer are retired
-    cudaError_t e = cudaMalloc(&p, want);
-    if (e != cudaSuccess) {
-        (void)cudaGetLastError();
-        e = cudaMalloc(&p, bytes);
-        want = bytes;
+    cudaError_t e = cudaSuccess;
+    auto take = [&](size_t want) {
+        e = limit && held + want > limit ? cudaErrorMemoryAllocation : cudaMalloc(&buf[s], want);
+        if (e != cudaSuccess) {
+            (void)cudaGetLastError();
+            buf[s] = nullptr;
+            return false;
+        }
+        cap[s] = want;
+        held += want;
+        return true;
+    };
+    // headroom for slightly larger calls, unless memory is short
+    if ((!lean && take(bytes + bytes / 8)) || take(bytes)) return buf[s];
+    if (!seeding && (buf[BUF_KPP0] || buf[BUF_KPP1] || buf[BUF_KPP2])) {
+        // the seedings' workspace, which nothing reads once the seeds are out
+        for (BufSlot q : {BUF_KPP0, BUF_KPP1, BUF_KPP2}) drop(q);
+        if (take(bytes)) return buf[s];
     }
-    if (e != cudaSuccess) {
-        (void)cudaGetLastError();
-        set_error("cudaMalloc of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
-        fail(FK_ERR_OOM);
-    }
-    buf[s] = p;
-    cap[s] = want;
-    return p;
+    set_error("cudaMalloc of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
+    fail(FK_ERR_OOM);
+}
+
+void Ctx::drop(BufSlot s) {
+    if (!buf[s]) return;
+    FK_CUDA(cudaStreamSynchronize(stream));
+    FK_CUDA(cudaFree(buf[s]));
+    held -= cap[s];
+    buf[s] = nullptr;
+    cap[s] = 0;
+}
+
+void Ctx::release() {
+    for (int q = 0; q < BUF_COUNT; q++) drop((BufSlot)q);
+    buf_gen++;
+    for (MixedPlan *p : {&mixed, &mixed2, &mixedm, &mixedm2, &mixedc, &mixedl}) p->n = -1;  // their maps name the buffers
 }
 
 // n_trials of kmeans.rs:198 (2 + floor(ln k), at least 1).
@@ -217,6 +232,15 @@ template <typename T>
 void copy_out(Ctx &ctx, T *dst, const T *dev_src, size_t count) {
     if (!count || !dst) return;
     FK_CUDA(cudaMemcpyAsync(dst, dev_src, sizeof(T) * count, cudaMemcpyDefault, ctx.stream));
+}
+
+// The caller's 64-bit labels. The first of a call's outputs: what it allocates may
+// send the call round again, and a caller may pass one buffer as input and output.
+void write_labels(Ctx &ctx, const int32_t *labels, int64_t n, uint64_t *out) {
+    const bool dev = is_device_ptr(out);
+    uint64_t *l64 = dev ? out : (uint64_t *)ctx.get(BUF_OUT, sizeof(uint64_t) * (size_t)n);
+    launch_labels_to_u64(labels, n, l64, ctx.stream);
+    if (!dev) copy_out<uint64_t>(ctx, out, l64, (size_t)n);
 }
 
 template <typename T> struct FMax;
@@ -369,10 +393,11 @@ void run_graphed(Ctx &ctx, const uint64_t (&key)[10], Body &&body) {
 // 1M x 127 against 1,000 centres 30.0 / 8.1 ms in BF16 and 43.4 / 11.9 in FP8,
 // 300,000 x 250 against 500 23.1 / 6.6 and 33.1 / 7.9 (d = 128 and 252 as they are:
 // 7.9, 11.6, 6.3, 7.4). nullptr: not needed, d beyond these forms, or no memory
-// for the copy (the kernels for single values run then).
+// for the copy and what else the call needs (the kernels for single values run then).
 const float *pad_rows(Ctx &ctx, const float *x, int64_t n, int64_t d, int64_t &dp) {
     dp = (d + 3) / 4 * 4;
-    if (dp > 256 || d == 0 || (dp == d && ((uintptr_t)x & 15u) == 0)) return nullptr;
+    if (ctx.lean || dp > 256 || d == 0 || (dp == d && ((uintptr_t)x & 15u) == 0)) return nullptr;
+    ctx.spared = true;
     float *xp;
     try {
         xp = (float *)ctx.get(BUF_XPAD, sizeof(float) * (size_t)n * dp);
@@ -388,7 +413,8 @@ const float *pad_rows(Ctx &ctx, const float *x, int64_t n, int64_t d, int64_t &d
 template <typename TX, typename TC>
 void assign_direct_labels(Ctx &ctx, const TX *x, int64_t n, int d, const TC *c, int k, int32_t *labels) {
     if constexpr (std::is_same<TX, float>::value && std::is_same<TC, float>::value) {
-        if (f32_scores_pay(n, d, k)) {
+        if (!ctx.lean && f32_scores_pay(n, d, k)) {
+            ctx.spared = true;
             try {
                 launch_assign_f32_scored(ctx, x, n, d, c, k, labels);
                 return;
@@ -637,7 +663,9 @@ fk_status fit_impl(fk_ctx *ctxp, const TX *x_in, int64_t n, int64_t d, const fk_
     // preparation has shown X finite and inside the split's exponent range.
     bool inc_candidate = false, incremental = false;
     // Plain forms of some size: centres that cannot win are left out
-    const bool prune = std::is_same<TX, TC>::value && p->precision == FK_PRECISION_PLAIN && prune_shape_ok(n, (int)d, (int)k);
+    const bool prune = std::is_same<TX, TC>::value && p->precision == FK_PRECISION_PLAIN && !ctx.lean &&
+                       prune_shape_ok(n, (int)d, (int)k);
+    if (prune) ctx.spared = true;
     if constexpr (std::is_same<TX, float>::value && std::is_same<TC, double>::value)
         inc_candidate = p->precision != FK_PRECISION_PLAIN && incremental_shape_ok((const float *)x, (int)d);
     for (int64_t run = 0; run < p->n_init; run++) {
@@ -690,7 +718,8 @@ fk_status fit_impl(fk_ctx *ctxp, const TX *x_in, int64_t n, int64_t d, const fk_
             count_ok = p->precision == FK_PRECISION_MIXED_BF16 || p->precision == FK_PRECISION_MIXED_FP8;
         bool bounds = false;  // this run's top-2 passes leave row bounds
         if constexpr (std::is_same<TX, float>::value && std::is_same<TC, double>::value)
-            bounds = count_ok && mixed_bounds_ok(n, (int)d, (int)k);
+            bounds = count_ok && !ctx.lean && mixed_bounds_ok(n, (int)d, (int)k);
+        if (bounds) ctx.spared = true;
         bool was_listed = false;
         int64_t kept = 0;  // rows kept, of the last iteration read
         bool was_count[2] = {false, false};
@@ -819,14 +848,8 @@ fk_status fit_impl(fk_ctx *ctxp, const TX *x_in, int64_t n, int64_t d, const fk_
         launch_repitch<TC>(cbest, k, (int)d, cb3[0], (int)d_in, s);
         cbest = cb3[0];
     }
+    write_labels(ctx, lbest, n, labels_out);
     copy_out<TC>(ctx, centers_out, cbest, (size_t)k * d_in);
-    if (is_device_ptr(labels_out)) {
-        launch_labels_to_u64(lbest, n, labels_out, s);
-    } else {
-        uint64_t *l64 = (uint64_t *)ctx.get(BUF_OUT, sizeof(uint64_t) * (size_t)n);
-        launch_labels_to_u64(lbest, n, l64, s);
-        copy_out<uint64_t>(ctx, labels_out, l64, (size_t)n);
-    }
     if (timing) {
         FK_CUDA(cudaEventRecord((*tev)[1], s));
         FK_CUDA(cudaEventSynchronize((*tev)[1]));
@@ -881,14 +904,8 @@ fk_status step_impl(fk_ctx *ctxp, const TX *x_in, int64_t n, int64_t d, const TC
     lloyd_iteration<TX, TC>(ctx, x, n, (int)d, c, (int)k, prec, nc, labels, sc, plan, true, rep, false);
     read_scalars(ctx, sc);
     accumulate_report(rep, *ctx.host_scalars, n);
+    write_labels(ctx, labels, n, labels_out);
     copy_out<TC>(ctx, centers_out, nc, kd);
-    if (is_device_ptr(labels_out)) {
-        launch_labels_to_u64(labels, n, labels_out, s);
-    } else {
-        uint64_t *l64 = (uint64_t *)ctx.get(BUF_OUT, sizeof(uint64_t) * (size_t)n);
-        launch_labels_to_u64(labels, n, l64, s);
-        copy_out<uint64_t>(ctx, labels_out, l64, (size_t)n);
-    }
     FK_CUDA(cudaStreamSynchronize(s));
     *inertia_out = (TC)ctx.host_scalars->inertia;
     *shift_out = shift_from_bits<TC>(ctx.host_scalars->shift_bits);
@@ -953,13 +970,7 @@ fk_status predict_impl(fk_ctx *ctxp, const TC *c_in, int64_t k, int64_t d_fit, c
             run_assign_mixed(ctx, xp ? xp : x, n, (int)(xp ? dp : d), c, (int)k, prec, labels, nullptr, sc, true);
         }
     }
-    if (is_device_ptr(labels_out)) {
-        launch_labels_to_u64(labels, n, labels_out, s);
-    } else {
-        uint64_t *l64 = (uint64_t *)ctx.get(BUF_OUT, sizeof(uint64_t) * (size_t)n);
-        launch_labels_to_u64(labels, n, l64, s);
-        copy_out<uint64_t>(ctx, labels_out, l64, (size_t)n);
-    }
+    write_labels(ctx, labels, n, labels_out);
     FK_CUDA(cudaStreamSynchronize(s));
     return FK_OK;
 }
@@ -1253,14 +1264,8 @@ fk_status minibatch_impl(fk_ctx *ctxp, const T *x_in, int64_t n, int64_t d, cons
             FK_CUDA(cudaMemcpyAsync(lbest, labels, sizeof(int32_t) * (size_t)n, cudaMemcpyDeviceToDevice, s));
         }
     }
+    write_labels(ctx, lbest, n, labels_out);
     copy_out<T>(ctx, centers_out, cbest, kd);
-    if (is_device_ptr(labels_out)) {
-        launch_labels_to_u64(lbest, n, labels_out, s);
-    } else {
-        uint64_t *l64 = (uint64_t *)ctx.get(BUF_OUT, sizeof(uint64_t) * (size_t)n);
-        launch_labels_to_u64(lbest, n, l64, s);
-        copy_out<uint64_t>(ctx, labels_out, l64, (size_t)n);
-    }
     FK_CUDA(cudaEventRecord(tev[1], s));
     FK_CUDA(cudaStreamSynchronize(s));
     if (rep) {
@@ -1354,6 +1359,9 @@ fk_status bisecting_impl(fk_ctx *ctxp, const T *x_in, int64_t n, int64_t d, cons
     FoldChain *dchains = (FoldChain *)ctx.get(BUF_BK_CHAINS, sizeof(FoldChain) * (nsum + runs + 2));
     T *fres = (T *)ctx.get(BUF_BK_FRES, sizeof(T) * (nsum + 8));
     long long *fcnt = (long long *)ctx.get(BUF_BK_FCNT, sizeof(long long) * (nsum + runs + 8));
+    // the outputs' buffers: taken before the folds', which make do with what is left
+    T *cout = (T *)ctx.get(BUF_OUT2, sizeof(T) * (size_t)k * d + 16);
+    int64_t *ldev = is_device_ptr(labels_out) ? labels_out : (int64_t *)ctx.get(BUF_BK_LABELS, sizeof(int64_t) * (size_t)n);
     std::vector<FoldChain> hchains;
     // feature j of the rows starts at rows + j * next, `stride` apart
     auto upload_sum_chains = [&](const T *rows, int64_t next, int64_t stride, int nr, bool gated) {
@@ -1509,10 +1517,8 @@ fk_status bisecting_impl(fk_ctx *ctxp, const T *x_in, int64_t n, int64_t d, cons
     }
     FK_CUDA(cudaMemcpyAsync(seg, hseg.data(), sizeof(int64_t) * hseg.size(), cudaMemcpyHostToDevice, s));
     FK_CUDA(cudaMemcpyAsync(scratch, hslot.data(), sizeof(int32_t) * hslot.size(), cudaMemcpyHostToDevice, s));
-    T *cout = (T *)ctx.get(BUF_OUT2, sizeof(T) * (size_t)nc * d + 16);
     launch_gather_rows<T>(centres, (int)d, scratch, nc, cout, s);
     copy_out<T>(ctx, centers_out, cout, (size_t)nc * d);
-    int64_t *ldev = is_device_ptr(labels_out) ? labels_out : (int64_t *)ctx.get(BUF_BK_LABELS, sizeof(int64_t) * (size_t)n);
     launch_bk_labels(perm, seg, nc, ldev, s);
     if (ldev != labels_out) copy_out<int64_t>(ctx, labels_out, ldev, (size_t)n);
     FK_CUDA(cudaStreamSynchronize(s));
@@ -1536,7 +1542,7 @@ void drop_call_state(fk_ctx *ctxp) {
 }
 
 template <typename F>
-fk_status guarded_body(fk_ctx *ctx, F &&f) {
+fk_status attempt(F &&f) {
     try {
         g_last_error.clear();
         return f();
@@ -1558,7 +1564,26 @@ fk_status guarded(fk_ctx *ctx, F &&f) {
         return FK_ERR_NULL_POINTER;
     }
     drop_call_state(ctx);
-    const fk_status st = guarded_body(ctx, f);
+    // A call that finds no room although the context holds buffers of earlier calls,
+    // or took a form that it can do without, gives everything back and runs once
+    // more in the forms that need least: what fits without them keeps running.
+    // (No call writes an output before it has all its buffers.)
+    Ctx &c = *reinterpret_cast<Ctx *>(ctx);
+    const bool held = c.held != 0;
+    c.spared = false;
+    fk_status st = attempt(f);
+    if (st == FK_ERR_OOM && (held || c.spared)) {
+        drop_call_state(ctx);
+        st = attempt([&] {
+            c.release();
+            return FK_OK;
+        });
+        if (st == FK_OK) {
+            c.lean = true;
+            st = attempt(f);
+            c.lean = false;
+        }
+    }
     drop_call_state(ctx);
     return st;
 }
@@ -1622,6 +1647,17 @@ const char *fk_last_error_message(void) { return fk::g_last_error.c_str(); }
 const char *fk_version(void) { return "ferrokmeans-gb300 0.1.0 (sm_103a)"; }
 
 uint64_t fk_debug_launch_count(void) { return __atomic_load_n(&fk::g_launch_count, __ATOMIC_RELAXED); }
+
+fk_status fk_debug_memory(fk_ctx *ctx, uint64_t limit, uint64_t *held) {
+    if (!ctx || !held) {
+        fk::set_error("required pointer is NULL");
+        return FK_ERR_NULL_POINTER;
+    }
+    fk::Ctx *c = reinterpret_cast<fk::Ctx *>(ctx);
+    c->limit = (size_t)limit;
+    *held = (uint64_t)c->held;
+    return FK_OK;
+}
 
 void fk_kmeans_params_default(fk_kmeans_params *p, int64_t n_clusters) {
     if (!p) return;

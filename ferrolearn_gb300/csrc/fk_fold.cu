@@ -369,24 +369,39 @@ void run_exact_folds(Ctx &ctx, const FoldChain *chains, int nchains, int64_t m, 
     if (nchains <= 0) return;
     cudaStream_t s = ctx.stream;
     const int64_t nch = m > 0 ? (m + FCH - 1) / FCH : 0;
-    float *csum = (float *)ctx.get(BUF_FOLD_SUM, sizeof(float) * (size_t)nchains * nch);
-    int32_t *ccnt = (int32_t *)ctx.get(BUF_FOLD_CNT, sizeof(int32_t) * (size_t)nchains * nch);
-    CMap *cmaps = (CMap *)ctx.get(BUF_FOLD_MAP, sizeof(CMap) * (size_t)nchains * nch);
+    // Chains at a time: gridDim.y holds 65,535, and their maps (48 bytes a chunk)
+    // stay within 1 GB, or as many as there is room for.
+    const int64_t room = (ctx.lean ? (int64_t)16 << 20 : (int64_t)1 << 30) / (48 * std::max<int64_t>(nch, 1));
+    int per = (int)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(nchains, 65535), room));
+    float *csum = nullptr;
+    int32_t *ccnt = nullptr;
+    CMap *cmaps = nullptr;
+    while (true) {
+        try {
+            csum = (float *)ctx.get(BUF_FOLD_SUM, sizeof(float) * (size_t)per * nch);
+            ccnt = (int32_t *)ctx.get(BUF_FOLD_CNT, sizeof(int32_t) * (size_t)per * nch);
+            cmaps = (CMap *)ctx.get(BUF_FOLD_MAP, sizeof(CMap) * (size_t)per * nch);
+            break;
+        } catch (const Error &e) {
+            if (e.code != FK_ERR_OOM || per == 1) throw;
+            per = (per + 1) / 2;
+        }
+    }
     const Chain<T> *ch = (const Chain<T> *)chains;
-    // gridDim.y holds 65,535 chains
-    for (int c0 = 0; c0 < nchains && nch > 0; c0 += 65535) {
-        const unsigned nc = (unsigned)std::min(65535, nchains - c0);
-        const dim3 grid((unsigned)((nch + FWARPS - 1) / FWARPS), nc);
-        float *cs = csum + (size_t)c0 * nch;
-        fold_sums_kernel<T><<<grid, FWARPS * 32, 0, s>>>(ch + c0, m, active, nch, cs, ccnt + (size_t)c0 * nch);
-        FK_LAUNCH_CHECK();
-        fold_prefix_kernel<T><<<nc, 32, 0, s>>>(ch + c0, active, nch, cs);
-        FK_LAUNCH_CHECK();
-        fold_compose_kernel<T><<<grid, FWARPS * 32, 0, s>>>(ch + c0, m, active, nch, cs, cmaps + (size_t)c0 * nch);
+    for (int c0 = 0; c0 < nchains; c0 += per) {
+        const unsigned nc = (unsigned)std::min(per, nchains - c0);
+        if (nch > 0) {
+            const dim3 grid((unsigned)((nch + FWARPS - 1) / FWARPS), nc);
+            fold_sums_kernel<T><<<grid, FWARPS * 32, 0, s>>>(ch + c0, m, active, nch, csum, ccnt);
+            FK_LAUNCH_CHECK();
+            fold_prefix_kernel<T><<<nc, 32, 0, s>>>(ch + c0, active, nch, csum);
+            FK_LAUNCH_CHECK();
+            fold_compose_kernel<T><<<grid, FWARPS * 32, 0, s>>>(ch + c0, m, active, nch, csum, cmaps);
+            FK_LAUNCH_CHECK();
+        }
+        fold_walk_kernel<T><<<nc, 32, 0, s>>>(ch + c0, m, active, nch, cmaps, ccnt, result + c0, count + c0);
         FK_LAUNCH_CHECK();
     }
-    fold_walk_kernel<T><<<(unsigned)nchains, 32, 0, s>>>(ch, m, active, nch, cmaps, ccnt, result, count);
-    FK_LAUNCH_CHECK();
 }
 
 template void run_exact_folds<double>(Ctx &, const FoldChain *, int, int64_t, const int *, double *, long long *);

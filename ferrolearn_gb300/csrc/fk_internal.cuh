@@ -189,6 +189,11 @@ struct Ctx {
     bool own_stream = false;
     void *buf[BUF_COUNT] = {};
     size_t cap[BUF_COUNT] = {};
+    size_t held = 0;        // bytes in all of them
+    size_t limit = 0;       // most bytes they may take (0: what the device has)
+    bool spared = false;    // this call took a form that it can do without
+    bool lean = false;      // this attempt takes the forms that need least memory
+    bool seeding = false;   // the seedings' workspace (BUF_KPP0 .. 2) is in use
     DevScalars *host_scalars = nullptr;  // pinned
     int num_sms = 0;
     int cc_major = 0, cc_minor = 0;
@@ -224,6 +229,8 @@ struct Ctx {
     double *count_acc = nullptr;     // when set: device time of the count passes among those
 
     void *get(BufSlot s, size_t bytes);  // grow-only device buffer
+    void drop(BufSlot s);                // gives one back
+    void release();                      // gives all of them back
     void bind();                         // make the device current
 };
 

@@ -1681,12 +1681,19 @@ void run_split(Ctx &ctx, const std::vector<KppJob> &jobs, const std::vector<int>
 }  // namespace
 
 // Seedings run together while their workspaces stay within this many bytes
-// (one larger seeding runs alone).
+// (one larger seeding runs alone, and each one where memory is short).
 constexpr size_t KPP_GROUP_BYTES = (size_t)6 << 30;
 
 template <typename T>
 void run_kmeanspp(Ctx &ctx, std::vector<KppJob> &jobs, int64_t *draws_used) {
     if (jobs.empty()) return;
+    struct Seeding {
+        Ctx &c;
+        explicit Seeding(Ctx &ctx) : c(ctx) { c.seeding = true; }
+        ~Seeding() { c.seeding = false; }
+    } use(ctx);
+    if (jobs.size() > 1) ctx.spared = true;
+    const size_t group_bytes = ctx.lean ? 0 : KPP_GROUP_BYTES;
     long long rows = 0;
     for (const KppJob &j : jobs) {
         const int trials = kpp_trials_host(j.k);
@@ -1722,7 +1729,7 @@ void run_kmeanspp(Ctx &ctx, std::vector<KppJob> &jobs, int64_t *draws_used) {
                                ? kpp_layout<T>(jobs[(size_t)order[q]], kpp_trials_host(jobs[(size_t)order[q]].k), scan).total
                                : 0;
         // (blockIdx.x counts the group's seedings too: far below its limit)
-        if (q > lo && (q == order.size() || bytes + add > KPP_GROUP_BYTES)) {
+        if (q > lo && (q == order.size() || bytes + add > group_bytes)) {
             run_split<T>(ctx, jobs, order, lo, q, scan, draws_used);
             lo = q;
             bytes = 0;

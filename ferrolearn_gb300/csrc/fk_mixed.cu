@@ -2056,7 +2056,7 @@ struct MixedBufs {
     void *xq;               // BF16 or E4M3 rows, n x d_pad
     __nv_bfloat16 *xaug;    // FP8: per-row augmentation rows, n x 16
     float4 *rowinfo;
-    float *xsq;             // ||x'||^2 of each row, f32 sums
+    float *xsq;             // ||x'||^2 of each row, f32 sums (where row bounds are kept)
     void *cq;               // BF16 or E4M3 centres, k_pad x d_pad
     __nv_bfloat16 *caug;    // k_pad x 16
     double *half_norm;
@@ -2071,7 +2071,8 @@ float mu_norm_up(double v) {
 
 // Plans the launch and prepares the rows (when X changed) and the centres.
 template <typename TX>
-MixedBufs prepare_mixed(Ctx &ctx, const TX *x, int64_t n, int d, const double *c, int k, bool fp8, bool x_changed) {
+MixedBufs prepare_mixed(Ctx &ctx, const TX *x, int64_t n, int d, const double *c, int k, bool fp8, bool x_changed,
+                        bool bounds) {
     cudaStream_t s = ctx.stream;
     MixedPlan &mp = ctx.mixed;
     const bool replan = x_changed || mp.n != n || mp.d != d || mp.k != k || mp.x != (const void *)x || mp.fp8 != fp8;
@@ -2085,7 +2086,7 @@ MixedBufs prepare_mixed(Ctx &ctx, const TX *x, int64_t n, int d, const double *c
     B.xq = ctx.get(BUF_XB, es * (size_t)n * mp.d_pad);
     B.xaug = fp8 ? (__nv_bfloat16 *)ctx.get(BUF_XAUG, sizeof(__nv_bfloat16) * 16 * (size_t)n) : nullptr;
     B.rowinfo = (float4 *)ctx.get(BUF_XNORM, sizeof(float4) * (size_t)n);
-    B.xsq = (float *)ctx.get(BUF_XSQ, sizeof(float) * (size_t)n);
+    B.xsq = bounds ? (float *)ctx.get(BUF_XSQ, sizeof(float) * (size_t)n) : nullptr;
     if (replan) {
         FK_CUDA(cudaMemsetAsync(B.stats, 0, sizeof(MixedStats), s));
         // the centring vector only needs to be finite: a strided sample of at
@@ -2334,7 +2335,8 @@ void run_assign_mixed(Ctx &ctx, const TX *x, int64_t n, int d, const double *c, 
         set_error("the tensor-core path supports 1 <= d <= 256 (got %d)", d);
         fail(FK_ERR_UNSUPPORTED);
     }
-    MixedBufs B = prepare_mixed<TX>(ctx, x, n, d, c, k, fp8, x_changed);
+    const bool bounds = main == MAIN_TOP2_BOUNDS || main == MAIN_LISTED;
+    MixedBufs B = prepare_mixed<TX>(ctx, x, n, d, c, k, fp8, x_changed, bounds);
     float *rowscale = nullptr;
     if (fp8) {
         rowscale = (float *)ctx.get(BUF_ROWSCALE, sizeof(float) * (size_t)n);
@@ -2359,7 +2361,7 @@ void run_assign_mixed(Ctx &ctx, const TX *x, int64_t n, int d, const double *c, 
         FK_LAUNCH_CHECK();
     }
     float *near2 = nullptr;
-    if (c_prev && (main == MAIN_TOP2_BOUNDS || main == MAIN_LISTED)) {
+    if (c_prev && bounds) {
         near2 = (float *)ctx.get(BUF_MX_NEAR, sizeof(float) * (size_t)k);
         FK_CUDA(cudaMemsetAsync(near2, 0x7F, sizeof(float) * (size_t)k, s));
         const unsigned t = (unsigned)((k + NT_ - 1) / NT_);
@@ -2368,7 +2370,7 @@ void run_assign_mixed(Ctx &ctx, const TX *x, int64_t n, int d, const double *c, 
     }
     const unsigned bound_grid =
         (unsigned)std::min<int64_t>((n + MBT * MB_ROWS - 1) / (MBT * MB_ROWS), (int64_t)ctx.num_sms * 6);
-    if (main == MAIN_TOP2_BOUNDS || main == MAIN_LISTED) {
+    if (bounds) {
         rb.xsq = B.xsq;
         rb.ub = (float *)ctx.get(BUF_MX_UB, sizeof(float) * 2 * (size_t)n);
         rb.lb = rb.ub + n;
@@ -2485,7 +2487,7 @@ void debug_tc_probe(Ctx &ctx, const float *x, int64_t n, int d, const double *c,
     const bool fp8 = precision == FK_PRECISION_MIXED_FP8;
     DevScalars *sc = (DevScalars *)ctx.get(BUF_SCALARS, sizeof(DevScalars));
     FK_CUDA(cudaMemsetAsync(sc, 0, sizeof(DevScalars), s));
-    MixedBufs B = prepare_mixed<float>(ctx, x, n, d, c, k, fp8, true);
+    MixedBufs B = prepare_mixed<float>(ctx, x, n, d, c, k, fp8, true, false);
     mp.x = nullptr;
     float *rowscale = nullptr;
     if (fp8) {

@@ -7,7 +7,9 @@
  * row-major and C-contiguous. Any input or output pointer may be host memory
  * or device memory of the context's GPU: the library checks each pointer and
  * copies only what lives on the host. Calls are synchronous (they return when
- * the results are in the caller's buffers), like the Rust methods.
+ * the results are in the caller's buffers), like the Rust methods. A call that
+ * the device has no room for gives the context's buffers back and tries once
+ * more in the forms that need least, before it returns FK_ERR_OOM.
  *
  * Status codes map one-to-one onto ferrolearn_core::error::FerroError
  * (ferrolearn-core/src/error.rs:30-91) plus CUDA-side failures; the message of
@@ -129,6 +131,10 @@ const char *fk_version(void);
 /* Diagnostics: number of kernel launches this library has issued so far in
  * the process (all contexts). No reference counterpart. */
 uint64_t fk_debug_launch_count(void);
+/* Diagnostics: sets the most bytes that the context's device buffers may take
+ * (0: what the device has) and returns what they take now. A call beyond it
+ * fails with FK_ERR_OOM as it would on a full device. No GPU needed. */
+fk_status fk_debug_memory(fk_ctx *ctx, uint64_t limit, uint64_t *held_out);
 
 /* KMeans::new(n_clusters) defaults (kmeans.rs:76-84). */
 void fk_kmeans_params_default(fk_kmeans_params *p, int64_t n_clusters);

@@ -143,6 +143,7 @@ unsafe extern "C" {
     pub fn fk_last_error_message() -> *const c_char;
     pub fn fk_version() -> *const c_char;
     pub fn fk_debug_launch_count() -> u64;
+    pub fn fk_debug_memory(ctx: *mut fk_ctx, limit: u64, held_out: *mut u64) -> i32;
     pub fn fk_kmeans_params_default(p: *mut fk_kmeans_params, n_clusters: i64);
     pub fn fk_draws_f64(seed: u64, count: i64, out: *mut f64) -> i32;
     pub fn fk_kmeans_fit_f64(ctx: *mut fk_ctx, x: *const f64, n: i64, d: i64, params: *const fk_kmeans_params,
