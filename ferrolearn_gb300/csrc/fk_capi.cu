@@ -13,12 +13,12 @@
 #include <cstring>
 #include <atomic>
 #include <memory>
-#include <system_error>
 #include <thread>
 #include <unordered_map>
 #include <vector>
 
 #include "fk_internal.cuh"
+#include "fk_workers.h"
 
 namespace fk {
 
@@ -207,23 +207,11 @@ bool copy_out_threads(Ctx &ctx, void *dst, const void *dev_src, size_t bytes) {
     const int workers = std::max(1, std::min(HostCopy::WORKERS, (int)(cores / 2)));
     FK_CUDA(cudaEventRecord(h.ready, ctx.stream));
     std::atomic<int> err{cudaSuccess};
-    auto work = [&](int w, int n) {
-        const cudaError_t e = host_copy_worker(h, ctx.device, w, n, (unsigned char *)dst, (const unsigned char *)dev_src, bytes);
+    run_workers<HostCopy::WORKERS>(workers, [&](int w) {
+        const cudaError_t e =
+            host_copy_worker(h, ctx.device, w, workers, (unsigned char *)dst, (const unsigned char *)dev_src, bytes);
         if (e != cudaSuccess) err.store((int)e);
-    };
-    std::thread pool[HostCopy::WORKERS];
-    std::vector<int> missing;
-    for (int w = 1; w < workers; w++) {
-        try {
-            pool[w] = std::thread(work, w, workers);
-        } catch (const std::system_error &) {
-            missing.push_back(w);  // no thread to be had: the caller does its share
-        }
-    }
-    work(0, workers);  // the caller is worker 0
-    for (int w : missing) work(w, workers);
-    for (int w = 1; w < workers; w++)
-        if (pool[w].joinable()) pool[w].join();
+    });
     FK_CUDA((cudaError_t)err.load());
     return true;
 }
