@@ -88,83 +88,175 @@ __global__ void prune_shift_kernel(const F *__restrict__ c, const F *__restrict_
     }
 }
 
-// The NROW nearest other centres of each centre (one block per centre): row
+// The NROW nearest other centres of each centre (A centres per block): row
 // thresholds in ascending order -- a row of this centre at computed squared
 // distance m < threshold cannot be nearer to, or as near as, that neighbour --
 // and the neighbours' indices. As in fk_kpp.cu: L a lower bound of D(c, q),
 // threshold = L (1 - rho) / 4, rho = (d + 8) 1e-6, which exceeds every rounding
 // of the two direct forms; bounds below 1e-30, where underflow would count, and
 // NaN give 0 (always compared).
+//
+// G lanes take a centre q (one up to 16 features, else eight): each reads its
+// features of q once for all A centres, and the lanes share the A thresholds.
+// Every lane of a group forming each centre's threshold, and one warp selecting
+// from all of them (or k ranks of k values), took 0.14 / 0.70 / 1.51 ms a launch at k
+// = 1,000 / 4,000 / 8,192 and d = 300 / 64 / 8, up to twice the pass that the lists
+// are to save; this takes 0.10 / 0.36 / 0.42 (256 centres of 64 features: 13 us as
+// before).
+template <int A, int G>
 __global__ void __launch_bounds__(PT)
     prune_near_lists_kernel(const float *__restrict__ c32, const float *__restrict__ cerr, int k, int d,
                             float *__restrict__ nthr, int *__restrict__ nidx) {
-    extern __shared__ float sm[];  // thr[k], then this centre's row
-    float *thr = sm, *row = sm + k;
-    const int a = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    for (int j = tid; j < d; j += PT) row[j] = c32[(int64_t)a * d + j];
+    extern __shared__ __align__(16) float sm[];  // thr[A][k], then (at 16 bytes) the centres' rows [A][d]
+    float *const row = sm + (((size_t)A * k + 3) & ~(size_t)3);
+    const int a0 = blockIdx.x * A, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    for (int e = tid; e < A * d; e += PT) {
+        const int a = e / d;
+        row[e] = c32[(int64_t)min(a0 + a, k - 1) * d + e - a * d];
+    }
     __syncthreads();
-    const float ea = cerr ? cerr[a] : 0.f, rho = (float)(d + 8) * 1e-6f;
-    // eight lanes a centre, their loads in flight together (256 centres of 64
-    // features: 13 us a launch, 25 with a warp a centre and the selection below)
-    for (int q0 = 4 * w; q0 < k; q0 += PT / 8) {
-        const int q = q0 + (lane >> 3);
+    const float rho = (float)(d + 8) * 1e-6f;
+    auto store = [&](int a, int q, float s) {
+        const float e = cerr ? __fadd_ru(cerr[min(a0 + a, k - 1)], cerr[q]) : 0.f;
+        const float th = 0.25f * __fsub_rd(s, bound32(s, e, d)) * (1.0f - rho);
+        sm[(size_t)a * k + q] = q == a0 + a ? INFINITY : (th > 1e-30f && th < FLT_MAX ? th : 0.f);
+    };
+    const bool vec = (d & 3) == 0 && ((reinterpret_cast<uintptr_t>(c32) | reinterpret_cast<uintptr_t>(row)) & 15) == 0;
+    // (one bound for every lane of a warp: the shuffles are warp-wide)
+    for (int q0 = w * (32 / G); q0 < k; q0 += PT / G) {
+        const int q = q0 + lane / G;
         const float *cq = c32 + (int64_t)min(q, k - 1) * d;
-        float s = 0.f;
-#pragma unroll 8
-        for (int j = lane & 7; j < d; j += 8) {
-            const float t = __fsub_rn(row[j], cq[j]);
-            s = __fmaf_rn(t, t, s);
-        }
+        float s[A];
 #pragma unroll
-        for (int o = 4; o >= 1; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if ((lane & 7) == 0 && q < k) {
-            const float e = cerr ? __fadd_ru(ea, cerr[q]) : 0.f;
-            const float th = 0.25f * __fsub_rd(s, bound32(s, e, d)) * (1.0f - rho);
-            thr[q] = q == a ? INFINITY : (th > 1e-30f && th < FLT_MAX ? th : 0.f);
+        for (int a = 0; a < A; a++) s[a] = 0.f;
+        if (vec) {
+            const float4 *c4 = reinterpret_cast<const float4 *>(cq);
+#pragma unroll 4
+            for (int j = lane % G; j < d / 4; j += G) {
+                const float4 cv = c4[j];
+#pragma unroll
+                for (int a = 0; a < A; a++) {
+                    const float4 r = *reinterpret_cast<const float4 *>(row + a * d + 4 * j);
+                    const float t0 = __fsub_rn(r.x, cv.x), t1 = __fsub_rn(r.y, cv.y), t2 = __fsub_rn(r.z, cv.z),
+                                t3 = __fsub_rn(r.w, cv.w);
+                    s[a] = __fmaf_rn(t3, t3, __fmaf_rn(t2, t2, __fmaf_rn(t1, t1, __fmaf_rn(t0, t0, s[a]))));
+                }
+            }
+        } else {
+#pragma unroll 8
+            for (int j = lane % G; j < d; j += G) {
+                const float cv = cq[j];
+#pragma unroll
+                for (int a = 0; a < A; a++) {
+                    const float t = __fsub_rn(row[a * d + j], cv);
+                    s[a] = __fmaf_rn(t, t, s[a]);
+                }
+            }
+        }
+        if (G == 1) {
+            if (q < k)
+#pragma unroll
+                for (int a = 0; a < A; a++) store(a, q, s[a]);
+        } else {
+            // the lanes' sums, each lane left with those of half the centres a step
+            int a = 0;
+            float v = s[0];
+            if constexpr (A == 4) {
+                const bool hi = lane & 4, hi2 = lane & 2;
+                const float k0 = (hi ? s[2] : s[0]) + __shfl_xor_sync(0xffffffffu, hi ? s[0] : s[2], 4);
+                const float k1 = (hi ? s[3] : s[1]) + __shfl_xor_sync(0xffffffffu, hi ? s[1] : s[3], 4);
+                v = (hi2 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, hi2 ? k0 : k1, 2);
+                a = (hi ? 2 : 0) + (hi2 ? 1 : 0);
+            } else if constexpr (A == 2) {
+                const bool hi = lane & 4;
+                v = (hi ? s[1] : s[0]) + __shfl_xor_sync(0xffffffffu, hi ? s[0] : s[1], 4);
+                v += __shfl_xor_sync(0xffffffffu, v, 2);
+                a = hi ? 1 : 0;
+            } else {
+                v += __shfl_xor_sync(0xffffffffu, v, 4);
+                v += __shfl_xor_sync(0xffffffffu, v, 2);
+            }
+            v += __shfl_xor_sync(0xffffffffu, v, 1);
+            if (q < k && (lane & (8 / A - 1)) == 0) store(a, q, v);
         }
     }
     __syncthreads();
-    if (k <= 4 * PT) {
+    if (k <= PT) {
         // each centre's rank among the others, ties by index
-        for (int q = tid; q < k; q += PT) {
-            const float v = thr[q];
-            int rank = 0;
+        for (int a = 0; a < A && a0 + a < k; a++) {
+            const float *thr = sm + (size_t)a * k;
+            for (int q = tid; q < k; q += PT) {
+                const float v = thr[q];
+                int rank = 0;
 #pragma unroll 8
-            for (int p = 0; p < k; p++) rank += thr[p] < v || (thr[p] == v && p < q);
-            if (rank < NROW) {
-                nthr[(int64_t)a * NROW + rank] = v;
-                if (rank < NEAR) nidx[(int64_t)a * NEAR + rank] = v < INFINITY ? q : -1;
+                for (int p = 0; p < k; p++) rank += thr[p] < v || (thr[p] == v && p < q);
+                if (rank < NROW) {
+                    nthr[(int64_t)(a0 + a) * NROW + rank] = v;
+                    if (rank < NEAR) nidx[(int64_t)(a0 + a) * NEAR + rank] = v < INFINITY ? q : -1;
+                }
             }
-        }
-        for (int t = k + tid; t < NROW; t += PT) {
-            nthr[(int64_t)a * NROW + t] = INFINITY;
-            if (t < NEAR) nidx[(int64_t)a * NEAR + t] = -1;
+            for (int t = k + tid; t < NROW; t += PT) {
+                nthr[(int64_t)(a0 + a) * NROW + t] = INFINITY;
+                if (t < NEAR) nidx[(int64_t)(a0 + a) * NEAR + t] = -1;
+            }
         }
         return;
     }
-    if (w != 0) return;
-    // the smallest NROW, one after the other (non-negative floats order as their bits)
-    for (int t = 0; t < NROW; t++) {
-        uint32_t best = 0xFFFFFFFFu;
-        int at = -1;
-        for (int q = lane; q < k; q += 32) {
-            const uint32_t b = __float_as_uint(thr[q]);
-            if (b < best) {
-                best = b;
-                at = q;
+    // More centres: each warp takes the smallest NROW of its part, one after the
+    // other (non-negative floats order as their bits), then the ranks among the
+    // parts' lists.
+    constexpr int NW = PT / 32, PARTS = NW / A;  // warps per centre
+    __shared__ uint32_t best_v[NW * NROW];
+    __shared__ int best_q[NW * NROW];
+    {
+        float *thr = sm + (size_t)(w / PARTS) * k;
+        for (int t = 0; t < NROW; t++) {
+            uint32_t best = 0xFFFFFFFFu;
+            int at = -1;
+#pragma unroll 4
+            for (int q = (w % PARTS) * 32 + lane; q < k; q += 32 * PARTS) {
+                const uint32_t b = __float_as_uint(thr[q]);
+                if (b < best) {
+                    best = b;
+                    at = q;
+                }
             }
+            const uint32_t m = __reduce_min_sync(0xffffffffu, best);
+            const int src = __ffs(__ballot_sync(0xffffffffu, best == m)) - 1;
+            at = __shfl_sync(0xffffffffu, at, src);
+            if (lane == 0) {
+                const bool any = m < 0x7F800000u;
+                best_v[w * NROW + t] = any ? m : 0x7F800000u;
+                best_q[w * NROW + t] = any ? at : -1;
+                if (any) thr[at] = __uint_as_float(0x7F800001u);  // taken: NaN, above every float's bits
+            }
+            __syncwarp();
         }
-        const uint32_t m = __reduce_min_sync(0xffffffffu, best);
-        const int src = __ffs(__ballot_sync(0xffffffffu, best == m)) - 1;
-        at = __shfl_sync(0xffffffffu, at, src);
-        if (lane == 0) {
-            const bool any = m < 0x7F800000u;
-            nthr[(int64_t)a * NROW + t] = any ? __uint_as_float(m) : INFINITY;
-            if (t < NEAR) nidx[(int64_t)a * NEAR + t] = any ? at : -1;
-            if (any) thr[at] = __uint_as_float(0x7F800001u);  // taken
-        }
-        __syncwarp();
     }
+    __syncthreads();
+    for (int e = tid; e < NW * NROW; e += PT) {
+        const int a = e / (PARTS * NROW), first = a * PARTS * NROW;
+        const uint32_t v = best_v[e];
+        int rank = 0;
+        for (int p = first; p < first + PARTS * NROW; p++) rank += best_v[p] < v || (best_v[p] == v && p < e);
+        if (rank < NROW && a0 + a < k) {
+            nthr[(int64_t)(a0 + a) * NROW + rank] = __uint_as_float(v);
+            if (rank < NEAR) nidx[(int64_t)(a0 + a) * NEAR + rank] = best_q[e];
+        }
+    }
+}
+
+template <int A>
+void launch_near_lists(const float *c32, const float *cerr, int k, int d, float *nthr, int *nidx, cudaStream_t s) {
+    const size_t smem = sizeof(float) * (A * ((size_t)k + d) + 3);
+    auto run = [&](auto kernel) {
+        if (smem > 48 * 1024)
+            FK_CUDA(cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kernel<<<(unsigned)((k + A - 1) / A), PT, smem, s>>>(c32, cerr, k, d, nthr, nidx);
+        FK_LAUNCH_CHECK();
+    };
+    if (d <= 16) run(prune_near_lists_kernel<A, 1>);
+    else run(prune_near_lists_kernel<A, 8>);
 }
 
 struct PruneLists {
@@ -509,8 +601,11 @@ constexpr int STM = 8, STN = 8;                // of a thread
 // Every centre for the listed rows (list null: all n rows): 128 x 128 tiles,
 // 8 x 8 distances a thread, 16 features staged at a time; a row's 16 threads
 // merge at the end. Bound by the FP32 pipe (3 operations a feature and pair in
-// f32, 2 in f64).
-template <typename F>
+// f32, 2 in f64), and where there is a tile an SM at most by the loads' latency:
+// FEW keeps the rows' numbers in registers then, not in shared memory before each
+// load (10,000 x 1,000 against 300 centres 1.32 ms -> 0.96, 66,000 x 64 against
+// 4,000 2.33 -> 2.43).
+template <typename F, bool FEW>
 __global__ void __launch_bounds__(PT)
     prune_scan_kernel(const float *__restrict__ x, const float *__restrict__ xerr, int64_t n, int d,
                       const float *__restrict__ c32, const float *__restrict__ cerr, int k,
@@ -526,6 +621,12 @@ __global__ void __launch_bounds__(PT)
         __syncthreads();  // the tile before is done with ids
         if (tid < SBM) ids[tid] = row0 + tid < cnt ? (list ? list[row0 + tid] : (int32_t)(row0 + tid)) : -1;
         __syncthreads();
+        constexpr int PER = (SBM * SDJ) / PT;  // values of a tile that a thread stages, one feature of PER rows
+        int32_t rid[FEW ? PER : 1];
+        if constexpr (FEW) {
+#pragma unroll
+            for (int e = 0; e < PER; e++) rid[e] = ids[tid / SDJ + e * (PT / SDJ)];
+        }
         B b[STM];
         float ex[STM];
 #pragma unroll
@@ -542,10 +643,9 @@ __global__ void __launch_bounds__(PT)
                 for (int q = 0; q < STN; q++) acc[a][q] = 0.f;
             for (int j0 = 0; j0 < d; j0 += SDJ) {
 #pragma unroll
-                for (int e = 0; e < (SBM * SDJ) / PT; e++) {
-                    const int idx = tid + e * PT;
-                    const int r = idx / SDJ, jj = idx % SDJ;
-                    const int gj = j0 + jj, id = ids[r], gc = ct + r;
+                for (int e = 0; e < PER; e++) {
+                    const int r = tid / SDJ + e * (PT / SDJ), jj = tid % SDJ;
+                    const int gj = j0 + jj, id = FEW ? rid[FEW ? e : 0] : ids[r], gc = ct + r;
                     xsm[jj][r] = (id >= 0 && gj < d) ? x[(int64_t)id * d + gj] : 0.f;
                     csm[jj][r] = (gc < k && gj < d) ? c32[(int64_t)gc * d + gj] : 0.f;
                 }
@@ -649,20 +749,24 @@ void launch_assign_pruned(Ctx &ctx, const F *x, int64_t n, int d, const F *c, co
     L.open_rows = L.scan_rows + n;
     L.count = (unsigned long long *)ctx.get(BUF_PF_CNT, sizeof(unsigned long long) * 4);
     FK_CUDA(cudaMemsetAsync(L.count, 0, sizeof(unsigned long long) * 4, s));
-    const unsigned tiles = (unsigned)std::min<int64_t>((n + SBM - 1) / SBM, (int64_t)ctx.num_sms * 4);
-    if (!c_prev) {
-        prune_scan_kernel<F><<<(unsigned)((n + SBM - 1) / SBM), PT, 0, s>>>(x32, xerr, n, d, c32, cerr, k, nullptr,
-                                                                           labels, ub, lb, L);
+    const int64_t tiles = (n + SBM - 1) / SBM;
+    auto scan = [&](const int32_t *list, int64_t blocks) {
+        if (tiles <= ctx.num_sms)
+            prune_scan_kernel<F, true><<<(unsigned)blocks, PT, 0, s>>>(x32, xerr, n, d, c32, cerr, k, list, labels, ub, lb, L);
+        else
+            prune_scan_kernel<F, false><<<(unsigned)blocks, PT, 0, s>>>(x32, xerr, n, d, c32, cerr, k, list, labels, ub, lb, L);
         FK_LAUNCH_CHECK();
+    };
+    if (!c_prev) {
+        scan(nullptr, tiles);
     } else {
         prune_shift_kernel<F><<<(unsigned)((k + 7) / 8), PT, 0, s>>>(c, c_prev, k, d, shift);
         FK_LAUNCH_CHECK();
-        const size_t smem = sizeof(float) * ((size_t)k + d);
-        if (smem > 48 * 1024)
-            FK_CUDA(cudaFuncSetAttribute((const void *)prune_near_lists_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        prune_near_lists_kernel<<<(unsigned)k, PT, smem, s>>>(c32, cerr, k, d, nthr, nidx);
-        FK_LAUNCH_CHECK();
+        // as many centres a block as leave two blocks for every SM, and room for three on
+        // it (k = 300, d = 1,000 with one: 64 us; 4,000 x 64 with one 417, with four 365)
+        if (k >= 8 * ctx.num_sms && k + d <= 4608) launch_near_lists<4>(c32, cerr, k, d, nthr, nidx, s);
+        else if (k >= 4 * ctx.num_sms && k + d <= 9216) launch_near_lists<2>(c32, cerr, k, d, nthr, nidx, s);
+        else launch_near_lists<1>(c32, cerr, k, d, nthr, nidx, s);
         const int64_t bound_blocks = std::min<int64_t>((n + BU * PT - 1) / (BU * PT), (int64_t)ctx.num_sms * 8);
         prune_bound_kernel<<<(unsigned)bound_blocks, PT, 0, s>>>(
             n, k, d, prev, labels, ub, lb, shift, nthr, L);
@@ -684,8 +788,7 @@ void launch_assign_pruned(Ctx &ctx, const F *x, int64_t n, int d, const F *c, co
         prune_near_kernel<F><<<(unsigned)std::min<int64_t>((n + tile - 1) / tile, (int64_t)ctx.num_sms * 8), PT, nsm,
                                s>>>(x32, xerr, d, c32, cerr, prev, nthr, nidx, labels, ub, lb, tile, xs, L);
         FK_LAUNCH_CHECK();
-        prune_scan_kernel<F><<<tiles, PT, 0, s>>>(x32, xerr, n, d, c32, cerr, k, L.scan_rows, labels, ub, lb, L);
-        FK_LAUNCH_CHECK();
+        scan(L.scan_rows, std::min<int64_t>(tiles, (int64_t)ctx.num_sms * 4));
     }
     if constexpr (!S) 
         launch_f64_open_rows(ctx, x, x32, xerr, d, c, c32, cerr, k, L.open_rows, L.count + 2, labels, nullptr);
