@@ -433,8 +433,14 @@ void lloyd_iteration(Ctx &ctx, const TX *x, int64_t n, int d, const TC *c, int k
         Timer t(timing, ctx, rep ? &rep->ms_assign : nullptr);
         if (pruned) {
             // a fit's labels alone: its inertia is formed once, at its end
-            if constexpr (std::is_same<TX, TC>::value)
-                launch_assign_pruned<TC>(ctx, x, n, d, c, prev_c, k, prev_labels, labels, x_changed);
+            if constexpr (std::is_same<TX, TC>::value) {
+                if (main != PLAIN_DIRECT)
+                    launch_assign_pruned<TC>(ctx, x, n, d, c, prev_c, k, prev_labels, labels, x_changed, sc);
+                else if constexpr (std::is_same<TC, double>::value)
+                    launch_assign_f64_filtered(ctx, x, n, d, c, k, labels, nullptr, x_changed);
+                else
+                    launch_assign_direct<TX, TC>(x, n, d, c, k, labels, nullptr, s);
+            }
         } else if (prec == FK_PRECISION_PLAIN) {
             TC *mind = (TC *)ctx.get(BUF_MIND, sizeof(TC) * (size_t)n);
             double *part = (double *)ctx.get(BUF_PARTIAL, sizeof(double) * (size_t)sum_fixed_partials(n));
@@ -712,6 +718,17 @@ fk_status fit_impl(fk_ctx *ctxp, const TX *x_in, int64_t n, int64_t d, const fk_
         int64_t kept = 0;  // rows kept, of the last iteration read
         bool was_count[2] = {false, false};
         int64_t count_from = FK_COUNT_FROM;
+        // Plain fits with bounds: where the lists of near centres cost more than a
+        // sixteenth of a pass (prune_may_rest) and an eighth of the rows or fewer are left
+        // out, the fit goes on without them for 2, then for 8 iterations at a time before
+        // it tries again (the iteration before a trial leaves the bounds, at no cost). The
+        // first bounded iteration follows the first moves and says nothing yet; the
+        // counts are read one iteration late, so a trial is two iterations.
+        int plain[2] = {PLAIN_DIRECT, PLAIN_DIRECT};  // the last two iterations' passes
+        int64_t rest_end = 0, rest = 2, trial = 2;
+        const bool may_rest = prune && prune_may_rest(n, (int)d, (int)k);
+        bool stop = false;
+        int64_t launched = 0, finished = 0;
         auto finish = [&](int64_t r) {
             FK_CUDA(cudaEventSynchronize(iter_done[r & 1]));
             const DevScalars &h = ctx.host_scalars[1 + (r & 1)];
@@ -724,12 +741,19 @@ fk_status fit_impl(fk_ctx *ctxp, const TX *x_in, int64_t n, int64_t d, const fk_
             if (was_count[r & 1] && ((int64_t)h.full_count > n / 10 || (int64_t)h.ex_count > n / 500))
                 count_from = std::max(count_from, r + 3);
             accumulate_report(rep, h, n);
+            if (may_rest && plain[r & 1] == PLAIN_BOUNDED && r >= trial) {
+                if ((int64_t)h.prune[1] > n - n / 8) {
+                    rest_end = launched + rest;
+                    trial = rest_end + 1;
+                    rest = 8;
+                } else {
+                    rest = 2;
+                }
+            }
             inertia = (TC)h.inertia;
             n_iter = r + 1;
             return shift_from_bits<TC>(h.shift_bits) < (TC)p->tol;
         };
-        bool stop = false;
-        int64_t launched = 0, finished = 0;
         auto finish_next = [&] {
             if (finished < launched && !stop) stop = finish(finished++);
         };
@@ -750,11 +774,16 @@ fk_status fit_impl(fk_ctx *ctxp, const TX *x_in, int64_t n, int64_t d, const fk_
             if (bounds && it >= FK_COUNT_FROM && (!pays || !reserve_listed(ctx, n, (int)d, p->precision))) bounds = false;
             // (the count pass carries every row's floor: a pass over listed rows left the others' behind)
             const bool count = count_ok && calm && it >= count_from && !bounds && !was_listed;
-            const int main = bounds ? (it >= FK_COUNT_FROM ? MAIN_LISTED : MAIN_TOP2_BOUNDS)
-                             : count ? MAIN_COUNT
-                                     : MAIN_TOP2;
-            const bool with_prev = main == MAIN_COUNT || main == MAIN_LISTED || (main == MAIN_TOP2_BOUNDS && it > 0) ||
-                                   (prune && it > 0);
+            plain[par] = it < rest_end                              ? PLAIN_DIRECT
+                         : it > 0 && plain[par ^ 1] != PLAIN_DIRECT ? PLAIN_BOUNDED
+                                                                    : PLAIN_START;
+            const int main = prune    ? plain[par]
+                             : bounds ? (it >= FK_COUNT_FROM ? MAIN_LISTED : MAIN_TOP2_BOUNDS)
+                             : count  ? MAIN_COUNT
+                                      : MAIN_TOP2;
+            const bool with_prev =
+                prune ? main == PLAIN_BOUNDED
+                      : main == MAIN_COUNT || main == MAIN_LISTED || (main == MAIN_TOP2_BOUNDS && it > 0);
             was_count[par] = count;
             was_listed = main == MAIN_LISTED;
             if (count && rep) rep->count_iterations++;
@@ -770,7 +799,8 @@ fk_status fit_impl(fk_ctx *ctxp, const TX *x_in, int64_t n, int64_t d, const fk_
                 // (phase timers record events, so timed fits run without graphs)
                 const uint64_t key[10] = {(uint64_t)(uintptr_t)x, (uint64_t)n, (uint64_t)d, (uint64_t)k,
                                           (uint64_t)p->precision, (uint64_t)(it % 6), (uint64_t)mode,
-                                          (uint64_t)main, (uint64_t)(uintptr_t)sc, sizeof(TX) * 16 + sizeof(TC)};
+                                          (uint64_t)main, (uint64_t)(uintptr_t)sc,
+                                          sizeof(TX) * 16 + sizeof(TC) + (prune ? 256 : 0)};
                 run_graphed(ctx, key, [&] {
                     FK_CUDA(cudaMemsetAsync(sc, 0, sizeof(DevScalars), s));
                     iteration();

@@ -71,6 +71,7 @@ struct DevScalars {
     unsigned long long pair2_count; // FP8 second pass: pairs its count pass left
     unsigned long long kept_rows;   // rows whose bounds keep their label (fits of some size)
     unsigned long long listed_rows; // rows listed for the main pass
+    unsigned long long prune[3];    // plain bounds: rows near their centre, rows against every centre, rows left to FP64
 };
 
 // --------------------------------------------------- mixed precision --
@@ -345,13 +346,17 @@ void launch_assign_f64_filtered(Ctx &ctx, const double *x, int64_t n, int d, con
 bool f32_scores_pay(int64_t n, int d, int k);
 void launch_assign_f32_scored(Ctx &ctx, const float *x, int64_t n, int d, const float *c, int k, int32_t *labels);
 // The plain assignment of a fit's iteration (fk_prune.cu): the labels of
-// launch_assign_direct<F, F>, without the distances. c_prev null: the first
-// iteration, every centre for every row; else prev are the labels against
-// c_prev, and the context's bounds are those the call before left.
+// launch_assign_direct<F, F>, without the distances. c_prev null: every centre for
+// every row; else prev are the labels against c_prev, and the context's bounds are
+// those the call before left. sc->prune (zero before) receives the rows' routes.
 bool prune_shape_ok(int64_t n, int d, int k);
+bool prune_may_rest(int64_t n, int d, int k);
 template <typename F>
 void launch_assign_pruned(Ctx &ctx, const F *x, int64_t n, int d, const F *c, const F *c_prev, int k,
-                          const int32_t *prev, int32_t *labels, bool fresh_x);
+                          const int32_t *prev, int32_t *labels, bool fresh_x, DevScalars *sc);
+// The assignment of an iteration of such a fit: as without bounds, every centre for
+// every row so that bounds are left, or only the rows that the bounds do not keep.
+enum PlainPass { PLAIN_DIRECT = 0, PLAIN_START = 1, PLAIN_BOUNDED = 2 };
 // Each row's direct-form distance to its label, F::MAX where it is not below.
 template <typename F>
 void launch_label_dist(Ctx &ctx, const F *x, int64_t n, int d, const F *c, const int32_t *labels, F *mind);

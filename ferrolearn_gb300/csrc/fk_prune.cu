@@ -711,16 +711,31 @@ __global__ void prune_dist_kernel(const F *__restrict__ x, int64_t n, int d, con
 
 }  // namespace
 
+// What the lists of near centres cost beside a pass over every centre (measured
+// from k = 300, d = 1,000 to k = 8,192, d = 8: 4e-12 s a pair of centres and 3e-13 a
+// feature of it, the pass 1.2e-13 s a row, centre and feature).
+static double lists_cost(int64_t n, int d, int k) { return k * (32.0 + 2.6 * d) / ((double)n * d); }
+
 bool prune_shape_ok(int64_t n, int d, int k) {
     // Below: the direct pass takes less than the lists' extra launches (about
-    // 25 us). k and d: a centre's thresholds and row fill shared memory, and k^2 d
-    // is small beside n k d.
-    return k >= 32 && k <= 8192 && d >= 1 && d <= 8192 && n >= 8 * (int64_t)k && (double)n * k * d >= 1e9;
+    // 25 us). k and d: a centre's thresholds and row fill shared memory. Lists that cost
+    // about half a pass pay on no data tried (66,000 x 8 against 8,192 centres,
+    // 0.8 of a pass: 20 iterations 25.8-29 ms, 24.8 without).
+    return k >= 32 && k <= 8192 && d >= 1 && d <= 8192 && n >= 8 * (int64_t)k && (double)n * k * d >= 1e9 &&
+           lists_cost(n, d, k) <= 0.45;
 }
+
+// Whether a bounded iteration that keeps few rows is worth leaving out. 20 iterations
+// on rows without structure, f32, beside the same without bounds, always bounded /
+// resting: 50,000 x 32 against 2,000 centres 1.19 / 1.10, 200,000 x 64 against 8,192
+// 1.09 / 1.03, 66,000 x 8 against 4,000 1.08 / 1.05 (on clusters 0.57, 0.39 and 0.97 either
+// way). Below the line resting loses more where the bounds come to pay late:
+// 400,000 x 80 against 32 wide clusters 0.60 / 0.66, 1M x 64 against 256 0.60 / 0.87.
+bool prune_may_rest(int64_t n, int d, int k) { return lists_cost(n, d, k) > 1.0 / 16; }
 
 template <typename F>
 void launch_assign_pruned(Ctx &ctx, const F *x, int64_t n, int d, const F *c, const F *c_prev, int k,
-                          const int32_t *prev, int32_t *labels, bool fresh_x) {
+                          const int32_t *prev, int32_t *labels, bool fresh_x, DevScalars *sc) {
     cudaStream_t s = ctx.stream;
     constexpr bool S = std::is_same<F, float>::value;
     const float *x32, *c32, *xerr = nullptr, *cerr = nullptr;
@@ -747,8 +762,7 @@ void launch_assign_pruned(Ctx &ctx, const F *x, int64_t n, int d, const F *c, co
     L.near_rows = (int32_t *)ctx.get(BUF_PR_LIST, sizeof(int32_t) * 3 * (size_t)n);
     L.scan_rows = L.near_rows + n;
     L.open_rows = L.scan_rows + n;
-    L.count = (unsigned long long *)ctx.get(BUF_PF_CNT, sizeof(unsigned long long) * 4);
-    FK_CUDA(cudaMemsetAsync(L.count, 0, sizeof(unsigned long long) * 4, s));
+    L.count = sc->prune;
     const int64_t tiles = (n + SBM - 1) / SBM;
     auto scan = [&](const int32_t *list, int64_t blocks) {
         if (tiles <= ctx.num_sms)
@@ -803,9 +817,9 @@ void launch_label_dist(Ctx &ctx, const F *x, int64_t n, int d, const F *c, const
 }
 
 template void launch_assign_pruned<float>(Ctx &, const float *, int64_t, int, const float *, const float *, int,
-                                          const int32_t *, int32_t *, bool);
+                                          const int32_t *, int32_t *, bool, DevScalars *);
 template void launch_assign_pruned<double>(Ctx &, const double *, int64_t, int, const double *, const double *, int,
-                                           const int32_t *, int32_t *, bool);
+                                           const int32_t *, int32_t *, bool, DevScalars *);
 template void launch_label_dist<float>(Ctx &, const float *, int64_t, int, const float *, const int32_t *, float *);
 template void launch_label_dist<double>(Ctx &, const double *, int64_t, int, const double *, const int32_t *, double *);
 
