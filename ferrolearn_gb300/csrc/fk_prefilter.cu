@@ -528,9 +528,12 @@ void launch_assign_f64_filtered(Ctx &ctx, const double *x, int64_t n, int d, con
     f32_copy_rows_kernel<<<(unsigned)std::min<int64_t>((k + 7) / 8, grid_rows), 256, 0, s>>>(c, k, d, c32, cerr);
     FK_LAUNCH_CHECK();
     FK_CUDA(cudaMemsetAsync(open_count, 0, sizeof(unsigned long long), s));
-    // 128-row tiles read the centres least often; below one tile an SM the small
-    // ones fill the chip (1,024 rows, k = 256, d = 64)
-    if ((n + PBM - 1) / PBM < ctx.num_sms)
+    // 128-row tiles read the centres least often; up to 5/8 of a tile an SM the small
+    // ones, which fill the chip, are faster (predict of 8,192 x 64 against 1,000 centres
+    // 163 us for 215, 12,288 rows 211 for 213, 16,384 237 for 216). Up to 64 centres, half
+    // of a 128-centre tile, they are up to one tile an SM (19,000 x 64 against 50: 70 for 78).
+    const int64_t tiles = (n + PBM - 1) / PBM;
+    if (8 * tiles < (k <= 64 && d >= 32 ? 8 : 5) * (int64_t)ctx.num_sms)
         f32_filter_few_kernel<<<(unsigned)((n + FBM - 1) / FBM), PNT, 0, s>>>(x32, xerr, n, d, c32, cerr, k, labels,
                                                                               open_list, open_count);
     else
