@@ -925,43 +925,31 @@ AssignFn assign_fn(int bucket, int v) {
     }
 }
 
-// Streams that a capture forks to (nothing runs on them outside it).
-struct Branches {
-    static constexpr int N = 4;
-    cudaStream_t stream[N] = {};
-    cudaEvent_t fork = nullptr, join[N] = {};
-    Branches() {
-        try {
-            FK_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
-            for (int q = 0; q < N; q++) {
-                FK_CUDA(cudaStreamCreateWithFlags(&stream[q], cudaStreamNonBlocking));
-                FK_CUDA(cudaEventCreateWithFlags(&join[q], cudaEventDisableTiming));
-            }
-        } catch (...) {
-            release();
-            throw;
-        }
-    }
-    Branches(const Branches &) = delete;
-    Branches &operator=(const Branches &) = delete;
-    ~Branches() { release(); }
-
-  private:
-    void release() {
-        for (int q = 0; q < N; q++) {
-            if (join[q]) cudaEventDestroy(join[q]);
-            if (stream[q]) cudaStreamDestroy(stream[q]);
-        }
-        if (fork) cudaEventDestroy(fork);
-    }
-};
-
 int n_variants(int bucket) {
     const int d = bucket_d(bucket);
     return d == 0 ? 1 : d == 64 ? 3 : NVARIANTS;
 }
 
 }  // namespace
+
+void Branches::make() {
+    if (!fork) FK_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+    for (int q = 0; q < N; q++) {
+        if (!stream[q]) FK_CUDA(cudaStreamCreateWithFlags(&stream[q], cudaStreamNonBlocking));
+        if (!join[q]) FK_CUDA(cudaEventCreateWithFlags(&join[q], cudaEventDisableTiming));
+    }
+}
+
+void Branches::release() {
+    for (int q = 0; q < N; q++) {
+        if (join[q]) cudaEventDestroy(join[q]);
+        if (stream[q]) cudaStreamDestroy(stream[q]);
+        join[q] = nullptr;
+        stream[q] = nullptr;
+    }
+    if (fork) cudaEventDestroy(fork);
+    fork = nullptr;
+}
 
 fk_status batched_fit_impl(Ctx &ctx, fk_batch_problem *P, int64_t np, int reduction, fk_batch_report *rep) {
     if (np < 0 || (np > 0 && !P)) {
@@ -1216,21 +1204,26 @@ fk_status batched_fit_impl(Ctx &ctx, fk_batch_problem *P, int64_t np, int reduct
     FK_CUDA(cudaEventRecord(ev[3], s));
 
     // ---- Lloyd iterations: one captured iteration, replayed. The buckets'
-    // assignments are independent: branches of the graph.
-    Branches side;
+    // assignments are independent: branches of the graph where there are several
+    // (streams made for every call took 0.1 ms of a call of two 200 x 8 problems).
+    int nbuckets = 0;
+    for (int b = 0; b < NBUCKETS; b++) nbuckets += bstart[b + 1] > bstart[b];
+    const int forks = nbuckets > 1 ? std::min(nbuckets, Branches::N) : 0;
+    Branches &side = ctx.branches;
+    if (forks) side.make();
     auto one_iteration = [&]() {
         FK_CUDA(cudaMemsetAsync(dctr, 0, sizeof(int) * 22, s));
-        FK_CUDA(cudaEventRecord(side.fork, s));
-        for (int q = 0; q < Branches::N; q++) FK_CUDA(cudaStreamWaitEvent(side.stream[q], side.fork, 0));
+        if (forks) FK_CUDA(cudaEventRecord(side.fork, s));
+        for (int q = 0; q < forks; q++) FK_CUDA(cudaStreamWaitEvent(side.stream[q], side.fork, 0));
         int at = 0;
         for (int b = 0; b < NBUCKETS; b++) {
             const int cnt = bstart[b + 1] - bstart[b];
             if (cnt == 0) continue;
             const int grid = std::min(cnt, ctx.num_sms * 8);
-            assign_fn(b, ctx.batch_variant[b])<<<grid, ASSIGN_T, bsmem[b], side.stream[at++ % Branches::N]>>>(
+            assign_fn(b, ctx.batch_variant[b])<<<grid, ASSIGN_T, bsmem[b], forks ? side.stream[at++ % forks] : s>>>(
                 X, dfits, dstate, ditems + bstart[b], cnt, dctr + b, dC, dthr, dlab, dpart + bstart[b]);
         }
-        for (int q = 0; q < Branches::N; q++) {
+        for (int q = 0; q < forks; q++) {
             FK_CUDA(cudaEventRecord(side.join[q], side.stream[q]));
             FK_CUDA(cudaStreamWaitEvent(s, side.join[q], 0));
         }

@@ -1653,6 +1653,7 @@ fk_status fk_ctx_destroy(fk_ctx *ctx) {
     }
     if (h.ready) cudaEventDestroy(h.ready);
     if (h.pinned) cudaFreeHost(h.pinned);
+    c->branches.release();
     for (auto &g : c->iter_graphs)
         if (g.exec) cudaGraphExecDestroy(g.exec);
     if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);

@@ -184,6 +184,16 @@ struct HostCopy {
     bool made = false, failed = false;
 };
 
+// Streams that the capture of batched fits forks to (fk_batched.cu; nothing runs on
+// them outside it). Made at the first call with several buckets.
+struct Branches {
+    static constexpr int N = 4;
+    cudaStream_t stream[N] = {};
+    cudaEvent_t fork = nullptr, join[N] = {};
+    void make();
+    void release();
+};
+
 struct Ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -206,6 +216,7 @@ struct Ctx {
     };
     std::vector<PendingTimer> pending;  // phase timers read after the loop
     HostCopy host_copy;
+    Branches branches;
     MixedPlan mixed;   // main pass
     MixedPlan mixed2;  // second pass (BF16 count pass) over the rows an FP8 main pass left open
     MixedPlan mixedm2; // its mask pass (BF16, the slicing of mixed2)
