@@ -838,14 +838,21 @@ __global__ void __launch_bounds__(UPDATE_T) batch_update_kernel(const float *__r
                 newc[pr] = oldc[pr];  // empty cluster keeps its centre
                 continue;
             }
-            // values of the cluster's rows in row order, loaded 8 ahead
+            // values of the cluster's rows in row order, loaded 8 ahead, their rows' numbers 16
             float cur8[8], nxt8[8];
+            int row8[8];
 #pragma unroll
-            for (int u = 0; u < 8; u++) cur8[u] = u < cnt ? x[(int64_t)M[o + u] * d + j] : 0.f;
+            for (int u = 0; u < 8; u++) {
+                cur8[u] = u < cnt ? x[(int64_t)M[o + u] * d + j] : 0.f;
+                row8[u] = 8 + u < cnt ? M[o + 8 + u] : -1;
+            }
             float acc = 0.f;
             for (int m = 0; m < cnt; m += 8) {
 #pragma unroll
-                for (int u = 0; u < 8; u++) nxt8[u] = m + 8 + u < cnt ? x[(int64_t)M[o + m + 8 + u] * d + j] : 0.f;
+                for (int u = 0; u < 8; u++) {
+                    nxt8[u] = row8[u] >= 0 ? x[(int64_t)row8[u] * d + j] : 0.f;
+                    row8[u] = m + 16 + u < cnt ? M[o + m + 16 + u] : -1;
+                }
 #pragma unroll
                 for (int u = 0; u < 8; u++)
                     if (m + u < cnt) acc = __fadd_rn(acc, cur8[u]);
