@@ -1022,6 +1022,7 @@ fk_status batched_fit_impl(Ctx &ctx, fk_batch_problem *P, int64_t np, int reduct
     std::vector<BFit> fits;
     std::vector<int> fit_prob, fit_run;
     int64_t soff = 0, coff = 0, koff = 0;
+    bool bounds_pay = false;
     for (int64_t p = 0; p < np; p++) {
         const fk_batch_problem &q = P[p];
         for (int64_t r = 0; r < q.n_init; r++) {
@@ -1038,9 +1039,10 @@ fk_status batched_fit_impl(Ctx &ctx, fk_batch_problem *P, int64_t np, int reduct
             F.tol = (float)q.tol;
             F.seed = q.random_state + (uint64_t)r;
             F.prob = (int32_t)p;
-            // the thresholds cost k^2 d in one CTA group a fit: little beside n k d
             F.keep_sums = q.n * std::max<int64_t>(q.max_iter, 1) <= ((int64_t)1 << 30);
+            // the thresholds cost k^2 d in one CTA group a fit: little beside n k d
             F.bounded = dbucket(F.d) < 4 && F.k <= BOUND_K && (int64_t)F.n >= 16 * (int64_t)F.k;
+            bounds_pay = bounds_pay || (F.bounded && F.n >= 2048 && F.k >= 8);
             fits.push_back(F);
             fit_prob.push_back((int)p);
             fit_run.push_back((int)r);
@@ -1049,6 +1051,10 @@ fk_status batched_fit_impl(Ctx &ctx, fk_batch_problem *P, int64_t np, int reduct
             koff += q.n_clusters;
         }
     }
+    // a call of small fits alone: the thresholds' launch is longer than what they save
+    // (100 fits of 1,000 x 8, 4 clusters: 30.1 us an iteration with, 26.1 without)
+    if (!bounds_pay)
+        for (BFit &F : fits) F.bounded = 0;
     const int nf = (int)fits.size();
     // work items: chunks of rows, grouped by (d, k) bucket, largest fits first
     auto cost = [&](int f) { return (double)fits[f].n * fits[f].k * fits[f].d; };

@@ -73,3 +73,24 @@ def test_fits_and_batches_of_small_seedings(kind):
     g = F.KMeans(7, dtype="f32").with_n_init(5).with_random_state(3).with_max_iter(4).fit(x)
     o = O.fit(x, 7, max_iter=4, n_init=5, seed=3)
     assert np.array_equal(g.cluster_centers(), o["centers"]) and np.array_equal(g.labels(), o["labels"])
+
+
+@pytest.mark.parametrize("reduction", ["reference", "f64"])
+@pytest.mark.parametrize("d", [8, 16, 20, 64])
+def test_batches_of_small_fits_take_no_bounds(d, reduction):
+    # (their thresholds' launch would take longer than it saves; larger fits in the call bring them back)
+    rng = np.random.default_rng(d)
+    probs = []
+    for i, (n, k) in enumerate([(1, 1), (127, 3), (1000, 9), (2047, 30), (40, 40)]):
+        x = rng.normal(size=(n, d)).astype(np.float32)
+        x[: n // 2] += 6
+        probs.append(dict(x=x, k=k, n_init=2, max_iter=25, tol=1e-4, random_state=i))
+    alone, _ = F.fit_batched(probs, reduction=reduction)
+    big = dict(x=rng.normal(size=(3000, d)).astype(np.float32), k=9, n_init=1, max_iter=25, tol=1e-4, random_state=1)
+    together, _ = F.fit_batched(probs + [big], reduction=reduction)
+    for a, b, p in zip(alone, together, probs):
+        assert np.array_equal(a.labels(), b.labels()) and np.array_equal(a.cluster_centers(), b.cluster_centers())
+        assert a.n_iter() == b.n_iter() and a.inertia() == b.inertia()
+        if reduction == "reference":
+            o = O.fit(p["x"], p["k"], max_iter=25, tol=1e-4, n_init=2, seed=p["random_state"])
+            assert np.array_equal(a.labels(), o["labels"]) and np.array_equal(a.cluster_centers(), o["centers"])
