@@ -1476,27 +1476,29 @@ __global__ void __launch_bounds__(KPP_THREADS) kpp_walk_kernel(const KppFit<T> *
 }
 
 // ---------------------------------------------------- small seedings --
-// F = f32 with at most SMALL_N rows and SMALL_D features: a seeding is one CTA's, its
+// F = f32 with at most SMALL_N rows, SMALL_D features and SMALL_ND values: a seeding is one CTA's, its
 // D^2 arrays in shared memory (slot `cur` and one for each trial), every centre in one
 // launch. A fold of 1,024 f32 values is 4,096 cycles: a thread per trial walks its
 // array value by value and records the running sum after every 32, which is where the
-// next candidates are found. Four launches a centre took 30-45 us: the seedings of a
-// batch of three problems of 300 to 500 rows, k up to 20, 0.71 ms, like this 0.17; of
-// 1,000 fits of 300 rows, k = 8, 0.72 and 0.14. From about 2,000 rows on the four
-// launches are faster.
-constexpr int SMALL_N = 1024, SMALL_D = 256;
+// next candidates are found. Four launches a centre took 30 to 60 us, this 3.4 (100 x 4)
+// to 49 (300 seedings of 1,000 x 64, k = 40; the four 73). Above SMALL_ND values the one CTA
+// is slower than the four launches where the seedings are few (1,000 x 128, k = 40 58 us
+// for 45).
+constexpr int SMALL_N = 1024, SMALL_D = 256, SMALL_ND = 65536;
+// (4 floats past a multiple of 32: the folds of eight trials meet no bank conflict)
+__host__ __device__ inline int small_stride(int n) { return (n + 31) / 32 * 32 + 4; }
 inline size_t small_smem(int n, int d, int trials) {
-    const size_t stride = (size_t)n | 1;  // odd: the trials' folds meet no bank conflict
-    return sizeof(float) * ((size_t)(trials + 1) * (stride + 32) + (size_t)trials * d);
+    return sizeof(float) * ((size_t)(trials + 1) * (small_stride(n) + 32) + (size_t)trials * ((d + 3) & ~3));
 }
 
 __global__ void __launch_bounds__(KPP_THREADS) kpp_small_kernel(const KppFit<float> *__restrict__ fits) {
     const KppFit<float> f = fits[blockIdx.x];
-    const int n = (int)f.n, d = f.d, ntr = f.trials, stride = n | 1, ng = (n + 31) / 32;
+    const int n = (int)f.n, d = f.d, ntr = f.trials, stride = small_stride(n), ng = (n + 31) / 32, dc = (d + 3) & ~3;
+    const bool vec = (d & 3) == 0 && (reinterpret_cast<uintptr_t>(f.x) & 15) == 0;
     extern __shared__ __align__(16) float small_sm[];
     float *const arr = small_sm;                     // [ntr + 1][stride] D^2 arrays
     float *const gs = arr + (ntr + 1) * stride;      // [ntr + 1][32] running sums after each 32 values
-    float *const crow = gs + (ntr + 1) * 32;         // [ntr][d] candidate rows
+    float *const crow = gs + (ntr + 1) * 32;         // [ntr][dc] candidate rows (at 16 bytes)
     __shared__ float pot[MAX_TRIALS + 1];
     __shared__ int cand[MAX_TRIALS];
     __shared__ int best_sh;
@@ -1570,7 +1572,7 @@ __global__ void __launch_bounds__(KPP_THREADS) kpp_small_kernel(const KppFit<flo
         }
         cursor += ntr;
         __syncthreads();
-        for (int e = tid; e < ntr * d; e += KPP_THREADS) crow[e] = f.x[(int64_t)cand[e / d] * d + e % d];
+        for (int e = tid; e < ntr * d; e += KPP_THREADS) crow[e / d * dc + e % d] = f.x[(int64_t)cand[e / d] * d + e % d];
         __syncthreads();
         for (int i = tid; i < n; i += KPP_THREADS) {
             const float *xr = f.x + (int64_t)i * d;
@@ -1579,14 +1581,31 @@ __global__ void __launch_bounds__(KPP_THREADS) kpp_small_kernel(const KppFit<flo
                 float acc[4] = {0.f, 0.f, 0.f, 0.f};
                 const float *cr[4];
 #pragma unroll
-                for (int u = 0; u < 4; u++) cr[u] = crow + min(t0 + u, ntr - 1) * d;
+                for (int u = 0; u < 4; u++) cr[u] = crow + min(t0 + u, ntr - 1) * dc;
+                if (vec) {
 #pragma unroll 4
-                for (int j = 0; j < d; j++) {
-                    const float xv = xr[j];
+                    for (int q = 0; q < d / 4; q++) {
+                        const float4 xv = reinterpret_cast<const float4 *>(xr)[q];
 #pragma unroll
-                    for (int u = 0; u < 4; u++) {
-                        const float t = __fsub_rn(xv, cr[u][j]);
-                        acc[u] = __fadd_rn(acc[u], __fmul_rn(t, t));
+                        for (int u = 0; u < 4; u++) {
+                            const float4 cv = *reinterpret_cast<const float4 *>(cr[u] + 4 * q);
+                            const float t1 = __fsub_rn(xv.x, cv.x), t2 = __fsub_rn(xv.y, cv.y);
+                            const float t3 = __fsub_rn(xv.z, cv.z), t4 = __fsub_rn(xv.w, cv.w);
+                            acc[u] = __fadd_rn(acc[u], __fmul_rn(t1, t1));
+                            acc[u] = __fadd_rn(acc[u], __fmul_rn(t2, t2));
+                            acc[u] = __fadd_rn(acc[u], __fmul_rn(t3, t3));
+                            acc[u] = __fadd_rn(acc[u], __fmul_rn(t4, t4));
+                        }
+                    }
+                } else {
+#pragma unroll 4
+                    for (int j = 0; j < d; j++) {
+                        const float xv = xr[j];
+#pragma unroll
+                        for (int u = 0; u < 4; u++) {
+                            const float t = __fsub_rn(xv, cr[u][j]);
+                            acc[u] = __fadd_rn(acc[u], __fmul_rn(t, t));
+                        }
                     }
                 }
 #pragma unroll
@@ -1605,7 +1624,7 @@ __global__ void __launch_bounds__(KPP_THREADS) kpp_small_kernel(const KppFit<flo
         }
         __syncthreads();
         const int best = best_sh;
-        for (int j = tid; j < d; j += KPP_THREADS) f.centers[(long long)c * d + j] = crow[best * d + j];
+        for (int j = tid; j < d; j += KPP_THREADS) f.centers[(long long)c * d + j] = crow[best * dc + j];
         cur = slot(best, cur);
         __syncthreads();  // crow and best_sh are rewritten
     }
@@ -1806,7 +1825,7 @@ bool run_group(Ctx &ctx, const std::vector<KppJob> &jobs, const std::vector<int>
     return true;
 }
 
-// Every seeding in one launch (small_ok).
+// Every seeding in one launch.
 void run_small(Ctx &ctx, const std::vector<KppJob> &jobs, int64_t *draws_used) {
     cudaStream_t s = ctx.stream;
     const size_t nf = jobs.size();
@@ -1877,7 +1896,7 @@ void run_kmeanspp(Ctx &ctx, std::vector<KppJob> &jobs, int64_t *draws_used) {
     }
     if constexpr (std::is_same<T, float>::value) {
         bool small = true;
-        for (const KppJob &j : jobs) small = small && j.n <= SMALL_N && j.d <= SMALL_D;
+        for (const KppJob &j : jobs) small = small && j.n <= SMALL_N && j.d <= SMALL_D && j.n * j.d <= SMALL_ND;
         if (small) return run_small(ctx, jobs, draws_used);
     }
     if constexpr (std::is_same<T, double>::value) {

@@ -1,4 +1,4 @@
-"""f32 k-means++ of up to 1,024 rows and 256 features, a seeding a CTA: the oracle's
+"""f32 k-means++ of up to 1,024 rows, 256 features and 65,536 values, a seeding a CTA: the oracle's
 centres and draws at the edges of the groups of 32 values, of the trials scored at
 a time (4) and of the form, on data with ties, equal rows, zero sums and values
 that are not finite."""
@@ -12,7 +12,7 @@ from oracle import oracle as O
 pytestmark = pytest.mark.gpu
 
 ROWS = [(1, 3, 1), (2, 1, 2), (31, 5, 4), (32, 8, 7), (33, 7, 20), (63, 2, 63), (64, 16, 12), (257, 33, 55), (992, 6, 30),
-        (1000, 255, 8), (1023, 256, 21), (1024, 64, 149)]
+        (257, 255, 8), (256, 256, 21), (1023, 64, 9), (1024, 63, 5), (1024, 64, 149)]
 
 
 def _rows(kind, n, d, seed):
@@ -49,7 +49,7 @@ def test_small_seeding_matches_oracle(n, d, k, kind):
     assert np.array_equal(F.kmeans_plus_plus(x, k, seed=n * 7 + k, dtype="f32")[0], oc, equal_nan=True)
 
 
-@pytest.mark.parametrize("n,d", [(1025, 8), (1024, 257)])
+@pytest.mark.parametrize("n,d", [(1025, 8), (1024, 65), (64, 257)])
 def test_beyond_the_line(n, d):
     x = _rows("blobs", n, d, 3)
     before = _native.lib().fk_debug_launch_count()
