@@ -703,10 +703,14 @@ fk_status fit_impl(fk_ctx *ctxp, const TX *x_in, int64_t n, int64_t d, const fk_
         // second pass, or 0.2% to the exhaustive re-score, holds it off for
         // the next two iterations (the centres still move too much for the
         // carried bound).
-        // Larger fits keep row bounds from the top-2 pass instead, counting from
-        // the second iteration on how many rows they would keep; from the fourth
-        // on, once that is a sixth, the main pass is over the other rows. Where
-        // it is less by then, the fit goes on with the count pass.
+        // Larger fits keep row bounds from the top-2 pass instead; the third iteration
+        // counts how many rows they would keep, and if that is a sixth, the main pass is
+        // over the other rows from the fourth on. Where it is less, the fit goes on
+        // with the count pass. (The sixth: 20 iterations of 2,000,000 x 128, k = 1,024,
+        // with 11-30% kept by then, 15.3-16.0 -> 11.3-12.0 ms; 1,000,000 x 64, k = 4,096
+        // 19.8 -> 13.9; in FP8 with 23% 19.7 -> 14.7: the share grows as the centres
+        // settle. With 4%, 15.8 -> 13.4, but with none 20.7 -> 23.0 and 21.4 -> 25.8, and
+        // which of the two a small share becomes is not known by the fourth iteration.)
         bool count_ok = false, calm = false;
         if constexpr (std::is_same<TX, float>::value && std::is_same<TC, double>::value)
             count_ok = p->precision == FK_PRECISION_MIXED_BF16 || p->precision == FK_PRECISION_MIXED_FP8;
@@ -783,7 +787,7 @@ fk_status fit_impl(fk_ctx *ctxp, const TX *x_in, int64_t n, int64_t d, const fk_
                                       : MAIN_TOP2;
             const bool with_prev =
                 prune ? main == PLAIN_BOUNDED
-                      : main == MAIN_COUNT || main == MAIN_LISTED || (main == MAIN_TOP2_BOUNDS && it > 0);
+                      : main == MAIN_COUNT || main == MAIN_LISTED || (main == MAIN_TOP2_BOUNDS && it == FK_COUNT_FROM - 1);
             was_count[par] = count;
             was_listed = main == MAIN_LISTED;
             if (count && rep) rep->count_iterations++;

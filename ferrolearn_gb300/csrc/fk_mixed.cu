@@ -732,8 +732,10 @@ __device__ __forceinline__ float pair_dist_down(float d32, float e) {
 
 // A lower bound of each centre's squared distance to its nearest other centre
 // (near2, set to a large value before): 64 x 64 tiles of the upper triangle in
-// FP32 with the bound of the f32 copies' distances, 4 x 4 pairs a thread. 2 k^2 d / 2
-// operations: 0.1 ms at k = 4096, d = 256, less than 1% of a full pass.
+// FP32 with the bound of the f32 copies' distances, 4 x 4 pairs a thread. k^2 d
+// operations at the FP32 rate beside a pass's 2 n k d on the tensor cores: its share
+// grows with k / n (0.1 ms at k = 4096, d = 256: under 1% of a pass over 8M rows, more
+// than the pass below some 50 rows a centre, where no fit keeps bounds).
 constexpr int NT_ = 64, NDJ = 16;
 __global__ void __launch_bounds__(256)
     centre_near_kernel(const float *__restrict__ c32, const float *__restrict__ ec32, int k, int d,
@@ -2298,9 +2300,25 @@ void second_pass(Ctx &ctx, const float *x, int64_t n, int d, const double *c, in
 
 }  // namespace
 
-// Fits whose main pass is long against the bounds' few launches (2e10: about 20
-// us of BF16 contraction) keep them.
-bool mixed_bounds_ok(int64_t n, int d, int k) { return (double)n * k * d >= 2e10; }
+// Fits whose main pass is long against what the bounds add to each iteration keep
+// them: the listing's launches (shifts, nearest centres, bounds, gather: 40 us and more),
+// the finalize's wait for the list, and centre_near's k^2 d, which is (k / n) of a pass
+// at the FP32 rate: more than the pass saves below some 64 rows a centre. Fits of 20
+// iterations on clusters, with bounds over without (BF16 / FP8):
+//   rows a centre  k = 4,096 and 16,384: 98: 0.73 - 0.86, 64: 0.77 - 0.88 / 0.82 - 0.99,
+//                  49: 0.98 / 1.09, 24: 1.25 / 1.28, 6: 2.2 / 1.8
+//   n k d          160,000 x 256, k = 1,024 (4.2e10) 0.95 / 1.00, 320,000 x 64 the same
+//                  product at d = 128 (narrower rows' passes take as long) 0.96 / 0.93,
+//                  2,000,000 x 128 (2.6e11) 0.75 / 0.74; 300,000 x 256, k = 512 (3.9e10)
+//                  1.02 / 1.04; 100,000 x 256, k = 1,024 (2.6e10) 1.04 - 1.07
+//   k below 512    (wide groups, whose rows the second pass still takes) 600,000 x 256,
+//                  k = 256 (3.9e10) 1.06 / 1.01; 1,200,000 x 256 (7.9e10) 0.96 / 0.97;
+//                  3,000,000 x 128 (9.8e10) 0.89 / 0.85; 4,000,000 x 64, k = 100
+//                  (5.1e10) 1.01 - 1.04 / 0.82
+// A fit whose rows the bounds do not keep drops them after three iterations, for 1-2%.
+bool mixed_bounds_ok(int64_t n, int d, int k) {
+    return (double)n * k * std::max(d, 128) >= (k < 512 ? 7.5e10 : 4e10) && n >= 64 * (int64_t)k;
+}
 
 bool reserve_listed(Ctx &ctx, int64_t n, int d, int precision) {
     const bool fp8 = precision == FK_PRECISION_MIXED_FP8;

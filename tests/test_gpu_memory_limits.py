@@ -79,7 +79,7 @@ CASES = {
     "ragged bf16 fit": (lambda: _fit("f32x64", 200000, 127, 64, "bf16"), 0.75),
     "ragged fp8 fit": (lambda: _fit("f32x64", 150000, 125, 64, "fp8"), 0.78),
     "ragged bf16 predict": (lambda: _predict("f32x64", 200000, 127, 64, "bf16"), 0.75),
-    "bounded bf16 fit": (lambda: _fit("f32x64", 200000, 128, 1024, "bf16"), 0.75),
+    "bounded bf16 fit": (lambda: _fit("f32x64", 320000, 128, 1024, "bf16"), 0.75),
     "bounded f32 fit": (lambda: _fit("f32", 400000, 16, 256), 0.75),
     "bounded f64 fit": (lambda: _fit("f64", 400000, 16, 256), 0.80),
     "seeded f64 fit": (lambda: _fit("f64", 20000, 8, 20, n_init=10), 0.50),
