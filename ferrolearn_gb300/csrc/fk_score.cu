@@ -257,51 +257,91 @@ __global__ void __launch_bounds__(SNT, 2)
     }
 }
 
-// Listed rows, a warp a row, lanes over 128 centres at a time (their features
-// read from ct in whole lines): the direct form against every centre, lowest
-// index among the smallest distances strictly below F::MAX, else 0.
+// A row against centres [c0 + 32 u, c0 + 32 u + 32) for u < U, lane by lane: the direct
+// form's sums over ascending features, and of them the smallest (the lowest index of
+// equals) taken into (bv, bi). 32 / U features' loads of ct, whole lines, are in flight.
+template <int U>
+__device__ __forceinline__ void direct_group(const float *__restrict__ xr, int d, const float *__restrict__ ct, int kp,
+                                             int k, int c0, int lane, float &bv, int &bi) {
+    float acc[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) acc[u] = 0.f;
+    const float *cp = ct + c0 + lane;
+#pragma unroll(32 / U)
+    for (int j = 0; j < d; j++) {
+        const float xv = xr[j];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const float t = __fsub_rn(xv, cp[(int64_t)j * kp + 32 * u]);
+            acc[u] = __fadd_rn(acc[u], __fmul_rn(t, t));
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const int cc = c0 + 32 * u + lane;
+        if (cc < k && acc[u] < bv) {  // ascending index: the lowest of equals stays
+            bv = acc[u];
+            bi = cc;
+        }
+    }
+}
+
+__device__ __forceinline__ void lowest_of(float &bv, int &bi, int o) {
+    const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+    if (ov < bv || (ov == bv && oi < bi)) {
+        bv = ov;
+        bi = oi;
+    }
+}
+
+// Listed rows: the direct form against every centre, lowest index among the
+// smallest distances strictly below F::MAX, else 0. A row is a chain of d dependent
+// sums behind d loads, so a short list is bound by latency: a CTA takes a row,
+// each warp 32 centres at a time. A long one has rows enough: a warp a row, 128
+// centres at a time (each feature of the row read once for four). Predict calls with
+// a few hundred open rows, a warp a row / as here (us): 12,000 x 50, 400 centres
+// 130 / 107, 19,000 x 100, 129: 106 / 86, 800 x 999, 300: 1,099 / 701.
 __global__ void __launch_bounds__(SNT)
     score_open_rows_kernel(const float *__restrict__ x, int d, const float *__restrict__ ct, int k, int kp,
                            const int32_t *__restrict__ list, const unsigned long long *__restrict__ count,
                            int32_t *__restrict__ labels) {
-    const int lane = threadIdx.x & 31;
+    __shared__ float wv[SNT / 32];
+    __shared__ int wi[SNT / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned long long cnt = *count;
+    if (cnt <= 2 * (unsigned long long)gridDim.x) {
+        for (unsigned long long q = blockIdx.x; q < cnt; q += gridDim.x) {
+            const int64_t r = list[q];
+            float bv = FLT_MAX;
+            int bi = INT32_MAX;
+            for (int c0 = 32 * warp; c0 < k; c0 += SNT) direct_group<1>(x + r * d, d, ct, kp, k, c0, lane, bv, bi);
+#pragma unroll
+            for (int o = 16; o >= 1; o >>= 1) lowest_of(bv, bi, o);
+            if (lane == 0) {
+                wv[warp] = bv;
+                wi[warp] = bi;
+            }
+            __syncthreads();
+            if (warp == 0) {
+                bv = wv[lane % (SNT / 32)];
+                bi = wi[lane % (SNT / 32)];
+#pragma unroll
+                for (int o = SNT / 64; o >= 1; o >>= 1) lowest_of(bv, bi, o);
+                if (lane == 0) labels[r] = bi == INT32_MAX ? 0 : bi;
+            }
+            __syncthreads();
+        }
+        return;
+    }
     const unsigned long long nw = ((unsigned long long)gridDim.x * SNT) >> 5;
     for (unsigned long long q = ((unsigned long long)blockIdx.x * SNT + threadIdx.x) >> 5; q < cnt; q += nw) {
         const int64_t r = list[q];
-        const float *xr = x + r * d;
         float bv = FLT_MAX;
         int bi = INT32_MAX;
-        for (int c0 = 0; c0 < k; c0 += 128) {
-            float acc[4] = {0.f, 0.f, 0.f, 0.f};
-            const float *cp = ct + c0 + lane;
-#pragma unroll 8
-            for (int j = 0; j < d; j++) {
-                const float xv = xr[j];
+        for (int c0 = 0; c0 < k; c0 += 128) direct_group<4>(x + r * d, d, ct, kp, k, c0, lane, bv, bi);
 #pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const float t = __fsub_rn(xv, cp[(int64_t)j * kp + 32 * u]);
-                    acc[u] = __fadd_rn(acc[u], __fmul_rn(t, t));
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const int cc = c0 + 32 * u + lane;
-                if (cc < k && acc[u] < bv) {  // ascending index: the lowest of equals stays
-                    bv = acc[u];
-                    bi = cc;
-                }
-            }
-        }
-#pragma unroll
-        for (int o = 16; o >= 1; o >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (ov < bv || (ov == bv && oi < bi)) {
-                bv = ov;
-                bi = oi;
-            }
-        }
+        for (int o = 16; o >= 1; o >>= 1) lowest_of(bv, bi, o);
         if (lane == 0) labels[r] = bi == INT32_MAX ? 0 : bi;
     }
 }
