@@ -401,7 +401,7 @@ const float *pad_rows(Ctx &ctx, const float *x, int64_t n, int64_t d, int64_t &d
 template <typename TX, typename TC>
 void assign_direct_labels(Ctx &ctx, const TX *x, int64_t n, int d, const TC *c, int k, int32_t *labels) {
     if constexpr (std::is_same<TX, float>::value && std::is_same<TC, float>::value) {
-        if (!ctx.lean && f32_scores_pay(n, d, k)) {
+        if (!ctx.lean && f32_scores_pay(n, d, k, ctx.num_sms)) {
             ctx.spared = true;
             try {
                 launch_assign_f32_scored(ctx, x, n, d, c, k, labels);

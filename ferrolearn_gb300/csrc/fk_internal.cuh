@@ -354,7 +354,7 @@ void launch_assign_f64_filtered(Ctx &ctx, const double *x, int64_t n, int d, con
 // The plain f32 labels -- launch_assign_direct<float, float>'s -- through FMA
 // scores with rigorous bounds (fk_score.cu): the direct form only for the rows
 // they cannot decide. Where it pays: f32_scores_pay.
-bool f32_scores_pay(int64_t n, int d, int k);
+bool f32_scores_pay(int64_t n, int d, int k, int num_sms);
 void launch_assign_f32_scored(Ctx &ctx, const float *x, int64_t n, int d, const float *c, int k, int32_t *labels);
 // The plain assignment of a fit's iteration (fk_prune.cu): the labels of
 // launch_assign_direct<F, F>, without the distances. c_prev null: every centre for

@@ -364,11 +364,15 @@ void launch_rows(const float *x, int64_t n, int d, int k, const ScorePlan &p, bo
 // at 1e8) costs little more than the two launches around the tiled one (7 us).
 // Predict calls at the line, direct / scored: 1,000,000 x 16, 24 centres 382 /
 // 184 us, 400,000 x 16, 32: 179 / 109, 2,000 x 256, 500: 383 / 257. Where the
-// direct pass's 128-row tiles fill the SMs about once it needs 3e8: 30,000 x 80, 100
-// (2.4e8) 92 / 81 us when few rows stay open, 92 / 97 when many do.
-bool f32_scores_pay(int64_t n, int d, int k) {
-    const double w = (double)n * d * k;
-    return d >= 16 && d <= 1024 && k >= 24 && n < INT32_MAX && w >= 2e8 && (w >= 3e8 || n < 16384 || n >= 38912);
+// row tiles fit the SMs at once, the direct pass takes as long as one tile does,
+// d k, and has the SMs full near their number: there 12,500. Direct / scored with
+// no row open / with hundreds open: two waves 25,000 x 80, 100 82 / 70 / 77 us,
+// 30,000 x 100, 100 96 / 74 / 86, 38,900 x 54, 100 69 / 61 / 72; one wave
+// 19,000 x 110, 100 (11,000) 72 / 70 / 80, 16,000 x 126, 100 (12,600) 81 / 70 / 84,
+// 19,000 x 64, 200 (12,800) 80 / 68 / 74, 10,500 x 100, 200 110 / 91 / 102.
+bool f32_scores_pay(int64_t n, int d, int k, int num_sms) {
+    return d >= 16 && d <= 1024 && k >= 24 && n < INT32_MAX && (double)n * d * k >= 2e8 &&
+           (n > (int64_t)SBM * num_sms || (int64_t)d * k >= 12500);
 }
 
 void launch_assign_f32_scored(Ctx &ctx, const float *x, int64_t n, int d, const float *c, int k, int32_t *labels) {

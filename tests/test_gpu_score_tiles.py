@@ -43,8 +43,12 @@ def test_scored_labels_over_tiles_and_slabs(n, d, k, kind):
 
 
 @pytest.mark.parametrize("n,d,k,form", [(520960, 16, 24, SCORED), (800, 999, 300, SCORED), (4001, 200, 257, SCORED),
-                                        (521000, 15, 26, DIRECT), (600000, 16, 23, DIRECT), (25000, 65, 129, DIRECT)])
+                                        (521000, 15, 26, DIRECT), (600000, 16, 23, DIRECT),
+                                        (24577, 64, 128, SCORED), (25000, 65, 129, SCORED),
+                                        # row tiles of one wave: from d k = 12,500 on
+                                        (0, 100, 124, DIRECT), (1, 100, 124, SCORED), (0, 125, 100, SCORED)])
 def test_the_line_between_the_forms(n, d, k, form):
+    n = n if n > 1 else n + 128 * torch.cuda.get_device_properties(0).multi_processor_count
     x, c = _case("blobs", n, d, k, np.random.default_rng(1))
     model = FittedKMeans(c, None, 0.0, 0, "f32")
     got, launches = _launches(lambda: model.predict(torch.from_numpy(x).cuda()))
