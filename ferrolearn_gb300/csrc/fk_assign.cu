@@ -403,15 +403,12 @@ void launch_convert(const TS *src, int64_t count, TD *dst, cudaStream_t s) {
 }
 
 template int assign_splits<float>(int64_t, int, int);
-template int assign_splits<double>(int64_t, int, int);
 template void launch_assign_direct<double, double>(const double *, int64_t, int, const double *, int,
                                                    int32_t *, double *, cudaStream_t);
 template void launch_assign_direct<float, float>(const float *, int64_t, int, const float *, int,
                                                  int32_t *, float *, cudaStream_t);
 template void launch_assign_direct<float, double>(const float *, int64_t, int, const double *, int,
                                                   int32_t *, double *, cudaStream_t);
-template void launch_assign_direct_split<double, double>(const double *, int64_t, int, const double *, int,
-                                                         int32_t *, double *, int, double *, int32_t *, cudaStream_t);
 template void launch_assign_direct_split<float, float>(const float *, int64_t, int, const float *, int, int32_t *,
                                                        float *, int, float *, int32_t *, cudaStream_t);
 template void launch_transform_direct<double>(const double *, int64_t, int, const double *, int,

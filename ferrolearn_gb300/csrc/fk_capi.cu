@@ -1123,7 +1123,8 @@ int64_t fisher_yates_picks(UniformStream &g, int64_t n, int64_t count, std::unor
 
 // MiniBatchKMeans::fit (mini_batch_kmeans.rs:492-591) on the GPU. Per run:
 // the initial centres, then per iteration the batch rows gathered, their
-// nearest centres (the direct-form assignment kernel), the in-order update
+// nearest centres (f32: the direct-form kernel, split over centres; f64: the
+// filtered form, FP64 only for rows its FP32 pass leaves open), the in-order update
 // and the max shift; the early stop reads the shift back only when tol > 0
 // (a shift is never below a tol <= 0). The batch indices come from the host
 // stream, uploaded a chunk of iterations at a time.
@@ -1189,10 +1190,17 @@ fk_status minibatch_impl(fk_ctx *ctxp, const T *x_in, int64_t n, int64_t d, cons
     int32_t *didx = (int32_t *)ctx.get(BUF_MB_IDX, sizeof(int32_t) * (size_t)std::max(m * chunk, k));
     T *xb = (T *)ctx.get(BUF_MB_XB, sizeof(T) * (size_t)m * d);
     int32_t *blab = (int32_t *)ctx.get(BUF_MB_LAB, sizeof(int32_t) * (size_t)m);
-    // f32: a batch is too few rows to fill the GPU by row tiles, so the centres are split too
-    const int splits = std::is_same<T, float>::value ? assign_splits<T>(m, (int)k, ctx.num_sms) : 1;
-    T *part_v = splits > 1 ? (T *)ctx.get(BUF_MB_PARTV, sizeof(T) * (size_t)splits * m) : nullptr;
-    int32_t *part_i = splits > 1 ? (int32_t *)ctx.get(BUF_MB_PARTI, sizeof(int32_t) * (size_t)splits * m) : nullptr;
+    int splits = 1;
+    T *part_v = nullptr;
+    int32_t *part_i = nullptr;
+    if constexpr (std::is_same<T, float>::value) {
+        // a batch is too few rows to fill the GPU by row tiles, so the centres are split too
+        splits = assign_splits<T>(m, (int)k, ctx.num_sms);
+        if (splits > 1) {
+            part_v = (T *)ctx.get(BUF_MB_PARTV, sizeof(T) * (size_t)splits * m);
+            part_i = (int32_t *)ctx.get(BUF_MB_PARTI, sizeof(int32_t) * (size_t)splits * m);
+        }
+    }
     std::vector<int32_t> hidx;
     std::unordered_map<int64_t, int64_t> moved;
     std::vector<int64_t> pool;
